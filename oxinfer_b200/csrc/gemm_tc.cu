@@ -231,6 +231,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Gives a staging buffer of packed weights back to the copy engine once the warp's loads from it have landed in registers. The
+// loads have only been issued when the warp gets here, and with the tensor cores reading shared memory at most of its rate they
+// can stay queued for longer than the next copy takes to arrive: an arrival that did not wait for them let that copy overwrite
+// words that were still to be read (a few weight rows of a tile then came from the next super-block). So the arrival takes an
+// operand that every lane's loaded words enter: `words` is an OR over them, `zero` a kernel argument that is always 0.
+__device__ __forceinline__ void release_raw(uint64_t* bar, uint32_t words, int zero, int lane) {
+    const uint32_t off = __reduce_or_sync(0xffffffffu, words) & (uint32_t)zero;
+    if (lane == 0) asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar) + off) : "memory");
+}
+
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 
 // TT: the instantiation that takes two-term operands (a_lo_row_arg, w_terms); the one-term kernel carries none of that code.
@@ -240,7 +250,7 @@ template <int FMT, bool SPLIT, bool TT, bool PAIR = false>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                    const __grid_constant__ CUtensorMap tmap_y, int K, int n_out, int t,
-                   int tile_n, int m_halves, void* __restrict__ y, int y_dtype_arg, GemmStatus* __restrict__ status, int dbg_arg,
+                   int tile_n, int m_halves, void* __restrict__ y, int y_dtype_arg, GemmStatus* __restrict__ status, int dbg_arg, int zero,
                    const int* __restrict__ tile_expert, F8Scales f8, int k_splits, const float* __restrict__ row_unscale, int a_lo_row_arg, int w_terms,
                    const CUtensorMap* __restrict__ y_more, int n_more) {
     // y_more[0 .. n_more): tensor maps (in global memory) of the other ranks' copies of y, for a row-sharded product whose
@@ -519,10 +529,8 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                         for (int c = 0; c < 4; c++) ql4[c] = my_raw[((uint32_t)(4 * n + c)) ^ swz];
 #pragma unroll
                         for (int c = 0; c < 2; c++) qh4[c] = my_qh[((uint32_t)(2 * n + c)) ^ swh];
-                        if (jj == 1) {  // the row's last read of this super-block's staging buffer
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&sh->raw_empty[rb]);
-                        }
+                        if (jj == 1)  // the row's last read of this super-block's staging buffer
+                            release_raw(&sh->raw_empty[rb], ql4[0].x | ql4[1].x | ql4[2].x | ql4[3].x | qh4[0].x | qh4[1].x, zero, lane);
                         const uint32_t sc4 = live ? __ldg((const uint32_t*)((const int8_t*)f8.s + wrow * (size_t)(K / 16) + (size_t)(sb0 + sb) * 16 + 4 * j)) : 0u;
                         __half2 mul[4];
 #pragma unroll
@@ -567,8 +575,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     uint4 qb[4];
 #pragma unroll
                     for (int c = 0; c < 4; c++) qb[c] = my_raw[((uint32_t)(4 * set + c)) ^ swz];
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sh->raw_empty[rb]);
+                    release_raw(&sh->raw_empty[rb], qb[0].x | qb[1].x | qb[2].x | qb[3].x, zero, lane);
                     const int ks = sb * 2 + set;
                     const int s = ks % STAGES;
                     const uint32_t ph = (uint32_t)((ks / STAGES) & 1);
@@ -631,8 +638,12 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     q[2 * jj] = my_raw[1 + 2 * (set + NSETS * jj)];
                     q[2 * jj + 1] = my_raw[2 + 2 * (set + NSETS * jj)];
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sh->raw_empty[rb]);
+                {
+                    uint32_t words = hdr.x;
+#pragma unroll
+                    for (int i = 0; i < 2 * (4 / NSETS); i++) words |= q[i].x;
+                    release_raw(&sh->raw_empty[rb], words, zero, lane);
+                }
 #pragma unroll
                 for (int jj = 0; jj < 4 / NSETS; jj++) {
                     const int j = set + NSETS * jj;
@@ -1217,7 +1228,7 @@ cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, i
                            cudaStream_t st, const float* row_unscale) {
     const bool split = p->k_splits > 1;
     const bool tt = p->a_lo_row0 > 0 || p->w_terms == 2;
-    using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, int, int, int, int, int, void*, int, GemmStatus*, int, const int*, F8Scales, int, const float*,
+    using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, int, int, int, int, int, void*, int, GemmStatus*, int, int, const int*, F8Scales, int, const float*,
                           int, int, const CUtensorMap*, int);
     Kern kern;
     if (tt)  // two-term operands never come with a K split
@@ -1250,7 +1261,7 @@ cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, i
         cfg.attrs = attr;
         cfg.numAttrs = 2;
         cudaError_t le = cudaLaunchKernelEx(&cfg, kern, p->tmap_x, p->tmap_w, p->tmap_y, (int)w.n_in, (int)w.n_out, (int)t, p->tile_n, p->m_halves, y,
-                                  y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), (const int*)nullptr, f8, 1, row_unscale, 0, 1, (const CUtensorMap*)nullptr, 0);
+                                  y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), 0, (const int*)nullptr, f8, 1, row_unscale, 0, 1, (const CUtensorMap*)nullptr, 0);
         return le;
     }
     if (cudaError_t e = ensure_dynamic_smem((const void*)kern, GEMM_SMEM); e != cudaSuccess) return e;
@@ -1261,7 +1272,7 @@ cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, i
     }
     // (a dependent launch: see the top of the kernel)
     return launch_k(kern, grid, dim3(GEMM_THREADS), GEMM_SMEM, st, true, p->tmap_x, p->tmap_w, p->tmap_y, (int)w.n_in, (int)w.n_out, (int)t, p->tile_n, p->m_halves, y,
-                    y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), p->tile_expert, f8, p->k_splits, row_unscale, (int)p->a_lo_row0, p->w_terms,
+                    y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), 0, p->tile_expert, f8, p->k_splits, row_unscale, (int)p->a_lo_row0, p->w_terms,
                     (const CUtensorMap*)p->y_more, p->n_more);
 }
 
