@@ -114,12 +114,12 @@ __host__ __device__ constexpr size_t attend_smem() {
 
 // A group of 256 threads (a CTA of the attention kernel; `bar_id` names its barrier) as unit (kvh, split): it runs the G
 // query heads of KV head kvh over its share of the key tiles with an online softmax, writes the unnormalized partial (o, m, l) of each head, and the last CTA of a KV head
-// to finish (a counter, no waiting) combines the partials, writes `out` and, if asked, the planes of `out`.
+// to finish (a counter, no waiting) combines the partials and writes `out`.
 template <int HD, int G, typename T>
 __device__ __forceinline__ void attend_unit(uint8_t* smem, const int tid, const int bar_id, const int kvh, const int split,
                                             const uint32_t max_splits, const uint32_t pos, const float* q,
                                             const T* kc, const T* vc, float* out, float* part,
-                                            uint32_t* counters, DecAttn p, XPlanes xp, uint32_t* status,
+                                            uint32_t* counters, DecAttn p, uint32_t* status,
                                             unsigned long long* prof = nullptr, const FusedRope* fr = nullptr, const uint32_t table_pos0 = 0,
                                             const bool wait_inside = false) {
     const long long pt0 = clock64();
@@ -445,9 +445,7 @@ __device__ __forceinline__ void attend_unit(uint8_t* smem, const int tid, const 
             float o = 0.0f;
 #pragma unroll
             for (int r2 = 0; r2 < R; r2++) o += red[(size_t)r2 * NC * 4 + idx];
-            const float r = o / mrun[idx / HD];
-            out[(size_t)h0 * HD + idx] = r;
-            if (p.planes) xplanes_block(r, (h0 * HD + idx) >> 5, tid & 31, (int)(p.nh * HD), xp);
+            out[(size_t)h0 * HD + idx] = o / mrun[idx / HD];
         }
     }
     stamp(5);

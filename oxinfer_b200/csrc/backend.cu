@@ -81,7 +81,7 @@ class Backend {
     uint64_t next_handle = 1;
     uint64_t launches = 0;
     // staging for the host-buffer entry points
-    Scratch x_dev, y_dev, x16, x8, xplanes, pair_tmp;
+    Scratch x_dev, y_dev, x16, x8, xprep, xrec;
     GemmStatus* gemm_status = nullptr;  // device
     // cached tensor maps of the tensor-core GEMM (see matmul_dev)
     std::vector<GemmPlan*> plans;
@@ -428,25 +428,31 @@ class Backend {
         return B2_OK;
     }
 
-    // The activation planes of one vector (kernels.h, XPlanes), computed once and read by every
-    // matrix-vector product over that vector: the role of quantize_act, which the reference's CPU
-    // driver also runs once per batch of jobs (src/kernels.rs:1731-1879, `xa`).
+    // The vector of b2_prepare_x_dev: a copy of its own, which the products made from it read (the role of quantize_act, which the
+    // reference's CPU driver runs once per batch of jobs, src/kernels.rs:1731-1879, `xa`; here every product splits the vector itself).
     size_t prepared_k = 0;
     int prepare_x(const float* x_dev_, size_t n_in) {
         if (!x_dev_ || n_in == 0 || n_in % 32) return fail(B2_ERR_ARG, "[b200qmm: prepare_x: n_in must be a positive multiple of 32]");
-        cudaError_t e = xplanes.reserve(xplanes_bytes(n_in));
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(planes)");
-        e = launch_xplanes(x_dev_, n_in, planes_at(xplanes.p, n_in), stream, chained);
-        launches++;
-        if (e != cudaSuccess) return cuda_fail(e, "xplanes");
+        cudaError_t e = xprep.reserve(n_in * 4);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(prepared vector)");
+        e = cudaMemcpyAsync(xprep.p, x_dev_, n_in * 4, cudaMemcpyDeviceToDevice, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "prepare_x");
         prepared_k = n_in;
         return B2_OK;
     }
 
-    // One token on the device over the prepared planes (FP8 weights read x itself).
-    // `after_planes`: the product directly follows the plane kernel of its own vector in the stream, so it is launched as
-    // that kernel's dependent (it fetches its first weights while the planes are written, and waits for them on the device).
-    int matvec_prepared(uint64_t h, uint64_t up, const float* x_dev_, float* y_dev_, int mode, const float* gate, bool after_planes = false) {
+    // One token on the device over the prepared vector (FP8 weights and the generic formats read x itself).
+    int matvec_prepared(uint64_t h, uint64_t up, const float* x_dev_, float* y_dev_, int mode, const float* gate) {
+        Weight* w = find(h);
+        if (!w) return fail(B2_ERR_ARG, "[b200qmm: matvec: unknown weight]");
+        if (w->dev.fmt == B2_FMT_F8E4M3 || fmt_is_other(w->dev.fmt)) return matvec_dev(h, up, x_dev_, y_dev_, mode, gate);
+        if (prepared_k != w->dev.n_in) return fail(B2_ERR_ARG, "[b200qmm: matvec: no planes prepared for n_in = %zu (b2_prepare_x_dev)]", w->dev.n_in);
+        return matvec_dev(h, up, (const float*)xprep.p, y_dev_, mode, gate);
+    }
+
+    // One token on the device. The launches are dependent ones (each may start while the one ahead drains and reads nothing but
+    // weights before it has waited for it).
+    int matvec_dev(uint64_t h, uint64_t up, const float* x_dev_, float* y_dev_, int mode, const float* gate) {
         Weight* w = find(h);
         if (!w) return fail(B2_ERR_ARG, "[b200qmm: matvec: unknown weight]");
         bool pair = mode == B2_MODE_SILU_PAIR || mode == B2_MODE_GELU_PAIR;
@@ -458,7 +464,7 @@ class Backend {
                 return fail(B2_DECLINED, "[b200qmm: matvec: the pair's matrices differ in shape or format]");
         }
         if (mode < 0 || mode > 4 || (mode == B2_MODE_ADD_GATED && !gate)) return fail(B2_ERR_ARG, "[b200qmm: matvec: bad mode]");
-        if (fmt_is_other(w->dev.fmt)) {  // the generic kernel reads x itself
+        if (fmt_is_other(w->dev.fmt)) {
             if (!gemv_other_supports(w->dev)) return fail(B2_DECLINED, "[b200qmm: matvec: shape not supported for this format]");
             cudaError_t eo = launch_gemv_other(w->dev, u ? &u->dev : nullptr, x_dev_, 0, y_dev_, 0, 1, mode, gate, sm_count, stream, chained);
             launches++;
@@ -466,30 +472,43 @@ class Backend {
             return B2_OK;
         }
         if (!gemv_supports(w->dev)) return fail(B2_DECLINED, "[b200qmm: matvec: shape not supported by the GEMV kernels]");
-        XPlanes xp{};
-        if (w->dev.fmt != B2_FMT_F8E4M3) {
-            if (prepared_k != w->dev.n_in) return fail(B2_ERR_ARG, "[b200qmm: matvec: no planes prepared for n_in = %zu (b2_prepare_x_dev)]", w->dev.n_in);
-            xp = planes_at(xplanes.p, w->dev.n_in);
+        cudaError_t e;
+        if (gemv_mma_supports(w->dev)) {
+            GemvIn in;
+            in.x = x_dev_;
+            in.fast = fast_planes && !exact;
+            e = launch_gemv_mma(w->dev, u ? &u->dev : nullptr, in, 1, y_dev_, 0, mode, gate, 0, sm_count, stream, true);
+        } else {
+            e = launch_gemv_f8_float(w->dev, u ? &u->dev : nullptr, x_dev_, y_dev_, mode, gate, sm_count, stream, true);
         }
-        cudaError_t e = launch_gemv(w->dev, u ? &u->dev : nullptr, x_dev_, xp, y_dev_, mode, gate, sm_count, stream, chained || after_planes,
-                                    NormScale{nullptr, 0, 0.0f, 0.0f}, EpiPlanes{XPlanes{nullptr, nullptr, nullptr}, nullptr, nullptr, 1.0f}, after_planes && !chained);
         launches++;
         if (e != cudaSuccess) return cuda_fail(e, "gemv");
         return B2_OK;
     }
 
-    int matvec_dev(uint64_t h, uint64_t up, const float* x_dev_, float* y_dev_, int mode, const float* gate) {
-        Weight* w = find(h);
-        if (!w) return fail(B2_ERR_ARG, "[b200qmm: matvec: unknown weight]");
-        bool planes = false;
-        if (w->dev.fmt != B2_FMT_F8E4M3 && !fmt_is_other(w->dev.fmt) && gemv_supports(w->dev)) {
-            int rc = prepare_x(x_dev_, w->dev.n_in);
-            if (rc) return rc;
-            // the product is launched as the plane kernel's dependent, in its register-load form (the 4-bit ring form loses when
-            // launched alone): its first weights travel while the planes are made
-            planes = true;
+    // Records (launch_split) of t rows for the products of several tokens, in `xrec`; the digits form and the halves form (FP8 weights)
+    // lie side by side when a call needs both.
+    size_t record_stride(size_t K, bool halves) const { return (split_bytes_of(K, halves) + 255) / 256 * 256; }
+    int make_records(const float* x, size_t t, size_t K, bool halves, uint8_t* at) {
+        cudaError_t e = launch_split(x, K, nullptr, 1.0f, K, (int)t, at, record_stride(K, halves), halves, fast_planes && !exact, stream, true);
+        launches++;
+        if (e != cudaSuccess) return cuda_fail(e, "activation split");
+        return B2_OK;
+    }
+    // t tokens of one matrix from their records, up to eight per launch (the weights are read once per launch). A matrix whose tiles
+    // fill no more than half the SMs goes four at a time: the launches run side by side, and a launch of four has half the arithmetic.
+    int small_products(const WeightDev& w, const WeightDev* up, const uint8_t* rec, size_t t, float* y, int mode) {
+        const size_t stride = record_stride(w.n_in, gemv_mma_halves(w)), tiles = (w.n_out + 15) / 16;
+        const size_t per = 2 * tiles <= (size_t)sm_count ? 4 : 8;
+        for (size_t i = 0; i < t; i += per) {
+            GemvIn in;
+            in.rec = rec + i * stride;
+            in.rec_stride = stride;
+            cudaError_t e = launch_gemv_mma(w, up, in, (int)std::min(per, t - i), y + i * w.n_out, w.n_out, mode, nullptr, 0, sm_count, stream, true);
+            launches++;
+            if (e != cudaSuccess) return cuda_fail(e, "gemv (several rows)");
         }
-        return matvec_prepared(h, up, x_dev_, y_dev_, mode, gate, planes);
+        return B2_OK;
     }
 
     int ensure_status() {
@@ -527,47 +546,23 @@ class Backend {
             }
             return B2_OK;
         }
-        // Two to eight tokens of a 4-bit format: four at a time through the several-token matrix-vector kernel (its integer
-        // dots on the tensor cores), every row equal to its one-token row bit for bit.
-        const bool few_4bit = t >= 2 && t <= 8 && x_dtype == B2_F32 && y_dtype == B2_F32 && (w->dev.fmt == B2_FMT_Q4_K || w->dev.fmt == B2_FMT_MLX4) &&
-                              gemv_supports(w->dev) && gemv_multi_pays(w->dev, (int)std::min<size_t>(t, 4));
-        if (!few_4bit && t <= 8 && x_dtype == B2_F32 && y_dtype == B2_F32 && gemv_supports(w->dev) && !(fp8_act && w->dev.fmt == B2_FMT_F8E4M3)) {
-            for (size_t i = 0; i < t; i++) {
-                int rc = matvec_dev(h, 0, (const float*)x + i * K, (float*)y + i * w->dev.n_out, B2_MODE_STORE, nullptr);
-                if (rc) return rc;
-            }
-            return B2_OK;
-        }
-        if (few_4bit || (rows_path(w->dev) && x_dtype == B2_F32 && y_dtype == B2_F32 && (exact || !gemm_tc_supports(w->dev, t)))) {
-            // Q6_K / Q8_0 under the exact switch (or at a shape the tensor-core kernel does not take): the tokens go four at a
-            // time through the multi-row matrix-vector kernel (the weights are read once per four tokens; every row equals its
-            // one-token result bit for bit).
-            const size_t stride = (xplanes_bytes(K) + 255) / 256 * 256;
-            cudaError_t e = xplanes.reserve(t * stride);
-            if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(planes)");
-            e = launch_xplanes_rows((const float*)x, t, K, (uint8_t*)xplanes.p, stride, stream);
-            launches++;
-            prepared_k = 0;  // the scratch holds many rows' planes now
-            if (e != cudaSuccess) return cuda_fail(e, "xplanes (rows)");
-            const size_t n_out = w->dev.n_out;
-            for (size_t i = 0; i < t; i += 4) {
-                const size_t nt = std::min<size_t>(4, t - i);
-                const float* xi = (const float*)x + i * K;
-                float* yi = (float*)y + i * n_out;
-                uint8_t* pi = (uint8_t*)xplanes.p + i * stride;
-                if (nt > 1 && gemv_multi_fits(w->dev, (int)nt)) {
-                    e = launch_gemv_multi(w->dev, nullptr, xi, K, planes_at(pi, K), stride, yi, n_out, (int)nt, B2_MODE_STORE, sm_count, stream);
-                    launches++;
-                    if (e != cudaSuccess) return cuda_fail(e, "gemv (several rows)");
-                    continue;
+        // Up to eight f32 rows: exact products on the small-batch kernel, every row equal to its one-token row bit for bit. Under the
+        // exact switch (or at a shape the tensor-core kernel does not take) Q6_K / Q8_0 matrices take it for any number of rows.
+        const bool f8_both = fp8_act && w->dev.fmt == B2_FMT_F8E4M3;
+        if (x_dtype == B2_F32 && y_dtype == B2_F32 && gemv_supports(w->dev) &&
+            ((t <= 8 && !f8_both) || (rows_path(w->dev) && (exact || !gemm_tc_supports(w->dev, t))))) {
+            if (t == 1 || !gemv_mma_supports(w->dev)) {
+                for (size_t i = 0; i < t; i++) {
+                    int rc = matvec_dev(h, 0, (const float*)x + i * K, (float*)y + i * w->dev.n_out, B2_MODE_STORE, nullptr);
+                    if (rc) return rc;
                 }
-                for (size_t r = 0; r < nt; r++) {  // one row, or the rows' planes do not fit in shared memory together
-                    e = launch_gemv(w->dev, nullptr, xi + r * K, planes_at(pi + r * stride, K), yi + r * n_out, B2_MODE_STORE, nullptr, sm_count, stream);
-                    launches++;
-                    if (e != cudaSuccess) return cuda_fail(e, "gemv");
-                }
+                return B2_OK;
             }
-            return B2_OK;
+            const bool halves = gemv_mma_halves(w->dev);
+            cudaError_t e = xrec.reserve(t * record_stride(K, halves));
+            if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(records)");
+            int rc = make_records((const float*)x, t, K, halves, (uint8_t*)xrec.p);
+            return rc ? rc : small_products(w->dev, nullptr, (const uint8_t*)xrec.p, t, (float*)y, B2_MODE_STORE);
         }
         if (fp8_act && !exact && gemm_f8_supports(w->dev, t)) {
             // FP8 on both sides: the activations are quantized per token and per 128 k to e4m3, and the tensor cores multiply
@@ -731,10 +726,11 @@ class Backend {
         if (e != cudaSuccess) return cuda_fail(e, "copy-in");
         ns_in += since(t0);
         auto t1 = clk::now();
-        // The planes of this call's rows are computed at most once, by the first job that reads them; a job that takes the
-        // row-by-row route writes one vector's planes into the same scratch, after which they must be computed again.
-        bool planes_ready = false;
-        const size_t stride = (xplanes_bytes(n_in) + 255) / 256 * 256;
+        // The records of this call's rows are made at most once per form, by the first job that reads them (one row: every product
+        // splits it itself).
+        const size_t digits = t * record_stride(n_in, false);
+        bool made[2] = {false, false};
+        if (t > 1 && (e = xrec.reserve(digits + t * record_stride(n_in, true))) != cudaSuccess) return cuda_fail(e, "cudaMalloc(records)");
         for (size_t j = 0; j < n_jobs; j++) {
             Weight* w = find(jobs[j].w);
             Weight* u = jobs[j].up ? find(jobs[j].up) : nullptr;
@@ -746,32 +742,20 @@ class Backend {
                 if (e != cudaSuccess) return cuda_fail(e, "gemv (generic)");
                 continue;
             }
-            // Two to four rows: one launch that reads the weights once (each row's result is the one-row result bit for bit),
-            // when the rows' vectors fit in shared memory together. FP8 rows go one by one: their single-row kernel is the
-            // tensor-core one, and the rows must match it bit for bit.
-            if (t > 1 && w->dev.fmt != B2_FMT_F8E4M3 && gemv_multi_fits(w->dev, (int)t)) {
-                if (!planes_ready) {
-                    e = xplanes.reserve(t * stride);
-                    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(planes)");
-                    e = launch_xplanes_rows((const float*)x_dev.p, t, n_in, (uint8_t*)xplanes.p, stride, stream);
-                    launches++;
-                    if (e != cudaSuccess) return cuda_fail(e, "xplanes (rows)");
-                    prepared_k = 0;  // the scratch now holds several rows' planes, not one prepared vector
-                    planes_ready = true;
-                }
-                e = launch_gemv_multi(w->dev, u ? &u->dev : nullptr, (const float*)x_dev.p, n_in, planes_at(xplanes.p, n_in), stride, yj, jobs[j].n_out,
-                                      (int)t, mode, sm_count, stream);
-                launches++;
-                if (e != cudaSuccess) return cuda_fail(e, "gemv (several rows)");
-                continue;
+            int rc = B2_OK;
+            if (t > 1 && gemv_mma_supports(w->dev)) {  // one launch reads the weights once for all rows
+                const bool halves = gemv_mma_halves(w->dev);
+                uint8_t* rec = (uint8_t*)xrec.p + (halves ? digits : 0);
+                if (!made[halves]) rc = make_records((const float*)x_dev.p, t, n_in, halves, rec);
+                made[halves] = true;
+                if (!rc) rc = small_products(w->dev, u ? &u->dev : nullptr, rec, t, yj, mode);
+            } else {
+                for (size_t i = 0; i < t && !rc; i++)
+                    rc = matvec_dev(jobs[j].w, jobs[j].up, (const float*)x_dev.p + i * n_in, yj + i * jobs[j].n_out, mode, nullptr);
             }
-            for (size_t i = 0; i < t; i++) {
-                if (w->dev.fmt != B2_FMT_F8E4M3) planes_ready = false;  // matvec_dev overwrites the planes scratch
-                int rc = matvec_dev(jobs[j].w, jobs[j].up, (const float*)x_dev.p + i * n_in, yj + i * jobs[j].n_out, mode, nullptr);
-                if (rc) {
-                    cudaStreamSynchronize(stream);
-                    return rc;
-                }
+            if (rc) {
+                cudaStreamSynchronize(stream);
+                return rc;
             }
         }
         // Every launch was accepted (a refused one returned above, before any y is touched): the results follow the kernels on
@@ -1338,7 +1322,7 @@ class Backend {
                 Weight* w = find(h);
                 return w ? &w->dev : nullptr;
             },
-            sm_count, planes_read(), tokens, prefill, &p, e);
+            sm_count, fast_planes && !exact, tokens, prefill, &p, e);
         if (rc) {
             err = e;
             return rc;
@@ -1442,8 +1426,8 @@ class Backend {
         y_dev.release();
         x16.release();
         x8.release();
-        xplanes.release();
-        pair_tmp.release();
+        xprep.release();
+        xrec.release();
         if (gemm_status) cudaFree(gemm_status);
         gemm_status = nullptr;
         for (GemmPlan* p : plans) gemm_tc_plan_destroy(p);

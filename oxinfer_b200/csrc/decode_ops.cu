@@ -3,7 +3,7 @@
 // launches that does not depend on the position: every kernel reads the position from a device word.
 //
 //   norm      : RMSNorm rows (dnorm, src/cuda_decode.cu:314-328; CPU rmsnorm_f32w, src/kernels.rs:2157),
-//               optionally writing the activation planes the next GEMV reads
+//               one CTA per row
 //   qk_rope   : per-head q/k norm, RoPE, KV-cache append (dqk_rope, src/cuda_decode.cu:349-395)
 //   attend    : one query per head over the cache (dattn / dattn_combine, src/cuda_decode.cu:396-536;
 //               CPU attention_ext, src/model.rs:2214-2309), split over the keys, combined by the last CTA
@@ -26,8 +26,7 @@ namespace {
 // One CTA per row. out (+)= (x * pre) * k * w with k = 1 / sqrt(mean((x pre)^2) + eps). Rows of up to
 // 8 * blockDim values stay in registers between the two passes; longer rows are read twice.
 constexpr int NORM_PER_THREAD = 8;
-__global__ void __launch_bounds__(1024) norm_kernel(const float* __restrict__ x, float* __restrict__ out, const float* __restrict__ w, DecNorm p,
-                                                    XPlanes xp) {
+__global__ void __launch_bounds__(1024) norm_kernel(const float* __restrict__ x, float* __restrict__ out, const float* __restrict__ w, DecNorm p) {
     __shared__ float red[32];
     pdl_launch_dependents();
     const float* xr = x + (size_t)blockIdx.x * p.x_stride;
@@ -61,12 +60,11 @@ __global__ void __launch_bounds__(1024) norm_kernel(const float* __restrict__ x,
 #pragma unroll
         for (int j = 0; j < NORM_PER_THREAD; j++) {
             const uint32_t i = threadIdx.x + j * blockDim.x;
-            if (i < p.n) {  // p.n % 32 == 0 when planes are asked for: whole warps stay together
+            if (i < p.n) {
                 float t = v[j] * k;
                 if (w) t *= wv[j];
                 if (p.add) t += o[i];
                 o[i] = t;
-                if (p.planes) xplanes_block(t, (int)(i >> 5), threadIdx.x & 31, (int)p.n, xp);
             }
         }
     } else {
@@ -75,7 +73,6 @@ __global__ void __launch_bounds__(1024) norm_kernel(const float* __restrict__ x,
             if (w) t *= w[i];
             if (p.add) t += o[i];
             o[i] = t;
-            if (p.planes) xplanes_block(t, (int)(i >> 5), threadIdx.x & 31, (int)p.n, xp);
         }
     }
 }
@@ -113,12 +110,12 @@ __global__ void __launch_bounds__(256) glu_kernel(const float* __restrict__ g, c
 }
 
 // ---- attention: grid (KV heads, splits), one unit per CTA (attend_core.cuh) --------------------------------
-// blockIdx.z: the token of a step of several tokens (AttnTokens: its queries, outputs and planes a fixed stride behind token
+// blockIdx.z: the token of a step of several tokens (AttnTokens: its queries and outputs a fixed stride behind token
 // 0's, its own step words, partials and counters); the keys of all the step's tokens are in the caches already.
 template <int HD, int G, typename T>
 __global__ void __launch_bounds__(ATT_THREADS) attend_kernel(const float* __restrict__ q, T* kc, T* vc, float* __restrict__ out, float* part,
-                                                             uint32_t* counters, const uint32_t* __restrict__ sp, DecAttn p, XPlanes xp,
-                                                             uint32_t* status, FusedRope fr, AttnTokens at) {
+                                                             uint32_t* counters, const uint32_t* __restrict__ sp, DecAttn p, uint32_t* status,
+                                                             FusedRope fr, AttnTokens at) {
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_launch_dependents();
     if (blockIdx.z) {
@@ -129,14 +126,9 @@ __global__ void __launch_bounds__(ATT_THREADS) attend_kernel(const float* __rest
         counters += z * p.nkv;
         sp += 4 * z;
         if (fr.qkv) fr.qkv += z * at.act_stride;
-        if (xp.planes) {
-            xp.planes = (int8_t*)((uint8_t*)xp.planes + z * at.planes_stride);
-            xp.sx = (float2*)((uint8_t*)xp.sx + z * at.planes_stride);
-            xp.v16 = (int32_t*)((uint8_t*)xp.v16 + z * at.planes_stride);
-        }
     }
     // the step words (position, RoPE table base) were written before this step's graph was launched
-    attend_unit<HD, G, T>(smem, threadIdx.x, 0, blockIdx.x, blockIdx.y, gridDim.y, sp[0], q, kc, vc, out, part, counters, p, xp, status, nullptr,
+    attend_unit<HD, G, T>(smem, threadIdx.x, 0, blockIdx.x, blockIdx.y, gridDim.y, sp[0], q, kc, vc, out, part, counters, p, status, nullptr,
                           fr.qkv ? &fr : nullptr, sp[1], true);
 }
 
@@ -325,10 +317,9 @@ cudaError_t launch_set_step(uint32_t* sp, uint32_t pos, uint32_t table_pos0, uin
     return cudaGetLastError();
 }
 
-cudaError_t launch_norm(const float* x, float* out, const float* w, const DecNorm& p, uint32_t rows, XPlanes xp, cudaStream_t st, bool pdl) {
-    if (p.planes && (p.n % 32 || rows != 1)) return cudaErrorInvalidValue;
+cudaError_t launch_norm(const float* x, float* out, const float* w, const DecNorm& p, uint32_t rows, cudaStream_t st, bool pdl) {
     unsigned threads = p.n >= 4096 ? 1024 : p.n >= 1024 ? 512 : ((p.n + 31) / 32) * 32;
-    return launch_k(norm_kernel, dim3(rows), dim3(threads), 0, st, pdl, x, out, w, p, xp);
+    return launch_k(norm_kernel, dim3(rows), dim3(threads), 0, st, pdl, x, out, w, p);
 }
 
 template <typename T>
@@ -352,31 +343,31 @@ size_t attend_part_floats(uint32_t nh, uint32_t hd) { return (size_t)nh * ATT_MA
 
 template <int HD, int G, typename T>
 static cudaError_t attend_t(const float* q, void* kc, void* vc, float* out, float* part, uint32_t* counters, const uint32_t* sp,
-                            const DecAttn& p, XPlanes xp, uint32_t* status, cudaStream_t st, bool pdl, const FusedRope& fr, const AttnTokens& at) {
+                            const DecAttn& p, uint32_t* status, cudaStream_t st, bool pdl, const FusedRope& fr, const AttnTokens& at) {
     constexpr size_t smem = attend_smem<HD, G, T>();
     if (cudaError_t e = ensure_dynamic_smem((const void*)attend_kernel<HD, G, T>, smem, 0); e != cudaSuccess) return e;
     uint32_t splits = (p.max_len + ATT_TILE - 1) / ATT_TILE;
     if (splits > ATT_MAX_SPLITS) splits = ATT_MAX_SPLITS;
     if (splits == 0) splits = 1;
     dim3 grid(p.nkv, splits, (unsigned)std::max(1, at.n));
-    return launch_k(attend_kernel<HD, G, T>, grid, dim3(ATT_THREADS), smem, st, pdl, q, (T*)kc, (T*)vc, out, part, counters, sp, p, xp, status, fr, at);
+    return launch_k(attend_kernel<HD, G, T>, grid, dim3(ATT_THREADS), smem, st, pdl, q, (T*)kc, (T*)vc, out, part, counters, sp, p, status, fr, at);
 }
 
 template <int HD, typename T>
 static cudaError_t attend_g(uint32_t g, const float* q, void* kc, void* vc, float* out, float* part, uint32_t* counters,
-                            const uint32_t* sp, const DecAttn& p, XPlanes xp, uint32_t* status, cudaStream_t st, bool pdl, const FusedRope& fr,
+                            const uint32_t* sp, const DecAttn& p, uint32_t* status, cudaStream_t st, bool pdl, const FusedRope& fr,
                             const AttnTokens& at) {
     switch (g) {
-        case 1: return attend_t<HD, 1, T>(q, kc, vc, out, part, counters, sp, p, xp, status, st, pdl, fr, at);
-        case 2: return attend_t<HD, 2, T>(q, kc, vc, out, part, counters, sp, p, xp, status, st, pdl, fr, at);
-        case 4: return attend_t<HD, 4, T>(q, kc, vc, out, part, counters, sp, p, xp, status, st, pdl, fr, at);
-        case 8: return attend_t<HD, 8, T>(q, kc, vc, out, part, counters, sp, p, xp, status, st, pdl, fr, at);
+        case 1: return attend_t<HD, 1, T>(q, kc, vc, out, part, counters, sp, p, status, st, pdl, fr, at);
+        case 2: return attend_t<HD, 2, T>(q, kc, vc, out, part, counters, sp, p, status, st, pdl, fr, at);
+        case 4: return attend_t<HD, 4, T>(q, kc, vc, out, part, counters, sp, p, status, st, pdl, fr, at);
+        case 8: return attend_t<HD, 8, T>(q, kc, vc, out, part, counters, sp, p, status, st, pdl, fr, at);
     }
     return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_attend(const float* q, void* kc, void* vc, int kv_f16, float* out, float* part, uint32_t* counters,
-                          const uint32_t* sp, const DecAttn& p, XPlanes xp, uint32_t* status, cudaStream_t st, bool pdl, const FusedRope* frp,
+                          const uint32_t* sp, const DecAttn& p, uint32_t* status, cudaStream_t st, bool pdl, const FusedRope* frp,
                           const AttnTokens* atp) {
     if (!attend_supports(p.nh, p.nkv, p.hd)) return cudaErrorInvalidValue;
     AttnTokens at{};
@@ -390,10 +381,10 @@ cudaError_t launch_attend(const float* q, void* kc, void* vc, int kv_f16, float*
     }
     const uint32_t g = p.nh / p.nkv;
     if (p.hd == 64)
-        return kv_f16 ? attend_g<64, __half>(g, q, kc, vc, out, part, counters, sp, p, xp, status, st, pdl, fr, at)
-                      : attend_g<64, float>(g, q, kc, vc, out, part, counters, sp, p, xp, status, st, pdl, fr, at);
-    return kv_f16 ? attend_g<128, __half>(g, q, kc, vc, out, part, counters, sp, p, xp, status, st, pdl, fr, at)
-                  : attend_g<128, float>(g, q, kc, vc, out, part, counters, sp, p, xp, status, st, pdl, fr, at);
+        return kv_f16 ? attend_g<64, __half>(g, q, kc, vc, out, part, counters, sp, p, status, st, pdl, fr, at)
+                      : attend_g<64, float>(g, q, kc, vc, out, part, counters, sp, p, status, st, pdl, fr, at);
+    return kv_f16 ? attend_g<128, __half>(g, q, kc, vc, out, part, counters, sp, p, status, st, pdl, fr, at)
+                  : attend_g<128, float>(g, q, kc, vc, out, part, counters, sp, p, status, st, pdl, fr, at);
 }
 
 cudaError_t launch_glu(const float* g, const float* u, float* out, uint32_t n, int gelu, cudaStream_t st, bool pdl) {

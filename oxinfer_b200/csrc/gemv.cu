@@ -679,14 +679,13 @@ cudaError_t launch_fmt(const WeightDev& w, const WeightDev* up, const float* x, 
 }  // namespace
 
 bool gemv_supports(const WeightDev& w) {
-    switch (w.fmt) {
-        case B2_FMT_MLX4:
-        case B2_FMT_Q4_K:
-        case B2_FMT_Q6_K: return w.n_in % 256 == 0 && xplanes_bytes(w.n_in) <= 200 * 1024;
-        case B2_FMT_Q8_0: return w.n_in % 64 == 0 && xplanes_bytes(w.n_in) <= 200 * 1024;
-        case B2_FMT_F8E4M3: return w.n_in % 16 == 0 && w.n_in * 4 <= 200 * 1024 && (w.p1 == nullptr || w.bs_cols % 16 == 0);
-        default: return false;
-    }
+    return gemv_mma_supports(w) ||
+           (w.fmt == B2_FMT_F8E4M3 && w.n_in % 16 == 0 && w.n_in * 4 <= 200 * 1024 && (w.p1 == nullptr || w.bs_cols % 16 == 0));
+}
+cudaError_t launch_gemv_f8_float(const WeightDev& w, const WeightDev* up, const float* x, float* y, int mode, const float* gate, int sm_count,
+                                 cudaStream_t st, bool pdl) {
+    if (w.fmt != B2_FMT_F8E4M3) return cudaErrorInvalidValue;
+    return launch_fmt<FmtF8_T, true>(w, up, x, XPlanes{}, y, mode, gate, sm_count, st, pdl, NormScale{nullptr, 0, 0.0f, 0.0f});
 }
 
 cudaError_t launch_xplanes(const float* x, size_t K, XPlanes out, cudaStream_t st, bool pdl, int tokens, size_t x_stride, size_t planes_stride) {

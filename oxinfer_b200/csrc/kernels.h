@@ -147,8 +147,37 @@ cudaError_t launch_xplanes_rows(const float* x, size_t rows, size_t K, uint8_t* 
 cudaError_t launch_gemv_multi(const WeightDev& w, const WeightDev* up, const float* x, size_t x_stride, XPlanes xp, size_t xp_stride, float* y,
                               size_t y_stride, int nt, int mode, int sm_count, cudaStream_t st, bool pdl = false,
                               NormScale ns = NormScale{nullptr, 0, 0.0f, 0.0f}, size_t ns_stride = 0);
-// Whether launch_gemv handles this format and shape.
+// Whether a one-token product of this format and shape has a kernel: launch_gemv_mma, or for FP8 matrices with other scale blocks
+// launch_gemv_f8_float.
 bool gemv_supports(const WeightDev& w);
+cudaError_t launch_gemv_f8_float(const WeightDev& w, const WeightDev* up, const float* x, float* y, int mode, const float* gate, int sm_count,
+                                 cudaStream_t st, bool pdl);
+
+// ---- gemv_mma.cu: products of one to eight tokens on mma.sync ----------------------------------------------------------------
+// Where a product's vectors come from: f32 vectors that the product splits itself (norm_w: multiplied by these weights first; norm:
+// the results multiplied by 1 / sqrt(mean square of x * pre + eps)), or records that launch_split made of them (rec set).
+struct GemvIn {
+    const float* x = nullptr;  // token i at x + i * x_stride
+    size_t x_stride = 0;
+    const float* norm_w = nullptr;
+    float pre = 1.0f;
+    int norm = 0;
+    float eps = 0.0f;
+    const uint8_t* rec = nullptr;  // token i at rec + i * rec_stride
+    size_t rec_stride = 0;
+    int fast = 0;  // 16 bits of every value
+};
+bool gemv_mma_supports(const WeightDev& w);
+size_t split_blocks_of(size_t K);
+size_t split_bytes_of(size_t K, bool halves);  // bytes of a vector's record
+bool gemv_mma_halves(const WeightDev& w);  // the form of split this format's products read
+// y[i] = mode(W x_i [, U x_i]) for T (1 .. 8) tokens, token i's results at y + i * y_stride; every row equals its one-token row bit
+// for bit, from records or not.
+cudaError_t launch_gemv_mma(const WeightDev& w, const WeightDev* up, const GemvIn& in, int T, float* y, size_t y_stride, int mode, const float* gate,
+                            size_t gate_stride, int sm_count, cudaStream_t st, bool pdl);
+// Records (split.cuh, split_bytes each) of `tokens` vectors of x * pre * norm_w.
+cudaError_t launch_split(const float* x, size_t x_stride, const float* norm_w, float pre, size_t K, int tokens, uint8_t* rec, size_t rec_stride, bool halves,
+                         bool fast, cudaStream_t st, bool pdl);
 
 // ---- gemv_other.cu: the other GGUF block formats (dq_other.cuh), raw rows, one generic kernel ---------------------------
 bool gemv_other_supports(const WeightDev& w);
@@ -244,7 +273,7 @@ cudaError_t launch_scatter_blocks(const float* gathered, size_t world, size_t t,
 // Every kernel reads the step words `sp` on the device: sp[0] position of the token, sp[1] position of row 0
 // of the RoPE table, sp[2] tokens generated so far (the argmax kernel advances [0] and [2]).
 struct DecNorm {
-    uint32_t n, x_stride, out_stride, add, planes;
+    uint32_t n, x_stride, out_stride, add;
     float pre, eps;
 };
 struct DecRope {
@@ -253,7 +282,7 @@ struct DecRope {
     float eps;
 };
 struct DecAttn {
-    uint32_t nh, nkv, hd, max_len, window, planes;
+    uint32_t nh, nkv, hd, max_len, window;
     float scale;
 };
 // The ranks of a tensor-parallel plan as one rank sees them: every rank's activation block and flag words, mapped
@@ -268,7 +297,7 @@ struct PeerSet {
 // wait_limit_cycles: how long a rank polls for its peers before it gives up and sets the status word (0: about half a second).
 cudaError_t launch_exchange(const PeerSet& ps, size_t off_floats, uint32_t n, uint32_t* lflags, uint32_t* status, cudaStream_t st,
                             bool pdl = false, bool meet_first = true, long long wait_limit_cycles = 0);
-cudaError_t launch_norm(const float* x, float* out, const float* w, const DecNorm& p, uint32_t rows, XPlanes xp, cudaStream_t st, bool pdl = false);
+cudaError_t launch_norm(const float* x, float* out, const float* w, const DecNorm& p, uint32_t rows, cudaStream_t st, bool pdl = false);
 // KV caches are [nkv][max_len][hd], f32 or (kv_f16) f16.
 cudaError_t launch_qk_rope(const float* qkv, float* qo, void* kc, void* vc, int kv_f16, const float* qn, const float* kn, const float* cs_table,
                            const uint32_t* sp, const DecRope& p, cudaStream_t st, bool pdl = false);
@@ -288,11 +317,11 @@ struct FusedRope {
 // part_stride floats, its counters nkv words, its step words 4 words.
 struct AttnTokens {
     int n;  // 0 or 1: one token
-    size_t act_stride, planes_stride, part_stride;
+    size_t act_stride, part_stride;
 };
 // counters: nkv zeroed words (left zero by every launch); status: set to 1 if a bounded wait gave up.
 cudaError_t launch_attend(const float* q, void* kc, void* vc, int kv_f16, float* out, float* part, uint32_t* counters,
-                          const uint32_t* sp, const DecAttn& p, XPlanes xp, uint32_t* status, cudaStream_t st, bool pdl = false,
+                          const uint32_t* sp, const DecAttn& p, uint32_t* status, cudaStream_t st, bool pdl = false,
                           const FusedRope* fr = nullptr, const AttnTokens* tokens = nullptr);
 // Host-order rows [n][nkv][hd] f32 <-> cache rows pos0 .. pos0 + n - 1.
 cudaError_t launch_kv_rows(float* rows, void* cache, int kv_f16, bool to_cache, uint32_t nkv, uint32_t hd, uint32_t max_len, uint32_t pos0,

@@ -1,6 +1,6 @@
-// Decode plan: resolves a b2_graph to device pointers, decides where the activation planes of each
-// matrix-vector product come from (written by the norm / attention kernel that produces the vector, or by
-// a plane kernel of their own), captures the op list into CUDA graphs, and runs steps.
+// Decode plan: resolves a b2_graph to device pointers, decides where each product's activation split is made (by
+// the product itself, with the RMS norm in front of it, or by a kernel of its own), captures the op list into CUDA
+// graphs, and runs steps.
 // What the reference does per token with ~11 cuLaunchKernel calls per layer from the host
 // (src/cuda_decode.rs:1466-1658) is one cudaGraphLaunch here.
 #include "plan.h"
@@ -18,11 +18,9 @@ namespace b2 {
 
 namespace {
 
-constexpr uint32_t OP_XPLANES = 100;
+constexpr uint32_t OP_SPLIT = 100;  // internal: the record of a vector (launch_split)
 constexpr int ATT_THREADS_HOST = 256;  // threads of an attention unit (a thread per head dimension makes the token's key row)
 static bool overlaps_f(const float* a, size_t na, const float* b, size_t nb) { return a && b && na && nb && a < b + nb && b < a + na; }
-constexpr uint32_t OP_NORM_DEFERRED = 101;  // internal: planes of x * w and per-block sums of squares; the products apply the factor  // internal: planes of a vector no producer kernel could write
-
 std::string fmt(const char* f, ...) {
     char buf[512];
     va_list ap;
@@ -60,7 +58,12 @@ void row_bytes(const WeightDev& w, size_t (&rb)[4]) {
             rb[0] = K;
             rb[1] = (K / 32) * 2;
             break;
+        case B2_FMT_F8E4M3: rb[0] = K; break;  // (its block scales: fuse_rows)
     }
+}
+// Whether a matrix's rows may be a part of a concatenation: FP8 parts have to be whole rows of scale blocks.
+bool fusable(const WeightDev& w) {
+    return w.fmt != B2_FMT_F8E4M3 || w.p1 == nullptr || (w.n_out % w.bs_rows == 0 && w.bs_row0 % w.bs_rows == 0);
 }
 
 // One matrix whose rows are the rows of `parts` in order (same format and n_in): device copies, owned by the plan.
@@ -85,6 +88,22 @@ cudaError_t fuse_rows(const std::vector<const WeightDev*>& parts, WeightDev* out
         }
         out->*planes[pl] = d;
     }
+    if (parts[0]->fmt == B2_FMT_F8E4M3 && parts[0]->p1) {
+        const size_t row = parts[0]->bs_ncb * 4;
+        uint8_t* d = nullptr;
+        cudaError_t e = cudaMalloc((void**)&d, total / parts[0]->bs_rows * row);
+        if (e != cudaSuccess) return e;
+        owned.push_back(d);
+        size_t at = 0;
+        for (const WeightDev* w : parts) {
+            const size_t bytes = w->n_out / w->bs_rows * row;
+            e = cudaMemcpy(d + at, w->p1 + w->bs_row0 / w->bs_rows * row, bytes, cudaMemcpyDeviceToDevice);
+            if (e != cudaSuccess) return e;
+            at += bytes;
+        }
+        out->p1 = d;
+        out->bs_row0 = 0;
+    }
     return cudaSuccess;
 }
 
@@ -106,7 +125,7 @@ DecodePlanImpl::~DecodePlanImpl() {
     for (void* m : peer_maps_) cudaIpcCloseMemHandle(m);
     for (auto& kv : gemm_plans_)
         for (GemmPlan* gp : kv.second) gemm_tc_plan_destroy(gp);
-    void* frees[] = {kv16_, x16_, unscale_, tmp_a_, tmp_b_, gemm_status_, norm_partials_, xflags_, bufs_, planes_, consts_, part_, words_, rope_table_, argmax_val_, argmax_idx_, token_, out_tokens_, stage_};
+    void* frees[] = {kv16_, x16_, unscale_, tmp_a_, tmp_b_, gemm_status_, xflags_, bufs_, records_, consts_, part_, words_, rope_table_, argmax_val_, argmax_idx_, token_, out_tokens_, stage_};
     for (void* p : frees)
         if (p) cudaFree(p);
 }
@@ -117,7 +136,7 @@ bool DecodePlanImpl::uses_weight(uint64_t h) const {
     return h != 0 && h == gen_embed_;
 }
 
-int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDev*(uint64_t)>& resolve, int sm_count, int planes, int tokens,
+int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDev*(uint64_t)>& resolve, int sm_count, bool fast, int tokens,
                            bool prefill, DecodePlanImpl** out, std::string& err) {
     if (!g || !g->bufs || !g->ops || g->n_bufs == 0 || g->n_ops == 0 || !out) {
         err = "[b200qmm: decode_plan: empty graph]";
@@ -137,20 +156,18 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
     }
     std::unique_ptr<DecodePlanImpl> p(new DecodePlanImpl());
     p->sm_count_ = sm_count;
+    p->fast_ = fast;
     p->tokens_ = tokens;
     const size_t T = (size_t)tokens;
     if (const char* e = getenv("B2_PLAN_PDL")) p->pdl_ = atoi(e) != 0;
     if (const char* e = getenv("B2_PLAN_FUSE")) p->fuse_ = atoi(e) != 0;
     if (const char* e = getenv("B2_PLAN_DEFER_NORM")) p->defer_norm_ = atoi(e) != 0;
-    int epi_level = 1;  // 1: products that add into the residual row (their split is a deferred norm); 2: gate / up pairs too
-    if (const char* e = getenv("B2_PLAN_EPILOGUE")) {
-        epi_level = atoi(e);
-        p->epilogue_ = epi_level != 0;
-    }
+    int self_level = 2;  // which products split their vectors themselves: 0 none, 1 those behind a norm, 2 all
+    if (const char* e = getenv("B2_PLAN_EPILOGUE")) self_level = atoi(e);
     if (const char* e = getenv("B2_PLAN_FUSE_ROPE")) p->fuse_rope_ = atoi(e) != 0;
     if (prefill) {  // the one-token kernels' fusions do not apply: the products are GEMMs
         p->prefill_ = true;
-        p->defer_norm_ = p->fuse_rope_ = p->epilogue_ = false;
+        p->defer_norm_ = p->fuse_rope_ = false;
         const char* e = getenv("B2_PREFILL_ATTEND");
         p->loop_attend_ = e && strcmp(e, "loop") == 0;
     }
@@ -222,18 +239,13 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
     };
 
     // ---- ops -------------------------------------------------------------------------------------
-    // Planes bookkeeping. key = (buffer, offset, length) of a vector; `valid` = planes of the current
-    // contents exist in that region; `writer` = index (in ops_) of the norm / attention op that wrote
-    // exactly this vector last and can still be told to write its planes.
-    using Key = std::tuple<uint32_t, uint32_t, uint32_t>;
-    std::map<Key, size_t> valid;    // -> region index
-    std::map<Key, size_t> writer;   // -> op index
-    std::vector<size_t> region_k;   // K of each planes region
-    auto touch = [&](uint32_t buf) {  // a write into `buf`: planes and writers of its vectors are stale
+    // Records of vectors. key = (buffer, offset, length, form); `valid` = the region that holds the record of the current contents.
+    using Key = std::tuple<uint32_t, uint32_t, uint32_t, bool>;
+    std::map<Key, size_t> valid;
+    std::vector<std::pair<size_t, bool>> regions;  // length and form
+    auto touch = [&](uint32_t buf) {  // a write into `buf`: records of its vectors are stale
         for (auto it = valid.begin(); it != valid.end();) it = std::get<0>(it->first) == buf ? valid.erase(it) : std::next(it);
-        for (auto it = writer.begin(); it != writer.end();) it = std::get<0>(it->first) == buf ? writer.erase(it) : std::next(it);
     };
-    std::vector<std::pair<size_t, size_t>> region_of_op;  // (op index, region): xp filled in once regions are allocated
 
     for (uint32_t i = 0; i < g->n_ops; i++) {
         const b2_op& o = g->ops[i];
@@ -248,11 +260,10 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
                 size_t xs = o.x_stride ? o.x_stride : o.n, os = o.out_stride ? o.out_stride : o.n;
                 op.x = view(o.x, (size_t)(o.rows - 1) * xs + o.n);
                 op.y = view(o.y, (size_t)(o.rows - 1) * os + o.n);
-                op.norm = DecNorm{o.n, (uint32_t)xs, (uint32_t)os, o.add ? 1u : 0u, 0u, o.pre == 0.0f ? 1.0f : o.pre, o.eps};
+                op.norm = DecNorm{o.n, (uint32_t)xs, (uint32_t)os, o.add ? 1u : 0u, o.pre == 0.0f ? 1.0f : o.pre, o.eps};
                 op.rows = o.rows;
                 if (o.p0) PLAN_CUDA(put_const(o.p0, o.n, &op.p0), "cudaMemcpy(norm weights)");
                 touch(o.y.buf);
-                if (o.rows == 1 && o.n % 32 == 0) writer[Key{o.y.buf, o.y.off, o.n}] = p->ops_.size();
                 break;
             }
             case B2_OP_LINEAR: {
@@ -300,7 +311,7 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
                 if (o.mode == B2_MODE_ADD_GATED) op.z = view(o.z, 1);
                 // Products of the same vector that store into consecutive ranges (q, k, v) run as one launch over
                 // a row-wise concatenation of their matrices (a device copy the plan owns).
-                if (p->fuse_ && o.mode == B2_MODE_STORE && w->fmt != B2_FMT_F8E4M3) {
+                if (p->fuse_ && o.mode == B2_MODE_STORE && fusable(*w)) {
                     std::vector<const WeightDev*> parts{w};
                     uint32_t end = o.y.off + o.n_out, j = i + 1;
                     for (; j < g->n_ops; j++) {
@@ -309,7 +320,9 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
                             n.y.buf != o.y.buf || n.y.off != end || n.y.buf == n.x.buf)
                             break;
                         const WeightDev* nw = resolve(n.w);
-                        if (!nw || nw->fmt != w->fmt || nw->n_in != w->n_in || nw->n_out != n.n_out || nw->group != w->group) break;
+                        if (!nw || nw->fmt != w->fmt || nw->n_in != w->n_in || nw->n_out != n.n_out || nw->group != w->group || !fusable(*nw) ||
+                            nw->bs_rows != w->bs_rows || nw->bs_cols != w->bs_cols || nw->bs_ncb != w->bs_ncb || !nw->p1 != !w->p1)
+                            break;
                         parts.push_back(nw);
                         p->weight_handles_.push_back(n.w);
                         end += n.n_out;
@@ -320,32 +333,22 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
                         i = j - 1;  // the fused ops are done
                     }
                 }
-                if (w->fmt != B2_FMT_F8E4M3 && !prefill) {
-                    Key key{o.x.buf, o.x.off, o.n_in};
-                    size_t region;
-                    auto v = valid.find(key);
-                    if (v != valid.end()) {
-                        region = v->second;
-                    } else {
-                        region = region_k.size();
-                        region_k.push_back(o.n_in);
-                        auto wr = writer.find(key);
-                        if (wr != writer.end()) {
-                            Op& prod = p->ops_[wr->second];
-                            if (prod.kind == B2_OP_NORM) prod.norm.planes = 1;
-                            else prod.attn.planes = 1;
-                            region_of_op.push_back({wr->second, region});
-                        } else {
-                            Op xp;
-                            xp.kind = OP_XPLANES;
-                            xp.x = op.x;
-                            xp.n = o.n_in;
-                            region_of_op.push_back({p->ops_.size(), region});
-                            p->ops_.push_back(xp);
-                        }
-                        valid[key] = region;
+                if (!prefill && gemv_mma_supports(op.w)) {
+                    const bool halves = gemv_mma_halves(op.w);
+                    auto [v, fresh] = valid.try_emplace(Key{o.x.buf, o.x.off, o.n_in, halves}, regions.size());
+                    if (fresh) {
+                        Op sp;
+                        sp.kind = OP_SPLIT;
+                        sp.x = sp.sx = op.x;
+                        sp.n = o.n_in;
+                        sp.halves = halves;
+                        sp.region = (int)regions.size();
+                        regions.push_back({o.n_in, halves});
+                        p->ops_.push_back(sp);
                     }
-                    region_of_op.push_back({p->ops_.size(), region});
+                    op.region = (int)v->second;
+                    op.sx = op.x;
+                    op.halves = halves;
                 }
                 if (o.y.buf == o.x.buf && !(o.y.off + o.n_out <= o.x.off || o.x.off + o.n_in <= o.y.off)) {
                     err = "[b200qmm: decode_plan: a linear op writes over its own input]";
@@ -390,11 +393,10 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
                 op.x = view(o.x, (size_t)o.nh * o.hd);
                 op.y = view(o.y, (size_t)o.nh * o.hd);
                 op.kv = o.kv;
-                op.attn = DecAttn{o.nh, o.nkv, o.hd, g->max_len, o.window, 0u, o.scale};
+                op.attn = DecAttn{o.nh, o.nkv, o.hd, g->max_len, o.window, o.scale};
                 max_nh = std::max(max_nh, o.nh);
                 max_hd = std::max(max_hd, o.hd);
                 touch(o.y.buf);
-                writer[Key{o.y.buf, o.y.off, o.nh * o.hd}] = p->ops_.size();
                 break;
             }
             case B2_OP_GLU: {
@@ -443,82 +445,103 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
         return B2_ERR_ARG;
     }
 
-    // ---- norms whose output only products read: the factor moves behind the product -----------------------------
-    // The one-CTA norm spends most of its time splitting the row into planes on a single SM; when nothing reads the
-    // normalized row itself (every reader is a product over its planes), a grid of independent warps splits x * w and
-    // leaves the blocks' sums of squares, and the products multiply by the factor (NormScale).
-    size_t norm_floats = 0;
+    // What an op reads and writes, as far as the passes below need it (they treat attention and RoPE as touching their whole views).
+    auto reads = [&](const Op& o, const float* v, size_t n) {
+        switch (o.kind) {
+            case B2_OP_LINEAR:
+                return (o.region < 0 && overlaps_f(v, n, o.x, o.w.n_in)) || (o.mode == B2_MODE_ADD_GATED && overlaps_f(v, n, o.z, 1)) ||
+                       ((o.mode == B2_MODE_ADD || o.mode == B2_MODE_ADD_GATED) && overlaps_f(v, n, o.y, o.w.n_out));
+            case OP_SPLIT: return overlaps_f(v, n, o.sx, o.n);
+            case B2_OP_NORM:
+                return overlaps_f(v, n, o.x, (size_t)(o.rows - 1) * o.norm.x_stride + o.norm.n) ||
+                       (o.norm.add && overlaps_f(v, n, o.y, (size_t)(o.rows - 1) * o.norm.out_stride + o.norm.n));
+            case B2_OP_EXCHANGE: return overlaps_f(v, n, o.x, o.n);
+            case B2_OP_GLU: return overlaps_f(v, n, o.x, o.n) || overlaps_f(v, n, o.z, o.n);
+            default: return overlaps_f(v, n, o.x, n) || overlaps_f(v, n, o.y, n) || overlaps_f(o.x, 1, v, n);
+        }
+    };
+    auto writes = [&](const Op& o, const float* v, size_t n) {
+        switch (o.kind) {
+            case B2_OP_LINEAR: return overlaps_f(v, n, o.y, o.w.n_out);
+            case OP_SPLIT: return false;
+            case B2_OP_NORM: return overlaps_f(v, n, o.y, (size_t)(o.rows - 1) * o.norm.out_stride + o.norm.n);
+            case B2_OP_EXCHANGE: return overlaps_f(v, n, o.x, o.n);
+            case B2_OP_GLU: return overlaps_f(v, n, o.y, o.n);
+            case B2_OP_ATTEND: return overlaps_f(v, n, o.y, (size_t)o.attn.nh * o.attn.hd);
+            default: return overlaps_f(v, n, o.y, (size_t)o.rope.nh * o.rope.hd);
+        }
+    };
+    // ---- norms whose output only splits read become part of the split: x times the weights is split, and the products multiply their
+    // results by the factor (nothing has to wait for the whole row first, and the norm is not launched) ----
     if (p->defer_norm_) {
-        auto overlaps = [](const float* a, size_t na, const float* b, size_t nb) { return a && b && a < b + nb && b < a + na; };
         for (size_t a = 0; a < p->ops_.size(); a++) {
-            Op& nrm = p->ops_[a];
-            if (nrm.kind != B2_OP_NORM || !nrm.norm.planes || nrm.rows != 1 || nrm.norm.add) continue;
+            const Op nrm = p->ops_[a];
+            if (nrm.kind != B2_OP_NORM || nrm.rows != 1 || nrm.norm.add || nrm.norm.n % 4) continue;
             const float* y = nrm.y;
             const size_t n = nrm.norm.n;
-            if (overlaps(y, n, p->hidden_, p->n_hidden_) || overlaps(y, n, p->logits_, p->n_logits_) || overlaps(y, n, p->input_, p->n_input_)) continue;
-            bool ok = true;
+            if (overlaps_f(y, n, p->hidden_, p->n_hidden_) || overlaps_f(y, n, p->logits_, p->n_logits_) || overlaps_f(y, n, p->input_, p->n_input_)) continue;
+            bool ok = true, stale = false;
             std::vector<size_t> users;
             for (size_t b = a + 1; b < p->ops_.size() && ok; b++) {
                 const Op& o = p->ops_[b];
-                bool writes = false;
-                switch (o.kind) {
-                    case B2_OP_LINEAR:
-                        if (o.x == y && o.w.n_in == n && o.w.fmt != B2_FMT_F8E4M3) users.push_back(b);
-                        else if (overlaps(y, n, o.x, o.w.n_in)) ok = false;
-                        if (overlaps(y, n, o.y, o.w.n_out)) {
-                            if (o.mode != B2_MODE_STORE && !o.pair) ok = false;  // reads what it adds to
-                            writes = true;
-                        }
-                        break;
-                    case B2_OP_NORM:
-                    case OP_NORM_DEFERRED:
-                        if (overlaps(y, n, o.x, (size_t)(o.rows - 1) * o.norm.x_stride + o.norm.n)) ok = false;
-                        writes = overlaps(y, n, o.y, (size_t)(o.rows - 1) * o.norm.out_stride + o.norm.n);
-                        break;
-                    case OP_XPLANES: ok = ok && !overlaps(y, n, o.x, o.n); break;
-                    case B2_OP_EXCHANGE:
-                        if (overlaps(y, n, o.x, o.n)) ok = false;
-                        break;
-                    case B2_OP_GLU:
-                        if (overlaps(y, n, o.x, o.n) || overlaps(y, n, o.z, o.n)) ok = false;
-                        writes = overlaps(y, n, o.y, o.n);
-                        break;
-                    default:  // RoPE, attention: any overlap of their views with the row disqualifies it
-                        if (overlaps(y, n, o.x, n) || overlaps(y, n, o.y, n)) ok = false;
-                        break;
-                }
-                if (writes) break;
+                if (o.kind == OP_SPLIT && o.sx == y && o.n == n && !o.normed && !stale) users.push_back(b);
+                else if (reads(o, y, n)) ok = false;
+                if (writes(o, y, n)) break;
+                stale = stale || writes(o, nrm.x, n);  // a split behind this point would read another x
             }
             if (!ok || users.empty()) continue;
-            nrm.kind = OP_NORM_DEFERRED;
-            nrm.ns = NormScale{(const float*)(uintptr_t)norm_floats, (uint32_t)(n / 32), 1.0f / (float)n, nrm.norm.eps};  // offset now, pointer below
-            for (size_t b : users) p->ops_[b].ns = nrm.ns;
-            norm_floats += (n / 32 + 63) / 64 * 64;
+            for (size_t b : users) {
+                Op& s = p->ops_[b];
+                s.sx = nrm.x;
+                s.nw = nrm.p0;
+                s.npre = nrm.norm.pre;
+                s.neps = nrm.norm.eps;
+                s.normed = 1;
+            }
+            p->ops_.erase(p->ops_.begin() + (ptrdiff_t)a);
+            a--;
         }
     }
-    p->partial_block_ = norm_floats;
-    if (norm_floats) {
-        PLAN_CUDA(cudaMalloc((void**)&p->norm_partials_, T * norm_floats * sizeof(float)), "cudaMalloc(norm partial sums)");
-        PLAN_CUDA(cudaMemset(p->norm_partials_, 0, T * norm_floats * sizeof(float)), "cudaMemset(norm partial sums)");
-        for (Op& o : p->ops_)
-            if ((o.kind == OP_NORM_DEFERRED || o.kind == B2_OP_LINEAR) && o.ns.count)
-                o.ns.partial = p->norm_partials_ + (size_t)(uintptr_t)o.ns.partial;
+    // ---- products that split their vector themselves: every product of the record must find the vector unchanged, and none may
+    // write over it (its CTAs read the vector at different times) ----
+    for (size_t a = 0; a < p->ops_.size(); a++) {
+        Op& s = p->ops_[a];
+        if (s.kind != OP_SPLIT) continue;
+        bool ok = self_level >= (s.normed ? 1 : 2);
+        std::vector<size_t> users;
+        bool stale = false;
+        for (size_t b = a + 1; b < p->ops_.size(); b++) {
+            Op& o = p->ops_[b];
+            const bool user = o.kind == B2_OP_LINEAR && o.region == s.region;
+            if (user) {
+                users.push_back(b);
+                if (stale || writes(o, s.sx, s.n)) ok = false;
+            }
+            stale = stale || writes(o, s.sx, s.n);
+        }
+        s.self = ok;
+        for (size_t b : users) {
+            Op& o = p->ops_[b];
+            o.sx = s.sx;
+            o.nw = s.nw;
+            o.npre = s.npre;
+            o.neps = s.neps;
+            o.normed = s.normed;
+            o.self = s.self;
+        }
     }
-
-    // ---- planes regions ---------------------------------------------------------------------------
-    size_t planes_total = 0;
-    std::vector<size_t> region_at(region_k.size());
-    for (size_t r = 0; r < region_k.size(); r++) {
-        region_at[r] = planes_total;
-        planes_total += align_up(xplanes_bytes(region_k[r]), 256);
+    // ---- records ---------------------------------------------------------------------------------
+    size_t rec_total = 0;
+    std::vector<size_t> region_at;
+    for (auto& [n, halves] : regions) {
+        region_at.push_back(rec_total);
+        rec_total += align_up(split_bytes_of(n, halves), 256);
     }
-    planes_total = std::max<size_t>(planes_total, 256);
-    p->planes_block_ = planes_total;
-    PLAN_CUDA(cudaMalloc((void**)&p->planes_, T * planes_total), "cudaMalloc(planes)");
-    for (auto& [oi, r] : region_of_op) {
-        p->ops_[oi].xp = xplanes_at(p->planes_ + region_at[r], region_k[r]);
-        p->ops_[oi].xp.np = planes;
-    }
+    rec_total = std::max<size_t>(rec_total, 256);
+    p->rec_block_ = rec_total;
+    PLAN_CUDA(cudaMalloc((void**)&p->records_, T * rec_total), "cudaMalloc(records)");
+    for (Op& o : p->ops_)
+        if (o.region >= 0) o.rec_at = region_at[(size_t)o.region];
 
     // ---- RoPE inside the attention kernel ----------------------------------------------------------------------
     // A QK_ROPE op without per-head norms whose rotated queries only the ATTEND op right behind it reads: the attention
@@ -543,9 +566,9 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
                     const float* q0 = rp->y;
                     const size_t qn = (size_t)rp->rope.nh * rp->rope.hd;
                     const size_t xn = o.kind == B2_OP_LINEAR ? o.w.n_in : o.kind == B2_OP_ATTEND ? (size_t)o.attn.nh * o.attn.hd
-                                      : (o.kind == B2_OP_NORM || o.kind == OP_NORM_DEFERRED) ? (size_t)(o.rows - 1) * o.norm.x_stride + o.norm.n : o.n;
+                                      : o.kind == B2_OP_NORM ? (size_t)(o.rows - 1) * o.norm.x_stride + o.norm.n : o.n;
                     if (o.kind == B2_OP_ATTEND && o.x == q0) continue;  // another layer's attention over its own fused queries
-                    if (overlaps_f(q0, qn, o.x, xn) || overlaps_f(q0, qn, o.z, o.n ? o.n : 1)) other_reader = true;
+                    if (overlaps_f(q0, qn, o.x, xn) || overlaps_f(q0, qn, o.z, o.n ? o.n : 1) || overlaps_f(q0, qn, o.sx, xn)) other_reader = true;
                 }
                 if (!other_reader) {
                     at.fr = FusedRope{rp->x, nullptr, rp->rope};  // the table's address is known at launch
@@ -554,30 +577,6 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
                 }
             }
             kept.push_back(at);
-        }
-        p->ops_ = std::move(kept);
-    }
-
-    // ---- planes written by the product ahead ---------------------------------------------------------------------
-    // A split kernel (deferred norm, or the planes of an MLP activation) that directly follows the 4-bit product which
-    // wrote its whole input is dropped: that product's CTAs then own whole blocks of 32 rows and split each block once
-    // its rows are done (EpiPlanes). Saves a launch per product whose output feeds another product.
-    if (p->epilogue_ && p->pdl_) {
-        std::vector<Op> kept;
-        kept.reserve(p->ops_.size());
-        for (size_t b = 0; b < p->ops_.size(); b++) {
-            const Op& nx = p->ops_[b];
-            Op* lin = kept.empty() ? nullptr : &kept.back();
-            if (lin && lin->kind == B2_OP_LINEAR && !lin->epi.out.planes && gemv_takes_epilogue(lin->w)) {
-                const size_t n = lin->w.n_out;
-                const bool norm = nx.kind == OP_NORM_DEFERRED && nx.x == lin->y && nx.norm.n == n && nx.rows == 1;
-                const bool split = nx.kind == OP_XPLANES && nx.x == lin->y && nx.n == n && (epi_level >= 2 || !lin->pair);
-                if (norm || split) {
-                    lin->epi = EpiPlanes{nx.xp, norm ? nx.p0 : nullptr, norm ? const_cast<float*>(nx.ns.partial) : nullptr, norm ? nx.norm.pre : 1.0f};
-                    continue;
-                }
-            }
-            kept.push_back(nx);
         }
         p->ops_ = std::move(kept);
     }
@@ -658,18 +657,40 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
     return B2_OK;
 }
 
+GemvIn DecodePlanImpl::product_in(const Op& o, bool self) const {
+    GemvIn in;
+    if (self) {
+        in.x = o.sx;
+        in.x_stride = block_floats_;
+        in.norm_w = o.nw;
+        in.pre = o.npre;
+    } else {
+        in.rec = records_ + o.rec_at;
+        in.rec_stride = rec_block_;
+    }
+    in.norm = o.normed;
+    in.eps = o.neps;
+    in.fast = fast_;
+    return in;
+}
+
 // `chained`: every launch but the first (`first_chained`: the first too) carries the programmatic-dependent-launch
 // attribute, so each kernel starts (and fetches its first weights) while the one before it drains.
 int DecodePlanImpl::run_ops(cudaStream_t st, std::string& err, bool chained, bool first_chained) {
+    launches_ = 0;
     for (size_t i = 0; i < ops_.size(); i++) {
         const Op& o = ops_[i];
-        const bool pdl = chained && (i > 0 || first_chained);
+        if (o.kind == OP_SPLIT && o.self) continue;
+        const bool pdl = chained && (launches_ > 0 || first_chained);
+        launches_++;
         cudaError_t e = cudaSuccess;
         switch (o.kind) {
-            case B2_OP_NORM: e = launch_norm(o.x, o.y, o.p0, o.norm, o.rows, o.xp, st, pdl); break;
-            case OP_XPLANES: e = launch_xplanes(o.x, o.n, o.xp, st, pdl); break;
-            case OP_NORM_DEFERRED: e = launch_norm_planes(o.x, o.p0, o.norm.pre, o.norm.n, o.xp, const_cast<float*>(o.ns.partial), st, pdl); break;
-            case B2_OP_LINEAR: e = launch_gemv(o.w, o.pair ? &o.w2 : nullptr, o.x, o.xp, o.y, o.mode, o.z, sm_count_, st, pdl, o.ns, o.epi); break;
+            case B2_OP_NORM: e = launch_norm(o.x, o.y, o.p0, o.norm, o.rows, st, pdl); break;
+            case OP_SPLIT: e = launch_split(o.sx, 0, o.nw, o.npre, o.n, 1, records_ + o.rec_at, 0, o.halves, fast_, st, pdl); break;
+            case B2_OP_LINEAR:
+                e = o.region >= 0 ? launch_gemv_mma(o.w, o.pair ? &o.w2 : nullptr, product_in(o, o.self), 1, o.y, 0, o.mode, o.z, 0, sm_count_, st, pdl)
+                                  : launch_gemv_f8_float(o.w, o.pair ? &o.w2 : nullptr, o.x, o.y, o.mode, o.z, sm_count_, st, pdl);
+                break;
             case B2_OP_QK_ROPE:
                 e = launch_qk_rope(o.x, o.y, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.p0, o.p1, rope_table_, sp_, o.rope, st, pdl);
                 break;
@@ -677,9 +698,9 @@ int DecodePlanImpl::run_ops(cudaStream_t st, std::string& err, bool chained, boo
                 if (o.fr.qkv) {
                     FusedRope fr = o.fr;
                     fr.cs_table = rope_table_;
-                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, part_, att_counters_, sp_, o.attn, o.xp, status_, st, pdl, &fr);
+                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, part_, att_counters_, sp_, o.attn, status_, st, pdl, &fr);
                 } else {
-                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, part_, att_counters_, sp_, o.attn, o.xp, status_, st, pdl);
+                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, part_, att_counters_, sp_, o.attn, status_, st, pdl);
                 }
                 break;
             case B2_OP_GLU: e = launch_glu(o.x, o.z, o.y, o.n, o.gelu, st, pdl); break;
@@ -696,25 +717,12 @@ int DecodePlanImpl::run_ops(cudaStream_t st, std::string& err, bool chained, boo
     return B2_OK;
 }
 
-// The ops for nt tokens at once, op by op: a product reads its weights once for all tokens where the tokens' vectors fit in
-// shared memory together (launch_gemv_multi: each token's sums are its one-token sums), every other op runs once per token
-// on that token's blocks (activations, planes, norm sums, step words). Attention and RoPE are ordinary launches, not
-// dependent ones: token i's attention reads the keys the launches just ahead of it appended, and its first key tile is
-// fetched before the dependency wait.
+// The ops for nt tokens at once, op by op: a product reads its weights once for all tokens (each token's sums are its one-token sums),
+// every other op runs once per token on that token's blocks (activations, records, step words) or has the token as a grid dimension.
+// Attention and RoPE are ordinary launches, not dependent ones: token i's attention reads the keys the launches just ahead of it
+// appended, and its first key tile is fetched before the dependency wait.
 int DecodePlanImpl::run_ops_multi(cudaStream_t st, int nt, std::string& err, bool chained) {
     auto A = [&](const float* p, int tk) -> float* { return p ? const_cast<float*>(p) + (size_t)tk * block_floats_ : nullptr; };
-    auto P = [&](XPlanes xp, int tk) {
-        if (!xp.planes) return xp;
-        const size_t off = (size_t)tk * planes_block_;
-        xp.planes = (int8_t*)((uint8_t*)xp.planes + off);
-        xp.sx = (float2*)((uint8_t*)xp.sx + off);
-        xp.v16 = (int32_t*)((uint8_t*)xp.v16 + off);
-        return xp;
-    };
-    auto N = [&](NormScale ns, int tk) {
-        if (ns.partial) ns.partial += (size_t)tk * partial_block_;
-        return ns;
-    };
     bool first = true;
     uint64_t count = 0;
     auto pdl = [&]() {
@@ -723,50 +731,32 @@ int DecodePlanImpl::run_ops_multi(cudaStream_t st, int nt, std::string& err, boo
         count++;
         return v;
     };
+    // A vector's record is made in a launch of its own where the products would have more than `self_blocks` blocks of 256 values per
+    // warp to split, every CTA all of them.
+    static const size_t self_blocks = [] {
+        const char* e = getenv("B2_PLAN_SELF_BLOCKS");
+        return e ? (size_t)atoi(e) : (size_t)2;
+    }();
+    auto self = [&](const Op& o, size_t n) { return o.self && split_blocks_of(n) * (size_t)nt <= 16 * self_blocks; };
     for (size_t i = 0; i < ops_.size(); i++) {
         const Op& o = ops_[i];
         cudaError_t e = cudaSuccess;
         switch (o.kind) {
             case B2_OP_NORM:
-                for (int tk = 0; tk < nt && e == cudaSuccess; tk++)
-                    e = launch_norm(A(o.x, tk), A(o.y, tk), o.p0, o.norm, o.rows, P(o.xp, tk), st, pdl());
+                for (int tk = 0; tk < nt && e == cudaSuccess; tk++) e = launch_norm(A(o.x, tk), A(o.y, tk), o.p0, o.norm, o.rows, st, pdl());
                 break;
-            case OP_XPLANES:  // one launch for all tokens (a block of a token's planes is made by one warp either way: the same bits)
-                e = launch_xplanes(o.x, o.n, o.xp, st, pdl(), nt, block_floats_, planes_block_);
+            case OP_SPLIT:
+                if (!self(o, o.n)) e = launch_split(o.sx, block_floats_, o.nw, o.npre, o.n, nt, records_ + o.rec_at, rec_block_, o.halves, fast_, st, pdl());
                 break;
-            case OP_NORM_DEFERRED:
-                e = launch_norm_planes(o.x, o.p0, o.norm.pre, o.norm.n, o.xp, const_cast<float*>(o.ns.partial), st, pdl(), nt, block_floats_, planes_block_,
-                                       partial_block_);
-                break;
-            case B2_OP_LINEAR: {
-                // FP8 products go token by token: their one-token kernel is the tensor-core one, and the tokens must match it.
-                // So do two tokens of a Q6_K / Q8_0 product: their several-token kernel does a token's arithmetic per token, and the
-                // one-token launches are the faster form inside a chain of dependent launches (gemv_multi_pays).
-                const bool together = o.mode != B2_MODE_ADD_GATED && o.w.fmt != B2_FMT_F8E4M3 && gemv_multi_pays(o.w, nt);
-                if (together) {
-                    e = launch_gemv_multi(o.w, o.pair ? &o.w2 : nullptr, o.x, block_floats_, o.xp, planes_block_, o.y, block_floats_, nt, o.mode,
-                                          sm_count_, st, pdl(), o.ns, partial_block_);
-                    // the split the one-token product does in its epilogue (the same bits as the kernels of their own)
-                    if (e == cudaSuccess && o.epi.out.planes) {
-                        if (o.epi.partial)
-                            e = launch_norm_planes(o.y, o.epi.w, o.epi.pre, o.w.n_out, o.epi.out, o.epi.partial, st, pdl(), nt, block_floats_, planes_block_,
-                                                   partial_block_);
-                        else
-                            e = launch_xplanes(o.y, o.w.n_out, o.epi.out, st, pdl(), nt, block_floats_, planes_block_);
-                    }
+            case B2_OP_LINEAR:
+                if (o.region >= 0) {
+                    e = launch_gemv_mma(o.w, o.pair ? &o.w2 : nullptr, product_in(o, self(o, o.w.n_in)), nt, o.y, block_floats_, o.mode, o.z, block_floats_, sm_count_,
+                                        st, pdl());
                     break;
                 }
-                for (int tk = 0; tk < nt && e == cudaSuccess; tk++) {
-                    EpiPlanes epi = o.epi;
-                    if (epi.out.planes) {
-                        epi.out = P(epi.out, tk);
-                        if (epi.partial) epi.partial += (size_t)tk * partial_block_;
-                    }
-                    e = launch_gemv(o.w, o.pair ? &o.w2 : nullptr, A(o.x, tk), P(o.xp, tk), A(o.y, tk), o.mode, A(o.z, tk), sm_count_, st, pdl(),
-                                    N(o.ns, tk), epi);
-                }
+                for (int tk = 0; tk < nt && e == cudaSuccess; tk++)
+                    e = launch_gemv_f8_float(o.w, o.pair ? &o.w2 : nullptr, A(o.x, tk), A(o.y, tk), o.mode, A(o.z, tk), sm_count_, st, pdl());
                 break;
-            }
             case B2_OP_QK_ROPE:  // all tokens in one launch (the one-token arithmetic per head)
                 e = launch_qk_rope_rows(o.x, o.y, block_floats_, (uint32_t)nt, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.p0, o.p1, rope_table_, sp_multi_, o.rope,
                                         st);
@@ -781,9 +771,9 @@ int DecodePlanImpl::run_ops_multi(cudaStream_t st, int nt, std::string& err, boo
                                             sp_multi_, o.fr.r, st);
                     count++;
                 }
-                const AttnTokens at{nt, block_floats_, planes_block_, part_stride_};
+                const AttnTokens at{nt, block_floats_, part_stride_};
                 if (e == cudaSuccess)
-                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, part_, att_counters_, sp_multi_, o.attn, o.xp, status_, st, false, nullptr,
+                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, part_, att_counters_, sp_multi_, o.attn, status_, st, false, nullptr,
                                       &at);
                 first = false;
                 count++;
@@ -971,11 +961,11 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
                 } else if (o.rows == 1) {
                     DecNorm n = o.norm;
                     n.x_stride = n.out_stride = (uint32_t)ld;
-                    e = launch_norm(o.x, o.y, o.p0, n, rows, XPlanes{}, st, false);
+                    e = launch_norm(o.x, o.y, o.p0, n, rows, st, false);
                     count++;
                 } else {
                     for (size_t tk = 0; tk < t && e == cudaSuccess; tk++, count++)
-                        e = launch_norm(o.x + tk * ld, o.y + tk * ld, o.p0, o.norm, o.rows, XPlanes{}, st, false);
+                        e = launch_norm(o.x + tk * ld, o.y + tk * ld, o.p0, o.norm, o.rows, st, false);
                 }
                 if (overlaps_f(o.y, (size_t)(o.rows - 1) * o.norm.out_stride + o.norm.n, x16_src, x16_k)) x16_src = nullptr;
                 break;
@@ -1025,7 +1015,7 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
                 if (loop_attend_) {
                     for (size_t tk = 0; tk < t && e == cudaSuccess; tk++, count++)
                         e = launch_attend(o.x + tk * ld, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y + tk * ld, part_, att_counters_, sp_multi_ + 4 * tk, o.attn,
-                                          XPlanes{}, status_, st, false, nullptr);
+                                          status_, st, false, nullptr);
                 } else {
                     e = launch_attend_rows(o.x, o.y, ld, rows, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, kv16_, (uint32_t)(pos + t), sp_, o.attn, st);
                     count += kv_f16_ ? 1 : 3;
@@ -1251,13 +1241,12 @@ int DecodePlanImpl::attach_peers(uint32_t rank, uint32_t world, const void* hand
                 if (o.kind == B2_OP_EXCHANGE) break;
                 switch (o.kind) {
                     case B2_OP_LINEAR:
-                        if (o.w.fmt == B2_FMT_F8E4M3) need = reads_outside(o.x, o.w.n_in, ex);
+                        if (o.self || o.region < 0) need = reads_outside(o.region < 0 ? o.x : o.sx, o.w.n_in, ex);
                         if (o.mode != B2_MODE_STORE && !o.pair) need = need || reads_outside(o.y, o.w.n_out, ex);
                         need = need || reads_outside(o.z, 1, ex);
                         break;
-                    case B2_OP_NORM:
-                    case OP_NORM_DEFERRED: need = reads_outside(o.x, (size_t)(o.rows - 1) * o.norm.x_stride + o.norm.n, ex); break;
-                    case OP_XPLANES: need = reads_outside(o.x, o.n, ex); break;
+                    case B2_OP_NORM: need = reads_outside(o.x, (size_t)(o.rows - 1) * o.norm.x_stride + o.norm.n, ex); break;
+                    case OP_SPLIT: need = !o.self && reads_outside(o.sx, o.n, ex); break;
                     case B2_OP_GLU: need = reads_outside(o.x, o.n, ex) || reads_outside(o.z, o.n, ex); break;
                     case B2_OP_QK_ROPE: need = reads_outside(o.x, (size_t)o.rope.v_off + (size_t)o.rope.nkv * o.rope.hd + (size_t)o.rope.nh * o.rope.q_stride, ex); break;
                     case B2_OP_ATTEND: need = reads_outside(o.x, (size_t)o.attn.nh * o.attn.hd, ex); break;

@@ -15,13 +15,13 @@ class DecodePlanImpl {
   public:
     // `resolve` maps a weight handle to its device description (nullptr: unknown handle).
     // Returns B2_OK, B2_DECLINED or an error code; `err` gets the reason.
-    // `planes`: how many planes of the activation split the plan's products read (2: the upper two, 16 bits; otherwise all three, 21 bits).
+    // `fast`: the plan's products read 16 bits of every activation (b2_set_fast_planes).
     // `tokens` (1..4): the most tokens of a step (Backend::decode_plan_multi, src/gpu.rs:273-276). A plan of several tokens keeps
-    // one activation block, planes block and block of norm sums per token.
+    // one activation block and block of records per token.
     // `prefill`: a prefill plan (Backend::decode_plan_prefill, src/gpu.rs:283-289): steps of up to `tokens` (1..8192) tokens on
     // batched kernels (tensor-core GEMMs for the products, tensor-core causal attention), whose results differ from one-token
     // steps in rounding. Such a plan takes no logits (the reference's prefill graph ends at the final norm).
-    static int create(const b2_graph* g, const std::function<const WeightDev*(uint64_t)>& resolve, int sm_count, int planes, int tokens,
+    static int create(const b2_graph* g, const std::function<const WeightDev*(uint64_t)>& resolve, int sm_count, bool fast, int tokens,
                       bool prefill, DecodePlanImpl** out, std::string& err);
     ~DecodePlanImpl();
 
@@ -39,13 +39,13 @@ class DecodePlanImpl {
                  const float* rope_cs_table, int32_t* out_tokens, float* elapsed_ms, std::string& err);
     int export_handle(void* out128, std::string& err);
     int attach_peers(uint32_t rank, uint32_t world, const void* handles, std::string& err);
-    uint64_t launches_per_step() const { return prefill_ ? prefill_launches_ : (uint64_t)ops_.size(); }
-    uint64_t launches_per_step(size_t t) const { return prefill_ ? prefill_launches_ : t >= 2 && t <= 4 ? multi_launches_[t] : (uint64_t)ops_.size(); }
+    uint64_t launches_per_step() const { return prefill_ ? prefill_launches_ : launches_; }
+    uint64_t launches_per_step(size_t t) const { return prefill_ ? prefill_launches_ : t >= 2 && t <= 4 ? multi_launches_[t] : launches_; }
     bool uses_weight(uint64_t h) const;
 
   private:
     struct Op {
-        uint32_t kind = 0;  // B2_OP_*, or OP_XPLANES
+        uint32_t kind = 0;  // B2_OP_*, or OP_SPLIT
         float *x = nullptr, *y = nullptr, *z = nullptr;
         WeightDev w{}, w2{};
         bool pair = false;
@@ -60,12 +60,20 @@ class DecodePlanImpl {
         int gelu = 0;
         bool meet_first = true;  // EXCHANGE: meet the peers before writing too
         size_t off = 0;  // EXCHANGE: offset of the vector in the activation block, in floats
-        NormScale ns{};      // LINEAR: the deferred norm factor of its vector; deferred NORM: where its partial sums go
-        XPlanes xp{};  // planes this op writes (norm, attend, xplanes) or reads (linear)
+        // Where a product's vector comes from (LINEAR) or what is split (SPLIT): f32 values, an RMS norm's weights and eps where the norm
+        // is part of the split, and the record; `self`: the products may split the vector themselves (the SPLIT op is then not
+        // launched).
+        float* sx = nullptr;
+        const float* nw = nullptr;
+        float npre = 1.0f, neps = 0.0f;
+        int normed = 0;
+        int region = -1;
+        size_t rec_at = 0;
+        bool halves = false, self = false;
         FusedRope fr{};   // ATTEND: RoPE and the cache append done by the attention kernel (the QK_ROPE op ahead of it is dropped)
-        EpiPlanes epi{};  // LINEAR: the planes of its output, written by its own last warps (the split kernel behind it is dropped)
     };
     DecodePlanImpl() = default;
+    GemvIn product_in(const Op& o, bool self) const;
     int run_ops(cudaStream_t st, std::string& err, bool chained, bool first_chained);
     int run_ops_multi(cudaStream_t st, int nt, std::string& err, bool chained);
     int run_prefill(cudaStream_t st, size_t pos, size_t t, std::string& err);
@@ -74,9 +82,11 @@ class DecodePlanImpl {
     int check_status(std::string& err);
 
     std::vector<Op> ops_;
-    // plans of several tokens: token i's activations, planes and norm sums sit these strides after token 0's
+    // plans of several tokens: token i's activations and records sit these strides after token 0's
     int tokens_ = 1;
-    size_t block_floats_ = 0, planes_block_ = 0, partial_block_ = 0;
+    size_t block_floats_ = 0, rec_block_ = 0;
+    bool fast_ = false;
+    uint64_t launches_ = 0;               // kernels of a one-token step
     uint32_t* sp_multi_ = nullptr;        // [tokens][4] step words, inside words_
     std::vector<uint32_t> cs_off_;        // start of each RoPE table's values inside a row of the device table
     cudaGraphExec_t multi_exec_[5] = {};  // [nt], nt = 2 .. tokens
@@ -102,17 +112,15 @@ class DecodePlanImpl {
     PeerSet peers_{};
     uint32_t* xflags_ = nullptr;  // this rank's flag words
     std::vector<void*> peer_maps_;  // what cudaIpcOpenMemHandle returned
-    bool defer_norm_ = true;  // norms that feed only products: factor applied after the product (B2_PLAN_DEFER_NORM=0: off)
-    float* norm_partials_ = nullptr;
+    bool defer_norm_ = true;  // norms that feed only products run inside the split of their vector (B2_PLAN_DEFER_NORM=0: off)
     bool fuse_ = true;  // q / k / v style products of one vector as one launch over concatenated rows (B2_PLAN_FUSE=0: off)
     std::vector<void*> fused_;  // device copies made for that
     bool fuse_rope_ = true;  // RoPE inside the attention kernel where no per-head norm is asked for (B2_PLAN_FUSE_ROPE=0: separate kernels)
-    bool epilogue_ = true;  // a 4-bit product writes the planes the next product reads (B2_PLAN_EPILOGUE=0: separate kernels)
     // one allocation each
     float* bufs_ = nullptr;
     std::vector<float*> buf_ptr_;
     std::vector<size_t> buf_len_;
-    uint8_t* planes_ = nullptr;
+    uint8_t* records_ = nullptr;
     float* consts_ = nullptr;  // norm weights
     struct Kv {
         void *k = nullptr, *v = nullptr;
