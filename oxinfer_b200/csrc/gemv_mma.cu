@@ -12,7 +12,6 @@
 // weights multiply before the split, the factor multiplies the results), or as records that launch_split made. Where the split vectors
 // of all tokens do not fit beside the rings, K is taken in parts and the slices' sums wait in shared memory between them.
 #include <algorithm>
-#include <cstdlib>
 
 #include "gemv_mma.cuh"
 
@@ -335,8 +334,6 @@ cudaError_t launch_t(Args& a, int sm_count, cudaStream_t st, bool pdl) {
     const int slices = 1 << a.slice_log;
     const size_t tiles = (a.w.n_out + ROWS - 1) / ROWS;
     a.ks = slices;
-    static const int ks_env = getenv("B2_KS") ? atoi(getenv("B2_KS")) : 0;
-    if (ks_env) a.ks = std::min(ks_env, slices);
     const int groups = WARPS / a.ks;
     const int span = std::max(slices, BPX), xblocks = (a.blocks + BPX - 1) / BPX;
     // the sums of a few tiles wait for one barrier: 8 KB of them, twice, over all groups
@@ -352,13 +349,17 @@ cudaError_t launch_t(Args& a, int sm_count, cudaStream_t st, bool pdl) {
         fixed -= comb;
         comb = (size_t)groups * slices * RES * 4;
         fixed += comb;
-        grid = std::max(grid, (tiles + (size_t)groups * MAX_TILES - 1) / ((size_t)groups * MAX_TILES));
-        a.hold_tiles = (int)((tiles + grid * groups - 1) / (grid * groups));
-        hold = (size_t)WARPS * a.hold_tiles * (slices / a.ks) * NT * 256;
         // parts of whole rounds of the slices where one fits, else of as many units as fit
         size_t step = (size_t)std::max(1, span * a.bpu / BPX);  // in blocks of the split
-        const size_t least = (size_t)std::max(1, a.bpu / BPX);
-        if (fixed + hold + least * per_block > SMEM_MAX) return cudaErrorInvalidValue;
+        const size_t least = (size_t)std::max(1, a.bpu / BPX), per_tile = (size_t)WARPS * (slices / a.ks) * NT * 256;
+        if (fixed + per_tile + least * per_block > SMEM_MAX) return cudaErrorInvalidValue;
+        // The waiting sums may take the room that a round leaves; a group that has more tiles than that goes in several waves of CTAs.
+        const size_t room = SMEM_MAX - fixed - (fixed + per_tile + step * per_block <= SMEM_MAX ? step : least) * per_block;
+        const size_t most = std::min<size_t>(MAX_TILES, room / per_tile), wave = (size_t)sm_count * groups;
+        const size_t waves = (tiles + wave * most - 1) / (wave * most);
+        if (waves > 1) grid = waves * sm_count;
+        a.hold_tiles = (int)((tiles + grid * groups - 1) / (grid * groups));
+        hold = a.hold_tiles * per_tile;
         part = (SMEM_MAX - fixed - hold) / per_block;
         if (part < step) step = least;
         part = part / step * step;
@@ -392,7 +393,8 @@ cudaError_t launch_f(Args& a, bool pair, int sm_count, cudaStream_t st, bool pdl
 }  // namespace
 
 bool gemv_mma_supports(const WeightDev& w) {
-    if ((uintptr_t)w.p0 & 15) return false;
+    // (the longest rows: a unit of eight tokens' activations has to fit beside the rings and the norm's sums, launch_t)
+    if (((uintptr_t)w.p0 & 15) || w.n_in > (w.fmt == B2_FMT_F8E4M3 ? 51200 : 58512)) return false;
     switch (w.fmt) {
         case B2_FMT_MLX4:
         case B2_FMT_Q4_K: return w.n_in % 256 == 0;

@@ -43,7 +43,8 @@ __device__ __forceinline__ SplitIn split_load(const float* x, const float* w, in
 
 // The values times pre and the weights, their largest magnitude's bits over the warp, and the sum of squares before the weights.
 __device__ __forceinline__ void split_values(const SplitIn& in, float pre, float (&v)[8], uint32_t& max_bits, float& ssq) {
-    float q = 0.0f, mx = 0.0f;
+    float q = 0.0f;
+    uint32_t mx = 0;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const float a[4] = {in.x[h].x * pre, in.x[h].y * pre, in.x[h].z * pre, in.x[h].w * pre};
@@ -52,10 +53,10 @@ __device__ __forceinline__ void split_values(const SplitIn& in, float pre, float
         for (int i = 0; i < 4; i++) {
             q = fmaf(a[i], a[i], q);
             v[4 * h + i] = a[i] * b[i];
-            mx = fmaxf(mx, fabsf(v[4 * h + i]));
+            mx = max(mx, __float_as_uint(v[4 * h + i]) & 0x7fffffffu);  // non-negative floats order like their bit patterns, NaN last
         }
     }
-    max_bits = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));  // non-negative floats order like their bit patterns
+    max_bits = __reduce_max_sync(0xffffffffu, mx);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
     ssq = q;
@@ -75,7 +76,7 @@ __device__ __forceinline__ SplitDigits split_digits(const SplitIn& in, float pre
     // the largest scales into (2^22, QMAX], or one power lower when it would exceed it
     const int up = mb == 0 ? 0 : min(126, max(-126, 149 - (int)(mb >> 23) - ((mb & 0x7fffffu) > 0x7efefeu ? 1 : 0)));
     const float k = __uint_as_float((uint32_t)(127 + up) << 23);
-    r.xs = __uint_as_float((uint32_t)(127 - up) << 23);
+    r.xs = mb >= 0x7f800000u ? __uint_as_float(0x7fffffffu) : __uint_as_float((uint32_t)(127 - up) << 23);  // (digits cannot hold an infinity or a NaN)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         uint32_t u[4];
