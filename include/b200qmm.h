@@ -103,18 +103,17 @@ const char* b2_open_error(void);
 /* Kernels are launched on `cuda_stream` (a cudaStream_t / CUstream; NULL = the default stream,
  * which is what src/cuda.rs:609-629 uses). Host-buffer entry points synchronize that stream. */
 int b2_set_stream(b2_ctx* ctx, void* cuda_stream);
-/* No counterpart in the reference. While on, the device-resident matrix-vector calls (b2_matvec_dev,
- * b2_matvec_prepared_dev, b2_prepare_x_dev) launch with the programmatic-dependent-launch attribute: each kernel may
- * start, and fetch its first weights, while the kernel ahead of it on the stream drains; it waits for that kernel before
- * it reads the vector or writes its output, so results are unchanged. Meant for a caller that queues a token's
- * products back to back (the decode plan does this by itself). Off by default. */
+/* No counterpart in the reference. The device-resident matrix-vector calls (b2_matvec_dev, b2_matvec_prepared_dev) launch with the
+ * programmatic-dependent-launch attribute: each kernel may start, and fetch its first weights, while the kernel ahead of it on
+ * the stream drains; it waits for that kernel before it reads the vector or writes its output, so results are unchanged. This
+ * switch asks the same of the generic kernels of the other GGUF formats, which launch the ordinary way by default. */
 int b2_set_chained(b2_ctx* ctx, int on);
 /* The boundary's exactness switch, `gpu::set_exact` / `exact()` (src/gpu.rs:313-338: "no reduced-precision matrix units").
  * Off (the default), a many-token matmul rounds activations and expanded weights to f16 operands once: results within 1e-3
  * of the f64 product per output row (FP8: 2e-3). On, the tensor-core GEMM takes every f32 / bf16 activation as two f16
  * terms and, for Q4_K, every weight as two f16 terms too (the other 4-bit and 8-bit formats' values need no second term):
  * results within 1e-4 per output row, the bound the reference holds its own f32 CUDA kernels to (src/cuda.rs:1684), at two to
- * four times the tensor-core work. Matrix-vector products (t <= 8) carry 21-bit activations either way. */
+ * four times the tensor-core work. Matrix-vector products (t <= 8) carry 23-bit activations either way. */
 int b2_set_exact(b2_ctx* ctx, int on);
 /* No counterpart in the reference, whose FP8 matrices multiply unquantized activations (src/ggml.rs:433-443; that stays the
  * default here and is what the 2e-3 parity bound refers to). On: b2_matmul / b2_matmul_dev over F8E4M3 weights with 128 x 128
@@ -125,11 +124,10 @@ int b2_set_exact(b2_ctx* ctx, int on);
  * e4m3's quantization noise (about 2e-2 per row). b2_set_exact takes precedence. */
 int b2_set_fp8_activations(b2_ctx* ctx, int on);
 /* No counterpart in the reference. Matrix-vector products (t <= 8, the decode plan, small MoE batches) multiply exact integer
- * digits of the activations, 21 bits per block of 32 in three planes; that is the default and holds a decoder layer to 1e-6
- * of the f64 oracle. On, the products read only the upper two planes (16 bits: every element rounded to 1.6e-5 of its
- * block's largest): a third fewer integer dot products, 5 % more decode tokens per second and 13 % on Q6_K, with errors of
- * 2e-5 .. 2e-4 per product row and 3e-4 through a decoder layer (inside the 1e-3 bound, not inside the default's). Read by
- * calls made, and by decode plans created, after it is set. b2_set_exact takes precedence. */
+ * digits of the activations, 23 to 24 bits of the largest value of each block of 256; that is the default and holds a decoder
+ * layer to 1e-6 of the f64 oracle. On, every element is rounded to 18 bits instead (at most 7.6e-6 of its block's largest): errors
+ * of 1e-5 .. 1e-4 per product row, inside the 1e-3 bound, not inside the default's, at the same speed (the digits are multiplied
+ * together). Read by calls made, and by decode plans created, after it is set. b2_set_exact takes precedence. */
 int b2_set_fast_planes(b2_ctx* ctx, int on);
 /* `Backend::stats`, src/cuda.rs:1120-1132: cumulative copy-in / kernel / copy-out time as text. */
 const char* b2_stats(b2_ctx* ctx);
@@ -221,11 +219,11 @@ int b2_moe_dev(b2_ctx* ctx, b2_moe_handle m, const float* x_dev, size_t t, const
  * of n_experts logits, the k largest (ties to the lower index) and exp(l - max) / sum over the chosen. */
 int b2_route_topk_dev(b2_ctx* ctx, const float* logits_dev, size_t t, size_t n_experts, size_t k, int32_t* ids_dev, float* w_dev);
 
-/* The two halves of b2_matvec_dev, for a plan in which one vector feeds several products (q, k, v;
- * gate and up): b2_prepare_x_dev splits x into the integer planes the 4- / 6- / 8-bit kernels read
- * (the role of quantize_act, which the reference's CPU driver runs once per batch of jobs,
- * src/kernels.rs:1731-1879), b2_matvec_prepared_dev runs one product over the planes prepared last.
- * n_in must match; FP8 weights read x_dev itself. */
+/* The two halves of b2_matvec_dev, for a caller in which one vector feeds several products (q, k, v;
+ * gate and up): b2_prepare_x_dev keeps a copy of x (the role of quantize_act, which the reference's CPU
+ * driver runs once per batch of jobs, src/kernels.rs:1731-1879; the products split it themselves),
+ * b2_matvec_prepared_dev runs one product over the vector prepared last. n_in must match; FP8 weights
+ * and the other GGUF formats read x_dev itself. */
 int b2_prepare_x_dev(b2_ctx* ctx, const float* x_dev, size_t n_in);
 int b2_matvec_prepared_dev(b2_ctx* ctx, b2_weight w, b2_weight up, const float* x_dev, float* y_dev, int mode, const float* gate_dev);
 
@@ -402,15 +400,13 @@ int b2_moe_ep(b2_ctx* ctx, b2_moe_handle m, size_t n_experts_global, const float
 /* No counterpart in the reference (its CUDA backend allocates staging and arena memory freely,
  * src/cuda.rs:572-699). One Q4_K matrix-vector product, y[n_out] = W x, that allocates nothing, for
  * hosts that cannot call cudaMalloc when they need it: a server whose own arena already owns the
- * whole device, or a decode loop that must stay out of the allocator. The activation planes the
- * kernel needs live in a fixed device array inside the library (57,344 bytes per GPU for as long as
- * the library is loaded), which limits n_in to B2_NOALLOC_MAX_K; larger inputs are refused with
+ * whole device, or a decode loop that must stay out of the allocator. The kernel splits the vector
+ * in its shared memory; n_in is limited to B2_NOALLOC_MAX_K, larger inputs are refused with
  * B2_ERR_ARG and a message, and go through b2_matvec_dev instead.
  *   w_blocks_dev : raw GGUF Q4_K super-blocks on the device, [n_out][n_in/256][144], 16-byte aligned
  *   x_dev, y_dev : f32 on the device; cuda_stream : the stream to launch on (NULL = default)
  *   err, err_len : optional buffer that receives the error text
- * The first call on a device looks up the array's device address; make it before any stream
- * capture. All calls share the one array: calls that may overlap on the GPU race on it. */
+ * The first call on a device sets the kernel up; make it before any stream capture. */
 #define B2_NOALLOC_MAX_K 16384
 int b2_matvec_q4k_noalloc(const void* w_blocks_dev, size_t n_out, size_t n_in, const float* x_dev, float* y_dev, void* cuda_stream,
                           char* err, size_t err_len);

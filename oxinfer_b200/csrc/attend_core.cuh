@@ -5,7 +5,7 @@
 
 #include "async_copy.cuh"
 #include "kernels.h"
-#include "xplanes.cuh"
+#include "pdl.cuh"
 
 namespace b2 {
 namespace attend_core {

@@ -114,14 +114,6 @@ class Backend {
     // only conditions are the kernels' shape rules.
     bool wants(size_t n_out, size_t n_in, size_t t) const { return t >= 1 && n_out >= 1 && n_in % 32 == 0; }
 
-    // The planes record at `base` as the products of this context read it: all three planes, or the upper two under
-    // b2_set_fast_planes (never under the exactness switch).
-    int planes_read() const { return fast_planes && !exact ? 2 : 3; }
-    XPlanes planes_at(void* base, size_t K) const {
-        XPlanes p = xplanes_at(base, K);
-        p.np = planes_read();
-        return p;
-    }
     int alloc_copy(const void* host, size_t bytes, void** out, std::vector<void*>& owned) {
         void* p = nullptr;
         cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
@@ -446,7 +438,7 @@ class Backend {
         Weight* w = find(h);
         if (!w) return fail(B2_ERR_ARG, "[b200qmm: matvec: unknown weight]");
         if (w->dev.fmt == B2_FMT_F8E4M3 || fmt_is_other(w->dev.fmt)) return matvec_dev(h, up, x_dev_, y_dev_, mode, gate);
-        if (prepared_k != w->dev.n_in) return fail(B2_ERR_ARG, "[b200qmm: matvec: no planes prepared for n_in = %zu (b2_prepare_x_dev)]", w->dev.n_in);
+        if (prepared_k != w->dev.n_in) return fail(B2_ERR_ARG, "[b200qmm: matvec: no vector prepared for n_in = %zu (b2_prepare_x_dev)]", w->dev.n_in);
         return matvec_dev(h, up, (const float*)xprep.p, y_dev_, mode, gate);
     }
 
@@ -497,9 +489,11 @@ class Backend {
     }
     // t tokens of one matrix from their records, up to eight per launch (the weights are read once per launch). A matrix whose tiles
     // fill no more than half the SMs goes four at a time: the launches run side by side, and a launch of four has half the arithmetic.
+    // So does one that has more tiles than the SMs have groups of warps, unless the activations of eight fit whole: the parts of K then
+    // pass over several tiles each. Q4_K 28672 x 4096, 8 tokens: 161 us in one launch, 63 in two; 4096 x 14336: 48 and 63.
     int small_products(const WeightDev& w, const WeightDev* up, const uint8_t* rec, size_t t, float* y, int mode) {
         const size_t stride = record_stride(w.n_in, gemv_mma_halves(w)), tiles = (w.n_out + 15) / 16;
-        const size_t per = 2 * tiles <= (size_t)sm_count ? 4 : 8;
+        const size_t per = 2 * tiles <= (size_t)sm_count || (tiles > 2 * (size_t)sm_count && w.n_in > GEMV_WHOLE_8) ? 4 : 8;
         for (size_t i = 0; i < t; i += per) {
             GemvIn in;
             in.rec = rec + i * stride;
@@ -858,26 +852,53 @@ class Backend {
     // ---- Backend::moe (src/gpu.rs:232-248, src/cuda.rs:798-966): y[i] += sum_j w_ij down_e(act(gate_e x_i) * up_e x_i).
     // The host builds the per-expert segments as the reference does (src/cuda.rs:810-857), padded to the
     // GEMM's 128-row token tile; x_dev / y_dev are device f32 [t][h].
-    // A few (token, route) pairs (decode): every pair is its own matrix-vector product, so the tensor-core GEMM's 128-row
-    // tiles would be almost empty. Five launches instead: planes of the tokens, one batched GEMV over the pairs' fused
-    // gate / up matrices (SiLU pair), planes of the activations, one batched GEMV over the down matrices, and the ordered
-    // combine (src/moe.rs:625-828 does the same per expert on the CPU; exact f32 / integer arithmetic, no f16 operands).
-    int moe_small(const Moe& m, const float* x_dev_, size_t t, const int32_t* ids, const float* rw, size_t k, float* y_dev_) {
+    // Few tokens per expert (decode, small batches): the 128-row tiles of the tensor-core GEMM would be almost empty. Three launches
+    // instead: the fused gate / up product and the down product of gemv_mma.cu over groups of up to eight pairs of one expert, and the
+    // ordered combine (src/moe.rs:625-828 does the same per expert on the CPU; f32-like arithmetic, no f16 operands). The routes travel as
+    // kernel arguments: no copy, no synchronization.
+    // Time of a group of up to 1 / 4 / 8 pairs of one expert, and of a 128-row tile of the tensor-core GEMM with one- and with two-term
+    // operands, in us per million weights of an expert; the GEMM path has a copy, a synchronization and two launches more.
+    static constexpr double GROUP_US[3] = {0.13, 0.195, 0.32}, TILE_US[2] = {0.55, 1.55}, TILES_US = 25.0;
+    // The cheapest group size that fits (8, 4, 1; 0: none does), and the time of the layer's groups.
+    int moe_group_size(const Moe& m, const std::vector<size_t>& count, double& us) {
+        const int fits = std::min(gemv_groups_most(m.h), gemv_groups_most(m.inter));
+        int best = 0;
+        for (int i = 0; i < 3; i++) {
+            const int size = i == 0 ? 1 : 4 * i;
+            size_t n = 0;
+            for (size_t c : count) n += (c + size - 1) / size;
+            const double v = n * GROUP_US[i] * (3e-6 * m.inter * m.h);
+            if (size <= fits && (best == 0 || v < us)) {
+                best = size;
+                us = v;
+            }
+        }
+        return best;
+    }
+    int moe_small(const Moe& m, const float* x_dev_, size_t t, const int32_t* ids, const float* rw, size_t k, float* y_dev_, const std::vector<size_t>& count,
+                  int size) {
         const size_t R = t * k;
-        const size_t sx = (xplanes_bytes(m.h) + 255) / 256 * 256, sa = (xplanes_bytes(m.inter) + 255) / 256 * 256;
-        cudaError_t e = moe_xg.reserve(t * sx);
-        if (e == cudaSuccess) e = moe_g.reserve(R * m.inter * 4);
-        if (e == cudaSuccess) e = moe_a.reserve(R * sa);
+        cudaError_t e = moe_g.reserve(R * m.inter * 4);
         if (e == cudaSuccess) e = moe_o.reserve(R * m.h * 4);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(moe scratch)");
-        // the routes travel as kernel arguments: no copy, no synchronization
-        GemvBatch b1{}, b2{};
+        // the pairs in the order of their experts
+        GemvGroups gr{};
         SmallRoutes routes{};
-        b1.n = b2.n = (int)R;
+        std::vector<size_t> at(m.experts, 0);
+        size_t rows = 0;
+        for (size_t x = 0; x < m.experts; x++) {
+            at[x] = rows;
+            for (size_t c = 0; size && c < count[x]; c += size) {
+                gr.expert[gr.n] = (uint16_t)x;
+                gr.row0[gr.n] = (uint16_t)(rows + c);
+                gr.count[gr.n++] = (uint8_t)std::min<size_t>(size, count[x] - c);
+            }
+            rows += count[x];
+        }
         for (size_t i = 0; i < R; i++) {
-            b1.expert[i] = b2.expert[i] = ids[i];
-            b1.xrow[i] = (int)(i / k);  // the pair's token
-            b2.xrow[i] = (int)i;        // the pair's own activations
+            const size_t slot = at[ids[i]]++;
+            gr.src[slot] = (uint16_t)(i / k);
+            routes.slot[i] = (uint16_t)slot;
             routes.w[i] = rw[i];
         }
         const size_t rb_h = m.h / 256 * 144, rb_i = m.inter / 256 * 144;
@@ -893,25 +914,35 @@ class Backend {
         down.n_out = m.h;
         down.n_in = m.inter;
         down.p0 = (const uint8_t*)m.down;
-        e = launch_xplanes_rows(x_dev_, t, m.h, (uint8_t*)moe_xg.p, sx, stream);
-        b1.w_stride = 2 * m.inter * rb_h;
-        b1.x_stride = sx;
-        b1.y_stride = m.inter;
-        b1.planes = (uint8_t*)moe_xg.p;
-        b2.w_stride = m.h * rb_i;
-        b2.x_stride = sa;
-        b2.y_stride = m.h;
-        b2.planes = (uint8_t*)moe_a.p;
-        if (e == cudaSuccess)
-            e = launch_gemv_batched(gate, &up, b1, R, (float*)moe_g.p, m.act == B2_ACT_GELU_TANH ? B2_MODE_GELU_PAIR : B2_MODE_SILU_PAIR, planes_read(), sm_count, stream,
-                                    true);
-        // (the five kernels are a chain of dependent launches: each may start while the one ahead drains and waits for it
-        // before it reads what that one wrote)
-        if (e == cudaSuccess) e = launch_xplanes_rows((const float*)moe_g.p, R, m.inter, (uint8_t*)moe_a.p, sa, stream, true);
-        if (e == cudaSuccess) e = launch_gemv_batched(down, nullptr, b2, R, (float*)moe_o.p, B2_MODE_STORE, planes_read(), sm_count, stream, true);
-        if (e == cudaSuccess) e = launch_moe_combine_small((const float*)moe_o.p, routes, t, k, m.h, y_dev_, stream, true);
-        launches += 5;
-        if (e != cudaSuccess) return cuda_fail(e, "moe (batched matrix-vector path)");
+        const int mode = m.act == B2_ACT_GELU_TANH ? B2_MODE_GELU_PAIR : B2_MODE_SILU_PAIR;
+        const bool fast = fast_planes && !exact;
+        float *g = (float*)moe_g.p, *o = (float*)moe_o.p;
+        if (size) {
+            gr.gather = 1;
+            gr.w_stride = 2 * m.inter * rb_h;
+            e = launch_gemv_groups(gate, &up, x_dev_, m.h, gr, size, g, m.inter, mode, fast, sm_count, stream);
+            gr.gather = 0;
+            gr.w_stride = m.h * rb_i;
+            if (e == cudaSuccess) e = launch_gemv_groups(down, nullptr, g, m.inter, gr, size, o, m.h, B2_MODE_STORE, fast, sm_count, stream);
+            launches += 2;
+        }
+        for (size_t i = 0; !size && i < R && e == cudaSuccess; i++) {  // rows longer than a group takes: pair by pair
+            const size_t x = (size_t)ids[i], slot = routes.slot[i];
+            WeightDev ge = gate, ue = up, de = down;
+            ge.p0 += x * 2 * m.inter * rb_h;
+            ue.p0 += x * 2 * m.inter * rb_h;
+            de.p0 += x * m.h * rb_i;
+            GemvIn in;
+            in.fast = fast;
+            in.x = x_dev_ + i / k * m.h;
+            e = launch_gemv_mma(ge, &ue, in, 1, g + slot * m.inter, 0, mode, nullptr, 0, sm_count, stream, true);
+            in.x = g + slot * m.inter;
+            if (e == cudaSuccess) e = launch_gemv_mma(de, nullptr, in, 1, o + slot * m.h, 0, B2_MODE_STORE, nullptr, 0, sm_count, stream, true);
+            launches += 2;
+        }
+        if (e == cudaSuccess) e = launch_moe_combine_small(o, routes, t, k, m.h, y_dev_, stream, true);
+        launches++;
+        if (e != cudaSuccess) return cuda_fail(e, "moe (grouped matrix-vector path)");
         return B2_OK;
     }
 
@@ -935,7 +966,15 @@ class Backend {
             count[(size_t)ids[i]]++;
         }
         // (the clamped SiLU has no fused pair mode in the matrix-vector kernels: those layers take the GEMM path at any batch)
-        if (t * k <= 64 && m.act != B2_ACT_SILU_CLAMP && !getenv("B2_MOE_NO_GEMV")) return moe_small(m, x_dev_, t, ids, rw, k, y_dev_);
+        if (t * k <= GEMV_GROUP_ROWS && m.experts <= 65536 && m.act != B2_ACT_SILU_CLAMP && !getenv("B2_MOE_NO_GEMV")) {
+            double us = 0.0;
+            const int size = moe_group_size(m, count, us);
+            size_t tiles = 0;
+            for (size_t c : count) tiles += (c + 127) / 128;
+            const bool two = m.fmt == B2_FMT_Q4_K || exact;
+            if (t * k <= 64 || (size && us <= TILES_US + tiles * TILE_US[two] * (3e-6 * m.inter * m.h)))
+                return moe_small(m, x_dev_, t, ids, rw, k, y_dev_, count, size);
+        }
         // Token tiles of 128 or 256 rows. A tile costs about the same either way (the kernel is bound by the expansion of
         // the tile's weights, which both heights share), so the taller tile wins as soon as it needs clearly fewer tiles:
         // large batches, where the experts hold more than a tile's worth of tokens each.

@@ -3,7 +3,7 @@
 // never fuses `d1 * v - m1` (src/ggml.rs:769), `(q - 8) * d + m` (src/quant.rs:601) or
 // `d * sc * q` (src/ggml.rs:787).
 #include "dq_core.cuh"
-#include "xplanes.cuh"
+#include "pdl.cuh"
 
 namespace b2 {
 

@@ -1,288 +1,9 @@
-// Dequant products of one to eight tokens: the role of dmv_* and dmvk_* in the reference (src/cuda_decode.cu:139-232). See
-// gemv_mma.cuh for the arithmetic and split.cuh for the activations.
-//
-// One CTA of 16 warps per SM. K is summed in eight slices (units of one or two blocks in turn, so that neighbouring warps read
-// neighbouring bytes); KS warps share a tile of 16 rows, each taking 8 / KS of the slices, and the 16 / KS groups of warps take tiles of
-// their own. Each warp keeps units of packed weights in flight in a ring of shared memory of its own (cp.async), filled before the
-// kernel waits for the one ahead of it in the stream. The slices' sums of a few tiles wait in shared memory and are then added, in the
-// order of the slices, by all threads of the group. Neither KS nor the number of tokens changes the order of a sum, so every row
-// equals its one-token row bit for bit, in a row shard too.
-//
-// The activations come as f32 vectors and are split by the CTA itself (an RMS norm in front of the product runs in the same pass: the
-// weights multiply before the split, the factor multiplies the results), or as records that launch_split made. Where the split vectors
-// of all tokens do not fit beside the rings, K is taken in parts and the slices' sums wait in shared memory between them.
-#include <algorithm>
-
-#include "gemv_mma.cuh"
+// The products of one to eight tokens of the five tuned formats, and the activation split's own kernel (gemv_mma_kernel.cuh).
+#include "gemv_mma_kernel.cuh"
 
 namespace b2 {
 
-using namespace gmma;
-
 namespace {
-
-constexpr int WARPS = 16, THREADS = WARPS * 32;
-constexpr int MAX_TILES = 8;           // most tiles of a group whose sums wait between parts
-constexpr size_t SMEM_MAX = 226 * 1024;
-
-__device__ __forceinline__ float silu(float a) { return a / (1.0f + __expf(-a)); }
-__device__ __forceinline__ float gelu_tanh(float a) {
-    const float t = 0.7978845608f * (a + 0.044715f * a * a * a);
-    return 0.5f * a * (1.0f + tanhf(t));
-}
-
-struct Args {
-    WeightDev w, w2;
-    const float* x;        // token i at x + i * x_stride
-    size_t x_stride;
-    const float* nw;       // norm weights (null: none)
-    float pre;
-    int norm;              // multiply the results by 1 / sqrt(mean square + eps)
-    float eps;
-    const uint8_t* rec;    // or token i's record at rec + i * rec_stride
-    size_t rec_stride;
-    float* y;
-    size_t y_stride;
-    const float* gate;     // token i's gate at gate + i * gate_stride
-    size_t gate_stride;
-    int mode, T, ks, fast;
-    int units, part_units;  // units of k in all, and in a part
-    int blocks, bpu, slice_log, batch, bufs;  // blocks of the format, blocks per unit, log2 of the slices, tiles whose sums are added together, buffers for them
-    int hold_tiles;
-    uint32_t frag_off, xs_off, ssq_off, sums_off, hold_off, comb_off;  // shared memory
-};
-
-template <class F, bool PAIR, int TP, bool PARTS>
-__global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_constant__ Args a) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    using X = typename F::template X<TP>;
-    constexpr int ROWS = PAIR ? 8 : 16, S = F::SLOTS, BPX = 256 / F::BLOCK_K, NT = X::NT;  // BPX: blocks of the format per block of the split
-    pdl_launch_dependents();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    // (uniform over the warp, and the compiler should know)
-    const int ks = a.ks, wq = __shfl_sync(0xffffffffu, warp, 0), group = wq / ks, q = wq - group * ks, groups = WARPS / ks;
-    const int T = a.T;
-    const size_t n_out = a.w.n_out;
-    const int tiles = (int)((n_out + ROWS - 1) / ROWS), tile0 = group * (int)gridDim.x + (int)blockIdx.x, tile_step = groups * (int)gridDim.x;
-    const int my_tiles = tile0 < tiles ? (tiles - tile0 + tile_step - 1) / tile_step : 0;
-    // unit u, of `bpu` blocks, belongs to slice u % slices (a power of two)
-    const int sl_log = a.slice_log, slices = 1 << sl_log, bpu = a.bpu;
-    const int parts = PARTS ? (a.units + a.part_units - 1) / a.part_units : 1;
-    auto j_at = [&](int s, int u) { return (u - s + slices - 1) >> sl_log; };  // a slice's units below u
-    auto j_beg = [&](int s, int p) { return PARTS ? j_at(s, p * a.part_units) : 0; };
-    auto j_end = [&](int s, int p) { return j_at(s, PARTS ? min(a.units, (p + 1) * a.part_units) : a.units); };
-    const size_t last_row0 = n_out > 8 ? n_out - 8 : 0;
-    auto row_of = [&](int i, int half) { return min((size_t)(tile0 + i * tile_step) * ROWS + (PAIR ? 0 : 8 * half), last_row0); };
-    const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(smem);
-    const uint32_t ring = smem0 + (uint32_t)wq * (S * F::UNIT_BYTES), ring_end = ring + S * F::UNIT_BYTES;
-    uint32_t islot = ring, slot = ring;
-
-    // the copies run ahead of the arithmetic in the same order: parts, tiles, slices, units
-    typename F::template Copy<PAIR> cp;
-    cp.init(a.w, bpu, lane);
-    int ip = 0, it = 0, is = q, ij = 0, ije = j_end(q, 0);
-    bool more = my_tiles > 0 && q < a.units;
-    if (more) cp.tile(a.w, a.w2, row_of(0, 0), row_of(0, 1), lane);
-    auto next_run = [&] {  // the next slice of a tile, tile of a part, part
-        is += ks;
-        if (is >= slices) {
-            is = q;
-            if (++it == my_tiles) {
-                it = 0;
-                ip++;
-            }
-            cp.tile(a.w, a.w2, row_of(it, 0), row_of(it, 1), lane);
-        }
-        more = ip < parts;
-        ij = j_beg(is, ip);
-        ije = j_end(is, ip);
-    };
-    if (PARTS)
-        while (more && ij >= ije) next_run();
-    auto issue = [&] {
-        if (more) {
-            const int b = (is + (ij << sl_log)) * bpu;
-            cp.issue(islot, b, b + 2 > a.blocks, lane);
-            islot = islot + F::UNIT_BYTES == ring_end ? ring : islot + F::UNIT_BYTES;
-            if (++ij >= ije) do next_run();
-                while (more && ij >= ije);
-        }
-        cp_commit();
-    };
-#pragma unroll
-    for (int s = 0; s < S; s++) issue();
-    pdl_wait();
-
-    float* const xs_s = (float*)(smem + a.xs_off);
-    float* const ssq_s = (float*)(smem + a.ssq_off);
-    float2* const hold = (float2*)(smem + a.hold_off);
-    // the slices' sums of `batch` tiles, `bufs` times: [tile][slice][instruction's tokens][row 16][token]
-    constexpr int RES = X::RES;
-    float* const comb = (float*)(smem + a.comb_off) + (size_t)group * a.bufs * a.batch * slices * RES;
-    X xv;
-    {
-        if constexpr (F::HALVES) {
-            const int ct = TP == 1 ? 0 : g >> 1, rt = TP == 1 ? 0 : t;
-            xv.frag = smem0 + a.frag_off + (uint32_t)(ct * 128 + (g & 1) * 64 + t * 16);
-            xv.xs = smem0 + a.xs_off + 4u * (uint32_t)rt;
-            xv.sums = 0;
-        } else {
-            const int ct = TP == 1 ? 0 : g >> 2, cd = min(g & 3, 2), rt = TP == 1 ? 0 : t >> 1;
-            xv.frag = smem0 + a.frag_off + (uint32_t)(ct * 192 + cd * 64 + t * 16);
-            xv.xs = smem0 + a.xs_off + 4u * (uint32_t)rt;
-            xv.sums = smem0 + a.sums_off + (F::SUMS_BY_COLUMN ? (uint32_t)(ct * 32 + (g & 3) * 8 + t * 4) : (uint32_t)(rt * 32 + (t & 1) * 8));
-        }
-    }
-    const int xblocks = (a.blocks + BPX - 1) / BPX;  // of the split
-    for (int p = 0; p < parts; p++) {
-        const int b0 = PARTS ? p * (a.part_units * bpu / BPX) : 0, nb = PARTS ? min(xblocks, b0 + a.part_units * bpu / BPX) - b0 : xblocks;
-        if (PARTS && p > 0) __syncthreads();  // every warp is done with the part before
-        auto load = [&](int i) {
-            const int b = i / T, tk = i - b * T, k = (b0 + b) * 256;
-            return split_load(a.x + (size_t)tk * a.x_stride + k, a.nw ? a.nw + k : nullptr, (int)a.w.n_in - k, lane);
-        };
-        SplitIn next;
-        if (!a.rec && wq < nb * T) next = load(wq);
-        for (int i = wq; i < nb * T; i += WARPS) {
-            const int b = i / T, tk = i - b * T, blk = b0 + b;
-            uint8_t* f0 = smem + a.frag_off + (size_t)b * (X::BLOCK * TP) + tk * X::TOKEN;
-            int s;
-            float xs, ssq;
-            if (a.rec) {
-                const uint8_t* r = a.rec + (size_t)tk * a.rec_stride;
-                const uint4* src = (const uint4*)(r + (size_t)blk * X::BLOCK);
-                constexpr int PIECES = X::BLOCK / 16, PER = X::TOKEN / 16;  // pieces of 16 bytes
-                const uint4 v0 = __ldcg(src + lane);
-                uint4 v1 = make_uint4(0, 0, 0, 0);
-                if (lane + 32 < PIECES) v1 = __ldcg(src + 32 + lane);
-                const uint8_t* aux = r + (size_t)xblocks * X::BLOCK + (size_t)blk * SPLIT_AUX;
-                const float2 h0 = __ldcg((const float2*)aux);
-                s = F::SUMS ? __ldcg((const int*)(aux + 16) + (lane & 7)) : 0;
-                xs = h0.x;
-                ssq = h0.y;
-                *(uint4*)(f0 + (size_t)(lane / PER) * X::STEP + (lane % PER) * 16) = v0;
-                if (lane + 32 < PIECES) *(uint4*)(f0 + (size_t)((lane + 32) / PER) * X::STEP + ((lane + 32) % PER) * 16) = v1;
-            } else {
-                const SplitIn in = next;
-                if (i + WARPS < nb * T) next = load(i + WARPS);
-                if constexpr (F::HALVES) {
-                    const SplitHalves d = split_halves(in, a.pre);
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        uint8_t* o = f0 + (size_t)(4 * h + (lane >> 3)) * X::STEP + (lane & 3) * 16 + ((lane >> 2) & 1) * 8;
-                        *(uint2*)o = d.hi[h];
-                        *(uint2*)(o + 64) = d.lo[h];
-                    }
-                    xs = d.xs;
-                    ssq = d.ssq;
-                    s = 0;
-                } else {
-                    const SplitDigits d = split_digits(in, a.pre, a.fast);
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        int pair, in16;
-                        split_digit_at(h, lane, pair, in16);
-                        uint8_t* o = f0 + (size_t)pair * X::STEP + in16;
-#pragma unroll
-                        for (int pl = 0; pl < 3; pl++) *(uint32_t*)(o + 64 * pl) = d.d[h][pl];
-                    }
-                    xs = d.xs;
-                    ssq = d.ssq;
-                    const int from = (lane & 3) * 8, sl = __shfl_sync(0xffffffffu, d.s[0], from), sh = __shfl_sync(0xffffffffu, d.s[1], from);
-                    s = (lane & 4) ? sh : sl;
-                }
-            }
-            if (lane == 0) {
-                xs_s[b * TP + tk] = xs;
-                ssq_s[blk * TP + tk] = ssq;
-            }
-            F::put_sums(smem + a.sums_off + (size_t)(b * TP + tk) * X::SUMS, xs, s, lane);
-        }
-        __syncthreads();
-        int in_batch = 0, buf = 0, batch0 = 0;
-        for (int i = 0; i < my_tiles; i++) {
-            float* cb = comb + (size_t)(buf * a.batch + in_batch) * slices * RES;
-            const uint32_t tag = F::tag(a.w, a.w2, row_of(i, 0), row_of(i, 1), g);
-            for (int sl = q; sl < slices; sl += ks) {
-                float acc[NT][2];
-                float2* h = PARTS ? hold + ((size_t)((wq * a.hold_tiles + i) * (slices / ks) + sl / ks) * NT) * 32 + lane : nullptr;
-#pragma unroll
-                for (int n = 0; n < NT; n++) {
-                    float2 v = make_float2(0.0f, 0.0f);
-                    if (PARTS && p > 0) v = h[n * 32];
-                    acc[n][0] = v.x;
-                    acc[n][1] = v.y;
-                }
-                const int b_part = PARTS ? p * a.part_units * bpu : 0, j1 = j_end(sl, p);
-                for (int j = j_beg(sl, p); j < j1; j++) {
-                    cp_wait<S - 1>();
-                    __syncwarp();
-                    const int b = (sl + (j << sl_log)) * bpu;
-                    const int bn = min(bpu, a.blocks - b);
-                    for (int k = 0; k < bn; k++) F::template block<TP>(slot + k * F::BLOCK_BYTES, b + k - b_part, ((b + k) & 1) ? ~tag : tag, a.w, xv, g, t, acc);
-                    __syncwarp();
-                    issue();  // into the slot just used
-                    slot = slot + F::UNIT_BYTES == ring_end ? ring : slot + F::UNIT_BYTES;
-                }
-                if (PARTS && p + 1 < parts) {
-#pragma unroll
-                    for (int n = 0; n < NT; n++) h[n * 32] = make_float2(acc[n][0], acc[n][1]);
-                } else {
-#pragma unroll
-                    for (int n = 0; n < NT; n++) {
-                        float* cr = cb + sl * RES + n * 16 * X::PER;
-                        if constexpr (F::HALVES) {
-                            if (TP > 1) cr[g * 4 + t] = acc[n][0], cr[(g + 8) * 4 + t] = acc[n][1];
-                            else if (t == 0) cr[g] = acc[n][0], cr[g + 8] = acc[n][1];
-                        } else {  // a token's two lanes together; one keeps row g, the other row g + 8
-                            const float v0 = acc[n][0] + __shfl_xor_sync(0xffffffffu, acc[n][0], 1), v1 = acc[n][1] + __shfl_xor_sync(0xffffffffu, acc[n][1], 1);
-                            const float v = (t & 1) ? v1 : v0;
-                            const int row = g + 8 * (t & 1);
-                            if (TP > 1) cr[row * 2 + (t >> 1)] = v;
-                            else if (t < 2) cr[row] = v;
-                        }
-                    }
-                }
-            }
-            if (PARTS && p + 1 < parts) continue;
-            if (++in_batch < a.batch && i + 1 < my_tiles) continue;
-            if (ks == 1) __syncwarp();
-            else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(ks * 32) : "memory");
-            // one thread per result (per pair of results in the pair form): the sums in the order of the slices
-            constexpr int PER = PAIR ? 8 : 16;
-            const float* c0 = comb + (size_t)buf * a.batch * slices * RES;
-            for (int e = q * 32 + lane; e < in_batch * PER * T; e += ks * 32) {
-                const int r = e % PER, et = e / PER, token = et % T, tl = et / T;
-                const size_t first = (size_t)(tile0 + (batch0 + tl) * tile_step) * ROWS + (r & 8), row = row_of(batch0 + tl, r >> 3) + (r & 7);
-                if (row < first || row >= n_out) continue;  // (the last tile's halves overlap the rows before them)
-                const float* pv = c0 + (size_t)tl * slices * RES + (TP == 1 ? r : token / X::PER * 16 * X::PER + r * X::PER + token % X::PER);
-                float v = 0.0f, v2 = 0.0f;
-                for (int s = 0; s < slices; s++) {
-                    v += pv[s * RES];
-                    if (PAIR) v2 += pv[s * RES + 8 * (TP == 1 ? 1 : X::PER)];
-                }
-                if (a.norm) {
-                    float sq = 0.0f;
-                    for (int b = 0; b < xblocks; b++) sq += ssq_s[b * TP + token];
-                    const float k = 1.0f / sqrtf(sq / (float)a.w.n_in + a.eps);
-                    v *= k;
-                    v2 *= k;
-                }
-                float* o = a.y + (size_t)token * a.y_stride + row;
-                if (PAIR) *o = (a.mode == B2_MODE_SILU_PAIR ? silu(v) : gelu_tanh(v)) * v2;
-                else if (a.mode == B2_MODE_STORE) *o = v;
-                else if (a.mode == B2_MODE_ADD) *o += v;
-                else *o += v * (1.0f / (1.0f + __expf(-a.gate[(size_t)token * a.gate_stride])));
-            }
-            batch0 = i + 1;
-            in_batch = 0;
-            if (a.bufs == 2) buf ^= 1;
-            else if (ks == 1) __syncwarp();
-            else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(ks * 32) : "memory");
-        }
-    }
-    cp_wait<0>();
-}
 
 __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x, size_t x_stride, const float* __restrict__ w, float pre, int K, uint8_t* out,
                                                     size_t out_stride, int fast, int halves) {
@@ -320,74 +41,12 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
     }
 }
 
-template <class F, bool PAIR, int TP>
-cudaError_t launch_t(Args& a, int sm_count, cudaStream_t st, bool pdl) {
-    using X = typename F::template X<TP>;
-    constexpr int ROWS = PAIR ? 8 : 16, BPX = 256 / F::BLOCK_K, NT = X::NT, RES = X::RES;
-    a.blocks = (int)((a.w.n_in + F::BLOCK_K - 1) / F::BLOCK_K);
-    // The order of a row's sum depends on K alone (a row shard has other tiles): eight slices, or as many as there are units, of units
-    // of two blocks where that leaves a unit per slice. How many warps share a tile does not change it.
-    a.bpu = a.blocks >= 8 * F::MAX_BLOCKS ? F::MAX_BLOCKS : 1;
-    a.units = (a.blocks + a.bpu - 1) / a.bpu;
-    a.slice_log = 3;
-    while ((1 << a.slice_log) > a.units) a.slice_log--;
-    const int slices = 1 << a.slice_log;
-    const size_t tiles = (a.w.n_out + ROWS - 1) / ROWS;
-    a.ks = slices;
-    const int groups = WARPS / a.ks;
-    const int span = std::max(slices, BPX), xblocks = (a.blocks + BPX - 1) / BPX;
-    // the sums of a few tiles wait for one barrier: 8 KB of them, twice, over all groups
-    a.batch = std::max(1, std::min(8, 8192 / (groups * slices * RES * 4)));
-    a.bufs = 2;
-    const size_t ring = (size_t)WARPS * F::SLOTS * F::UNIT_BYTES;
-    size_t comb = (size_t)groups * a.bufs * a.batch * slices * RES * 4;
-    size_t grid = std::min(tiles, (size_t)sm_count);
-    const size_t ssq = xblocks * TP * 4, per_block = TP * (X::BLOCK + 4 + X::SUMS), slack = 512;
-    size_t fixed = ring + comb + ssq + slack, hold = 0, part = xblocks;
-    if (fixed + xblocks * per_block > SMEM_MAX) {
-        a.batch = a.bufs = 1;  // (a tile's arithmetic is long here: the second barrier costs little and the room holds activations)
-        fixed -= comb;
-        comb = (size_t)groups * slices * RES * 4;
-        fixed += comb;
-        // parts of whole rounds of the slices where one fits, else of as many units as fit
-        size_t step = (size_t)std::max(1, span * a.bpu / BPX);  // in blocks of the split
-        const size_t least = (size_t)std::max(1, a.bpu / BPX), per_tile = (size_t)WARPS * (slices / a.ks) * NT * 256;
-        if (fixed + per_tile + least * per_block > SMEM_MAX) return cudaErrorInvalidValue;
-        // The waiting sums may take the room that a round leaves; a group that has more tiles than that goes in several waves of CTAs.
-        const size_t room = SMEM_MAX - fixed - (fixed + per_tile + step * per_block <= SMEM_MAX ? step : least) * per_block;
-        const size_t most = std::min<size_t>(MAX_TILES, room / per_tile), wave = (size_t)sm_count * groups;
-        const size_t waves = (tiles + wave * most - 1) / (wave * most);
-        if (waves > 1) grid = waves * sm_count;
-        a.hold_tiles = (int)((tiles + grid * groups - 1) / (grid * groups));
-        hold = a.hold_tiles * per_tile;
-        part = (SMEM_MAX - fixed - hold) / per_block;
-        if (part < step) step = least;
-        part = part / step * step;
-    }
-    const bool parts = part < (size_t)xblocks;
-    a.part_units = parts ? (int)part * BPX / a.bpu : a.units;
-    size_t at = ring;
-    auto take = [&](size_t n) {
-        const size_t r = at;
-        at += (n + 15) / 16 * 16;
-        return (uint32_t)r;
-    };
-    a.frag_off = take(part * TP * X::BLOCK);
-    a.comb_off = take(comb);
-    a.hold_off = take(hold);
-    a.sums_off = take(part * TP * X::SUMS + 64);
-    a.ssq_off = take(ssq);
-    a.xs_off = take(part * TP * 4 + 64);
-    auto kern = parts ? gemv_mma_kernel<F, PAIR, TP, true> : gemv_mma_kernel<F, PAIR, TP, false>;
-    if (cudaError_t e = ensure_dynamic_smem((const void*)kern, at); e != cudaSuccess) return e;
-    return launch_k(kern, dim3((unsigned)grid), dim3(THREADS), at, st, pdl, a);
-}
-
 template <class F>
-cudaError_t launch_f(Args& a, bool pair, int sm_count, cudaStream_t st, bool pdl) {
-    if (a.T == 1) return pair ? launch_t<F, true, 1>(a, sm_count, st, pdl) : launch_t<F, false, 1>(a, sm_count, st, pdl);
-    if (a.T <= 4) return pair ? launch_t<F, true, 4>(a, sm_count, st, pdl) : launch_t<F, false, 4>(a, sm_count, st, pdl);
-    return pair ? launch_t<F, true, 8>(a, sm_count, st, pdl) : launch_t<F, false, 8>(a, sm_count, st, pdl);
+cudaError_t launch_f(Args& a, bool pair, int sm_count, cudaStream_t st, bool pdl, const GemvGroups* gt = nullptr) {
+    if (a.T == 1) return pair ? launch_t<F, true, 1>(a, sm_count, st, pdl, gt) : launch_t<F, false, 1>(a, sm_count, st, pdl, gt);
+    if (a.T <= 4) return pair ? launch_t<F, true, 4>(a, sm_count, st, pdl, gt) : launch_t<F, false, 4>(a, sm_count, st, pdl, gt);
+    if (a.T <= 6) return pair ? launch_t<F, true, 6>(a, sm_count, st, pdl, gt) : launch_t<F, false, 6>(a, sm_count, st, pdl, gt);
+    return pair ? launch_t<F, true, 8>(a, sm_count, st, pdl, gt) : launch_t<F, false, 8>(a, sm_count, st, pdl, gt);
 }
 
 }  // namespace
@@ -439,6 +98,33 @@ cudaError_t launch_gemv_mma(const WeightDev& w, const WeightDev* up, const GemvI
         case B2_FMT_F8E4M3: return launch_f<F8B<true>>(a, pair, sm_count, st, pdl);
         default: return cudaErrorInvalidValue;
     }
+}
+
+// The most rows of K values that a group's activations fit for beside the rings (launch_t: two warp groups' sums are 16 KB).
+int gemv_groups_most(size_t K) {
+    const size_t nb = split_blocks(K), fixed = (size_t)WARPS * F4<false>::SLOTS * F4<false>::UNIT_BYTES + 16384 + 512;
+    for (size_t tp : {8, 4, 1})
+        if (fixed + nb * tp * (SPLIT_DIGITS + 4 + 4 + 32) <= SMEM_MAX) return (int)tp;
+    return 0;
+}
+cudaError_t launch_gemv_groups(const WeightDev& w, const WeightDev* up, const float* x, size_t x_stride, const GemvGroups& groups, int most, float* y,
+                               size_t y_stride, int mode, bool fast, int sm_count, cudaStream_t st) {
+    if (!gemv_mma_supports(w) || groups.n < 1 || most < 1 || most > 8) return cudaErrorInvalidValue;
+    const bool pair = mode == B2_MODE_SILU_PAIR || mode == B2_MODE_GELU_PAIR;
+    Args a{};
+    a.w = w;
+    a.w2 = pair ? *up : w;
+    a.x = x;
+    a.x_stride = x_stride;
+    a.pre = 1.0f;
+    a.fast = fast;
+    a.y = y;
+    a.y_stride = y_stride;
+    a.mode = mode;
+    a.T = most;
+    if (w.fmt == B2_FMT_MLX4) return launch_f<F4<true>>(a, pair, sm_count, st, true, &groups);
+    if (w.fmt == B2_FMT_Q4_K) return launch_f<F4<false>>(a, pair, sm_count, st, true, &groups);
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_split(const float* x, size_t x_stride, const float* norm_w, float pre, size_t K, int tokens, uint8_t* rec, size_t rec_stride, bool halves,

@@ -107,7 +107,7 @@ template <bool MLX>
 struct F4 {
     template <int TP>
     using X = XView<TP, false>;
-    static constexpr bool HALVES = false, SUMS = true;
+    static constexpr bool HALVES = false, SUMS = true, PARTS = true;
     static constexpr int BLOCK_K = 256, SLOTS = 2, MAX_BLOCKS = 2;  // a unit is one or two blocks
     static constexpr int BLOCK_BYTES = 16 * 144, UNIT_BYTES = MAX_BLOCKS * BLOCK_BYTES;
     static constexpr bool SUMS_BY_COLUMN = !MLX;
@@ -159,7 +159,7 @@ struct F4 {
     };
     // acc[n][row g | g + 8]: this lane's share (its two columns) of the results
     template <int TP>
-    __device__ static __forceinline__ void block(uint32_t slot, int u, uint32_t, const WeightDev&, const X<TP>& x, int g, int t, float (&acc)[X<TP>::NT][2]) {
+    __device__ static __forceinline__ void block(uint32_t slot, int u, uint32_t, const WeightDev&, const WeightDev&, const X<TP>& x, int g, int t, float (&acc)[X<TP>::NT][2]) {
         constexpr int NT = X<TP>::NT;
         const uint32_t ra = slot + g * 144, rb = ra + 8 * 144;
         const uint4 ha = lds128(ra), hb = lds128(rb);
@@ -255,7 +255,7 @@ template <bool FP8>
 struct F8B {
     template <int TP>
     using X = XView<TP, FP8>;
-    static constexpr bool HALVES = FP8, SUMS = false, SUMS_BY_COLUMN = false;
+    static constexpr bool HALVES = FP8, SUMS = false, SUMS_BY_COLUMN = false, PARTS = true;
     static constexpr int BLOCK_K = 128, SLOTS = 2, MAX_BLOCKS = 2;
     static constexpr int BLOCK_BYTES = 16 * 144, UNIT_BYTES = MAX_BLOCKS * BLOCK_BYTES;
     __device__ static __forceinline__ void put_sums(uint8_t*, float, int, int) {}
@@ -319,7 +319,7 @@ struct F8B {
         }
     };
     template <int TP>
-    __device__ static __forceinline__ void block(uint32_t slot, int u, uint32_t, const WeightDev& w, const X<TP>& x, int g, int t, float (&acc)[X<TP>::NT][2]) {
+    __device__ static __forceinline__ void block(uint32_t slot, int u, uint32_t, const WeightDev& w, const WeightDev&, const X<TP>& x, int g, int t, float (&acc)[X<TP>::NT][2]) {
         constexpr int NT = X<TP>::NT;
         const uint32_t ra = slot + g * 144, rb = ra + 8 * 144;
         if constexpr (FP8) {
@@ -402,7 +402,7 @@ struct F8B {
 struct F6 {
     template <int TP>
     using X = XView<TP, false>;
-    static constexpr bool HALVES = false, SUMS = false, SUMS_BY_COLUMN = false;
+    static constexpr bool HALVES = false, SUMS = false, SUMS_BY_COLUMN = false, PARTS = true;
     static constexpr int BLOCK_K = 256, SLOTS = 3, MAX_BLOCKS = 1;
     static constexpr int BLOCK_BYTES = 16 * 208 + 64, UNIT_BYTES = BLOCK_BYTES;
     __device__ static __forceinline__ void put_sums(uint8_t*, float, int, int) {}
@@ -457,7 +457,7 @@ struct F6 {
     // Element 128 n + 32 k4 + e of a block: nibble k4 / 2 of ql[64 n + 32 (k4 & 1) + e] under bit pair k4 of qh[32 n + e], minus 32 (src/ggml.rs
     // Q6_K decode). As signed bytes of four times the value: the pair and the nibble shifted up by two, the sign bit turned.
     template <int TP>
-    __device__ static __forceinline__ void block(uint32_t slot, int u, uint32_t tag, const WeightDev&, const X<TP>& x, int g, int t, float (&acc)[X<TP>::NT][2]) {
+    __device__ static __forceinline__ void block(uint32_t slot, int u, uint32_t tag, const WeightDev&, const WeightDev&, const X<TP>& x, int g, int t, float (&acc)[X<TP>::NT][2]) {
         constexpr int NT = X<TP>::NT;
         constexpr uint32_t N = 0x3C3C3C3Cu, P = 0xC0C0C0C0u, S = 0x80808080u;
         const uint32_t ra = slot + g * 208, rb = ra + 8 * 208;

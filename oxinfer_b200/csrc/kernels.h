@@ -61,92 +61,7 @@ cudaError_t launch_repack_q4a(const uint8_t* q, const uint16_t* scales, const ui
                               uint8_t* out, int* mismatch, cudaStream_t st);
 cudaError_t launch_repack_q8_0(const uint8_t* raw, size_t n_out, size_t n_in, int8_t* qs, uint16_t* d, cudaStream_t st);
 
-// ---- gemv.cu: one-token dequant matrix-vector products ---------------------------------------
-// Activation vector split into three int8 planes per block of 32 (x ~= xs * (q0 + 32 q1 + 8192 q2),
-// 21 significant bits per block; q1 and q2 alone carry 16), plus block scales and sums. The record in global memory is the image the product
-// kernels keep in shared memory, so staging it is a plain copy (bulk copies in the ring form). For n_in = K, in bytes:
-//   planes 3K | sx 8K/32 | v16 4K/16
-// Element k of plane p sits at p * K + 16 * xplanes_slot(k / 16) + k % 16: the 16-byte slots of each 64 bytes are
-// permuted so that the product kernels' shared-memory reads spread over the banks.
-struct XPlanes {
-    int8_t* planes;   // [3][K], slots permuted
-    float2* sx;       // [K/32]  (block scale, scale * sum of the block's integers = the quantized block sum)
-    int32_t* v16;     // [K/16]  integer sums of each 16 elements
-    int np;           // planes a product reads: 2 = the upper two (16 bits), anything else = all three (21 bits, the default)
-};
-// Slot g -> g with its low two bits xor-ed by bits 3 and 4: lanes L = 0..7 of a phase that read slots 4 L + i (a 64-byte
-// stride) then cover all eight 16-byte bank groups for every i.
-__host__ __device__ inline int xplanes_slot(int g) { return g ^ ((((g >> 3) & 1) << 1) | ((g >> 4) & 1)); }
-__host__ __device__ inline size_t xplanes_bytes(size_t K) { return 3 * K + 4 * (K / 32) * 2 + 4 * (K / 16); }
-__host__ __device__ inline XPlanes xplanes_at(void* base, size_t K) {
-    XPlanes p;
-    uint8_t* b = (uint8_t*)base;
-    p.planes = (int8_t*)b;
-    p.sx = (float2*)(b + 3 * K);
-    p.v16 = (int32_t*)(b + 3 * K + 8 * (K / 32));
-    p.np = 0;
-    return p;
-}
-// tokens > 1: token i's vector x_stride floats and its planes planes_stride bytes behind token 0's, one launch for all.
-cudaError_t launch_xplanes(const float* x, size_t K, XPlanes out, cudaStream_t st, bool pdl = false, int tokens = 1, size_t x_stride = 0,
-                           size_t planes_stride = 0);
-// A vector whose RMS-norm factor is applied after the product instead of before the split: the planes hold the split of
-// x * w (no factor), `partial` holds the sum of squares of every block of 32 of x, and the product kernel multiplies its
-// sums by k = 1 / sqrt(sum(partial) * inv_n + eps). The split of a block does not depend on a common factor, so this
-// equals the product over the normalized vector up to rounding; it lets the norm run as independent warps on many SMs
-// instead of one CTA that must first reduce the whole row. partial == nullptr: no factor.
-struct NormScale {
-    const float* partial;
-    uint32_t count;
-    float inv_n, eps;
-};
-// planes(x * pre * w) and the blocks' sums of squares of x * pre; K a multiple of 32, w may be null.
-// tokens > 1 as for launch_xplanes; token i's sums partial_stride floats behind token 0's.
-cudaError_t launch_norm_planes(const float* x, const float* w, float pre, size_t K, XPlanes out, float* partial, cudaStream_t st, bool pdl = false,
-                               int tokens = 1, size_t x_stride = 0, size_t planes_stride = 0, size_t partial_stride = 0);
-// What a product may do with its finished output, so that the kernel which would split it for the next product is not
-// launched: the CTAs then own whole blocks of 32 consecutive rows (four per warp), the warps leave their results in
-// shared memory, and after a CTA barrier one warp writes the planes of y * pre * w (w may be null) and, with `partial`,
-// the block's sum of squares of y * pre: what launch_xplanes / launch_norm_planes would have written, bit for bit.
-// n_out must be a multiple of 32. out.planes == nullptr: nothing.
-struct EpiPlanes {
-    XPlanes out;
-    const float* w;
-    float* partial;
-    float pre;
-};
-// Whether launch_gemv takes an EpiPlanes for this matrix (the 4-bit formats whose planes and rings fit in shared memory).
-bool gemv_takes_epilogue(const WeightDev& w);
-// y[n_out] = mode(W x [, U x]). `xp` holds the planes of x (launch_xplanes); the
-// FP8 kernel reads `x` (f32) directly and ignores `xp`. plain_form: never the ring form (a lone product behind its own plane
-// kernel: launched as that kernel's dependent, the register-load form fetches its first weights while the planes are made).
-cudaError_t launch_gemv(const WeightDev& w, const WeightDev* up, const float* x, XPlanes xp, float* y, int mode, const float* gate,
-                        int sm_count, cudaStream_t st, bool pdl = false, NormScale ns = NormScale{nullptr, 0, 0.0f, 0.0f},
-                        EpiPlanes epi = EpiPlanes{XPlanes{nullptr, nullptr, nullptr}, nullptr, nullptr, 1.0f},
-                        bool plain_form = false);
-// A batch of products in one launch (the routed experts of a few tokens): entry b multiplies matrix expert[b] of a stack
-// of equally shaped 4-bit matrices (w describes matrix 0; w_stride bytes apart) by the planes block xrow[b] (x_stride
-// bytes apart, laid out as xplanes_at) into y + b * y_stride. The tables travel as kernel arguments (up to 64 entries),
-// so a call needs no copy of its own and no synchronization.
-constexpr int GEMV_BATCH_MAX = 64;
-struct GemvBatch {
-    int n;  // 0: not a batch
-    int expert[GEMV_BATCH_MAX];
-    int xrow[GEMV_BATCH_MAX];
-    size_t w_stride, x_stride, y_stride;
-    uint8_t* planes;
-};
-cudaError_t launch_gemv_batched(const WeightDev& w, const WeightDev* up, const GemvBatch& b, size_t batch, float* y, int mode, int np, int sm_count,
-                                cudaStream_t st, bool pdl = false);
-// Planes of `rows` vectors of K values (row r at x + r * K) into blocks `stride` bytes apart.
-cudaError_t launch_xplanes_rows(const float* x, size_t rows, size_t K, uint8_t* planes, size_t stride, cudaStream_t st, bool pdl = false);
-// nt (1..4) tokens in one launch, the weights read once: token i's f32 vector at x + i * x_stride (FP8 weights) or planes
-// at xp + i * xp_stride bytes (the other formats), outputs at y + i * y_stride. Each token's result equals its
-// single-token result bit for bit. cudaErrorInvalidValue if the tokens' vectors do not fit in shared memory together, or for
-// the gated mode. `ns`: token 0's deferred norm factor (see NormScale), token i's partial sums ns_stride floats further.
-cudaError_t launch_gemv_multi(const WeightDev& w, const WeightDev* up, const float* x, size_t x_stride, XPlanes xp, size_t xp_stride, float* y,
-                              size_t y_stride, int nt, int mode, int sm_count, cudaStream_t st, bool pdl = false,
-                              NormScale ns = NormScale{nullptr, 0, 0.0f, 0.0f}, size_t ns_stride = 0);
+// ---- gemv.cu: one-token products of FP8 matrices with other scale blocks ---------------------
 // Whether a one-token product of this format and shape has a kernel: launch_gemv_mma, or for FP8 matrices with other scale blocks
 // launch_gemv_f8_float.
 bool gemv_supports(const WeightDev& w);
@@ -165,9 +80,10 @@ struct GemvIn {
     float eps = 0.0f;
     const uint8_t* rec = nullptr;  // token i at rec + i * rec_stride
     size_t rec_stride = 0;
-    int fast = 0;  // 16 bits of every value
+    int fast = 0;  // 18 bits of every value (split.cuh)
 };
 bool gemv_mma_supports(const WeightDev& w);
+constexpr size_t GEMV_WHOLE_8 = 2048;  // rows of up to this many values are held whole by a launch of eight tokens, whatever the format
 size_t split_blocks_of(size_t K);
 size_t split_bytes_of(size_t K, bool halves);  // bytes of a vector's record
 bool gemv_mma_halves(const WeightDev& w);  // the form of split this format's products read
@@ -175,6 +91,19 @@ bool gemv_mma_halves(const WeightDev& w);  // the form of split this format's pr
 // for bit, from records or not.
 cudaError_t launch_gemv_mma(const WeightDev& w, const WeightDev* up, const GemvIn& in, int T, float* y, size_t y_stride, int mode, const float* gate,
                             size_t gate_stride, int sm_count, cudaStream_t st, bool pdl);
+// Products over a stack of equally shaped 4-bit matrices (the routed experts of a batch; w describes matrix 0, the others w_stride bytes
+// apart): group g multiplies matrix expert[g] by rows row0[g] .. + count[g] - 1 (at most `most`, 1 .. 8) of the pairs' list. Row i reads the
+// vector of x's row src[i] (gather) or i and writes row i of y. The table travels as a kernel argument: no copy, no synchronization.
+constexpr int GEMV_GROUP_ROWS = 512;
+struct GemvGroups {
+    int n, gather;
+    size_t w_stride;
+    uint16_t expert[GEMV_GROUP_ROWS], row0[GEMV_GROUP_ROWS], src[GEMV_GROUP_ROWS];
+    uint8_t count[GEMV_GROUP_ROWS];
+};
+int gemv_groups_most(size_t K);  // 8, 4, 1, or 0: not even one row of K values fits
+cudaError_t launch_gemv_groups(const WeightDev& w, const WeightDev* up, const float* x, size_t x_stride, const GemvGroups& groups, int most, float* y,
+                               size_t y_stride, int mode, bool fast, int sm_count, cudaStream_t st);
 // Records (split.cuh, split_bytes each) of `tokens` vectors of x * pre * norm_w.
 cudaError_t launch_split(const float* x, size_t x_stride, const float* norm_w, float pre, size_t K, int tokens, uint8_t* rec, size_t rec_stride, bool halves,
                          bool fast, cudaStream_t st, bool pdl);
@@ -229,13 +158,6 @@ cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, i
 // x_ld: elements between the rows of x (0: K, the rows are contiguous).
 cudaError_t launch_to_f16(const void* x, int x_dtype, size_t t, size_t K, void* x16, float* unscale, cudaStream_t st, size_t lo_row0 = 0,
                           size_t x_ld = 0);
-// Whether nt (1..4) token rows' vectors fit in shared memory together for launch_gemv_multi.
-bool gemv_multi_fits(const WeightDev& w, int nt);
-// Whether one launch for nt tokens beats nt one-token launches inside a chain of dependent launches: from two tokens on
-// for the 4-bit formats (integer dots on the tensor cores), from three for the others (their several-token kernel does a
-// token's arithmetic per token and is not the bulk-copy form).
-bool gemv_multi_pays(const WeightDev& w, int nt);
-
 // ---- gemm_f8.cu: FP8 weights x FP8 activations (tcgen05 kind::f8f6f4), 128 x 128 weight scale blocks, activations quantized
 // per token and per 128 k -----------------------------------------------------------------------------------------------
 bool gemm_f8_supports(const WeightDev& w, size_t t);
@@ -257,9 +179,10 @@ cudaError_t launch_moe_gather(const float* x, const int* src, size_t rows, size_
 // kind: B2_ACT_* (0 SiLU, 1 tanh GELU, 2 SiLU with clamp `limit`).
 cudaError_t launch_moe_act(const float* g, const int* src, size_t rows, size_t inter, void* a_f16, float* unscale, size_t lo_row0, cudaStream_t st,
                            int kind = 0, float limit = 0.0f);
-// The same with the routes as kernel arguments (at most GEMV_BATCH_MAX pairs): slot of pair (i, j) = i k + j, no row scale.
+// The same with the routes as kernel arguments (at most GEMV_GROUP_ROWS pairs).
 struct SmallRoutes {
-    float w[GEMV_BATCH_MAX];
+    float w[GEMV_GROUP_ROWS];
+    uint16_t slot[GEMV_GROUP_ROWS];
 };
 cudaError_t launch_moe_combine_small(const float* o, const SmallRoutes& r, size_t t, size_t k, size_t h, float* y, cudaStream_t st, bool pdl = false);
 cudaError_t launch_moe_combine(const float* o, const int* slots, const float* w, size_t t, size_t k, size_t h, float* y, cudaStream_t st);

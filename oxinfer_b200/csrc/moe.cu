@@ -10,7 +10,7 @@
 #include <algorithm>
 
 #include "kernels.h"
-#include "xplanes.cuh"
+#include "pdl.cuh"
 
 namespace b2 {
 
@@ -321,19 +321,23 @@ __global__ void moe_combine_kernel(const float* __restrict__ o, const int* __res
     *(float4*)(y + (size_t)tok * h + c) = acc;
 }
 
-// y[tok][c] += sum over the token's k routes, in order, of w * o[tok k + j][c]; the weights are kernel arguments.
-__global__ void moe_combine_small_kernel(const float* __restrict__ o, SmallRoutes r, int k, int h, float* __restrict__ y) {
+// The same with the routes as kernel arguments.
+__global__ void __launch_bounds__(256) moe_combine_small_kernel(const float* __restrict__ o, const __grid_constant__ SmallRoutes r, int k, int h, float* __restrict__ y) {
     pdl_launch_dependents();
     pdl_wait();
     const int tok = blockIdx.y;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (c >= h) return;
-    float acc = y[(size_t)tok * h + c];
+    float4 acc = *(const float4*)(y + (size_t)tok * h + c);
     for (int j = 0; j < k; j++) {
-        const int slot = tok * k + j;
-        acc = __fadd_rn(acc, __fmul_rn(r.w[slot], o[(size_t)slot * h + c]));
+        const float wj = r.w[tok * k + j];
+        const float4 v = *(const float4*)(o + (size_t)r.slot[tok * k + j] * h + c);
+        acc.x = __fadd_rn(acc.x, __fmul_rn(wj, v.x));
+        acc.y = __fadd_rn(acc.y, __fmul_rn(wj, v.y));
+        acc.z = __fadd_rn(acc.z, __fmul_rn(wj, v.z));
+        acc.w = __fadd_rn(acc.w, __fmul_rn(wj, v.w));
     }
-    y[(size_t)tok * h + c] = acc;
+    *(float4*)(y + (size_t)tok * h + c) = acc;
 }
 
 // out[r][h] = x[idx[r]][h] (f32 rows gathered by index), and the all-gather's rank-major blocks into column blocks.
@@ -370,8 +374,8 @@ cudaError_t launch_scatter_blocks(const float* gathered, size_t world, size_t t,
 }
 
 cudaError_t launch_moe_combine_small(const float* o, const SmallRoutes& r, size_t t, size_t k, size_t h, float* y, cudaStream_t st, bool pdl) {
-    if (t * k > GEMV_BATCH_MAX) return cudaErrorInvalidValue;
-    dim3 grid((unsigned)((h + 255) / 256), (unsigned)t);
+    if (t * k > GEMV_GROUP_ROWS) return cudaErrorInvalidValue;
+    dim3 grid((unsigned)((h / 4 + 255) / 256), (unsigned)t);
     return launch_k(moe_combine_small_kernel, grid, dim3(256), 0, st, pdl, o, r, (int)k, (int)h, y);
 }
 

@@ -15,7 +15,7 @@ class DecodePlanImpl {
   public:
     // `resolve` maps a weight handle to its device description (nullptr: unknown handle).
     // Returns B2_OK, B2_DECLINED or an error code; `err` gets the reason.
-    // `fast`: the plan's products read 16 bits of every activation (b2_set_fast_planes).
+    // `fast`: the plan's products read 18 bits of every activation (b2_set_fast_planes).
     // `tokens` (1..4): the most tokens of a step (Backend::decode_plan_multi, src/gpu.rs:273-276). A plan of several tokens keeps
     // one activation block and block of records per token.
     // `prefill`: a prefill plan (Backend::decode_plan_prefill, src/gpu.rs:283-289): steps of up to `tokens` (1..8192) tokens on

@@ -11,7 +11,7 @@
 //   Record of a block: [chunk of 32 k: 8][hi | lo][t][16 bytes] (two mma.m16n8k16: values 4 t .. 4 t + 3 of either half of the chunk), then SPLIT_AUX bytes as above without the sums.
 #pragma once
 #include "kernels.h"
-#include "xplanes.cuh"
+#include "pdl.cuh"
 
 namespace b2 {
 
@@ -67,7 +67,7 @@ struct SplitDigits {
     int s[2];          // sums of q over chunks lane / 8 and 4 + lane / 8
     float xs, ssq;
 };
-// fast: 16 bits of every value (the two upper digits)
+// fast: the upper 18 of the 24 bits of every value
 __device__ __forceinline__ SplitDigits split_digits(const SplitIn& in, float pre, bool fast) {
     SplitDigits r;
     float v[8];
@@ -84,7 +84,7 @@ __device__ __forceinline__ SplitDigits split_digits(const SplitIn& in, float pre
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             int q = __float2int_rn(v[4 * h + i] * k);
-            if (fast) q = (q + 128) & ~255;
+            if (fast) q = (q + 32) & ~63;
             s += q;
             u[i] = (uint32_t)(q + 0x808080);  // q + 128 (1 + 256 + 65536): its bytes are the digits plus 128
         }
