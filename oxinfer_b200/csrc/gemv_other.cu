@@ -210,6 +210,8 @@ cudaError_t launch_dequantize_other(const WeightDev& w, size_t r0, size_t nrows,
 cudaError_t launch_gemv_other(const WeightDev& w, const WeightDev* up, const float* x, size_t x_stride, float* y, size_t y_stride, int nt, int mode,
                               const float* gate, int sm_count, cudaStream_t st, bool pdl) {
     if (!gemv_other_supports(w) || nt < 1 || nt > 4) return cudaErrorInvalidValue;
+    // Rows of whole 256-value runs go to the integer tensor cores: Q5_K 14336 x 4096 11.7 us there, 39 here.
+    if (gemv_mma_other_tokens(w)) return launch_gemv_mma_other(w, up, x, x_stride, y, y_stride, nt, mode, gate, sm_count, st);
     if (nt > 1 && w.n_in * 4 * (size_t)nt > 160 * 1024) {  // the vectors of nt tokens do not fit together: fewer per launch
         const int half = nt / 2;
         if (cudaError_t e = launch_gemv_other(w, up, x, x_stride, y, y_stride, half, mode, gate, sm_count, st, pdl); e != cudaSuccess) return e;

@@ -108,6 +108,11 @@ cudaError_t launch_gemv_groups(const WeightDev& w, const WeightDev* up, const fl
 cudaError_t launch_split(const float* x, size_t x_stride, const float* norm_w, float pre, size_t K, int tokens, uint8_t* rec, size_t rec_stride, bool halves,
                          bool fast, cudaStream_t st, bool pdl);
 
+// ---- gemv_mma_other.cu: the other GGUF block formats on the same kernel, for rows of whole runs of 256 values ------------
+int gemv_mma_other_tokens(const WeightDev& w);  // 4, 1, or 0 where the generic kernel of gemv_other.cu is the only one
+cudaError_t launch_gemv_mma_other(const WeightDev& w, const WeightDev* up, const float* x, size_t x_stride, float* y, size_t y_stride, int nt, int mode,
+                                  const float* gate, int sm_count, cudaStream_t st);
+
 // ---- gemv_other.cu: the other GGUF block formats (dq_other.cuh), raw rows, one generic kernel ---------------------------
 bool gemv_other_supports(const WeightDev& w);
 cudaError_t launch_dequantize_other(const WeightDev& w, size_t r0, size_t nrows, float* out, cudaStream_t st, const int* row_dev = nullptr,

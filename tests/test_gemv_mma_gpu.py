@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import oxinfer_b200 as ob
+from oracle import oracle as O
 from oxinfer_b200 import synth
 
 from util import FORMATS, make_pair, row_err
@@ -79,3 +80,45 @@ def test_values_that_are_not_finite_and_vectors_off_16_bytes(backend, fmt):
         y = products(backend, dev, x)
         assert not np.isfinite(y[1]).any()
         assert np.array_equal(y[0], want[0])
+
+
+OTHERS = list(O.OTHER_KINDS) + [O.NVFP4]
+
+
+def other(kind, n_out, n_in, seed):
+    data, _ = O.random_blocks(kind, n_out * n_in // O.block_size(kind), seed)
+    scale = np.array([[0.03 + 0.001 * (seed % 7)]], np.float32) if kind == O.NVFP4 else None
+    dims = (n_out, n_in) if kind == O.NVFP4 else (0, 0)
+    return ob.Gguf(kind, data, scale, *dims), O.Matrix.gguf(kind, data, n_out, n_in, scale, *dims)
+
+
+@pytest.mark.parametrize("kind", OTHERS, ids=lambda k: O.KIND_NAMES[k])
+# as above; 20,480 values do not fit beside the rings in every format, whose generic kernel takes them then
+@pytest.mark.parametrize("shape", [(5, 256), (20, 768), (1201, 1280), (37, 14336), (19, 20480)])
+def test_other_formats_of_one_to_four_tokens(backend, kind, shape):
+    n_out, n_in = shape
+    ref, m = other(kind, n_out, n_in, 940 + kind)
+    dev = backend.upload(ref, n_out, n_in)
+    w = m.dequantize_rows().astype(np.float64)
+    x = (synth.activations(4, n_in, 941) * np.float32(1.2345)).astype(np.float32)
+    one = np.concatenate([products(backend, dev, x[i : i + 1]) for i in range(4)])
+    # (rows of up to 20,480 terms, summed in one slice by the generic kernel: sqrt(20480 / 32) f32 roundings per lane)
+    assert row_err(one, x.astype(np.float64) @ w.T) < 4e-6
+    for t in (2, 4):
+        assert np.array_equal(products(backend, dev, x[:t]), one[:t])
+
+
+@pytest.mark.parametrize("kind", OTHERS, ids=lambda k: O.KIND_NAMES[k])
+def test_other_formats_as_a_pair_and_as_a_shard(backend, kind):
+    n_out, n_in = 77, 768
+    (g, gm), (u, um) = other(kind, n_out, n_in, 950), other(kind, n_out, n_in, 951)
+    dg, du = backend.upload(g, n_out, n_in), backend.upload(u, n_out, n_in)
+    x = synth.activations(3, n_in, 952)
+    a, b = (x.astype(np.float64) @ m.dequantize_rows().astype(np.float64).T for m in (gm, um))
+    x = (x / np.abs(a).max()).astype(np.float32)  # silu stays in range
+    a, b = (x.astype(np.float64) @ m.dequantize_rows().astype(np.float64).T for m in (gm, um))
+    y = np.zeros((3, n_out), np.float32)
+    assert backend.matvec_rows(x, [ob.RowsJob(dg, y, du)])
+    assert row_err(y, a / (1.0 + np.exp(-a)) * b) < 1e-5
+    plain = products(backend, dg, x)
+    assert np.array_equal(products(backend, backend.shard_rows(dg, 13, n_out), x), plain[:, 13:])
