@@ -82,6 +82,10 @@ class Backend {
     uint64_t launches = 0;
     // staging for the host-buffer entry points
     Scratch x_dev, y_dev, x16, x8, xprep, xrec;
+    // page-locked staging of the host-buffer entry points, for vectors and results of up to HOST_STAGE bytes: [x | y]
+    static constexpr size_t HOST_STAGE = 256 * 1024;
+    uint8_t* host_stage = nullptr;
+    bool stage_busy = false;  // a call that failed half-way may have left a copy from it in flight
     GemmStatus* gemm_status = nullptr;  // device
     // cached tensor maps of the tensor-core GEMM (see matmul_dev)
     std::vector<GemmPlan*> plans;
@@ -643,6 +647,39 @@ class Backend {
     using clk = std::chrono::steady_clock;
     static double since(clk::time_point t0) { return std::chrono::duration<double, std::nano>(clk::now() - t0).count(); }
 
+    // Host vectors to x_dev, and the jobs' results back with the stream synchronized. Small ones go through page-locked memory, the
+    // results in one copy: a copy to pageable memory is a round trip of its own (the q / k / v products of
+    // one token: 67 us with four of them, 44 this way). Above a few hundred KB the bytes count, and a second
+    // copy on the host loses.
+    bool stage_host() {
+        if (!host_stage && cudaHostAlloc((void**)&host_stage, 2 * HOST_STAGE, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            host_stage = nullptr;
+        }
+        return host_stage != nullptr;
+    }
+    cudaError_t copy_in(const float* x, size_t bytes) {
+        const void* src = x;
+        if (bytes <= HOST_STAGE && stage_host()) {
+            if (stage_busy) cudaDeviceSynchronize();
+            src = std::memcpy(host_stage, x, bytes);
+            stage_busy = true;
+        }
+        return cudaMemcpyAsync(x_dev.p, src, bytes, cudaMemcpyHostToDevice, stream);
+    }
+    template <typename Job>
+    cudaError_t copy_out(const Job* jobs, size_t n_jobs, size_t t, const std::vector<size_t>& y_off, size_t y_total) {
+        const bool staged = y_total <= HOST_STAGE && stage_host();
+        cudaError_t e = cudaSuccess;
+        if (staged) e = cudaMemcpyAsync(host_stage + HOST_STAGE, y_dev.p, y_total, cudaMemcpyDeviceToHost, stream);
+        for (size_t j = 0; j < n_jobs && !staged && e == cudaSuccess; j++)
+            e = cudaMemcpyAsync(jobs[j].y, (uint8_t*)y_dev.p + y_off[j], t * jobs[j].n_out * 4, cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e == cudaSuccess) stage_busy = false;
+        for (size_t j = 0; j < n_jobs && staged && e == cudaSuccess; j++) std::memcpy(jobs[j].y, host_stage + HOST_STAGE + y_off[j], t * jobs[j].n_out * 4);
+        return e;
+    }
+
     // ---- Backend::matmul (src/cuda.rs:1428-1493)
     int matmul(const float* x, size_t t, size_t n_in, b2_job* jobs, size_t n_jobs) {
         if (t == 0 || n_jobs == 0) return B2_OK;
@@ -667,7 +704,7 @@ class Backend {
         cudaError_t e = x_dev.reserve(t * n_in * 4);
         if (e == cudaSuccess) e = y_dev.reserve(y_total);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(staging)");
-        e = cudaMemcpyAsync(x_dev.p, x, t * n_in * 4, cudaMemcpyHostToDevice, stream);
+        e = copy_in(x, t * n_in * 4);
         if (e != cudaSuccess) return cuda_fail(e, "copy-in");
         ns_in += since(t0);
         auto t1 = clk::now();
@@ -683,9 +720,7 @@ class Backend {
         if (int rc = check_gemm_status()) return rc;
         ns_gpu += since(t1);
         auto t2 = clk::now();
-        for (size_t j = 0; j < n_jobs && e == cudaSuccess; j++)
-            e = cudaMemcpyAsync(jobs[j].y, (uint8_t*)y_dev.p + y_off[j], t * jobs[j].n_out * 4, cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        e = copy_out(jobs, n_jobs, t, y_off, y_total);
         if (e != cudaSuccess) return cuda_fail(e, "copy-out");
         ns_out += since(t2);
         calls++;
@@ -716,7 +751,7 @@ class Backend {
         cudaError_t e = x_dev.reserve(t * n_in * 4);
         if (e == cudaSuccess) e = y_dev.reserve(y_total);  // all jobs run before any result goes back to the host
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(staging)");
-        e = cudaMemcpyAsync(x_dev.p, x, t * n_in * 4, cudaMemcpyHostToDevice, stream);
+        e = copy_in(x, t * n_in * 4);
         if (e != cudaSuccess) return cuda_fail(e, "copy-in");
         ns_in += since(t0);
         auto t1 = clk::now();
@@ -756,9 +791,7 @@ class Backend {
         // the stream and the call synchronizes once. (The matrix-vector kernels have no status word to consult in between; a
         // product of a few microseconds would otherwise pay two host round trips.) The kernels' and the copies' time are
         // booked together as kernel time.
-        for (size_t j = 0; j < n_jobs && e == cudaSuccess; j++)
-            e = cudaMemcpyAsync(jobs[j].y, (uint8_t*)y_dev.p + y_off[j], t * jobs[j].n_out * 4, cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        e = copy_out(jobs, n_jobs, t, y_off, y_total);
         if (e != cudaSuccess) return cuda_fail(e, "matvec_rows kernels / copy-out");
         ns_gpu += since(t1);
         calls++;
@@ -1466,6 +1499,8 @@ class Backend {
         x16.release();
         x8.release();
         xprep.release();
+        if (host_stage) cudaFreeHost(host_stage);
+        host_stage = nullptr;
         xrec.release();
         if (gemm_status) cudaFree(gemm_status);
         gemm_status = nullptr;
