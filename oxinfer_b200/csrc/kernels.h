@@ -274,9 +274,11 @@ cudaError_t launch_attend_rows(const float* q, float* out, size_t stride, uint32
 // RMS norm of `rows` rows (p.n values each, p.pre / p.eps / p.add as for launch_norm; the strides here replace p's). With
 // x16 / unscale the rows also leave as the f16 operands launch_to_f16 would make of the result (rows of p.n halves).
 bool norm_rows_supports(uint32_t n, const float* x, const float* out, const float* w, size_t x_stride, size_t out_stride);
-cudaError_t launch_norm_rows(const float* x, size_t x_stride, float* out, size_t out_stride, const float* w, const DecNorm& p, uint32_t rows,
-                             void* x16, float* unscale, cudaStream_t st);
-// With x16 / unscale (glu_rows_f16_supports(n)) the rows also leave as the f16 operands launch_to_f16 would make of the result.
+// `out` may be null then. addend: rows of p.n values that are added to x (in place) first.
+cudaError_t launch_norm_rows(float* x, size_t x_stride, float* out, size_t out_stride, const float* w, const DecNorm& p, uint32_t rows,
+                             void* x16, float* unscale, const float* addend, cudaStream_t st);
+// With x16 / unscale (glu_rows_f16_supports(n)) the rows also leave as the f16 operands launch_to_f16 would make of the result; `out`
+// may be null then.
 bool glu_rows_f16_supports(uint32_t n);
 cudaError_t launch_glu_rows(const float* g, size_t g_stride, const float* u, size_t u_stride, float* out, size_t out_stride, uint32_t n,
                             uint32_t rows, int gelu, cudaStream_t st, void* x16 = nullptr, float* unscale = nullptr);

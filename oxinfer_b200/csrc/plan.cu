@@ -471,6 +471,27 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
             default: return overlaps_f(v, n, o.y, (size_t)o.rope.nh * o.rope.hd);
         }
     };
+    // whether an op writes all of v
+    auto covers = [&](const Op& o, const float* v, size_t n) {
+        const float* y = o.kind == B2_OP_EXCHANGE ? nullptr : o.y;
+        const size_t len = o.kind == B2_OP_LINEAR ? o.w.n_out : o.kind == B2_OP_NORM ? (o.rows == 1 ? o.norm.n : 0) : o.kind == B2_OP_GLU ? o.n : 0;
+        return y && y <= v && v + n <= y + len;
+    };
+    // Whether anything from op b on reads v before it is written anew, a step following on a step, up to op a.
+    auto read_later = [&](size_t b, size_t a, const float* v, size_t n) {
+        for (size_t c = b; c != a; c = c + 1 < p->ops_.size() ? c + 1 : 0) {
+            const Op& o = p->ops_[c];
+            const size_t rope = o.kind == B2_OP_QK_ROPE ? std::max({(size_t)(o.rope.nh - 1) * o.rope.q_stride + o.rope.hd, (size_t)o.rope.k_off + (size_t)o.rope.nkv * o.rope.hd,
+                                                                    (size_t)o.rope.v_off + (size_t)o.rope.nkv * o.rope.hd})
+                                                        : 0;
+            const bool reading = o.kind == B2_OP_QK_ROPE  ? overlaps_f(v, n, o.x, rope)
+                                 : o.kind == B2_OP_ATTEND ? overlaps_f(v, n, o.x, (size_t)o.attn.nh * o.attn.hd)
+                                                          : reads(o, v, n);
+            if (reading) return true;
+            if (covers(o, v, n)) return false;
+        }
+        return false;
+    };
     // ---- norms whose output only splits read become part of the split: x times the weights is split, and the products multiply their
     // results by the factor (nothing has to wait for the whole row first, and the norm is not launched) ----
     if (p->defer_norm_) {
@@ -486,7 +507,8 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
                 const Op& o = p->ops_[b];
                 if (o.kind == OP_SPLIT && o.sx == y && o.n == n && !o.normed && !stale) users.push_back(b);
                 else if (reads(o, y, n)) ok = false;
-                if (writes(o, y, n)) break;
+                if (covers(o, y, n)) break;
+                if (writes(o, y, n)) ok = false;  // a part of it: what the rest holds would have to be known
                 stale = stale || writes(o, nrm.x, n);  // a split behind this point would read another x
             }
             if (!ok || users.empty()) continue;
@@ -612,6 +634,16 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
     PLAN_CUDA(cudaEventCreate(&p->ev1_), "cudaEventCreate");
 
     if (prefill) {
+        for (size_t a = 0; a + 1 < p->ops_.size(); a++) {
+            Op& o = p->ops_[a];
+            if (!(o.kind == B2_OP_NORM && o.rows == 1 && !o.norm.add) && !(o.kind == B2_OP_LINEAR && o.pair)) continue;
+            const size_t n = o.kind == B2_OP_NORM ? o.norm.n : o.w.n_out;
+            size_t b = a + 1;
+            while (b < p->ops_.size() && p->ops_[b].kind == B2_OP_LINEAR && p->ops_[b].x == o.y && p->ops_[b].w.n_in == n && !writes(p->ops_[b], o.y, n))
+                if (p->ops_[b++].pair) break;  // (its own result may take the f16 rows' place)
+            o.x16_only = b > a + 1 && b < p->ops_.size() && !overlaps_f(o.y, n, p->hidden_, p->n_hidden_) && !overlaps_f(o.y, n, p->input_, p->n_input_) &&
+                         !read_later(b, a, o.y, n);
+        }
         size_t max_k = 64, max_n = 64;
         for (const Op& o : p->ops_)
             if (o.kind == B2_OP_LINEAR) {
@@ -733,16 +765,19 @@ int DecodePlanImpl::run_ops_multi(cudaStream_t st, int nt, std::string& err, boo
     };
     // A vector's record is made in a launch of its own where the products would have more than `self_blocks` blocks of 256 values per
     // warp to split, every CTA all of them.
-    static const size_t self_blocks = [] {
-        const char* e = getenv("B2_PLAN_SELF_BLOCKS");
-        return e ? (size_t)atoi(e) : (size_t)2;
-    }();
+    constexpr size_t self_blocks = 2;
     auto self = [&](const Op& o, size_t n) { return o.self && split_blocks_of(n) * (size_t)nt <= 16 * self_blocks; };
     for (size_t i = 0; i < ops_.size(); i++) {
         const Op& o = ops_[i];
         cudaError_t e = cudaSuccess;
         switch (o.kind) {
             case B2_OP_NORM:
+                if (o.rows == 1) {  // all tokens in one launch: a CTA per row either way
+                    DecNorm n = o.norm;
+                    n.x_stride = n.out_stride = (uint32_t)block_floats_;
+                    e = launch_norm(o.x, o.y, o.p0, n, (uint32_t)nt, st, pdl());
+                    break;
+                }
                 for (int tk = 0; tk < nt && e == cudaSuccess; tk++) e = launch_norm(A(o.x, tk), A(o.y, tk), o.p0, o.norm, o.rows, st, pdl());
                 break;
             case OP_SPLIT:
@@ -922,6 +957,7 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
     const uint32_t rows = (uint32_t)t;
     const float* x16_src = nullptr;  // the vector whose f16 rows the scratch holds
     size_t x16_k = 0;
+    const float* addend = nullptr;  // rows that the norm behind a product still has to add to its own
     auto gemm = [&](const WeightDev& w, float* y, size_t y_ld) -> cudaError_t {
         GemmPlan* gp = nullptr;
         if (build) {
@@ -951,7 +987,8 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
                     // a product right behind it that reads exactly this vector gets its f16 rows from the norm kernel
                     const Op* nx = i + 1 < ops_.size() ? &ops_[i + 1] : nullptr;
                     const bool feeds = nx && nx->kind == B2_OP_LINEAR && nx->x == o.y && nx->w.n_in == o.norm.n && o.norm.n % 8 == 0;
-                    e = launch_norm_rows(o.x, ld, o.y, ld, o.p0, o.norm, rows, feeds ? x16_ : nullptr, unscale_, st);
+                    e = launch_norm_rows(o.x, ld, feeds && o.x16_only ? nullptr : o.y, ld, o.p0, o.norm, rows, feeds ? x16_ : nullptr, unscale_, addend, st);
+                    addend = nullptr;
                     count++;
                     if (feeds) {
                         x16_src = o.y;
@@ -986,7 +1023,7 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
                     const Op* nx = i + 1 < ops_.size() ? &ops_[i + 1] : nullptr;
                     const bool feeds = nx && nx->kind == B2_OP_LINEAR && nx->x == o.y && nx->w.n_in == n_out && glu_rows_f16_supports((uint32_t)n_out);
                     if (e == cudaSuccess)
-                        e = launch_glu_rows(tmp_a_, n_out, tmp_b_, n_out, o.y, ld, (uint32_t)n_out, rows, o.mode == B2_MODE_GELU_PAIR, st,
+                        e = launch_glu_rows(tmp_a_, n_out, tmp_b_, n_out, feeds && o.x16_only ? nullptr : o.y, ld, (uint32_t)n_out, rows, o.mode == B2_MODE_GELU_PAIR, st,
                                             feeds ? x16_ : nullptr, unscale_);
                     count++;
                     if (feeds && e == cudaSuccess) {
@@ -1000,8 +1037,15 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
                     // (a product that adds goes through the scratch matrix: its dense rows let the GEMM pick its widest tiles, which
                     // the strided destination's copy-engine stores cannot take; measured 63 + 13 us against 95 us at 4096 x 4096)
                     e = gemm(o.w, tmp_a_, n_out);
-                    if (e == cudaSuccess) e = launch_rows_op(o.y, ld, tmp_a_, n_out, (uint32_t)n_out, rows, o.mode == B2_MODE_ADD, st);
-                    count++;
+                    // (a norm right behind it that reads exactly these rows makes the sum on its way)
+                    const Op* nx = i + 1 < ops_.size() ? &ops_[i + 1] : nullptr;
+                    if (o.mode == B2_MODE_ADD && nx && nx->kind == B2_OP_NORM && nx->rows == 1 && nx->x == o.y && nx->norm.n == n_out &&
+                        norm_rows_supports(nx->norm.n, nx->x, nx->y, nx->p0, ld, ld)) {
+                        addend = tmp_a_;
+                    } else if (e == cudaSuccess) {
+                        e = launch_rows_op(o.y, ld, tmp_a_, n_out, (uint32_t)n_out, rows, o.mode == B2_MODE_ADD, st);
+                        count++;
+                    }
                 }
                 if (overlaps_f(o.y, n_out, x16_src, x16_k)) x16_src = nullptr;
                 break;

@@ -281,3 +281,40 @@ def test_prefill_over_fp8_weights(backend):
     assert row_err(hp, h1.astype(np.float64)) < 4e-3   # two FP8 paths against each other: twice the 2e-3 of an FP8 row
     one.close()
     pre.close()
+
+
+@pytest.mark.parametrize("again", ["nothing", "norm", "pair", "rows"])
+def test_rows_that_only_products_read_stay_f16_and_the_others_do_not(backend, again):
+    """A prefill plan leaves out the f32 rows of a norm or a gate / up pair that only the products behind it read (in f16), and folds a
+    residual add into the norm behind it. Whatever else reads those rows later in the step still finds them."""
+    h, inter, t = 256, 512, 37
+    gate, up, down, last = (backend.upload(synth.q4_k_model(n, k, 70 + i, k**-0.5), n, k) for i, (n, k) in enumerate([(inter, h), (inter, h), (h, inter), (h, h)]))
+    rng = np.random.default_rng(71)
+    w1, w2 = (1.0 + 0.1 * rng.standard_normal((2, h))).astype(np.float32)
+
+    def graph():
+        g = D.Graph()
+        x, y, m, z, o, out = g.buf(h), g.buf(h), g.buf(inter), g.buf(h), g.buf(h), g.buf(inter)
+        n_out = inter if again == "pair" else h
+        g.input, g.n_input, g.hidden, g.n_hidden = x, h, (o if again == "nothing" else out), n_out
+        g.norm(x, y, w1, h, 1e-5)
+        g.linear(gate, y, m, ob.MODE_SILU_PAIR, up)
+        g.linear(down, m, x, ob.MODE_ADD)
+        g.norm(x, z, w2, h, 1e-5)
+        g.linear(last, z, o)
+        if again != "nothing":
+            a = {"norm": y, "pair": m, "rows": x}[again]
+            g.glu(a, m if again == "pair" else o, out, n_out)
+        return g
+
+    one, pre = D.decode_plan(backend, graph(), 64), D.decode_plan_prefill(backend, graph(), 64, t)
+    assert one is not None and pre is not None, backend.last_declined
+    xs = rng.standard_normal((t, h)).astype(np.float32)
+    none = np.zeros((t, 0), np.float32)
+    for _ in range(2):  # the second step finds the first one's buffers
+        got, _ = pre.step_multi(0, xs, none, want_logits=False)
+        want = np.stack([one.step(i, xs[i], none[i], want_logits=False)[0] for i in range(t)])
+        # zero-mean weights of unit gain: the roundings of three products in a row, 2e-3 of a row's largest magnitude each, add
+        assert row_err(got, want) < 6e-3
+    one.close()
+    pre.close()
