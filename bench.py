@@ -828,7 +828,7 @@ def decode_extras(be, peaks, n_tokens=256, ctx=2048, n_layers=32, kv_f16=False, 
             many.close()
         except Exception as e:
             out["multi_token_steps"] = {"error": str(e)}
-        # the same model with the products reading 16 of the activations' 21 bits (b2_set_fast_planes; not the default)
+        # the same model with the products reading 18 of the activations' 24 bits (b2_set_fast_planes; not the default)
         try:
             be.set_fast_planes(True)
             fast = D.decode_plan(be, g, max_len, kv_f16=kv_f16)

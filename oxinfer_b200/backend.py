@@ -193,7 +193,7 @@ class Backend:
         self._check(self._L.b2_set_chained(self._ctx, int(on)))
 
     def set_fast_planes(self, on: bool) -> None:
-        """Matrix-vector products over 16 of the activations' 21 bits (no counterpart in the reference; off by default)."""
+        """Matrix-vector products over 18 of the activations' 24 bits (no counterpart in the reference; off by default)."""
         self._check(self._L.b2_set_fast_planes(self._ctx, int(on)))
 
     def set_exact(self, on: bool) -> None:

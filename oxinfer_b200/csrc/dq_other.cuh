@@ -2,8 +2,8 @@
 // non-linear IQ4_NL / IQ4_XS and the microscaling MXFP4): bit-exact decode of 32 consecutive weights, the arithmetic of the
 // matching arms of the reference's dequantize_row (src/ggml.rs:665-706, 713-773, 915-960) with explicit round-to-nearest
 // multiplies and adds. These formats stay in their raw GGUF layout on the device (blocks of 17 .. 176 bytes, only
-// byte-aligned in general), are read with byte loads, and run through one generic dequantize-and-multiply matrix-vector
-// kernel (gemv_other.cu): every format has a device path, none of them is tuned.
+// byte-aligned in general). Their products run on the integer tensor cores where rows are whole runs of 256 values
+// (gemv_mma_other.cuh), else through one generic dequantize-and-multiply kernel (gemv_other.cu).
 #pragma once
 #include "formats.cuh"
 

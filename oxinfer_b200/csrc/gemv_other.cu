@@ -3,7 +3,8 @@
 // no repack: the rows stay as they are in the GGUF file). It takes the five output modes of dmv_out
 // (src/cuda_decode.cu:131-137), the SiLU / GELU pair, and up to four tokens per launch with the weights read once (each
 // token's row equals its one-token row bit for bit). The reference declines every GGUF type on its CUDA backend
-// (src/cuda.rs:642); these formats get a correct device path here, not a tuned one: a warp brings 1024 weights' worth of
+// (src/cuda.rs:642); rows of whole 256-value runs take
+// gemv_mma_other.cuh, the others this kernel: a warp brings 1024 weights' worth of
 // its row's bytes into shared memory with aligned 16-byte loads (the next run is in flight while this one is decoded), and a
 // lane decodes one 32-weight chunk of it with byte reads, five to seven instructions per weight.
 #include "dq_other.cuh"
