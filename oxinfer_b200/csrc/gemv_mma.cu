@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
         if (lane == 0) *(float4*)(r + (size_t)nb * SPLIT_HALVES + (size_t)blk * SPLIT_AUX) = make_float4(d.xs, d.ssq, 0.0f, 0.0f);
         return;
     }
-    const SplitDigits d = split_digits(in, pre, fast);
+    const SplitDigits<3> d = split_digits(in, pre, fast);
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         int pair, in16;

@@ -85,16 +85,17 @@ __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0
 
 // The activations of the CTA in shared memory for TP token places (1, 4 or 8), as this lane reads them.
 // Digits: lane (g, t) feeds column g of an instruction (token g / 4 of its pair, digit g % 4) and holds the sums of columns 2 t and
-// 2 t + 1: token t / 2 of the pair, digits 0 and 1 (t even) or 2 and none (t odd).
+// 2 t + 1: token t / 2 of the pair, digits 0 and 1 (t even) or 2 and (of four) 3 (t odd).
 // Halves: column g is token g / 2 of its four, hi or lo; lane t holds both of token t.
-template <int TP, bool HALVES>
+template <int TP, bool HALVES, int DIGITS = 3>
 struct XView {
     static constexpr int PER = HALVES ? 4 : 2;               // tokens of an instruction
     static constexpr int NT = (TP + PER - 1) / PER;          // instructions for all of them
-    static constexpr uint32_t TOKEN = HALVES ? 128 : 192;    // bytes of a token in a chunk of 32 k (halves) or a pair of chunks (digits)
+    static constexpr uint32_t TOKEN = HALVES ? 128 : 64 * DIGITS;  // bytes of a token in a chunk of 32 k (halves) or a pair of chunks (digits)
     static constexpr uint32_t STEP = TOKEN * TP;             // from one such to the next
     static constexpr uint32_t NEXT = TOKEN * PER;            // from an instruction's tokens to the next one's
-    static constexpr uint32_t BLOCK = HALVES ? SPLIT_HALVES : SPLIT_DIGITS;
+    static constexpr uint32_t BLOCK = HALVES ? SPLIT_HALVES : DIGITS * 256;
+    static constexpr int COLUMNS = DIGITS;                   // of a token that carry digits; a fourth one repeats the third where there are three
     static constexpr uint32_t SUMS = HALVES ? 0 : 32;        // bytes of a (block, token) in `sums`
     static constexpr int RES = 16 * (TP == 1 ? 1 : NT * PER);  // results of a tile of 16 rows
     uint32_t frag;   // this lane's first B fragment

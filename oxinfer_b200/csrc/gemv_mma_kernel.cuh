@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
             xv.xs = smem0 + a.xs_off + 4u * (uint32_t)rt;
             xv.sums = 0;
         } else {
-            const int ct = TP == 1 ? 0 : g >> 2, cd = min(g & 3, 2), rt = TP == 1 ? 0 : t >> 1;
-            xv.frag = smem0 + a.frag_off + (uint32_t)(ct * 192 + cd * 64 + t * 16);
+            const int ct = TP == 1 ? 0 : g >> 2, cd = min(g & 3, X::COLUMNS - 1), rt = TP == 1 ? 0 : t >> 1;
+            xv.frag = smem0 + a.frag_off + ct * X::TOKEN + (uint32_t)(cd * 64 + t * 16);
             xv.xs = smem0 + a.xs_off + 4u * (uint32_t)rt;
             xv.sums = smem0 + a.sums_off + (F::SUMS_BY_COLUMN ? (uint32_t)(ct * 32 + (g & 3) * 8 + t * 4) : (uint32_t)(rt * 32 + (t & 1) * 8));
         }
@@ -214,14 +214,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
                     ssq = d.ssq;
                     s = 0;
                 } else {
-                    const SplitDigits d = split_digits(in, a.pre, a.fast);
+                    const auto d = split_digits<X::COLUMNS>(in, a.pre, a.fast);
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         int pair, in16;
                         split_digit_at(h, lane, pair, in16);
                         uint8_t* o = f0 + (size_t)pair * X::STEP + in16;
 #pragma unroll
-                        for (int pl = 0; pl < 3; pl++) *(uint32_t*)(o + 64 * pl) = d.d[h][pl];
+                        for (int pl = 0; pl < X::COLUMNS; pl++) *(uint32_t*)(o + 64 * pl) = d.d[h][pl];
                     }
                     xs = d.xs;
                     ssq = d.ssq;

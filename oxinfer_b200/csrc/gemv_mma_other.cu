@@ -11,7 +11,7 @@ bool fits(const WeightDev& w, int T) {
     using F = Fo<FMT>;
     const uintptr_t align = FMT == B2_FMT_Q3_K ? 2 : F::PIECE;
     const size_t tp = T == 1 ? 1 : 4, fixed = (size_t)WARPS * F::SLOTS * F::UNIT_BYTES + 16384 + 512;
-    return w.n_in % 256 == 0 && (uintptr_t)w.p0 % align == 0 && fixed + split_blocks(w.n_in) * tp * (SPLIT_DIGITS + 32 + 4 + 4) <= SMEM_MAX;
+    return w.n_in % 256 == 0 && (uintptr_t)w.p0 % align == 0 && fixed + split_blocks(w.n_in) * tp * (4 * 256 + 32 + 4 + 4) <= SMEM_MAX;
 }
 
 template <int FMT>

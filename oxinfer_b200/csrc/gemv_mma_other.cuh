@@ -46,7 +46,7 @@ __device__ __forceinline__ void cp8(uint32_t dst, const void* src) {
 template <int FMT>
 struct Fo {
     template <int TP>
-    using X = XView<TP, false>;
+    using X = XView<TP, false, 4>;  // (four digits: the float kernel, which these formats had before, rounds nothing of x)
     static constexpr bool ONE = FMT == B2_FMT_Q4_1 || FMT == B2_FMT_Q5_1;  // a float minimum per 32
     static constexpr bool HALVES = false, SUMS = ONE || FMT == B2_FMT_Q5_K, SUMS_BY_COLUMN = FMT == B2_FMT_Q5_K;
     static constexpr int BS = FMT == B2_FMT_Q2_K || FMT == B2_FMT_Q3_K || FMT == B2_FMT_Q5_K || FMT == B2_FMT_IQ4_XS ? 256 : FMT == B2_FMT_NVFP4 ? 64 : 32;
@@ -58,7 +58,7 @@ struct Fo {
     // of a row in a slot: an odd multiple of 16 bytes, so that eight rows of four words each fall on 32 banks
     static constexpr int STRIDE = RUN <= 112 ? 112 : RUN <= 144 ? 144 : RUN <= 176 ? 176 : 208;
     static constexpr bool PARTS = false;  // long rows of several tokens go token by token instead
-    static constexpr int BLOCK_K = 256, SLOTS = 3, MAX_BLOCKS = 1;
+    static constexpr int BLOCK_K = 256, SLOTS = STRIDE > 176 ? 2 : 3, MAX_BLOCKS = 1;
     static constexpr int BLOCK_BYTES = 16 * STRIDE, UNIT_BYTES = BLOCK_BYTES;
     // One: eight sums of 32 times the block scale. Q5_K: as for Q4_K.
     __device__ static __forceinline__ void put_sums(uint8_t* e, float xs, int s, int lane) {
@@ -174,7 +174,7 @@ struct Fo {
         constexpr int NT = X<TP>::NT;
         const uint32_t row[2] = {slot + g * STRIDE, slot + (g + 8) * STRIDE};
         const uint32_t xf = x.frag + (uint32_t)u * (4 * X<TP>::STEP);
-        const float w0 = (t & 1) ? 65536.0f : 1.0f, w1 = (t & 1) ? 0.0f : 256.0f;  // what this lane's two digits stand for
+        const float w0 = (t & 1) ? 65536.0f : 1.0f, w1 = (t & 1) ? 16777216.0f : 256.0f;  // what this lane's two digits stand for
         if constexpr (BS != 256) {
             float f[NT][2], mins[2][4] = {};  // mins: of the four chunks that this lane of its token's two takes
 #pragma unroll
@@ -396,8 +396,6 @@ struct Fo {
 #pragma unroll
                     for (int n = 0; n < NT; n++) mma_us16(e[n], mb[0], mb[1], lds32(x.sums + (u * TP + 2 * n) * 32));  // mins times the chunk sums' digits
             }
-            // Q5_K's chunk sums have four digits, Q2_K's minimums meet the activations' three
-            const float m0 = w0, m1 = FMT == B2_FMT_Q5_K ? ((t & 1) ? 16777216.0f : 256.0f) : w1;
 #pragma unroll
             for (int n = 0; n < NT; n++) {
                 const float xs = ldsf(x.xs + (u * TP + 2 * n) * 4);
@@ -405,7 +403,7 @@ struct Fo {
                 for (int r = 0; r < 2; r++) {
                     const float p = fmaf((float)lo[n][2 * r + 1], w1, (float)lo[n][2 * r] * w0);
                     float v = dd[r] * p;
-                    if constexpr (FMT == B2_FMT_Q2_K || FMT == B2_FMT_Q5_K) v = fmaf(dd[r], p, -(dm[r] * fmaf((float)e[n][2 * r + 1], m1, (float)e[n][2 * r] * m0)));
+                    if constexpr (FMT == B2_FMT_Q2_K || FMT == B2_FMT_Q5_K) v = fmaf(dd[r], p, -(dm[r] * fmaf((float)e[n][2 * r + 1], w1, (float)e[n][2 * r] * w0)));
                     acc[n][r] = fmaf(xs, v, acc[n][r]);
                 }
             }

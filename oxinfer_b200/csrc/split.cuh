@@ -2,7 +2,7 @@
 // l holds values 4 l .. 4 l + 3 and 128 + 4 l ... Two forms, chosen by the weights' format:
 //
 // Digits (integer weights). x ~ xs q with xs a power of two per block and |q| <= 8355711 = 127 (1 + 256 + 65536), 23 to 24 bits of
-// the block's largest value; q = q0 + 256 q1 + 65536 q2 in signed bytes. The products run on the integer tensor cores, exactly.
+// the block's largest value (other GGUF formats: a fourth digit, 25 to 26 bits); q = q0 + 256 q1 + 65536 q2 in signed bytes. The products run on the integer tensor cores, exactly.
 //   Record of a block: [pair of chunks of 32 k: 4][digit: 3][lane-in-four t][16 bytes] (the B fragments of two mma.m16n8k32: bytes
 //   4 t .. of either half of the one chunk, then of the other), then SPLIT_AUX bytes of {xs, sum of squares of x, 0, 0, the sums of
 //   q over the eight chunks (int32)}.
@@ -62,19 +62,22 @@ __device__ __forceinline__ void split_values(const SplitIn& in, float pre, float
     ssq = q;
 }
 
+template <int DIGITS>
 struct SplitDigits {
-    uint32_t d[2][3];  // a lane's four digits of each plane, for either half of the block
+    uint32_t d[2][DIGITS];  // a lane's four digits of each plane, for either half of the block
     int s[2];          // sums of q over chunks lane / 8 and 4 + lane / 8
     float xs, ssq;
 };
 // fast: the upper 18 of the 24 bits of every value
-__device__ __forceinline__ SplitDigits split_digits(const SplitIn& in, float pre, bool fast) {
-    SplitDigits r;
+// Four digits: |q| <= 2^25, so that a chunk's sum stays inside 31 bits; the largest values are exact then.
+template <int DIGITS = 3>
+__device__ __forceinline__ SplitDigits<DIGITS> split_digits(const SplitIn& in, float pre, bool fast) {
+    SplitDigits<DIGITS> r;
     float v[8];
     uint32_t mb;
     split_values(in, pre, v, mb, r.ssq);
     // the largest scales into (2^22, QMAX], or one power lower when it would exceed it
-    const int up = mb == 0 ? 0 : min(126, max(-126, 149 - (int)(mb >> 23) - ((mb & 0x7fffffu) > 0x7efefeu ? 1 : 0)));
+    const int up = mb == 0 ? 0 : min(126, max(-126, (DIGITS == 4 ? 151 : 149 - ((mb & 0x7fffffu) > 0x7efefeu ? 1 : 0)) - (int)(mb >> 23)));
     const float k = __uint_as_float((uint32_t)(127 + up) << 23);
     r.xs = mb >= 0x7f800000u ? __uint_as_float(0x7fffffffu) : __uint_as_float((uint32_t)(127 - up) << 23);  // (digits cannot hold an infinity or a NaN)
 #pragma unroll
@@ -86,12 +89,18 @@ __device__ __forceinline__ SplitDigits split_digits(const SplitIn& in, float pre
             int q = __float2int_rn(v[4 * h + i] * k);
             if (fast) q = (q + 32) & ~63;
             s += q;
-            u[i] = (uint32_t)(q + 0x808080);  // q + 128 (1 + 256 + 65536): its bytes are the digits plus 128
+            u[i] = (uint32_t)q + (DIGITS == 4 ? 0x80808080u : 0x808080u);  // q + 128 (1 + 256 + 65536 ..): its bytes are the digits plus 128
         }
         const uint32_t a = __byte_perm(u[0], u[1], 0x5140), b = __byte_perm(u[2], u[3], 0x5140);
         r.d[h][0] = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
         r.d[h][1] = __byte_perm(a, b, 0x7632) ^ 0x80808080u;
-        r.d[h][2] = __byte_perm(__byte_perm(u[0], u[1], 0x0062), __byte_perm(u[2], u[3], 0x0062), 0x5410) ^ 0x80808080u;
+        if constexpr (DIGITS == 4) {
+            const uint32_t c = __byte_perm(u[0], u[1], 0x7362), e = __byte_perm(u[2], u[3], 0x7362);
+            r.d[h][2] = __byte_perm(c, e, 0x5410) ^ 0x80808080u;
+            r.d[h][3] = __byte_perm(c, e, 0x7632) ^ 0x80808080u;
+        } else {
+            r.d[h][2] = __byte_perm(__byte_perm(u[0], u[1], 0x0062), __byte_perm(u[2], u[3], 0x0062), 0x5410) ^ 0x80808080u;
+        }
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         r.s[h] = s;
