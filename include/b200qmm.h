@@ -213,7 +213,9 @@ int b2_free_moe(b2_ctx* ctx, b2_moe_handle m);
  * (route_ids[i k + j], route_w[i k + j]) and y[i] += sum_j w_ij down(silu(gate x_i) * up x_i), added in
  * route order. Host x and y (y is read and written); routes are host arrays in both forms. */
 int b2_moe(b2_ctx* ctx, b2_moe_handle m, const float* x, size_t t, const int32_t* route_ids, const float* route_w, size_t k, float* y);
-/* Same with x and y resident on the device (no synchronization of the result). */
+/* Same with x and y resident on the device (no synchronization of the result). Layers of up to 64 (token, route) pairs run on the
+ * matrix-vector kernels (f32-like arithmetic), larger ones on the tensor-core GEMM (f16 operands); nothing else decides it, so a part of a
+ * layer's pairs over a part of its experts gives the bits that the whole layer gives wherever both counts lie on the same side of 64. */
 int b2_moe_dev(b2_ctx* ctx, b2_moe_handle m, const float* x_dev, size_t t, const int32_t* route_ids, const float* route_w, size_t k, float* y_dev);
 /* route_top_k (src/moe.rs:180-193) / dtopk (src/cuda_decode.cu:285-312) on the device: for each of t rows
  * of n_experts logits, the k largest (ties to the lower index) and exp(l - max) / sum over the chosen. */
@@ -392,8 +394,8 @@ int b2_matmul_sharded_peer(b2_ctx* ctx, b2_weight w_shard, const void* x_dev, in
  * and `m` holds this rank's (b2_upload_moe over them, local numbering); x_dev / y_dev [t][h] are THIS rank's tokens,
  * route_ids [t][k] (host) are global expert numbers, route_w [t][k] (host) their weights. Every (token, route) pair goes to
  * the rank that owns its expert and its result comes back (counts by ncclAllGather, rows by grouped ncclSend / ncclRecv),
- * then y[i] += sum_j w_ij o_ij in route order: bit-identical to b2_moe_dev over all experts on one GPU. Synchronizes the
- * stream (the route tables are host arrays). */
+ * then y[i] += sum_j w_ij o_ij in route order: bit-identical to b2_moe_dev over all experts and all ranks' tokens on one GPU.
+ * Synchronizes the stream (the route tables are host arrays). */
 int b2_moe_ep(b2_ctx* ctx, b2_moe_handle m, size_t n_experts_global, const float* x_dev, size_t t, const int32_t* route_ids,
               const float* route_w, size_t k, float* y_dev);
 

@@ -885,22 +885,26 @@ class Backend {
     // ---- Backend::moe (src/gpu.rs:232-248, src/cuda.rs:798-966): y[i] += sum_j w_ij down_e(act(gate_e x_i) * up_e x_i).
     // The host builds the per-expert segments as the reference does (src/cuda.rs:810-857), padded to the
     // GEMM's 128-row token tile; x_dev / y_dev are device f32 [t][h].
-    // Few tokens per expert (decode, small batches): the 128-row tiles of the tensor-core GEMM would be almost empty. Three launches
+    // A few (token, route) pairs (decode): the 128-row tiles of the tensor-core GEMM would be almost empty. Three launches
     // instead: the fused gate / up product and the down product of gemv_mma.cu over groups of up to eight pairs of one expert, and the
     // ordered combine (src/moe.rs:625-828 does the same per expert on the CPU; f32-like arithmetic, no f16 operands). The routes travel as
     // kernel arguments: no copy, no synchronization.
-    // Time of a group of up to 1 / 4 / 8 pairs of one expert, and of a 128-row tile of the tensor-core GEMM with one- and with two-term
-    // operands, in us per million weights of an expert; the GEMM path has a copy, a synchronization and two launches more.
-    static constexpr double GROUP_US[3] = {0.13, 0.195, 0.32}, TILE_US[2] = {0.55, 1.55}, TILES_US = 25.0;
-    // The cheapest group size that fits (8, 4, 1; 0: none does), and the time of the layer's groups.
-    int moe_group_size(const Moe& m, const std::vector<size_t>& count, double& us) {
+    // The two paths round differently, so the line between them is a number of pairs and nothing else: expert-parallel ranks, which hold
+    // other experts and other counts of them than the layer on one GPU, have to take the path that it takes. (Groups of up to 512
+    // pairs where they are faster, by the counts of the experts, took 64 tokens of 128 experts, top-8, from 202 to 162 us; a shard's
+    // results then differed from the layer's.)
+    // Time of a group of up to 1 / 4 / 8 pairs of one expert, in us per million weights of an expert.
+    static constexpr double GROUP_US[3] = {0.13, 0.195, 0.32};
+    // The cheapest group size that fits (8, 4, 1; 0: none does).
+    int moe_group_size(const Moe& m, const std::vector<size_t>& count) {
         const int fits = std::min(gemv_groups_most(m.h), gemv_groups_most(m.inter));
         int best = 0;
+        double us = 0.0;
         for (int i = 0; i < 3; i++) {
             const int size = i == 0 ? 1 : 4 * i;
             size_t n = 0;
             for (size_t c : count) n += (c + size - 1) / size;
-            const double v = n * GROUP_US[i] * (3e-6 * m.inter * m.h);
+            const double v = n * GROUP_US[i];
             if (size <= fits && (best == 0 || v < us)) {
                 best = size;
                 us = v;
@@ -908,9 +912,9 @@ class Backend {
         }
         return best;
     }
-    int moe_small(const Moe& m, const float* x_dev_, size_t t, const int32_t* ids, const float* rw, size_t k, float* y_dev_, const std::vector<size_t>& count,
-                  int size) {
+    int moe_small(const Moe& m, const float* x_dev_, size_t t, const int32_t* ids, const float* rw, size_t k, float* y_dev_, const std::vector<size_t>& count) {
         const size_t R = t * k;
+        const int size = moe_group_size(m, count);
         cudaError_t e = moe_g.reserve(R * m.inter * 4);
         if (e == cudaSuccess) e = moe_o.reserve(R * m.h * 4);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(moe scratch)");
@@ -922,7 +926,7 @@ class Backend {
         for (size_t x = 0; x < m.experts; x++) {
             at[x] = rows;
             for (size_t c = 0; size && c < count[x]; c += size) {
-                gr.expert[gr.n] = (uint16_t)x;
+                gr.expert[gr.n] = (uint32_t)x;
                 gr.row0[gr.n] = (uint16_t)(rows + c);
                 gr.count[gr.n++] = (uint8_t)std::min<size_t>(size, count[x] - c);
             }
@@ -985,7 +989,8 @@ class Backend {
         return rows;
     }
 
-    int moe_dev(uint64_t handle, const float* x_dev_, size_t t, const int32_t* ids, const float* rw, size_t k, float* y_dev_) {
+    // layer_pairs: the pairs of the layer that this call computes a part of (0: all of it).
+    int moe_dev(uint64_t handle, const float* x_dev_, size_t t, const int32_t* ids, const float* rw, size_t k, float* y_dev_, size_t layer_pairs = 0) {
         auto it = moes.find(handle);
         if (it == moes.end()) return fail(B2_ERR_ARG, "[b200qmm: moe: unknown handle]");
         const Moe& m = it->second;
@@ -999,15 +1004,8 @@ class Backend {
             count[(size_t)ids[i]]++;
         }
         // (the clamped SiLU has no fused pair mode in the matrix-vector kernels: those layers take the GEMM path at any batch)
-        if (t * k <= GEMV_GROUP_ROWS && m.experts <= 65536 && m.act != B2_ACT_SILU_CLAMP && !getenv("B2_MOE_NO_GEMV")) {
-            double us = 0.0;
-            const int size = moe_group_size(m, count, us);
-            size_t tiles = 0;
-            for (size_t c : count) tiles += (c + 127) / 128;
-            const bool two = m.fmt == B2_FMT_Q4_K || exact;
-            if (t * k <= 64 || (size && us <= TILES_US + tiles * TILE_US[two] * (3e-6 * m.inter * m.h)))
-                return moe_small(m, x_dev_, t, ids, rw, k, y_dev_, count, size);
-        }
+        if (std::max(t * k, layer_pairs) <= GEMV_GROUP_ROWS && m.act != B2_ACT_SILU_CLAMP && !getenv("B2_MOE_NO_GEMV"))
+            return moe_small(m, x_dev_, t, ids, rw, k, y_dev_, count);
         // Token tiles of 128 or 256 rows. A tile costs about the same either way (the kernel is bound by the expansion of
         // the tile's weights, which both heights share), so the taller tile wins as soon as it needs clearly fewer tiles:
         // large batches, where the experts hold more than a tile's worth of tokens each.
@@ -1274,8 +1272,8 @@ class Backend {
     //      send / receive (a receiver knows each row's expert from the counts alone, so no ids travel);
     //   3. the local experts over the received rows (moe_dev with one route of weight 1 per row);
     //   4. the results back the same way, and the combine y[i] += sum_j w_ij o_ij in route order.
-    // Each pair runs the kernels it runs on one GPU with the same inputs, and the combine keeps the route order: bit-identical
-    // to the single-GPU layer.
+    // Each pair runs the kernels it runs on one GPU with the same inputs (moe_dev chooses them by the pairs of all ranks), and the
+    // combine keeps the route order: bit-identical to the single-GPU layer.
     int moe_ep(uint64_t handle, size_t n_experts_global, const float* x_dev_, size_t t, const int32_t* ids, const float* rw, size_t k, float* y_dev_) {
         auto it = moes.find(handle);
         if (it == moes.end()) return fail(B2_ERR_ARG, "[b200qmm: moe_ep: unknown handle]");
@@ -1316,7 +1314,8 @@ class Backend {
                 }
         }
         std::vector<size_t> send_rows(W, 0), recv_rows(W, 0);
-        size_t n_recv = 0;
+        size_t n_recv = 0, layer_pairs = 0;
+        for (int32_t c : all) layer_pairs += (size_t)c;
         for (size_t r = 0; r < W; r++) {
             for (size_t x = r * per; x < (r + 1) * per; x++) send_rows[r] += (size_t)mine[x];
             for (size_t x = (size_t)rank * per; x < ((size_t)rank + 1) * per; x++) recv_rows[r] += (size_t)all[r * E + x];
@@ -1358,7 +1357,7 @@ class Backend {
                     for (int32_t c = 0; c < all[r * E + (size_t)rank * per + x]; c++) lid[at++] = (int32_t)x;
             e = cudaMemsetAsync(ep_out.p, 0, n_recv * hdim * 4, stream);
             if (e != cudaSuccess) return cuda_fail(e, "ep memset");
-            int rc = moe_dev(handle, (const float*)ep_recv.p, n_recv, lid.data(), one.data(), 1, (float*)ep_out.p);
+            int rc = moe_dev(handle, (const float*)ep_recv.p, n_recv, lid.data(), one.data(), 1, (float*)ep_out.p, layer_pairs);
             if (rc) return rc;
         }
         // 4. back, and the combine in route order

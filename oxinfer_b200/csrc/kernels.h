@@ -94,11 +94,12 @@ cudaError_t launch_gemv_mma(const WeightDev& w, const WeightDev* up, const GemvI
 // Products over a stack of equally shaped 4-bit matrices (the routed experts of a batch; w describes matrix 0, the others w_stride bytes
 // apart): group g multiplies matrix expert[g] by rows row0[g] .. + count[g] - 1 (at most `most`, 1 .. 8) of the pairs' list. Row i reads the
 // vector of x's row src[i] (gather) or i and writes row i of y. The table travels as a kernel argument: no copy, no synchronization.
-constexpr int GEMV_GROUP_ROWS = 512;
+constexpr int GEMV_GROUP_ROWS = 64;
 struct GemvGroups {
     int n, gather;
     size_t w_stride;
-    uint16_t expert[GEMV_GROUP_ROWS], row0[GEMV_GROUP_ROWS], src[GEMV_GROUP_ROWS];
+    uint32_t expert[GEMV_GROUP_ROWS];
+    uint16_t row0[GEMV_GROUP_ROWS], src[GEMV_GROUP_ROWS];
     uint8_t count[GEMV_GROUP_ROWS];
 };
 int gemv_groups_most(size_t K);  // 8, 4, 1, or 0: not even one row of K values fits

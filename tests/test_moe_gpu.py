@@ -132,6 +132,61 @@ def test_separate_up_matrices_and_the_other_activations(backend, act, limit, t):
     assert backend.upload_moe(devs[0], devs[2], h, inter, up=devs[1], act=3) is None
 
 
+@pytest.mark.parametrize("fmt", ["mlx4", "q4_k"])
+@pytest.mark.parametrize("t", [16, 50, 203])
+def test_parts_of_the_experts_give_the_whole_layers_bits(backend, fmt, t):
+    """What expert-parallel ranks do, one after the other: every rank's experts over the pairs that reach them, each with weight 1, and the
+    combine in route order. The whole layer has 64, 200 and 812 pairs, the parts fewer."""
+    n_experts, k, h, inter, parts = 16, 4, 512, 256, 2
+    refs = [(synth.make(fmt, 2 * inter, h, 770 + 2 * e), synth.make(fmt, h, inter, 771 + 2 * e)) for e in range(n_experts)]
+    devs = [(backend.upload(g, 2 * inter, h), backend.upload(d, h, inter)) for g, d in refs]
+    _, ids, w = routes(t, n_experts, k, 772)
+    x = torch.from_numpy(synth.activations(t, h, 773)).cuda()
+    want = torch.zeros((t, h), device="cuda")
+    assert backend.moe_dev(x, ids, w, backend.upload_moe([g for g, _ in devs], [d for _, d in devs], h, inter), want)
+    pairs = torch.zeros((t * k, h), device="cuda")
+    flat, per = ids.reshape(-1), n_experts // parts
+    for p in range(parts):
+        mine = np.flatnonzero(flat // per == p)
+        part = backend.upload_moe([g for g, _ in devs[p * per : (p + 1) * per]], [d for _, d in devs[p * per : (p + 1) * per]], h, inter)
+        o = torch.zeros((len(mine), h), device="cuda")
+        assert len(mine) > 64 or t < 50
+        assert backend.moe_dev(x[torch.from_numpy(mine // k).cuda()], (flat[mine] - p * per).reshape(-1, 1), np.ones((len(mine), 1), np.float32), part, o)
+        pairs[torch.from_numpy(mine).cuda()] = o
+    got = torch.zeros((t, h), device="cuda")
+    for j in range(k):
+        got += torch.from_numpy(w[:, j : j + 1]).cuda() * pairs[j::k]
+    torch.cuda.synchronize()
+    backend.check_status()
+    assert torch.equal(got, want)
+
+
+# pairs per expert: a lone one, fewer and more than a group of four and of eight, runs of groups; 21,248 values do not fit a group
+@pytest.mark.parametrize("counts,h,inter", [([1, 3, 4, 5, 8, 9, 0, 34], 512, 256), ([31, 0, 33], 768, 1024), ([2, 1], 256, 21248)])
+@pytest.mark.parametrize("fmt", ["mlx4", "q4_k"])
+@pytest.mark.parametrize("act", [0, 1])
+def test_groups_of_pairs(backend, fmt, act, counts, h, inter):
+    """Up to 64 pairs: every row is its one-token row bit for bit, and the layer is as close to the f64 one as two products of 2e-6 of a
+    row each with an activation between them are."""
+    n = len(counts)
+    refs = [[synth.make(fmt, inter, h, 780 + 3 * e), synth.make(fmt, inter, h, 781 + 3 * e), synth.make(fmt, h, inter, 782 + 3 * e)] for e in range(n)]
+    shapes = [(inter, h), (inter, h), (h, inter)]
+    devs, mats = ([[f(r[i], *shapes[i]) for r in refs] for i in range(3)] for f in (backend.upload, oracle_matrix))
+    moe = backend.upload_moe(devs[0], devs[2], h, inter, up=devs[1], act=act)
+    flat = np.random.default_rng(783).permutation(np.repeat(np.arange(n, dtype=np.int32), counts))
+    ids, t = flat.reshape(-1, 1), len(flat)
+    w = np.random.default_rng(784).uniform(0.1, 1.0, (t, 1)).astype(np.float32)
+    x = synth.activations(t, h, 785) * np.float32(0.25)
+    xd = torch.from_numpy(x).cuda()
+    y, one = torch.zeros((t, h), device="cuda"), torch.zeros((t, h), device="cuda")
+    assert backend.moe_dev(xd, ids, w, moe, y)
+    for i in range(t):
+        assert backend.moe_dev(xd[i : i + 1], ids[i : i + 1], w[i : i + 1], moe, one[i : i + 1])
+    torch.cuda.synchronize()
+    assert torch.equal(y, one)
+    assert row_err(y.cpu().numpy(), _layer_f64(mats[0], mats[1], mats[2], x, ids, w, act, 0.0)) < 1e-5
+
+
 def test_route_topk_matches_oracle(backend):
     t, n, k = 70, 128, 8
     logits, ids, w = routes(t, n, k, 720)
