@@ -87,7 +87,7 @@ __device__ __forceinline__ SplitDigits<DIGITS> split_digits(const SplitIn& in, f
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             int q = __float2int_rn(v[4 * h + i] * k);
-            if (fast) q = (q + 32) & ~63;
+            if (DIGITS == 3 && fast) q = min((q + 32) & ~63, 0x7f7f40);  // (the next multiple of 64 has no three signed digits)
             s += q;
             u[i] = (uint32_t)q + (DIGITS == 4 ? 0x80808080u : 0x808080u);  // q + 128 (1 + 256 + 65536 ..): its bytes are the digits plus 128
         }

@@ -82,6 +82,33 @@ def test_values_that_are_not_finite_and_vectors_off_16_bytes(backend, fmt):
         assert np.array_equal(y[0], want[0])
 
 
+@pytest.mark.parametrize("fmt", ["mlx4", "q4_k", "q6_k", "q8_0"])
+def test_fast_digits_of_the_largest_values_of_a_block(backend, fmt):
+    """Under b2_set_fast_planes a value is rounded to 18 bits, at most 7.6e-6 of its block's largest. 8355680 .. 8355711 units of the split
+    would round to a number that three signed digits cannot hold."""
+    n_out, n_in = 40, 2048
+    ref, m = make_pair(fmt, n_out, n_in, 960)
+    dev = backend.upload(ref, n_out, n_in)
+    x = 0.25 * synth.activations(3, n_in, 961)
+    tops = np.array([8355679, 8355680, 8355696, 8355710, 8355711, 8355647, 8355648, 8355672], np.float64)
+    blocks = x.reshape(3, 8, 256)
+    blocks[:, np.arange(8), 17 * np.arange(8)] = np.stack([tops, -tops, tops[::-1]]) * 2.0**-22
+    x = (blocks * 2.0 ** np.array([0, 5, -9, 3, 0, -20, 11, 1])[None, :, None]).reshape(3, n_in).astype(np.float32)
+    w = np.abs(m.dequantize_rows().astype(np.float64))
+    lost = 7.6e-6 * np.abs(x.reshape(3, 8, 256)).max(axis=2).astype(np.float64)
+    bound = np.einsum("tb,nb->tn", lost, w.reshape(n_out, 8, 256).sum(axis=2))
+    want = m.matmul_f64(x)
+    try:
+        backend.set_fast_planes(True)
+        y = products(backend, dev, x)
+        one = np.concatenate([products(backend, dev, x[i : i + 1]) for i in range(3)])
+    finally:
+        backend.set_fast_planes(False)
+    # (a thousandth of the bound for the f32 sums: 2e-6 of a row against 7.6e-6 of every block's largest, 2048 times)
+    assert (np.abs(y - want) <= 1.001 * bound + 2e-6 * np.abs(want)).all()
+    assert np.array_equal(y, one)
+
+
 OTHERS = list(O.OTHER_KINDS) + [O.NVFP4]
 
 
