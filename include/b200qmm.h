@@ -185,9 +185,10 @@ int b2_matvec_rows(b2_ctx* ctx, const float* x, size_t t, size_t n_in, b2_rows_j
 
 /* Device-resident forms of the two calls above (what a decode plan issues per op,
  * src/cuda_decode.rs:1233-1410): no copies, no synchronization, launched on the context's stream.
- * x_dev is [t][n_in] of x_dtype, y_dev is [t][n_out] of y_dtype. */
+ * x_dev is [t][n_in] of x_dtype, y_dev is [t][n_out] of y_dtype. In calls of up to eight f32 rows y_dev may overlap x_dev. */
 int b2_matmul_dev(b2_ctx* ctx, b2_weight w, const void* x_dev, int x_dtype, size_t t, void* y_dev, int y_dtype);
-/* One token: y = mode(W x [, U x]). x_dev f32 [n_in]; y_dev f32 [n_out]; gate_dev f32[1] or NULL. */
+/* One token: y = mode(W x [, U x]). x_dev f32 [n_in]; y_dev f32 [n_out], which may overlap x_dev (x is copied first then);
+ * gate_dev f32[1] or NULL. */
 int b2_matvec_dev(b2_ctx* ctx, b2_weight w, b2_weight up, const float* x_dev, float* y_dev, int mode, const float* gate_dev);
 
 /* ---- routed experts (MoE) ----------------------------------------------------------------- */
@@ -404,7 +405,9 @@ int b2_moe_ep(b2_ctx* ctx, b2_moe_handle m, size_t n_experts_global, const float
  * hosts that cannot call cudaMalloc when they need it: a server whose own arena already owns the
  * whole device, or a decode loop that must stay out of the allocator. The kernel splits the vector
  * in its shared memory; n_in is limited to B2_NOALLOC_MAX_K, larger inputs are refused with
- * B2_ERR_ARG and a message, and go through b2_matvec_dev instead.
+ * B2_ERR_ARG and a message, and go through b2_matvec_dev instead. y_dev may overlap x_dev: such calls
+ * copy x into one fixed array of the library (65,536 bytes per GPU for as long as it is loaded) and
+ * race on it where they may overlap on the GPU; the others share nothing.
  *   w_blocks_dev : raw GGUF Q4_K super-blocks on the device, [n_out][n_in/256][144], 16-byte aligned
  *   x_dev, y_dev : f32 on the device; cuda_stream : the stream to launch on (NULL = default)
  *   err, err_len : optional buffer that receives the error text

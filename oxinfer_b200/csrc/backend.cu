@@ -81,7 +81,7 @@ class Backend {
     uint64_t next_handle = 1;
     uint64_t launches = 0;
     // staging for the host-buffer entry points
-    Scratch x_dev, y_dev, x16, x8, xprep, xrec;
+    Scratch x_dev, y_dev, x16, x8, xprep, xrec, xapart;
     // page-locked staging of the host-buffer entry points, for vectors and results of up to HOST_STAGE bytes: [x | y]
     static constexpr size_t HOST_STAGE = 256 * 1024;
     uint8_t* host_stage = nullptr;
@@ -446,6 +446,16 @@ class Backend {
         return matvec_dev(h, up, (const float*)xprep.p, y_dev_, mode, gate);
     }
 
+    // Every CTA of a product reads x for itself, while others may already store y: an x that y overlaps is read from a copy.
+    int apart(const float*& x, size_t nx, const float* y, size_t ny) {
+        if ((uintptr_t)(y + ny) <= (uintptr_t)x || (uintptr_t)(x + nx) <= (uintptr_t)y) return B2_OK;
+        cudaError_t e = xapart.reserve(nx * 4);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(xapart.p, x, nx * 4, cudaMemcpyDeviceToDevice, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "copy of x");
+        x = (const float*)xapart.p;
+        return B2_OK;
+    }
+
     // One token on the device. The launches are dependent ones (each may start while the one ahead drains and reads nothing but
     // weights before it has waited for it).
     int matvec_dev(uint64_t h, uint64_t up, const float* x_dev_, float* y_dev_, int mode, const float* gate) {
@@ -462,12 +472,14 @@ class Backend {
         if (mode < 0 || mode > 4 || (mode == B2_MODE_ADD_GATED && !gate)) return fail(B2_ERR_ARG, "[b200qmm: matvec: bad mode]");
         if (fmt_is_other(w->dev.fmt)) {
             if (!gemv_other_supports(w->dev)) return fail(B2_DECLINED, "[b200qmm: matvec: shape not supported for this format]");
+            if (int rc = apart(x_dev_, w->dev.n_in, y_dev_, w->dev.n_out)) return rc;
             cudaError_t eo = launch_gemv_other(w->dev, u ? &u->dev : nullptr, x_dev_, 0, y_dev_, 0, 1, mode, gate, sm_count, stream, chained);
             launches++;
             if (eo != cudaSuccess) return cuda_fail(eo, "gemv (generic)");
             return B2_OK;
         }
         if (!gemv_supports(w->dev)) return fail(B2_DECLINED, "[b200qmm: matvec: shape not supported by the GEMV kernels]");
+        if (int rc = apart(x_dev_, w->dev.n_in, y_dev_, w->dev.n_out)) return rc;
         cudaError_t e;
         if (gemv_mma_supports(w->dev)) {
             GemvIn in;
@@ -535,9 +547,11 @@ class Backend {
             // no tensor-core kernel for these formats: four tokens at a time through the generic matrix-vector kernel (the weights
             // are read once per four tokens; every row equals its one-token row bit for bit)
             if (x_dtype != B2_F32 || y_dtype != B2_F32 || !gemv_other_supports(w->dev)) return fail(B2_DECLINED, "[b200qmm: matmul: this format takes f32 activations and results]");
+            const float* xf = (const float*)x;
+            if (int rc = apart(xf, t * K, (const float*)y, t * w->dev.n_out)) return rc;
             for (size_t i = 0; i < t; i += 4) {
                 const int nt = (int)std::min<size_t>(4, t - i);
-                cudaError_t eo = launch_gemv_other(w->dev, nullptr, (const float*)x + i * K, K, (float*)y + i * w->dev.n_out, w->dev.n_out, nt, B2_MODE_STORE, nullptr,
+                cudaError_t eo = launch_gemv_other(w->dev, nullptr, xf + i * K, K, (float*)y + i * w->dev.n_out, w->dev.n_out, nt, B2_MODE_STORE, nullptr,
                                                    sm_count, stream);
                 launches++;
                 if (eo != cudaSuccess) return cuda_fail(eo, "gemv (generic, several rows)");
@@ -550,11 +564,10 @@ class Backend {
         if (x_dtype == B2_F32 && y_dtype == B2_F32 && gemv_supports(w->dev) &&
             ((t <= 8 && !f8_both) || (rows_path(w->dev) && (exact || !gemm_tc_supports(w->dev, t))))) {
             if (t == 1 || !gemv_mma_supports(w->dev)) {
-                for (size_t i = 0; i < t; i++) {
-                    int rc = matvec_dev(h, 0, (const float*)x + i * K, (float*)y + i * w->dev.n_out, B2_MODE_STORE, nullptr);
-                    if (rc) return rc;
-                }
-                return B2_OK;
+                const float* xf = (const float*)x;
+                int rc = apart(xf, t * K, (const float*)y, t * w->dev.n_out);
+                for (size_t i = 0; i < t && !rc; i++) rc = matvec_dev(h, 0, xf + i * K, (float*)y + i * w->dev.n_out, B2_MODE_STORE, nullptr);
+                return rc;
             }
             const bool halves = gemv_mma_halves(w->dev);
             cudaError_t e = xrec.reserve(t * record_stride(K, halves));
@@ -1498,6 +1511,7 @@ class Backend {
         x16.release();
         x8.release();
         xprep.release();
+        xapart.release();
         if (host_stage) cudaFreeHost(host_stage);
         host_stage = nullptr;
         xrec.release();

@@ -129,13 +129,17 @@ cudaError_t launch_gemv_f8_float(const WeightDev& w, const WeightDev* up, const 
 // every buffer out of one arena they own, src/cuda_decode.rs:372-383) has nothing left for the
 // runtime to give, and a latency-critical decode loop must not enter the allocator at all. The
 // product splits its vector in shared memory, so the call needs no device memory of its own, and
-// calls on different streams do not meet. n_in is limited to B2_NOALLOC_MAX_K = 16384.
+// calls on different streams do not meet. A call whose y overlaps x reads x from a copy in a fixed
+// array of the library (every CTA reads x for itself, while others may already store y); all such
+// calls share the array. n_in is limited to its B2_NOALLOC_MAX_K = 16384 values.
 // =============================================================================================
 namespace b2 {
 namespace {
 constexpr size_t NOALLOC_MAX_K = 16384;
 constexpr int NOALLOC_MAX_DEVICES = 64;
 std::atomic<int> g_noalloc_sms[NOALLOC_MAX_DEVICES];
+static __device__ __align__(256) float g_noalloc_x[NOALLOC_MAX_K];
+std::atomic<float*> g_noalloc_ptr[NOALLOC_MAX_DEVICES];  // its address on each device
 
 int noalloc_fail(char* err, size_t err_len, int code, const char* text, cudaError_t e = cudaSuccess) {
     if (err && err_len) {
@@ -167,11 +171,15 @@ extern "C" __attribute__((visibility("default"))) int b2_matvec_q4k_noalloc(cons
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return noalloc_fail(err, err_len, B2_ERR_CUDA, "cudaGetDevice", e);
     if (dev < 0 || dev >= NOALLOC_MAX_DEVICES) return noalloc_fail(err, err_len, B2_ERR_ARG, "device ordinal out of range");
-    int sms = g_noalloc_sms[dev].load(std::memory_order_relaxed);
+    int sms = g_noalloc_sms[dev].load(std::memory_order_acquire);
     if (!sms) {
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess || sms <= 0) return noalloc_fail(err, err_len, B2_ERR_CUDA, "cudaDeviceGetAttribute", e);
-        g_noalloc_sms[dev].store(sms, std::memory_order_relaxed);
+        void* p = nullptr;
+        e = cudaGetSymbolAddress(&p, g_noalloc_x);
+        if (e != cudaSuccess || !p) return noalloc_fail(err, err_len, B2_ERR_CUDA, "cudaGetSymbolAddress(scratch)", e);
+        g_noalloc_ptr[dev].store((float*)p, std::memory_order_relaxed);
+        g_noalloc_sms[dev].store(sms, std::memory_order_release);
     }
     WeightDev w{};
     w.fmt = B2_FMT_Q4_K;
@@ -180,6 +188,12 @@ extern "C" __attribute__((visibility("default"))) int b2_matvec_q4k_noalloc(cons
     w.p0 = (const uint8_t*)w_blocks_dev;
     GemvIn in;
     in.x = x_dev;
+    if ((uintptr_t)(y_dev + n_out) > (uintptr_t)x_dev && (uintptr_t)(x_dev + n_in) > (uintptr_t)y_dev) {
+        float* copy = g_noalloc_ptr[dev].load(std::memory_order_relaxed);
+        e = cudaMemcpyAsync(copy, x_dev, n_in * sizeof(float), cudaMemcpyDeviceToDevice, (cudaStream_t)cuda_stream);
+        if (e != cudaSuccess) return noalloc_fail(err, err_len, B2_ERR_CUDA, "copy of x", e);
+        in.x = copy;
+    }
     e = launch_gemv_mma(w, nullptr, in, 1, y_dev, 0, B2_MODE_STORE, nullptr, 0, sms, (cudaStream_t)cuda_stream, false);
     if (e != cudaSuccess) return noalloc_fail(err, err_len, B2_ERR_CUDA, "gemv kernel", e);
     return B2_OK;

@@ -62,6 +62,43 @@ def test_longest_rows(backend):
     assert not backend.matvec_rows(synth.activations(1, 58624, 923), [ob.RowsJob(dev, np.zeros((1, 24), np.float32))])
 
 
+@pytest.mark.parametrize("fmt", FORMATS + ["q5_k"])
+@pytest.mark.parametrize("shift", [0, 8])
+def test_results_over_their_own_vector(backend, fmt, shift):
+    """y on top of x, whole or from its ninth value on: the bits of a y apart. GEMMs on another stream hold most SMs when the product
+    starts, so that its first CTAs have stored their rows before the others read x."""
+    n = 6144
+    ref = synth.make(fmt, n, n, 970) if fmt in FORMATS else other(O.Q5_K, n, n, 970)[0]
+    dev = backend.upload(ref, n, n)
+    x = synth.activations(3, n, 971)
+    want = products(backend, dev, x)
+    side, busy = torch.cuda.Stream(), ob.Backend(0)
+    busy.set_stream(side.cuda_stream)
+    gw = busy.upload(synth.q4_k(14336, 4096, 972), 14336, 4096)
+    gx, gy = torch.zeros((512, 4096), device="cuda", dtype=torch.float16), torch.zeros((512, 14336), device="cuda")
+
+    def beside(run):
+        torch.cuda.synchronize()
+        for _ in range(4):
+            assert busy.matmul_dev(gw, gx, gy)
+        assert run()
+        torch.cuda.synchronize()
+
+    xd = torch.from_numpy(x).cuda()
+    buf = torch.zeros(n + shift, device="cuda")
+    buf[:n] = xd[0]
+    beside(lambda: backend.matvec_dev(dev, buf[:n], buf[shift:]))
+    assert np.array_equal(buf[shift:].cpu().numpy(), want[0])
+    if shift == 0:  # a residual add in place, and several rows
+        buf[:] = xd[0]
+        beside(lambda: backend.matvec_dev(dev, buf, buf, ob.MODE_ADD))
+        assert np.array_equal(buf.cpu().numpy(), x[0] + want[0])
+        rows = xd.clone()
+        beside(lambda: backend.matmul_dev(dev, rows, rows))
+        assert np.array_equal(rows.cpu().numpy(), want)
+    busy.close()
+
+
 @pytest.mark.parametrize("fmt", FORMATS)
 def test_values_that_are_not_finite_and_vectors_off_16_bytes(backend, fmt):
     n_out, n_in = 40, 1024

@@ -89,6 +89,20 @@ def test_noalloc_matches_the_cpu_oracle_and_leaves_device_memory_alone(n_out, n_
         assert O.row_err(got[i].cpu().numpy()[None], want) < TOL
 
 
+def test_noalloc_result_over_its_own_vector():
+    n = 8192
+    ref = synth.q4_k(n, n, 930)
+    w_dev, x = torch.from_numpy(ref.data).cuda(), torch.from_numpy(synth.activations(1, n, 931)[0]).cuda()
+    want = torch.zeros(n, device="cuda")
+    assert _call(w_dev, n, n, x, want)[0] == ob.OK
+    for shift in (0, 8):
+        buf = torch.zeros(n + shift, device="cuda")
+        buf[:n] = x
+        assert _call(w_dev, n, n, buf[:n], buf[shift:])[0] == ob.OK
+        torch.cuda.synchronize()
+        assert torch.equal(buf[shift:], want)
+
+
 def test_noalloc_refuses_sizes_beyond_its_scratch():
     n_out, n_in = 4, 16384 + 256
     w = torch.zeros(n_out * (n_in // 256) * 144, dtype=torch.uint8, device="cuda")
