@@ -9,11 +9,12 @@ __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ x,
                                                     size_t out_stride, int fast, int halves) {
     pdl_launch_dependents();
     pdl_wait();
-    const int blk = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, nb = (K + 255) / 256;
+    // (the tokens along x: there may be more than the 65,535 that y holds)
+    const int blk = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, nb = (K + 255) / 256;
     if (blk >= nb) return;
     const int k = blk * 256;
-    const SplitIn in = split_load(x + (size_t)blockIdx.y * x_stride + k, w ? w + k : nullptr, K - k, lane);
-    uint8_t* r = out + (size_t)blockIdx.y * out_stride;
+    const SplitIn in = split_load(x + (size_t)blockIdx.x * x_stride + k, w ? w + k : nullptr, K - k, lane);
+    uint8_t* r = out + (size_t)blockIdx.x * out_stride;
     if (halves) {
         const SplitHalves d = split_halves(in, pre);
 #pragma unroll
@@ -131,7 +132,7 @@ cudaError_t launch_split(const float* x, size_t x_stride, const float* norm_w, f
                          bool fast, cudaStream_t st, bool pdl) {
     if (tokens < 1 || K == 0 || K % 4) return cudaErrorInvalidValue;
     const unsigned nb = (unsigned)split_blocks(K);
-    return launch_k(split_kernel, dim3((nb + 7) / 8, (unsigned)tokens), dim3(256), 0, st, pdl, x, x_stride, norm_w, pre, (int)K, rec, rec_stride, (int)fast, (int)halves);
+    return launch_k(split_kernel, dim3((unsigned)tokens, (nb + 7) / 8), dim3(256), 0, st, pdl, x, x_stride, norm_w, pre, (int)K, rec, rec_stride, (int)fast, (int)halves);
 }
 
 }  // namespace b2

@@ -50,6 +50,20 @@ def test_many_tiles_whose_sums_wait_for_the_next_part_of_k(backend, fmt, shape):
         assert np.array_equal(products(backend, dev, x[:t]), one[:t])
 
 
+def test_more_rows_than_a_grid_dimension_has(backend):
+    """65,537 rows under the exactness switch, whose products take any number of rows from the same split."""
+    n_out, n_in, t = 24, 256, 65537
+    ref, _ = make_pair("q6_k", n_out, n_in, 925)
+    dev = backend.upload(ref, n_out, n_in)
+    x = np.tile(synth.activations(64, n_in, 926), (1025, 1))[:t]
+    backend.set_exact(True)
+    try:
+        y, few = products(backend, dev, x), products(backend, dev, x[:64])
+    finally:
+        backend.set_exact(False)
+    assert np.array_equal(y, np.tile(few, (1025, 1))[:t])
+
+
 def test_longest_rows(backend):
     ref, m = make_pair("q8_0", 24, 58368, 920)
     dev = backend.upload(ref, 24, 58368)
