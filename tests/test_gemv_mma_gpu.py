@@ -200,3 +200,44 @@ def test_other_formats_as_a_pair_and_as_a_shard(backend, kind):
     assert row_err(y, a / (1.0 + np.exp(-a)) * b) < 1e-5
     plain = products(backend, dg, x)
     assert np.array_equal(products(backend, backend.shard_rows(dg, 13, n_out), x), plain[:, 13:])
+
+
+def f32_product(w, x):
+    """W x as an f32 kernel adds it: 32 lanes take 16 values at a time, a sum from zero with a fused multiply-add each (the product of a
+    weight of 4 and an activation of 24 bits is exact in f64), the lanes' sums in a tree."""
+    n_out, n_in = w.shape
+    steps = -(-n_in // 512)
+    terms = np.zeros((n_out, steps * 512), np.float64)
+    terms[:, :n_in] = w.astype(np.float64) * x.astype(np.float64)
+    terms = terms.reshape(n_out, steps, 32, 16)
+    acc = np.zeros((n_out, 32), np.float32)
+    for s in range(steps):
+        part = np.zeros((n_out, 32), np.float32)
+        for j in range(16):
+            part = (part + terms[:, s, :, j]).astype(np.float32)
+        acc += part
+    while acc.shape[1] > 1:
+        acc = acc[:, : acc.shape[1] // 2] + acc[:, acc.shape[1] // 2 :]
+    return acc[:, 0]
+
+
+@pytest.mark.parametrize("n_in", [256, 1024, 2816, 14336])
+@pytest.mark.parametrize("pair", [False, True])
+def test_fp8_products_are_as_close_as_f32_ones(backend, n_in, pair):
+    """The 2-norm of the error against f64 is no larger than an f32 product's."""
+    n_out, tokens = 1024, 4
+    refs = [make_pair("f8_e4m3", n_out, n_in, 980 + i) for i in range(2 if pair else 1)]
+    devs, w = [backend.upload(r, n_out, n_in) for r, _ in refs], [m.dequantize_rows() for _, m in refs]
+    x = synth.activations(tokens, n_in, 982)
+    x /= np.abs(w[0] @ x.T).max()  # silu stays in range
+    got, f32, want = [], [], []
+    for v in x:
+        y = torch.zeros(n_out, device="cuda")
+        assert backend.matvec_dev(devs[0], torch.from_numpy(v).cuda(), y, ob.MODE_SILU_PAIR if pair else ob.MODE_STORE, devs[1] if pair else None)
+        got.append(y.cpu().numpy())
+        d = [f32_product(m, v) for m in w]
+        f32.append(d[0] / (np.float32(1) + np.exp(-d[0])) * d[1] if pair else d[0])
+        d = [m.astype(np.float64) @ v.astype(np.float64) for m in w]
+        want.append(d[0] / (1.0 + np.exp(-d[0])) * d[1] if pair else d[0])
+    error = lambda v: np.linalg.norm(np.stack(v) - np.stack(want))  # noqa: E731
+    assert error(got) < error(f32)
