@@ -501,7 +501,29 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             const uint32_t row_off = (uint32_t)(r + (is_lo ? 128 : 0)) * 128u;
             const uint32_t swz = (uint32_t)(r & 7);
             const uint4* my_raw0 = (const uint4*)(raw + (size_t)(in_tile ? r : 0) * (FMT == B2_FMT_Q6_K ? 128 : RAW_ROW));
+            // The scales that lie beside the packed rows come straight from global memory, a super-block ahead: this row's f16 d and eight i8
+            // scales of this set's two stages (Q6_K), two f16 d (Q8_0), one f32 (FP8). Loaded where they are used they stand behind
+            // release_raw, which waits for the staged words: 512 x 4096 x 14336 in 69.9 us (Q6_K) and 66.6 (Q8_0), this way 61.9 and 60.8.
+            const bool live = in_tile && n0 + r < n_out;
+            uint32_t next_scales[3] = {0u, 0u, 0u};
+            auto load_scales = [&](int sb) {
+                if (!PRE_SCALED || !live || sb >= nsb) return;
+                const size_t wrow = (size_t)(n0 + r);
+                if constexpr (FMT == B2_FMT_Q6_K) {
+                    const uint32_t* sc = (const uint32_t*)((const int8_t*)f8.s + wrow * (size_t)(K / 16) + (size_t)(sb0 + sb) * 16);
+                    next_scales[0] = __ldg((const unsigned short*)f8.s2 + wrow * (size_t)(K / 256) + sb0 + sb);
+                    next_scales[1] = __ldg(sc + set);
+                    next_scales[2] = __ldg(sc + set + 2);
+                } else if constexpr (FMT == B2_FMT_Q8_0) {
+                    next_scales[0] = __ldg((const uint32_t*)((const unsigned short*)f8.s + wrow * (size_t)f8.ncb + (size_t)(sb0 + sb) * 4 + set * 2));
+                } else if (f8.s) {
+                    next_scales[0] = __float_as_uint(__ldg(f8.s + (size_t)((f8.row0 + n0 + r) / f8.rows) * f8.ncb + sb0 + sb));
+                }
+            };
+            load_scales(0);
             for (int sb = 0; sb < nsb && ok; sb++) {
+                const uint32_t scales[3] = {next_scales[0], next_scales[1], next_scales[2]};
+                load_scales(sb + 1);
                 const int rb = sb % NRAW;
                 const uint4* my_raw = (const uint4*)((const uint8_t*)my_raw0 + (size_t)rb * RAW_BYTES);
                 // this row's packed super-block: staging buffer -> registers (only the two 64-groups this set
@@ -518,9 +540,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     // c ^ ((r >> 1) & 3). w = f16(d sc pre) * (q - 32), q - 32 exact in f16.
                     const uint4* my_qh = (const uint4*)(raw + (size_t)my_rows * 128 + (size_t)(in_tile ? r : 0) * 64);
                     const uint32_t swh = (uint32_t)((r >> 1) & 3);
-                    const size_t wrow = (size_t)(n0 + r);
-                    const bool live = in_tile && n0 + r < n_out;
-                    const float d = live ? __half2float(__ushort_as_half(__ldg((const unsigned short*)f8.s2 + wrow * (size_t)(K / 256) + sb0 + sb))) : 0.0f;
+                    const float d = __half2float(__ushort_as_half((unsigned short)scales[0]));
 #pragma unroll
                     for (int jj = 0; jj < 2; jj++) {
                         const int j = set + 2 * jj, n = j >> 1, odd = j & 1;
@@ -531,7 +551,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                         for (int c = 0; c < 2; c++) qh4[c] = my_qh[((uint32_t)(2 * n + c)) ^ swh];
                         if (jj == 1)  // the row's last read of this super-block's staging buffer
                             release_raw(&sh->raw_empty[rb], ql4[0].x | ql4[1].x | ql4[2].x | ql4[3].x | qh4[0].x | qh4[1].x, zero, lane);
-                        const uint32_t sc4 = live ? __ldg((const uint32_t*)((const int8_t*)f8.s + wrow * (size_t)(K / 16) + (size_t)(sb0 + sb) * 16 + 4 * j)) : 0u;
+                        const uint32_t sc4 = scales[1 + jj];
                         __half2 mul[4];
 #pragma unroll
                         for (int i = 0; i < 4; i++) mul[i] = __float2half2_rn(d * (float)(int8_t)(sc4 >> (8 * i)) * f8.pre);
@@ -583,9 +603,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     if constexpr (FMT == B2_FMT_Q8_0) {
                         // 64 int8 of this set's stage = two blocks of 32 with an f16 scale each (src/ggml.rs Q8_0 decode): byte b ^ 0x80
                         // under the exponent 0x64 is the f16 1024 + (q + 128), minus 1152 = q exactly, times f16(d pre)
-                        uint32_t d2 = 0u;
-                        if (in_tile && n0 + r < n_out)
-                            d2 = __ldg((const uint32_t*)((const unsigned short*)f8.s + (size_t)(n0 + r) * (size_t)f8.ncb + (size_t)(sb0 + sb) * 4 + set * 2));
+                        const uint32_t d2 = scales[0];
                         const __half2 m0 = __float2half2_rn(__half2float(__ushort_as_half((unsigned short)(d2 & 0xffffu))) * f8.pre);
                         const __half2 m1 = __float2half2_rn(__half2float(__ushort_as_half((unsigned short)(d2 >> 16))) * f8.pre);
                         const __half2 bias = __float2half2_rn(1152.0f);
@@ -601,9 +619,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                             }
                         }
                     }
-                    float scale = 1.0f;
-                    if (FMT == B2_FMT_F8E4M3 && f8.s && in_tile && n0 + r < n_out) scale = __ldg(f8.s + (size_t)((f8.row0 + n0 + r) / f8.rows) * f8.ncb + sb0 + sb);
-                    const __half2 sc2 = __float2half2_rn(scale * f8.pre);
+                    const __half2 sc2 = __float2half2_rn((f8.s ? __uint_as_float(scales[0]) : 1.0f) * f8.pre);
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
                         if (FMT != B2_FMT_F8E4M3) break;
