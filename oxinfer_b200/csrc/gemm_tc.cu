@@ -269,9 +269,9 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     constexpr int dbg = 0;
     (void)dbg_arg;
 #endif
-    // A "raw block" is what one weight copy brings per row: a 144-byte 4-bit block (256 k, four pipeline
-    // stages) or 128 e4m3 bytes (128 k = one column of FP8 scale blocks, two stages).
-    // Q8_0 rows are 128 int8 per copy like the FP8 rows; a Q6_K copy brings a row's 128 bytes of low nibbles and, through a
+    // A "raw block" is a row's part of the packed weights that are expanded in one round: a 144-byte 4-bit block (256 k, four pipeline
+    // stages) or 128 e4m3 bytes (128 k = one column of FP8 scale blocks, two stages), which come in two copies.
+    // Q8_0 rows are 128 int8 like the FP8 rows; a Q6_K copy brings a row's 128 bytes of low nibbles and, through a
     // second tensor map (y_more[n_more]), its 64 bytes of high bit pairs (the planes of formats.cuh), 256 k = four stages.
     constexpr bool BYTE_ROWS = FMT == B2_FMT_F8E4M3 || FMT == B2_FMT_Q8_0;
     constexpr bool PRE_SCALED = BYTE_ROWS || FMT == B2_FMT_Q6_K;  // the f16 weights carry the factor f8.pre, the epilogue takes it out
@@ -290,7 +290,12 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     constexpr int RAW_BYTES = PAIR ? PAIR_RAW_BYTES : (FMT == B2_FMT_Q6_K ? Q6K_MAX_TILE_N * 192 : b2::RAW_BYTES);
     static_assert(1024 + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + (PAIR ? 2 : 1) * RAW_BYTES + sizeof(Shared) <= (PAIR ? PAIR_SMEM : GEMM_SMEM),
                   "the format's buffers fit the launch's shared memory");
-    constexpr int NRAW = PAIR ? 2 : 1;  // staging buffers of packed weights
+    // Staging buffers of packed weights. Rows of bytes: one for each dequantizer set, with the 64 k of the set's stage. (One buffer with
+    // the 128 k of both sets is free for the next copy only when the later set has read it, half a round after the earlier one, and the
+    // copy then lands when the earlier set is already waiting for it: Q8_0 512 x 4096 x 14336 60.8 us,
+    // this way 58.8.)
+    constexpr int NRAW = PAIR || BYTE_ROWS ? 2 : 1;
+    constexpr int RAW_STRIDE = BYTE_ROWS ? b2::MAX_TILE_N * 64 : RAW_BYTES;  // from a buffer to the next
     // dequantizer sets: groups of warps that take the pipeline stages in turn, one thread per weight row of the CTA's tile
     constexpr int NSETS = PAIR ? 4 : 2, SET_THREADS = 512 / NSETS, SET_WARPS = SET_THREADS / 32;
     extern __shared__ uint8_t smem_raw[];
@@ -298,7 +303,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     uint8_t* a_tiles = smem;
     uint8_t* b_tiles = smem + (size_t)STAGES * A_STAGE_BYTES;
     uint8_t* raw = b_tiles + (size_t)STAGES * B_STAGE_BYTES;
-    Shared* sh = (Shared*)(raw + NRAW * RAW_BYTES);
+    Shared* sh = (Shared*)(raw + (PAIR ? 2 : 1) * RAW_BYTES);
     // pair form: this CTA's rank in its pair (the even CTA issues the instructions) and the rows of the pair's tile it expands
     const uint32_t rank = PAIR ? cluster_rank() : 0u;
     const int my_rows = PAIR ? tile_n / 2 : tile_n;
@@ -332,7 +337,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         }
         for (int b = 0; b < NRAW; b++) {
             mbar_init(&sh->raw_full[b], 1);
-            mbar_init(&sh->raw_empty[b], (uint32_t)(NSETS * set_warps));
+            mbar_init(&sh->raw_empty[b], (uint32_t)(BYTE_ROWS ? set_warps : NSETS * set_warps));
         }
         mbar_init(&sh->acc_full, 1);
         sh->abort_flag = 0;
@@ -399,30 +404,31 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     } else if (warp == 18) {
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-            const uint32_t w_bytes = (uint32_t)(my_rows * RAW_ROW);
+            constexpr int COPIES = BYTE_ROWS ? 2 : 1, COPY_ROW = RAW_ROW / COPIES;  // copies of a super-block
+            const uint32_t w_bytes = (uint32_t)(my_rows * COPY_ROW);
             int w_issued = 0;
-            for (int sb = 0; sb < nsb; sb++) {
-                // the staging buffer is free once every dequant warp has taken its copy of super-block sb - 1,
-                // which they do at the start of that super-block: this copy runs a whole super-block ahead
-                const int rb = sb % NRAW;
-                if (!mbar_wait(&sh->raw_empty[rb], (uint32_t)(((sb / NRAW) & 1) ^ 1), sh, status, 8, (uint32_t)sb)) break;
+            for (int c = 0; c < nsb * COPIES; c++) {
+                // the staging buffer is free once every dequant warp that reads it has taken its copy of the one before,
+                // which they do at the start of a super-block: this copy runs a whole super-block ahead
+                const int rb = c % NRAW;
+                if (!mbar_wait(&sh->raw_empty[rb], (uint32_t)(((c / NRAW) & 1) ^ 1), sh, status, 8, (uint32_t)c)) break;
                 if (dbg & 2) {
                     mbar_arrive(&sh->raw_full[rb]);
                     continue;
                 }
                 mbar_arrive_expect_tx(&sh->raw_full[rb], w_bytes);
                 if constexpr (FMT == B2_FMT_Q6_K) {  // [rows][128] low nibbles, then [rows][64] high bit pairs
-                    tma_load_2d(raw, &tmap_w, &sh->raw_full[rb], (sb0 + sb) * 128, n0);
-                    tma_load_2d(raw + (size_t)my_rows * 128, y_more + n_more, &sh->raw_full[rb], (sb0 + sb) * 64, n0);
-                    w_issued = sb + 1;
+                    tma_load_2d(raw, &tmap_w, &sh->raw_full[rb], (sb0 + c) * 128, n0);
+                    tma_load_2d(raw + (size_t)my_rows * 128, y_more + n_more, &sh->raw_full[rb], (sb0 + c) * 64, n0);
+                    w_issued = c + 1;
                     continue;
                 }
-                tma_load_2d(raw + (size_t)rb * RAW_BYTES, &tmap_w, &sh->raw_full[rb], (sb0 + sb) * RAW_ROW, w_row0 + n0 + (int)rank * my_rows);
-                w_issued = sb + 1;
+                tma_load_2d(raw + (size_t)rb * RAW_STRIDE, &tmap_w, &sh->raw_full[rb], (sb0 * COPIES + c) * COPY_ROW, w_row0 + n0 + (int)rank * my_rows);
+                w_issued = c + 1;
             }
             if (sh->abort_flag)
-                for (int sb = max(0, w_issued - NRAW); sb < w_issued; sb++)
-                    mbar_wait(&sh->raw_full[sb % NRAW], (uint32_t)((sb / NRAW) & 1), sh, status, 9, (uint32_t)sb, false);
+                for (int c = max(0, w_issued - NRAW); c < w_issued; c++)
+                    mbar_wait(&sh->raw_full[c % NRAW], (uint32_t)((c / NRAW) & 1), sh, status, 9, (uint32_t)c, false);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -500,35 +506,39 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             const uint32_t b_full_even = PAIR ? cluster_addr(&sh->b_full[0], 0) : 0u;  // the even CTA's b_full[0]
             const uint32_t row_off = (uint32_t)(r + (is_lo ? 128 : 0)) * 128u;
             const uint32_t swz = (uint32_t)(r & 7);
-            const uint4* my_raw0 = (const uint4*)(raw + (size_t)(in_tile ? r : 0) * (FMT == B2_FMT_Q6_K ? 128 : RAW_ROW));
+            const uint4* my_raw0 = (const uint4*)(raw + (size_t)(in_tile ? r : 0) * (FMT == B2_FMT_Q6_K ? 128 : BYTE_ROWS ? 64 : RAW_ROW));
+            const uint32_t swh = (uint32_t)((r >> 1) & 3);  // the copy engine's swizzle of rows of 64 bytes
             // The scales that lie beside the packed rows come straight from global memory, a super-block ahead: this row's f16 d and eight i8
             // scales of this set's two stages (Q6_K), two f16 d (Q8_0), one f32 (FP8). Loaded where they are used they stand behind
-            // release_raw, which waits for the staged words: 512 x 4096 x 14336 in 69.9 us (Q6_K) and 66.6 (Q8_0), this way 61.9 and 60.8.
+            // release_raw, which waits for the staged words: 512 x 4096 x 14336 in 69.9 us (Q6_K) and 66.6 (Q8_0), this way 61.9 and 60.8 (58.8 with a
+            // staging buffer per set, see NRAW).
             const bool live = in_tile && n0 + r < n_out;
+            const size_t wrow = (size_t)(live ? n0 + r : 0);
+            const uint8_t* sc_row = (const uint8_t*)f8.s;
+            if constexpr (FMT == B2_FMT_Q6_K) sc_row += wrow * (size_t)(K / 16) + (size_t)sb0 * 16 + 4 * set;
+            if constexpr (FMT == B2_FMT_Q8_0) sc_row += (wrow * (size_t)f8.ncb + (size_t)sb0 * 4 + set * 2) * 2;
+            if constexpr (FMT == B2_FMT_F8E4M3) sc_row = f8.s ? sc_row + ((wrow + f8.row0) / f8.rows * f8.ncb + sb0) * 4 : nullptr;
+            const unsigned short* d_row = FMT == B2_FMT_Q6_K ? (const unsigned short*)f8.s2 + wrow * (size_t)(K / 256) + sb0 : nullptr;
             uint32_t next_scales[3] = {0u, 0u, 0u};
             auto load_scales = [&](int sb) {
                 if (!PRE_SCALED || !live || sb >= nsb) return;
-                const size_t wrow = (size_t)(n0 + r);
                 if constexpr (FMT == B2_FMT_Q6_K) {
-                    const uint32_t* sc = (const uint32_t*)((const int8_t*)f8.s + wrow * (size_t)(K / 16) + (size_t)(sb0 + sb) * 16);
-                    next_scales[0] = __ldg((const unsigned short*)f8.s2 + wrow * (size_t)(K / 256) + sb0 + sb);
-                    next_scales[1] = __ldg(sc + set);
-                    next_scales[2] = __ldg(sc + set + 2);
-                } else if constexpr (FMT == B2_FMT_Q8_0) {
-                    next_scales[0] = __ldg((const uint32_t*)((const unsigned short*)f8.s + wrow * (size_t)f8.ncb + (size_t)(sb0 + sb) * 4 + set * 2));
-                } else if (f8.s) {
-                    next_scales[0] = __float_as_uint(__ldg(f8.s + (size_t)((f8.row0 + n0 + r) / f8.rows) * f8.ncb + sb0 + sb));
+                    next_scales[0] = __ldg(d_row + sb);
+                    next_scales[1] = __ldg((const uint32_t*)(sc_row + (size_t)sb * 16));
+                    next_scales[2] = __ldg((const uint32_t*)(sc_row + (size_t)sb * 16 + 8));
+                } else if (FMT == B2_FMT_Q8_0 || sc_row) {
+                    next_scales[0] = __ldg((const uint32_t*)(sc_row + (size_t)sb * (FMT == B2_FMT_Q8_0 ? 8 : 4)));
                 }
             };
             load_scales(0);
             for (int sb = 0; sb < nsb && ok; sb++) {
                 const uint32_t scales[3] = {next_scales[0], next_scales[1], next_scales[2]};
                 load_scales(sb + 1);
-                const int rb = sb % NRAW;
-                const uint4* my_raw = (const uint4*)((const uint8_t*)my_raw0 + (size_t)rb * RAW_BYTES);
+                const int rb = BYTE_ROWS ? set : sb % NRAW;
+                const uint4* my_raw = (const uint4*)((const uint8_t*)my_raw0 + (size_t)rb * RAW_STRIDE);
                 // this row's packed super-block: staging buffer -> registers (only the two 64-groups this set
                 // expands), then release the buffer
-                if (!mbar_wait(&sh->raw_full[rb], (uint32_t)((sb / NRAW) & 1), sh, status, 10, (uint32_t)sb)) {
+                if (!mbar_wait(&sh->raw_full[rb], (uint32_t)((BYTE_ROWS ? sb : sb / NRAW) & 1), sh, status, 10, (uint32_t)sb)) {
                     ok = false;
                     break;
                 }
@@ -539,7 +549,6 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     // The staged tiles are swizzled by the copy engine: 16-byte chunk c of a ql row at c ^ (r & 7), of a qh row at
                     // c ^ ((r >> 1) & 3). w = f16(d sc pre) * (q - 32), q - 32 exact in f16.
                     const uint4* my_qh = (const uint4*)(raw + (size_t)my_rows * 128 + (size_t)(in_tile ? r : 0) * 64);
-                    const uint32_t swh = (uint32_t)((r >> 1) & 3);
                     const float d = __half2float(__ushort_as_half((unsigned short)scales[0]));
 #pragma unroll
                     for (int jj = 0; jj < 2; jj++) {
@@ -589,12 +598,12 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     continue;
                 }
                 if constexpr (BYTE_ROWS) {
-                    // 64 e4m3 bytes of this set's stage (the raw tile is 128-byte swizzled: chunk c of row r sits
-                    // at c ^ (r & 7)), the block scale of this row and k-block, then hardware e4m3x2 -> f16x2
+                    // 64 e4m3 bytes of this set's stage (the raw tile is 64-byte swizzled: chunk c of row r sits
+                    // at c ^ ((r >> 1) & 3)), the block scale of this row and k-block, then hardware e4m3x2 -> f16x2
                     // and one multiply by the scale per pair.
                     uint4 qb[4];
 #pragma unroll
-                    for (int c = 0; c < 4; c++) qb[c] = my_raw[((uint32_t)(4 * set + c)) ^ swz];
+                    for (int c = 0; c < 4; c++) qb[c] = my_raw[(uint32_t)c ^ swh];
                     release_raw(&sh->raw_empty[rb], qb[0].x | qb[1].x | qb[2].x | qb[3].x, zero, lane);
                     const int ks = sb * 2 + set;
                     const int s = ks % STAGES;
@@ -1151,14 +1160,15 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
     }
     {
         // the packed weights as a byte matrix [n_out][row_bytes]; one box = one super-block column of the tile
-        const bool f8 = w.fmt == B2_FMT_F8E4M3 || new_fmt;  // rows of bytes, 128 per copy, swizzled
+        // rows of bytes, swizzled: 128 per copy (Q6_K's nibbles) or 64 (FP8, Q8_0)
+        const bool f8 = w.fmt == B2_FMT_F8E4M3 || new_fmt;
         size_t row_bytes = w.fmt == B2_FMT_Q6_K ? w.n_in / 2 : f8 ? w.n_in : w.n_in / 256 * 144;
         cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)(w.n_out * experts)};
         cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-        cuuint32_t box[2] = {f8 ? 128u : 144u, (cuuint32_t)(p->pair ? p->tile_n / 2 : p->tile_n)};
+        cuuint32_t box[2] = {w.fmt == B2_FMT_Q6_K ? 128u : f8 ? 64u : 144u, (cuuint32_t)(p->pair ? p->tile_n / 2 : p->tile_n)};
         cuuint32_t estr[2] = {1, 1};
         CUresult r = enc(&p->tmap_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)w.p0, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         f8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                         w.fmt == B2_FMT_Q6_K ? CU_TENSOR_MAP_SWIZZLE_128B : f8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) {
             snprintf(err, errlen, "cuTensorMapEncodeTiled(w) failed with CUresult %d", (int)r);
             delete p;
