@@ -2,11 +2,11 @@
 // gemv_mma.cuh for the arithmetic and split.cuh for the activations.
 //
 // One CTA of 16 warps per SM. K is summed in eight slices (units of one or two blocks in turn, so that neighbouring warps read
-// neighbouring bytes); KS warps share a tile of 16 rows, each taking 8 / KS of the slices, and the 16 / KS groups of warps take tiles of
-// their own. Each warp keeps units of packed weights in flight in a ring of shared memory of its own (cp.async), filled before the
+// neighbouring bytes; fewer where there are fewer units), a warp each; the two groups of eight warps take tiles of 16 rows of their own.
+// Each warp keeps units of packed weights in flight in a ring of shared memory of its own (cp.async), filled before the
 // kernel waits for the one ahead of it in the stream. The slices' sums of a few tiles wait in shared memory and are then added, in the
-// order of the slices, by all threads of the group. Neither KS nor the number of tokens changes the order of a sum, so every row
-// equals its one-token row bit for bit, in a row shard too.
+// order of the slices, by all threads of the group. The number of tokens does not change the order of a sum, so every row equals its
+// one-token row bit for bit, in a row shard too.
 //
 // The activations come as f32 vectors and are split by the CTA itself (an RMS norm in front of the product runs in the same pass: the
 // weights multiply before the split, the factor multiplies the results), or as records that launch_split made. Where the split vectors
@@ -47,7 +47,7 @@ struct Args {
     size_t y_stride;
     const float* gate;     // token i's gate at gate + i * gate_stride
     size_t gate_stride;
-    int mode, T, ks, fast;
+    int mode, T, fast;
     int units, part_units;  // units of k in all, and in a part
     int blocks, bpu, slice_log, batch, bufs;  // blocks of the format, blocks per unit, log2 of the slices, tiles whose sums are added together, buffers for them
     int hold_tiles;
@@ -67,8 +67,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
     constexpr int ROWS = PAIR ? 8 : 16, S = F::SLOTS, BPX = 256 / F::BLOCK_K, NT = X::NT;  // BPX: blocks of the format per block of the split
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    // (uniform over the warp, and the compiler should know)
-    const int ks = a.ks, wq = __shfl_sync(0xffffffffu, warp, 0), group = wq / ks, q = wq - group * ks, groups = WARPS / ks;
+    const int sl_log = a.slice_log, slices = 1 << sl_log, bpu = a.bpu;
+    // (uniform over the warp, and the compiler should know) q: the warp's slice
+    const int wq = __shfl_sync(0xffffffffu, warp, 0), group = wq >> sl_log, q = wq & (slices - 1), groups = WARPS >> sl_log;
     const size_t n_out = a.w.n_out;
     const int tiles = (int)((n_out + ROWS - 1) / ROWS);
     // this group of warps: tiles tile0, tile0 + tile_step, ... below tile_end
@@ -85,11 +86,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
     }
     const int my_tiles = tile0 < tile_end ? (tile_end - tile0 + tile_step - 1) / tile_step : 0;
     // unit u, of `bpu` blocks, belongs to slice u % slices (a power of two)
-    const int sl_log = a.slice_log, slices = 1 << sl_log, bpu = a.bpu;
     const int parts = PARTS ? (a.units + a.part_units - 1) / a.part_units : 1;
-    auto j_at = [&](int s, int u) { return (u - s + slices - 1) >> sl_log; };  // a slice's units below u
-    auto j_beg = [&](int s, int p) { return PARTS ? j_at(s, p * a.part_units) : 0; };
-    auto j_end = [&](int s, int p) { return j_at(s, PARTS ? min(a.units, (p + 1) * a.part_units) : a.units); };
+    auto j_at = [&](int u) { return (u - q + slices - 1) >> sl_log; };  // the slice's units below u
+    auto j_beg = [&](int p) { return PARTS ? j_at(p * a.part_units) : 0; };
+    auto j_end = [&](int p) { return j_at(PARTS ? min(a.units, (p + 1) * a.part_units) : a.units); };
     const size_t last_row0 = n_out > 8 ? n_out - 8 : 0;
     auto tile_of = [&](int i) { return GROUPED ? (tile0 + i * tile_step) % tiles : tile0 + i * tile_step; };
     auto row_of = [&](int i, int half) { return min((size_t)tile_of(i) * ROWS + (PAIR ? 0 : 8 * half), last_row0); };
@@ -97,10 +97,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
     const uint32_t ring = smem0 + (uint32_t)wq * (S * F::UNIT_BYTES), ring_end = ring + S * F::UNIT_BYTES;
     uint32_t islot = ring, slot = ring;
 
-    // the copies run ahead of the arithmetic in the same order: parts, tiles, slices, units
+    // the copies run ahead of the arithmetic in the same order: parts, tiles, units
     typename F::template Copy<PAIR> cp;
     cp.init(a.w, bpu, lane);
-    int ip = 0, it = 0, is = q, ij = 0, ije = j_end(q, 0);
+    int ip = 0, it = 0, ij = 0, ije = j_end(0);
     bool more = my_tiles > 0 && q < a.units;
     auto copy_tile = [&](int i) {
         if constexpr (GROUPED) {
@@ -114,25 +114,21 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
         }
     };
     if (more) copy_tile(0);
-    auto next_run = [&] {  // the next slice of a tile, tile of a part, part
-        is += ks;
-        if (is >= slices) {
-            is = q;
-            if (++it == my_tiles) {
-                it = 0;
-                ip++;
-            }
-            copy_tile(it);
+    auto next_run = [&] {  // the next tile of a part, part
+        if (++it == my_tiles) {
+            it = 0;
+            ip++;
         }
+        copy_tile(it);
         more = ip < parts;
-        ij = j_beg(is, ip);
-        ije = j_end(is, ip);
+        ij = j_beg(ip);
+        ije = j_end(ip);
     };
     if (PARTS)
         while (more && ij >= ije) next_run();
     auto issue = [&] {
         if (more) {
-            const int b = (is + (ij << sl_log)) * bpu;
+            const int b = (q + (ij << sl_log)) * bpu;
             cp.issue(islot, b, b + 2 > a.blocks, lane);
             islot = islot + F::UNIT_BYTES == ring_end ? ring : islot + F::UNIT_BYTES;
             if (++ij >= ije) do next_run();
@@ -240,55 +236,53 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
         for (int i = batch0; i < i_end; i++) {
             float* cb = comb + (size_t)(buf * a.batch + in_batch) * slices * RES;
             const uint32_t tag = F::tag(a.w, a.w2, row_of(i, 0), row_of(i, 1), g);
-            for (int sl = q; sl < slices; sl += ks) {
-                float acc[NT][2];
-                float2* h = PARTS ? hold + ((size_t)((wq * a.hold_tiles + i) * (slices / ks) + sl / ks) * NT) * 32 + lane : nullptr;
+            float acc[NT][2];
+            float2* h = PARTS ? hold + (size_t)(wq * a.hold_tiles + i) * NT * 32 + lane : nullptr;
+#pragma unroll
+            for (int n = 0; n < NT; n++) {
+                float2 v = make_float2(0.0f, 0.0f);
+                if (PARTS && p > 0) v = h[n * 32];
+                acc[n][0] = v.x;
+                acc[n][1] = v.y;
+            }
+            const int b_part = PARTS ? p * a.part_units * bpu : 0, j1 = j_end(p);
+            for (int j = j_beg(p); j < j1; j++) {
+                cp_wait<S - 1>();
+                __syncwarp();
+                const int b = (q + (j << sl_log)) * bpu;
+                const int bn = min(bpu, a.blocks - b);
+                for (int k = 0; k < bn; k++) F::template block<TP>(slot + k * F::BLOCK_BYTES, b + k - b_part, ((b + k) & 1) ? ~tag : tag, a.w, a.w2, xv, g, t, acc);
+                __syncwarp();
+                issue();  // into the slot just used
+                slot = slot + F::UNIT_BYTES == ring_end ? ring : slot + F::UNIT_BYTES;
+            }
+            if (PARTS && p + 1 < parts) {
+#pragma unroll
+                for (int n = 0; n < NT; n++) h[n * 32] = make_float2(acc[n][0], acc[n][1]);
+            } else {
 #pragma unroll
                 for (int n = 0; n < NT; n++) {
-                    float2 v = make_float2(0.0f, 0.0f);
-                    if (PARTS && p > 0) v = h[n * 32];
-                    acc[n][0] = v.x;
-                    acc[n][1] = v.y;
-                }
-                const int b_part = PARTS ? p * a.part_units * bpu : 0, j1 = j_end(sl, p);
-                for (int j = j_beg(sl, p); j < j1; j++) {
-                    cp_wait<S - 1>();
-                    __syncwarp();
-                    const int b = (sl + (j << sl_log)) * bpu;
-                    const int bn = min(bpu, a.blocks - b);
-                    for (int k = 0; k < bn; k++) F::template block<TP>(slot + k * F::BLOCK_BYTES, b + k - b_part, ((b + k) & 1) ? ~tag : tag, a.w, a.w2, xv, g, t, acc);
-                    __syncwarp();
-                    issue();  // into the slot just used
-                    slot = slot + F::UNIT_BYTES == ring_end ? ring : slot + F::UNIT_BYTES;
-                }
-                if (PARTS && p + 1 < parts) {
-#pragma unroll
-                    for (int n = 0; n < NT; n++) h[n * 32] = make_float2(acc[n][0], acc[n][1]);
-                } else {
-#pragma unroll
-                    for (int n = 0; n < NT; n++) {
-                        float* cr = cb + sl * RES + n * 16 * X::PER;
-                        if constexpr (F::HALVES) {
-                            if (TP > 1) cr[g * 4 + t] = acc[n][0], cr[(g + 8) * 4 + t] = acc[n][1];
-                            else if (t == 0) cr[g] = acc[n][0], cr[g + 8] = acc[n][1];
-                        } else {  // a token's two lanes together; one keeps row g, the other row g + 8
-                            const float v0 = acc[n][0] + __shfl_xor_sync(0xffffffffu, acc[n][0], 1), v1 = acc[n][1] + __shfl_xor_sync(0xffffffffu, acc[n][1], 1);
-                            const float v = (t & 1) ? v1 : v0;
-                            const int row = g + 8 * (t & 1);
-                            if (TP > 1) cr[row * 2 + (t >> 1)] = v;
-                            else if (t < 2) cr[row] = v;
-                        }
+                    float* cr = cb + q * RES + n * 16 * X::PER;
+                    if constexpr (F::HALVES) {
+                        if (TP > 1) cr[g * 4 + t] = acc[n][0], cr[(g + 8) * 4 + t] = acc[n][1];
+                        else if (t == 0) cr[g] = acc[n][0], cr[g + 8] = acc[n][1];
+                    } else {  // a token's two lanes together; one keeps row g, the other row g + 8
+                        const float v0 = acc[n][0] + __shfl_xor_sync(0xffffffffu, acc[n][0], 1), v1 = acc[n][1] + __shfl_xor_sync(0xffffffffu, acc[n][1], 1);
+                        const float v = (t & 1) ? v1 : v0;
+                        const int row = g + 8 * (t & 1);
+                        if (TP > 1) cr[row * 2 + (t >> 1)] = v;
+                        else if (t < 2) cr[row] = v;
                     }
                 }
             }
             if (PARTS && p + 1 < parts) continue;
             if (++in_batch < a.batch && i + 1 < i_end) continue;
-            if (ks == 1) __syncwarp();
-            else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(ks * 32) : "memory");
+            if (slices == 1) __syncwarp();
+            else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(slices * 32) : "memory");
             // one thread per result (per pair of results in the pair form): the sums in the order of the slices
             constexpr int PER = PAIR ? 8 : 16;
             const float* c0 = comb + (size_t)buf * a.batch * slices * RES;
-            for (int e = q * 32 + lane; e < in_batch * PER * T; e += ks * 32) {
+            for (int e = q * 32 + lane; e < in_batch * PER * T; e += slices * 32) {
                 const int r = e % PER, et = e / PER, token = et % T, tl = et / T;
                 const size_t first = (size_t)tile_of(batch0 + tl) * ROWS + (r & 8), row = row_of(batch0 + tl, r >> 3) + (r & 7);
                 if (row < first || row >= n_out) continue;  // (the last tile's halves overlap the rows before them)
@@ -314,8 +308,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
             batch0 = i + 1;
             in_batch = 0;
             if (a.bufs == 2) buf ^= 1;
-            else if (ks == 1) __syncwarp();
-            else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(ks * 32) : "memory");
+            else if (slices == 1) __syncwarp();
+            else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(slices * 32) : "memory");
         }
         tile_at = i_end;
     }
@@ -328,15 +322,14 @@ cudaError_t launch_t(Args& a, int sm_count, cudaStream_t st, bool pdl, const Gem
     constexpr int ROWS = PAIR ? 8 : 16, BPX = 256 / F::BLOCK_K, NT = X::NT, RES = X::RES;
     a.blocks = (int)((a.w.n_in + F::BLOCK_K - 1) / F::BLOCK_K);
     // The order of a row's sum depends on K alone (a row shard has other tiles): eight slices, or as many as there are units, of units
-    // of two blocks where that leaves a unit per slice. How many warps share a tile does not change it.
+    // of two blocks where that leaves a unit per slice.
     a.bpu = a.blocks >= 8 * F::MAX_BLOCKS ? F::MAX_BLOCKS : 1;
     a.units = (a.blocks + a.bpu - 1) / a.bpu;
     a.slice_log = 3;
     while ((1 << a.slice_log) > a.units) a.slice_log--;
     const int slices = 1 << a.slice_log;
     const size_t tiles = (a.w.n_out + ROWS - 1) / ROWS;
-    a.ks = slices;
-    const int groups = WARPS / a.ks;
+    const int groups = WARPS / slices;
     const int span = std::max(slices, BPX), xblocks = (a.blocks + BPX - 1) / BPX;
     // the sums of a few tiles wait for one barrier: 8 KB of them, twice, over all groups
     a.batch = std::max(1, std::min(8, 8192 / (groups * slices * RES * 4)));
@@ -354,7 +347,7 @@ cudaError_t launch_t(Args& a, int sm_count, cudaStream_t st, bool pdl, const Gem
         fixed += comb;
         // parts of whole rounds of the slices where one fits, else of as many units as fit
         size_t step = (size_t)std::max(1, span * a.bpu / BPX);  // in blocks of the split
-        const size_t least = (size_t)std::max(1, a.bpu / BPX), per_tile = (size_t)WARPS * (slices / a.ks) * NT * 256;
+        const size_t least = (size_t)std::max(1, a.bpu / BPX), per_tile = (size_t)WARPS * NT * 256;
         if (fixed + per_tile + least * per_block > SMEM_MAX) return cudaErrorInvalidValue;
         // The waiting sums may take the room that a round leaves; a group that has more tiles than that goes in several waves of CTAs.
         const size_t room = SMEM_MAX - fixed - (fixed + per_tile + step * per_block <= SMEM_MAX ? step : least) * per_block;
