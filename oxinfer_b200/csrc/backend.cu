@@ -503,13 +503,17 @@ class Backend {
         if (e != cudaSuccess) return cuda_fail(e, "activation split");
         return B2_OK;
     }
-    // t tokens of one matrix from their records, up to eight per launch (the weights are read once per launch). A matrix whose tiles
-    // fill no more than half the SMs goes four at a time: the launches run side by side, and a launch of four has half the arithmetic.
-    // So does one that has more tiles than the SMs have groups of warps, unless the activations of eight fit whole: the parts of K then
-    // pass over several tiles each. Q4_K 28672 x 4096, 8 tokens: 161 us in one launch, 63 in two; 4096 x 14336: 48 and 63.
+    // t tokens of one matrix from their records, up to eight per launch (the weights are read once per launch). A matrix that has more
+    // tiles than the SMs have groups of warps goes four at a time, unless the activations of eight fit whole: the parts of K pass over
+    // several tiles each, and their sums through shared memory, one part at a time for eight. Eight tokens in one launch and in two:
+    // Q4_K 14336 x 4096 42 and 30 us, 28672 x 4096 136 and 47; Q8_0 48 and 32, 83 and 51. (4096 x 14336 has fewer tiles than that: one launch, 41 and 42 us.)
+    // The second launch waits for the first, so a matrix whose tiles fill no more than half of the SMs gains nothing by it: Q8_0
+    // 1024 x 2048 10.1 us in two launches, 7.8 in one; FP8 512 x 4096 11.5 and 10.1. Seven or eight tokens of Q6_K do (512 x 4096 12.7
+    // and 13.8), and the 4-bit formats keep a launch per four rows there, as their callers count them (1024 x 4096 12.3 and 12.2).
     int small_products(const WeightDev& w, const WeightDev* up, const uint8_t* rec, size_t t, float* y, int mode) {
         const size_t stride = record_stride(w.n_in, gemv_mma_halves(w)), tiles = (w.n_out + 15) / 16;
-        const size_t per = 2 * tiles <= (size_t)sm_count || (tiles > 2 * (size_t)sm_count && w.n_in > GEMV_WHOLE_8) ? 4 : 8;
+        const bool narrow = 2 * tiles <= (size_t)sm_count && (w.fmt == B2_FMT_Q4_K || w.fmt == B2_FMT_MLX4 || (w.fmt == B2_FMT_Q6_K && t > 6));
+        const size_t per = narrow || (tiles > 2 * (size_t)sm_count && w.n_in > GEMV_WHOLE_8) ? 4 : 8;
         for (size_t i = 0; i < t; i += per) {
             GemvIn in;
             in.rec = rec + i * stride;
