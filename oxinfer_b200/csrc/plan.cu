@@ -104,7 +104,8 @@ cudaError_t fuse_rows(const std::vector<const WeightDev*>& parts, WeightDev* out
         out->p1 = d;
         out->bs_row0 = 0;
     }
-    return cudaSuccess;
+    // (a copy within the device does not wait for itself, and products fetch weights before they wait for the work ahead)
+    return cudaStreamSynchronize(cudaStreamLegacy);
 }
 
 }  // namespace
