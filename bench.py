@@ -177,7 +177,7 @@ def gemv_extras(be, torch, peaks, steps, only=None, use_graph=True):
             be.matvec_dev(devs[i % copies], x, y)
         torch.cuda.synchronize()
         # One GEMV is a few microseconds, less than a host launch: time a CUDA graph of n back-to-back
-        # GEMVs (each with its activation-plane kernel) over the rotating weight copies.
+        # GEMVs over the rotating weight copies.
         n = max(steps, 2 * copies)
         graph, timing = torch.cuda.CUDAGraph(), "cuda graph"
         main_stream = torch.cuda.current_stream().cuda_stream
@@ -208,9 +208,9 @@ def gemv_extras(be, torch, peaks, steps, only=None, use_graph=True):
         us = ev[0].elapsed_time(ev[1]) * 1e3 / (n * reps)
         algo = wbytes + 4 * n_in + 4 * n_out
         out[name] = {"us_per_gemv": us, "bytes": algo, "gbs": algo / us / 1e3, "frac_of_hbm_peak": algo / us / 1e3 / peaks["hbm_gbs"],
-                     "launches_per_gemv": 1 if fmt == "f8_e4m3" else 2, "timing": timing}
+                     "launches_per_gemv": 1, "timing": timing}
         traffic, commit = profiled_traffic(f"gemv_{name}.txt")
-        out[name]["roofline"] = {"kernel": "gemv_f8_mma_kernel" if fmt == "f8_e4m3" else "xplanes_kernel + gemv_kernel (one matrix-vector product)",
+        out[name]["roofline"] = {"kernel": "gemv_mma_kernel (one matrix-vector product)",
                                  "bound": "hbm", "achieved": algo / us / 1e3, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                                  "frac": algo / us / 1e3 / peaks["hbm_gbs"], "frac_of_nominal_8000": algo / us / 1e3 / 8000.0, "traffic": traffic,
                                  "traffic_unit": f"bytes per product, from profiles/gemv_{name}.txt" + (f" captured at {commit}" if commit else ""),
@@ -249,8 +249,7 @@ def gemv_extras(be, torch, peaks, steps, only=None, use_graph=True):
                                              "path": O.decode_kernel_name()}
             except Exception as e:
                 out[name]["cpu_baseline_error"] = str(e)
-        # The GEMV kernel alone, over planes prepared once (what a decode plan sees when one vector feeds
-        # several products): a second graph with n GEMV launches and no plane kernels.
+        # The same over a vector prepared once (the form for one vector that feeds several products): a second graph.
         if use_graph and fmt != "f8_e4m3":
             try:
                 be.prepare_x_dev(x)
@@ -270,8 +269,7 @@ def gemv_extras(be, torch, peaks, steps, only=None, use_graph=True):
                 us2 = ev[0].elapsed_time(ev[1]) * 1e3 / (n * 5)
                 out[name].update({"us_kernel_only": us2, "gbs_kernel_only": algo / us2 / 1e3,
                                   "frac_kernel_only": algo / us2 / 1e3 / peaks["hbm_gbs"]})
-                # the same as a dependent-launch chain (how a decode step queues its products): every kernel may start while
-                # the one ahead drains, and the 4-bit kernels fetch their first weights before they wait for it
+                # and with b2_set_chained, which asks dependent launches of every kernel (these products have them anyway)
                 be.set_chained(True)
                 g3 = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g3):

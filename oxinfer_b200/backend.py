@@ -356,11 +356,11 @@ class Backend:
         return self._check(self._L.b2_moe_ep(self._ctx, dev.handle, n_experts_global, _ptr(x), t, _ptr(ids), _ptr(w), k, _ptr(y)))
 
     def prepare_x_dev(self, x) -> bool:
-        """Splits a device vector into the integer planes the GEMV kernels read (once per vector)."""
+        """Keeps a copy of a device vector for the products that ``matvec_prepared_dev`` makes of it."""
         return self._check(self._L.b2_prepare_x_dev(self._ctx, _ptr(x), x.numel()))
 
     def matvec_prepared_dev(self, dev: DeviceWeight, x, y, mode: int = MODE_STORE, up: DeviceWeight | None = None, gate=None) -> bool:
-        """One product over the planes prepared last by ``prepare_x_dev`` (same vector length)."""
+        """One product over the vector prepared last by ``prepare_x_dev`` (same length)."""
         return self._check(self._L.b2_matvec_prepared_dev(self._ctx, dev.handle, up.handle if up else 0, _ptr(x), _ptr(y), mode,
                                                           _ptr(gate) if gate is not None else None))
 

@@ -1,5 +1,5 @@
 // The other GGUF block formats on the device (dq_other.cuh): bit-exact dequantization, and one generic matrix-vector
-// kernel that decodes 32 weights at a time in registers and multiplies them with the f32 activations (no integer planes,
+// kernel that decodes 32 weights at a time in registers and multiplies them with the f32 activations (no split of the vector,
 // no repack: the rows stay as they are in the GGUF file). It takes the five output modes of dmv_out
 // (src/cuda_decode.cu:131-137), the SiLU / GELU pair, and up to four tokens per launch with the weights read once (each
 // token's row equals its one-token row bit for bit). The reference declines every GGUF type on its CUDA backend
@@ -211,7 +211,7 @@ cudaError_t launch_dequantize_other(const WeightDev& w, size_t r0, size_t nrows,
 cudaError_t launch_gemv_other(const WeightDev& w, const WeightDev* up, const float* x, size_t x_stride, float* y, size_t y_stride, int nt, int mode,
                               const float* gate, int sm_count, cudaStream_t st, bool pdl) {
     if (!gemv_other_supports(w) || nt < 1 || nt > 4) return cudaErrorInvalidValue;
-    // Rows of whole 256-value runs go to the integer tensor cores: Q5_K 14336 x 4096 11.7 us there, 39 here.
+    // Rows of whole 256-value runs go to the integer tensor cores, always as dependent launches: Q5_K 14336 x 4096 11.7 us there, 39 here.
     if (gemv_mma_other_tokens(w)) return launch_gemv_mma_other(w, up, x, x_stride, y, y_stride, nt, mode, gate, sm_count, st);
     if (nt > 1 && w.n_in * 4 * (size_t)nt > 160 * 1024) {  // the vectors of nt tokens do not fit together: fewer per launch
         const int half = nt / 2;

@@ -28,7 +28,7 @@ inline cudaError_t ensure_dynamic_smem(const void* kern, size_t bytes, size_t df
 }
 
 // Launch with or without the programmatic-dependent-launch attribute. With it the kernel may begin while the
-// kernel ahead of it in the stream is still running; every kernel launched this way calls pdl_wait() (xplanes.cuh)
+// kernel ahead of it in the stream is still running; every kernel launched this way calls pdl_wait() (pdl.cuh)
 // before it reads what that kernel wrote or writes anything.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, Args... args) {
@@ -242,7 +242,7 @@ struct FusedRope {
     DecRope r;
 };
 // Several tokens of a step in one launch (only without FusedRope: every token's key and value must be in the caches
-// already): token i's queries / outputs act_stride floats behind token 0's, its planes planes_stride bytes, its partials
+// already): token i's queries / outputs act_stride floats behind token 0's, its partials
 // part_stride floats, its counters nkv words, its step words 4 words.
 struct AttnTokens {
     int n;  // 0 or 1: one token

@@ -64,7 +64,7 @@ __device__ __forceinline__ void split_values(const SplitIn& in, float pre, float
 
 template <int DIGITS>
 struct SplitDigits {
-    uint32_t d[2][DIGITS];  // a lane's four digits of each plane, for either half of the block
+    uint32_t d[2][DIGITS];  // of each digit, a lane's four bytes for either half of the block
     int s[2];          // sums of q over chunks lane / 8 and 4 + lane / 8
     float xs, ssq;
 };
@@ -107,7 +107,7 @@ __device__ __forceinline__ SplitDigits<DIGITS> split_digits(const SplitIn& in, f
     }
     return r;
 }
-// Where a lane's digits go in the block's record: half h at split_digit_at(h, lane) + plane * plane_bytes (64 in the record).
+// Where a lane's digits go in the block's record: half h at split_digit_at(h, lane) + 64 * digit.
 __device__ __forceinline__ void split_digit_at(int h, int lane, int& pair, int& in16) {
     const int chunk = 4 * h + (lane >> 3);
     pair = chunk >> 1;
