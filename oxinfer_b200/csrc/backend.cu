@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "dq_other.cuh"
+#include "gemm_wt.h"
 #include "kernels.h"
 #include "nccl_dyn.h"
 #include "plan.h"
@@ -635,7 +636,7 @@ class Backend {
                 plans.clear();
             }
             char msg[256] = {0};
-            e = gemm_tc_plan_create(w->dev, xh, t, y, y_dtype, &plan, msg, sizeof msg, 1, nullptr, lo_row0 ? 1 : 0, lo_row0, w_terms, peer_y);
+            e = gemm_tc_plan_create(w->dev, xh, t, y, y_dtype, &plan, msg, sizeof msg, lo_row0 ? 1 : 0, lo_row0, w_terms, peer_y);
             if (e != cudaSuccess) return fail(B2_ERR_CUDA, "[b200qmm: %s]", msg);
             plans.push_back(plan);
         }
@@ -880,21 +881,19 @@ class Backend {
         return B2_OK;
     }
 
-    // One grouped GEMM: rows of xg (f16, segments of whole 128-row tiles per expert) times the stacked matrices.
-    int grouped_gemm(int fmt, const void* stacked, size_t experts, size_t n_out, size_t n_in, const void* xg, size_t rows, const int* tile_expert,
-                     float* out_dev, int m_halves, const float* row_unscale, size_t a_lo_row0) {
+    // One grouped GEMM: the rows of xg (f16, expert by expert, the second terms lo_row0 rows below) times the stacked matrices.
+    int grouped_gemm(int fmt, const void* stacked, size_t experts, size_t n_out, size_t n_in, const void* xg, size_t rows, size_t longest, const WtTile* tiles,
+                     size_t n_tiles, float* out_dev, const float* row_unscale, size_t lo_row0) {
         WeightDev w{};
         w.fmt = fmt;
         w.n_out = n_out;
         w.n_in = n_in;
         w.p0 = (const uint8_t*)stacked;
-        GemmPlan* plan = nullptr;
-        char msg[256] = {0};
-        cudaError_t e = gemm_tc_plan_create(w, xg, rows, out_dev, B2_F32, &plan, msg, sizeof msg, experts, tile_expert, m_halves, a_lo_row0, a_lo_row0 ? 2 : 1);
-        if (e != cudaSuccess) return fail(B2_ERR_CUDA, "[b200qmm: %s]", msg);
-        e = launch_gemm_tc(plan, w, rows, out_dev, B2_F32, gemm_status, sm_count, stream, row_unscale);
+        GemmWt g;
+        if (!gemm_wt_encode(&g, w, experts, xg, lo_row0 ? lo_row0 + rows : rows, longest, lo_row0 ? 2 : 1, lo_row0, lo_row0 && fmt == B2_FMT_Q4_K, true))
+            return fail(B2_ERR_CUDA, "[b200qmm: the tensor maps of a grouped product could not be made]");
+        cudaError_t e = launch_gemm_wt(g, w, rows, tiles, (int)n_tiles, out_dev, B2_F32, n_out, nullptr, 0, gemm_status, row_unscale, stream);
         launches++;
-        gemm_tc_plan_destroy(plan);  // the tensor maps were copied into the launch's parameters
         if (e != cudaSuccess) return cuda_fail(e, "grouped gemm");
         return B2_OK;
     }
@@ -1000,12 +999,6 @@ class Backend {
         return B2_OK;
     }
 
-    static size_t rows_for(const std::vector<size_t>& count, size_t tile) {
-        size_t rows = 0;
-        for (size_t c : count) rows += (c + tile - 1) / tile * tile;
-        return rows;
-    }
-
     // layer_pairs: the pairs of the layer that this call computes a part of (0: all of it).
     int moe_dev(uint64_t handle, const float* x_dev_, size_t t, const int32_t* ids, const float* rw, size_t k, float* y_dev_, size_t layer_pairs = 0) {
         auto it = moes.find(handle);
@@ -1023,76 +1016,58 @@ class Backend {
         // (the clamped SiLU has no fused pair mode in the matrix-vector kernels: those layers take the GEMM path at any batch)
         if (std::max(t * k, layer_pairs) <= GEMV_GROUP_ROWS && m.act != B2_ACT_SILU_CLAMP && !getenv("B2_MOE_NO_GEMV"))
             return moe_small(m, x_dev_, t, ids, rw, k, y_dev_, count);
-        // Token tiles of 128 or 256 rows. A tile costs about the same either way (the kernel is bound by the expansion of
-        // the tile's weights, which both heights share), so the taller tile wins as soon as it needs clearly fewer tiles:
-        // large batches, where the experts hold more than a tile's worth of tokens each.
-        size_t tiles128 = 0, tiles256 = 0;
-        for (size_t e = 0; e < m.experts; e++) {
-            tiles128 += (count[e] + 127) / 128;
-            tiles256 += (count[e] + 255) / 256;
-        }
-        static const int force_tile = [] {
-            const char* e = getenv("B2_MOE_TILE");
-            return e ? atoi(e) : 0;
-        }();
-        // Two-term operands (activations of both projections as two f16 terms, Q4_K weights as two f16 terms) need the
-        // 128-row tile. Q4_K experts always take them: Q4_K values round harder to f16 than MLX-4's, and one-term operands
-        // through two chained projections leave that layer above 1e-3 per output row (MLX-4 stays near 3e-4 with one term).
+        // The pairs' rows lie expert by expert without padding; a token tile is up to 128 rows of one expert, and an expert's tiles are
+        // about equally long. Long tiles come first: the short ones then fill the gaps that they leave at the end of the launch.
+        // Two-term operands (activations of both projections as two f16 terms, Q4_K weights as two f16 terms): Q4_K experts always
+        // take them. Q4_K values round harder to f16 than MLX-4's, and one-term operands through two chained projections leave that
+        // layer above 1e-3 per output row (MLX-4 stays near 3e-4 with one term).
         const bool two_term = m.fmt == B2_FMT_Q4_K || exact;
-        const size_t TILE = two_term ? 128
-                            : force_tile == 128 || force_tile == 256 ? (size_t)force_tile
-                            : tiles256 * 10 <= tiles128 * 8 ? 256 : 128;
-        const int m_halves = (int)(TILE / 128);
-        const size_t lo_row0 = two_term ? rows_for(count, 128) : 0;
-        std::vector<size_t> off(m.experts, 0);
-        std::vector<int32_t> tile_expert;
-        size_t rows = 0;
-        const size_t terms = lo_row0 ? 2 : 1;
-        for (size_t e = 0; e < m.experts; e++) {
-            off[e] = rows;
-            size_t tiles = (count[e] + TILE - 1) / TILE;
-            for (size_t i = 0; i < tiles; i++) tile_expert.push_back((int32_t)e);
-            rows += tiles * TILE;
+        const size_t rows = t * k, terms = two_term ? 2 : 1, lo_row0 = two_term ? rows : 0;
+        std::vector<size_t> at(m.experts, 0);
+        std::vector<WtTile> tiles;
+        size_t longest = 0;
+        for (size_t e = 0, row = 0; e < m.experts; e++) {
+            at[e] = row;
+            const size_t n = (count[e] + 127) / 128, size = n ? ((count[e] + n - 1) / n + 15) / 16 * 16 : 0;
+            for (size_t c = 0; c < count[e]; c += size)
+                tiles.push_back(WtTile{(int)e, (int)(row + c), (int)std::min(size, count[e] - c), 0});
+            longest = std::max(longest, std::min(size, count[e]));
+            row += count[e];
         }
-        std::vector<int32_t> src(rows, -1), slots(t * k);
-        std::vector<size_t> fill(m.experts, 0);
-        for (size_t i = 0; i < t; i++)
-            for (size_t j = 0; j < k; j++) {
-                size_t e = (size_t)ids[i * k + j];
-                size_t r = off[e] + fill[e]++;
-                src[r] = (int32_t)i;
-                slots[i * k + j] = (int32_t)r;
-            }
-        // index block on the device: src | slots | tile_expert | route weights
-        const size_t n_idx = rows + t * k + tile_expert.size();
-        cudaError_t e = moe_idx.reserve(n_idx * 4 + t * k * 4);
+        std::stable_sort(tiles.begin(), tiles.end(), [](const WtTile& a, const WtTile& b) { return a.count > b.count; });
+        // index block on the device: tiles | src | slots | route weights
+        const size_t n_idx = tiles.size() * 4 + 3 * rows;
+        cudaError_t e = moe_idx.reserve(n_idx * 4);
         if (e == cudaSuccess) e = moe_xg.reserve(terms * rows * m.h * 2 + rows * 4);
         if (e == cudaSuccess) e = moe_g.reserve(rows * 2 * m.inter * 4);
         if (e == cudaSuccess) e = moe_a.reserve(terms * rows * m.inter * 2 + rows * 4);
         if (e == cudaSuccess) e = moe_o.reserve(rows * m.h * 4);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(moe scratch)");
-        int32_t* d_src = (int32_t*)moe_idx.p;
-        int32_t* d_slots = d_src + rows;
-        int32_t* d_tiles = d_slots + t * k;
-        float* d_w = (float*)(d_tiles + tile_expert.size());
         std::vector<int32_t> host(n_idx);
-        std::memcpy(host.data(), src.data(), rows * 4);
-        std::memcpy(host.data() + rows, slots.data(), t * k * 4);
-        std::memcpy(host.data() + rows + t * k, tile_expert.data(), tile_expert.size() * 4);
-        e = cudaMemcpyAsync(d_src, host.data(), n_idx * 4, cudaMemcpyHostToDevice, stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(d_w, rw, t * k * 4, cudaMemcpyHostToDevice, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);  // the host vectors go out of scope
+        std::memcpy(host.data(), tiles.data(), tiles.size() * sizeof(WtTile));
+        int32_t *src = host.data() + tiles.size() * 4, *slots = src + rows;
+        for (size_t i = 0; i < rows; i++) {
+            const size_t r = at[(size_t)ids[i]]++;
+            src[r] = (int32_t)(i / k);
+            slots[i] = (int32_t)r;
+        }
+        std::memcpy(slots + rows, rw, rows * 4);
+        const WtTile* d_tiles = (const WtTile*)moe_idx.p;
+        const int32_t *d_src = (const int32_t*)moe_idx.p + tiles.size() * 4, *d_slots = d_src + rows;
+        const float* d_w = (const float*)(d_slots + rows);
+        e = cudaMemcpyAsync(moe_idx.p, host.data(), n_idx * 4, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);  // the host vector goes out of scope
         if (e != cudaSuccess) return cuda_fail(e, "moe index upload");
         float* x_unscale = (float*)((uint8_t*)moe_xg.p + terms * rows * m.h * 2);
         float* a_unscale = (float*)((uint8_t*)moe_a.p + terms * rows * m.inter * 2);
         e = launch_moe_gather(x_dev_, d_src, rows, m.h, moe_xg.p, x_unscale, lo_row0, stream);
         launches++;
         if (e != cudaSuccess) return cuda_fail(e, "moe_gather");
-        if ((rc = grouped_gemm(m.fmt, m.gate_up, m.experts, 2 * m.inter, m.h, moe_xg.p, rows, d_tiles, (float*)moe_g.p, m_halves, x_unscale, lo_row0))) return rc;
-        e = launch_moe_act((const float*)moe_g.p, d_src, rows, m.inter, moe_a.p, a_unscale, lo_row0, stream, m.act, m.act_limit);
+        if ((rc = grouped_gemm(m.fmt, m.gate_up, m.experts, 2 * m.inter, m.h, moe_xg.p, rows, longest, d_tiles, tiles.size(), (float*)moe_g.p, x_unscale, lo_row0))) return rc;
+        e = launch_moe_act((const float*)moe_g.p, rows, m.inter, moe_a.p, a_unscale, lo_row0, stream, m.act, m.act_limit);
         launches++;
         if (e != cudaSuccess) return cuda_fail(e, "moe_act");
-        if ((rc = grouped_gemm(m.fmt, m.down, m.experts, m.h, m.inter, moe_a.p, rows, d_tiles, (float*)moe_o.p, m_halves, a_unscale, lo_row0))) return rc;
+        if ((rc = grouped_gemm(m.fmt, m.down, m.experts, m.h, m.inter, moe_a.p, rows, longest, d_tiles, tiles.size(), (float*)moe_o.p, a_unscale, lo_row0))) return rc;
         e = launch_moe_combine((const float*)moe_o.p, d_slots, d_w, t, k, m.h, y_dev_, stream);
         launches++;
         if (e != cudaSuccess) return cuda_fail(e, "moe_combine");

@@ -38,7 +38,9 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "gemm_wt.h"
 #include "kernels.h"
+#include "tcgen05.cuh"
 
 namespace b2 {
 
@@ -51,7 +53,6 @@ constexpr int A_STAGE_BYTES = 256 * 128;   // up to 256 tokens
 constexpr int B_STAGE_BYTES = MAX_TILE_N * 128;
 constexpr int RAW_BYTES = MAX_TILE_N * 144;  // one super-block column of the weight tile, packed
 constexpr int GEMM_THREADS = 608;          // activation producer, MMA issuer, 16 dequant / epilogue warps, weight producer
-constexpr long long WAIT_LIMIT_CYCLES = 4000000000ll;  // about two seconds of SM clock
 
 struct F8Scales {  // block scales of an FP8 matrix (formats.cuh); s == nullptr for the 4-bit formats.
                    // Q8_0: s = the f16 block scales [n_out][ncb]. Q6_K: s = the i8 scales [n_out][K / 16], s2 = the f16 d [n_out][K / 256].
@@ -89,160 +90,6 @@ static_assert(GEMM_SMEM <= 227 * 1024, "shared memory budget");
 constexpr size_t PAIR_SMEM = 1024 + (size_t)PAIR_STAGES * (A_STAGE_BYTES + PAIR_B_STAGE_BYTES) + 2 * PAIR_RAW_BYTES + sizeof(Shared);
 static_assert(PAIR_SMEM <= 227 * 1024, "shared memory budget (pair form)");
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// The same test with acquire semantics at cluster scope: for barriers that a peer CTA's threads or copies complete.
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// The address, in the cluster's shared window, of the CTA of rank `cta`'s copy of a shared-memory object of this CTA.
-__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t cta) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(cta));
-    return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {  // every thread of both CTAs
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Bounded wait. Returns false when the CTA is aborting or the limit passed (in which case it records
-// `where` and raises the abort flag). `heed_abort` = false is for the teardown waits. The limit is
-// counted on the SM's own cycle counter (a cheap register read; the global nanosecond timer costs
-// about a microsecond per read, as long as a whole pipeline stage).
-template <bool CLUSTER = false>
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, Shared* sh, GemmStatus* status, uint32_t where, uint32_t iter,
-                                          bool heed_abort = true) {
-    auto test = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
-    if (test()) return true;
-    const long long t0 = clock64();
-    for (uint32_t spin = 1;; spin++) {
-        if (test()) return true;
-        if ((spin & 255) == 0) {
-            if (heed_abort && sh->abort_flag) return false;
-            if (clock64() - t0 > WAIT_LIMIT_CYCLES) {
-                if (atomicCAS(&status->code, 0u, 1u) == 0u) {
-                    status->where = where;
-                    status->cta = blockIdx.x + gridDim.x * blockIdx.y;
-                    status->iter = iter;
-                }
-                sh->abort_flag = 1;
-                return false;
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-        "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
-        : "memory");
-}
-
-// The copy of a CTA pair: the data lands in this CTA's shared memory, the bytes are counted on the barrier at the cluster
-// address `cluster_bar` (the even CTA's: its MMA thread waits for both CTAs' tiles on one barrier).
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-        "l"(map), "r"(cluster_bar), "r"(x), "r"(y)
-        : "memory");
-}
-
-// K-major operand tile, 128-byte swizzle, rows 128 bytes apart, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFF);         // start address
-    d |= (uint64_t)1 << 16;                        // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;              // stride byte offset: 8 rows * 128 B
-    d |= (uint64_t)1 << 46;                        // descriptor version (Blackwell)
-    d |= (uint64_t)2 << 61;                        // SWIZZLE_128B
-    return d;
-}
-
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// M = 256 over a CTA pair: A rows 0..127 and B rows 0..N/2-1 from the even CTA's shared memory, the rest from the odd CTA's
-// (same offsets in both), accumulator rows 0..127 in the even CTA's tensor memory, 128..255 in the odd CTA's.
-__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Arrives, when the pair's instructions issued so far have completed, on the barrier at cluster address `cluster_bar`
-// (issued once per CTA of the pair: each CTA's producers and epilogue wait on their own copy of the barrier).
-__device__ __forceinline__ void mma_commit_pair(uint32_t cluster_bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar) : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Gives a staging buffer of packed weights back to the copy engine once the warp's loads from it have landed in registers. The
-// loads have only been issued when the warp gets here, and with the tensor cores reading shared memory at most of its rate they
-// can stay queued for longer than the next copy takes to arrive: an arrival that did not wait for them let that copy overwrite
-// words that were still to be read (a few weight rows of a tile then came from the next super-block). So the arrival takes an
-// operand that every lane's loaded words enter: `words` is an OR over them, `zero` a kernel argument that is always 0.
-__device__ __forceinline__ void release_raw(uint64_t* bar, uint32_t words, int zero, int lane) {
-    const uint32_t off = __reduce_or_sync(0xffffffffu, words) & (uint32_t)zero;
-    if (lane == 0) asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar) + off) : "memory");
-}
-
-__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-
 // TT: the instantiation that takes two-term operands (a_lo_row_arg, w_terms); the one-term kernel carries none of that code.
 // PAIR: the CTA-pair form (4-bit formats, one-term operands, no K split, dense launches of an even number of 256-token
 // tiles): launched as clusters of two CTAs along x = the token tiles; tile_n is then the pair's tile width.
@@ -251,7 +98,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                    const __grid_constant__ CUtensorMap tmap_y, int K, int n_out, int t,
                    int tile_n, int m_halves, void* __restrict__ y, int y_dtype_arg, GemmStatus* __restrict__ status, int dbg_arg, int zero,
-                   const int* __restrict__ tile_expert, F8Scales f8, int k_splits, const float* __restrict__ row_unscale, int a_lo_row_arg, int w_terms,
+                   F8Scales f8, int k_splits, const float* __restrict__ row_unscale, int a_lo_row_arg, int w_terms,
                    const CUtensorMap* __restrict__ y_more, int n_more) {
     // y_more[0 .. n_more): tensor maps (in global memory) of the other ranks' copies of y, for a row-sharded product whose
     // result every rank wants whole: each staging tile is stored once per destination.
@@ -318,9 +165,6 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     // tiles run along x and the weight tiles along y)
     const int n0 = (PAIR ? blockIdx.y : blockIdx.x) * tile_n;
     const int m0 = (PAIR ? blockIdx.x : blockIdx.y) * 128 * m_halves;
-    // grouped (MoE) launches: the weights of all experts are stacked, n_out rows each, and every token tile
-    // belongs to one expert
-    const int w_row0 = tile_expert ? tile_expert[blockIdx.y] * n_out : 0;
     // w_terms == 2 (Q4_K, tile_n <= 112): every weight goes into the B operand as two f16 terms, hi in rows 0 .. tile_n - 1 of
     // the stage and lo (what the rounding of hi left of the exact f32 value) in rows 128 .. 128 + tile_n - 1; both are
     // multiplied by the activations into the same accumulator. In each dequantizer set warps 0..3 then write the hi terms of
@@ -423,7 +267,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     w_issued = c + 1;
                     continue;
                 }
-                tma_load_2d(raw + (size_t)rb * RAW_STRIDE, &tmap_w, &sh->raw_full[rb], (sb0 * COPIES + c) * COPY_ROW, w_row0 + n0 + (int)rank * my_rows);
+                tma_load_2d(raw + (size_t)rb * RAW_STRIDE, &tmap_w, &sh->raw_full[rb], (sb0 * COPIES + c) * COPY_ROW, n0 + (int)rank * my_rows);
                 w_issued = c + 1;
             }
             if (sh->abort_flag)
@@ -957,21 +801,6 @@ __global__ void __launch_bounds__(256) to_f16_rows_kernel(const T* __restrict__ 
     if (threadIdx.x == 0) unscale[blockIdx.x] = inv;
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    }
-    return fn;
-}
-
 // Only in builds made with -DB2_DEBUG (make EXTRA=-DB2_DEBUG), B2_GEMM_DEBUG selects diagnostic switches for timing
 // experiments (the results are WRONG when any of the first five is set): 1 skip the dequantizers' shared-memory
 // stores, 2 skip the weight copies, 4 skip the MMAs, 8 skip the epilogue's stores, 16 skip the activation copies;
@@ -988,10 +817,21 @@ int debug_switches() {
 
 }  // namespace
 
+TensorMapEncodeFn tensor_map_encode() {
+    static TensorMapEncodeFn fn = nullptr;
+    if (!fn) {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = (TensorMapEncodeFn)p;
+    }
+    return fn;
+}
+
 struct GemmPlan {
     CUtensorMap tmap_x, tmap_w, tmap_y;
-    const int* tile_expert = nullptr;  // grouped launches: expert of each token tile (device)
-    size_t experts = 1;
+    bool wt_form = false;  // weights in tensor memory (gemm_wt.cu); only `wt` below and the shapes are then in use
+    GemmWt wt;
     const void* x16;
     const void* wptr;
     const void* y;
@@ -1010,6 +850,9 @@ struct GemmPlan {
     size_t a_lo_row0 = 0;  // two-term activations: the lo rows start this many rows below the hi rows (0: one term)
     int split_asked = 1;  // B2_GEMM_SPLIT_K when the plan was made (a cached plan is reused only under the same setting)
 };
+
+// Dense products of up to this many tokens take gemm_wt.cu.
+static constexpr size_t WT_MOST = 128;
 
 bool gemm_tc_supports(const WeightDev& w, size_t t) {
     if (w.fmt == B2_FMT_F8E4M3) return w.n_in % 128 == 0 && t >= 1 && ((uintptr_t)w.p0 & 15) == 0 && (w.p1 == nullptr || w.bs_cols == 128);
@@ -1057,7 +900,7 @@ static int pick_tile_n(size_t n_out, int m_tiles, int sm_count, size_t K, int wi
 }
 
 // Q6_K's qh plane [n_out][K / 4] bytes: boxes of 64 bytes x tile rows, 64-byte swizzle (conflict-free 16-byte reads by row).
-static CUresult encode_q6k_qh(EncodeTiledFn enc, CUtensorMap* m, const WeightDev& w, int tile_n) {
+static CUresult encode_q6k_qh(TensorMapEncodeFn enc, CUtensorMap* m, const WeightDev& w, int tile_n) {
     cuuint64_t dims[2] = {(cuuint64_t)(w.n_in / 4), (cuuint64_t)w.n_out};
     cuuint64_t strides[1] = {(cuuint64_t)(w.n_in / 4)};
     cuuint32_t box[2] = {64u, (cuuint32_t)tile_n};
@@ -1067,11 +910,11 @@ static CUresult encode_q6k_qh(EncodeTiledFn enc, CUtensorMap* m, const WeightDev
 }
 
 cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, void* y, int y_dtype, GemmPlan** out, char* err,
-                                size_t errlen, size_t experts, const int* tile_expert, int force_m_halves, size_t a_lo_row0, int w_terms,
+                                size_t errlen, int force_m_halves, size_t a_lo_row0, int w_terms,
                                 const GemmPeerY* peer_y) {
-    EncodeTiledFn enc = encode_tiled_fn();
+    TensorMapEncodeFn enc = tensor_map_encode();
     const bool gathered = peer_y && peer_y->ld != 0;
-    if (gathered && (y_dtype != B2_F32 || experts != 1 || tile_expert || peer_y->n_more < 0 || peer_y->n_more > 7 || peer_y->ld < w.n_out ||
+    if (gathered && (y_dtype != B2_F32 || peer_y->n_more < 0 || peer_y->n_more > 7 || peer_y->ld < w.n_out ||
                      peer_y->ld % 4 || w.n_out % 4 || ((uintptr_t)y & 15))) {
         snprintf(err, errlen, "a gathered product needs a dense f32 result with 16-byte aligned column blocks");
         return cudaErrorInvalidValue;
@@ -1089,8 +932,6 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
     p->t = t;
     p->K = w.n_in;
     p->n_out = w.n_out;
-    p->experts = experts;
-    p->tile_expert = tile_expert;
     p->m_halves = force_m_halves ? force_m_halves : (t > 128 ? 2 : 1);
     p->a_lo_row0 = a_lo_row0;
     if (a_lo_row0 && (p->m_halves != 1 || a_lo_row0 % 128 || a_lo_row0 < t)) {
@@ -1105,10 +946,25 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (w_terms == 2 && w.fmt != B2_FMT_Q4_K) w_terms = 1;  // the other formats' weights round to f16 far below the bound
     p->w_terms = w_terms;
+    if (w_terms == 1 && t <= WT_MOST && split_k_asked() == 1 && ((uintptr_t)w.p2 & 7) == 0) {
+        p->wt_form = true;
+        p->split_asked = 1;
+        p->pair_asked = pair_form_enabled();
+        p->y_ld = gathered ? peer_y->ld : 0;
+        p->n_more = gathered ? peer_y->n_more : 0;
+        for (int d = 0; d < p->n_more; d++) p->more_ptr[d] = peer_y->more[d];
+        if (!gemm_wt_encode(&p->wt, w, 1, x16, a_lo_row0 ? a_lo_row0 + t : t, t, a_lo_row0 ? 2 : 1, a_lo_row0, false, false)) {
+            snprintf(err, errlen, "the tensor maps of a product of up to 128 tokens could not be made");
+            delete p;
+            return cudaErrorInvalidValue;
+        }
+        *out = p;
+        return cudaSuccess;
+    }
     // (a gathered product stores every tile through the copy engine, whose staging tiles are 32 columns wide)
     const bool new_fmt = w.fmt == B2_FMT_Q6_K || w.fmt == B2_FMT_Q8_0;
-    if (new_fmt && (experts != 1 || tile_expert || a_lo_row0 || w_terms == 2)) {
-        snprintf(err, errlen, "Q6_K / Q8_0 products are dense, with one-term operands");
+    if (new_fmt && (a_lo_row0 || w_terms == 2)) {
+        snprintf(err, errlen, "Q6_K / Q8_0 products of more than 128 tokens have one-term operands");
         delete p;
         return cudaErrorInvalidValue;
     }
@@ -1124,7 +980,7 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
         p->split_asked = want;
         const int sb_k = w.fmt == B2_FMT_F8E4M3 ? 128 : 256;
         const size_t nsb_all = w.n_in / sb_k;
-        if (want == 2 && !new_fmt && y_dtype == B2_F32 && !a_lo_row0 && w_terms == 1 && !tile_expert && !gathered && nsb_all % 2 == 0 && nsb_all >= 8) {
+        if (want == 2 && !new_fmt && y_dtype == B2_F32 && !a_lo_row0 && w_terms == 1 && !gathered && nsb_all % 2 == 0 && nsb_all >= 8) {
             const int tn2 = pick_tile_n(w.n_out, p->m_tiles * 2, sm_count, w.n_in / 2);
             const size_t tiles1 = (w.n_out + p->tile_n - 1) / p->tile_n * (size_t)p->m_tiles;
             const size_t tiles2 = (w.n_out + tn2 - 1) / tn2 * (size_t)p->m_tiles * 2;
@@ -1138,7 +994,7 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
     // The CTA-pair form: dense one-term 4-bit launches of more than one 256-token tile. The token tiles are rounded up to an
     // even count (a CTA whose tokens are all out of range multiplies zeros and stores nothing).
     p->pair_asked = pair_form_enabled();
-    p->pair = p->pair_asked && !gathered && (w.fmt == B2_FMT_Q4_K || w.fmt == B2_FMT_MLX4) && !tile_expert && experts == 1 && !a_lo_row0 && w_terms == 1 &&
+    p->pair = p->pair_asked && !gathered && (w.fmt == B2_FMT_Q4_K || w.fmt == B2_FMT_MLX4) && !a_lo_row0 && w_terms == 1 &&
               p->k_splits == 1 && p->m_halves == 2 && p->m_tiles >= 2;
     if (p->pair) {
         p->m_tiles = (p->m_tiles + 1) / 2 * 2;
@@ -1163,7 +1019,7 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
         // rows of bytes, swizzled: 128 per copy (Q6_K's nibbles) or 64 (FP8, Q8_0)
         const bool f8 = w.fmt == B2_FMT_F8E4M3 || new_fmt;
         size_t row_bytes = w.fmt == B2_FMT_Q6_K ? w.n_in / 2 : f8 ? w.n_in : w.n_in / 256 * 144;
-        cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)(w.n_out * experts)};
+        cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)w.n_out};
         cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
         cuuint32_t box[2] = {w.fmt == B2_FMT_Q6_K ? 128u : f8 ? 64u : 144u, (cuuint32_t)(p->pair ? p->tile_n / 2 : p->tile_n)};
         cuuint32_t estr[2] = {1, 1};
@@ -1246,15 +1102,17 @@ bool gemm_tc_plan_matches(const GemmPlan* p, const WeightDev& w, const void* x16
         for (int d = 0; d < nm; d++)
             if (p->more_ptr[d] != peer_y->more[d]) return false;
     }
-    return p && p->experts == 1 && p->a_lo_row0 == a_lo_row0 && p->w_terms == w_terms && (m_halves == 0 || p->m_halves == m_halves) && p->y == y && p->y_dtype == y_dtype && p->x16 == x16 && p->wptr == w.p0 && p->t == t && p->K == w.n_in && p->n_out == w.n_out &&
+    return p && p->a_lo_row0 == a_lo_row0 && p->w_terms == w_terms && (m_halves == 0 || p->m_halves == m_halves) && p->y == y && p->y_dtype == y_dtype && p->x16 == x16 && p->wptr == w.p0 && p->t == t && p->K == w.n_in && p->n_out == w.n_out &&
            p->split_asked == split_k_asked() && p->pair_asked == pair_form_enabled();
 }
 
 cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, int y_dtype, GemmStatus* status_dev, int /*sm_count*/,
                            cudaStream_t st, const float* row_unscale) {
+    if (p->wt_form)
+        return launch_gemm_wt(p->wt, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, p->more_ptr, p->n_more, status_dev, row_unscale, st);
     const bool split = p->k_splits > 1;
     const bool tt = p->a_lo_row0 > 0 || p->w_terms == 2;
-    using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, int, int, int, int, int, void*, int, GemmStatus*, int, int, const int*, F8Scales, int, const float*,
+    using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, int, int, int, int, int, void*, int, GemmStatus*, int, int, F8Scales, int, const float*,
                           int, int, const CUtensorMap*, int);
     Kern kern;
     if (tt)  // two-term operands never come with a K split
@@ -1287,7 +1145,7 @@ cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, i
         cfg.attrs = attr;
         cfg.numAttrs = 2;
         cudaError_t le = cudaLaunchKernelEx(&cfg, kern, p->tmap_x, p->tmap_w, p->tmap_y, (int)w.n_in, (int)w.n_out, (int)t, p->tile_n, p->m_halves, y,
-                                  y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), 0, (const int*)nullptr, f8, 1, row_unscale, 0, 1, (const CUtensorMap*)nullptr, 0);
+                                  y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), 0, f8, 1, row_unscale, 0, 1, (const CUtensorMap*)nullptr, 0);
         return le;
     }
     if (cudaError_t e = ensure_dynamic_smem((const void*)kern, GEMM_SMEM); e != cudaSuccess) return e;
@@ -1298,7 +1156,7 @@ cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, i
     }
     // (a dependent launch: see the top of the kernel)
     return launch_k(kern, grid, dim3(GEMM_THREADS), GEMM_SMEM, st, true, p->tmap_x, p->tmap_w, p->tmap_y, (int)w.n_in, (int)w.n_out, (int)t, p->tile_n, p->m_halves, y,
-                    y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), 0, p->tile_expert, f8, p->k_splits, row_unscale, (int)p->a_lo_row0, p->w_terms,
+                    y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), 0, f8, p->k_splits, row_unscale, (int)p->a_lo_row0, p->w_terms,
                     (const CUtensorMap*)p->y_more, p->n_more);
 }
 

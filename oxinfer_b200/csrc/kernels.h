@@ -131,6 +131,10 @@ struct GemmStatus {   // written by the kernel when a bounded wait gives up
     uint32_t t[8];    // cycle stamps of one CTA (diagnostics, B2_GEMM_DEBUG & 32768)
 };
 bool gemm_tc_supports(const WeightDev& w, size_t t);
+// A token tile of a grouped launch (gemm_wt.cu): `count` rows (1 .. 128) from row0, all of one expert.
+struct WtTile {
+    int expert, row0, count, pad;
+};
 // y[t][n_out] (f32 or bf16) = x[t][n_in] (f16, row-major, t padded by the caller to a multiple of
 // 256 rows in `x16`) * W^T. `tmap_x` is the host-encoded tensor map of x16 (see make_tmap_x).
 struct GemmPlan;
@@ -138,9 +142,6 @@ struct GemmPlan;
 // terms feed the same accumulator, so the activations enter with 22 significant bits.
 // w_terms == 2 (Q4_K only; other formats ignore it): every weight enters as two f16 terms, hi + lo = the reference's f32
 // value to about 22 bits; tiles are then at most 112 rows wide.
-// `experts` > 1 makes a grouped plan: w.p0 holds `experts` stacked matrices of w.n_out rows, x16 / y hold the
-// token rows of all experts in segments that are multiples of 128 * m_halves rows, and tile_expert[i]
-// (device) names the expert of token tile i.
 // Where a row-sharded product's f32 result goes when every rank is to end up with the whole y [t][ld]: this rank's columns
 // of its own y (`y` of the call, already offset to them) and of n_more peers' copies (device pointers mapped from the
 // peers, offset the same way). The GEMM's epilogue then issues each staging tile's bulk store once per destination, so the
@@ -151,7 +152,7 @@ struct GemmPeerY {
     float* more[7] = {};
 };
 cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, void* y, int y_dtype, GemmPlan** out, char* err,
-                                size_t errlen, size_t experts = 1, const int* tile_expert = nullptr, int force_m_halves = 0, size_t a_lo_row0 = 0, int w_terms = 1, const GemmPeerY* peer_y = nullptr);
+                                size_t errlen, int force_m_halves = 0, size_t a_lo_row0 = 0, int w_terms = 1, const GemmPeerY* peer_y = nullptr);
 void gemm_tc_plan_destroy(GemmPlan* p);
 bool gemm_tc_plan_matches(const GemmPlan* p, const WeightDev& w, const void* x16, size_t t, const void* y, int y_dtype, size_t a_lo_row0 = 0,
                           int w_terms = 1, int m_halves = 0, const GemmPeerY* peer_y = nullptr);
@@ -183,7 +184,7 @@ cudaError_t launch_route_topk(const float* logits, size_t t, size_t n, size_t k,
 // rows, the second term lo_row0 rows below the first (see launch_to_f16).
 cudaError_t launch_moe_gather(const float* x, const int* src, size_t rows, size_t h, void* xg_f16, float* unscale, size_t lo_row0, cudaStream_t st);
 // kind: B2_ACT_* (0 SiLU, 1 tanh GELU, 2 SiLU with clamp `limit`).
-cudaError_t launch_moe_act(const float* g, const int* src, size_t rows, size_t inter, void* a_f16, float* unscale, size_t lo_row0, cudaStream_t st,
+cudaError_t launch_moe_act(const float* g, size_t rows, size_t inter, void* a_f16, float* unscale, size_t lo_row0, cudaStream_t st,
                            int kind = 0, float limit = 0.0f);
 // The same with the routes as kernel arguments (at most GEMV_GROUP_ROWS pairs).
 struct SmallRoutes {

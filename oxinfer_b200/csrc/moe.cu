@@ -1,7 +1,7 @@
 // Element-wise pieces of the routed-expert layer around the grouped tensor-core GEMM:
 //   route_topk   : top-k of the router logits with the reference's order and weights
 //                  (route_top_k, src/moe.rs:180-193; dtopk, src/cuda_decode.cu:285-312)
-//   moe_gather   : token rows -> per-expert segments, f32 -> f16, pad rows zero
+//   moe_gather   : token rows -> per-expert segments, f32 -> f16
 //                  (moe_gather, src/cuda.rs:293-297)
 //   moe_act      : act(gate) * up over the fused gate_up output, to f16 for the down projection
 //                  (moe_act, src/cuda.rs:300-316; SiLU with expf as on the reference's GPU path)
@@ -88,7 +88,7 @@ __device__ __forceinline__ void store_terms(float4 v, float f, __half* hi, __hal
     }
 }
 
-// xg[row][h] (f16) = x[src[row]][h] (f32) * factor[row], zeros where src[row] < 0; unscale[row] = 1 / factor, which the
+// xg[row][h] (f16) = x[src[row]][h] (f32) * factor[row]; unscale[row] = 1 / factor, which the
 // GEMM's epilogue multiplies the row's results by. lo_off > 0: two-term rows (see launch_to_f16), the second term
 // lo_off elements behind the first. One CTA of 256 threads per row; h is a multiple of 256 and at most 8192.
 constexpr int GATHER_KEEP = 8;
@@ -100,14 +100,6 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const float* __restrict
     const int row = blockIdx.x;
     const int s = src[row];
     __half* o = xg + (size_t)row * h;
-    if (s < 0) {
-        for (int c = threadIdx.x * 4; c < h; c += 1024) {
-            *(uint2*)(o + c) = make_uint2(0u, 0u);
-            if (lo_off) *(uint2*)(o + lo_off + c) = make_uint2(0u, 0u);
-        }
-        if (threadIdx.x == 0) unscale[row] = 1.0f;
-        return;
-    }
     const float4* in = (const float4*)(x + (size_t)s * h);
     float4 v[GATHER_KEEP];
     float mx = 0.0f;
@@ -148,16 +140,6 @@ __global__ void __launch_bounds__(256) moe_gather_warp_kernel(const float* __res
     if (row >= rows) return;
     const int s = src[row];
     __half* o = xg + (size_t)row * H;
-    if (s < 0) {
-#pragma unroll
-        for (int j = 0; j < VPL; j++) {
-            const int c = (j * 32 + lane) * 4;
-            *(uint2*)(o + c) = make_uint2(0u, 0u);
-            if (lo_off) *(uint2*)(o + lo_off + c) = make_uint2(0u, 0u);
-        }
-        if (lane == 0) unscale[row] = 1.0f;
-        return;
-    }
     const float4* in = (const float4*)(x + (size_t)s * H);
     float4 v[VPL];
     float mx = 0.0f;
@@ -179,8 +161,7 @@ __global__ void __launch_bounds__(256) moe_gather_warp_kernel(const float* __res
 
 // a[row][inter] (f16) = silu(g[row][c]) * g[row][inter + c] * factor[row] over the fused gate_up output g [rows][2 inter]
 // (f32); factor[row] is the power of two of row_factor and unscale[row] = 1 / factor is what the down projection's epilogue
-// multiplies the row's results by. lo_off as for the gather. src[row] < 0 marks a padding row (src may be null: no
-// padding). One CTA per row; the row is read once (a thread keeps its products in registers between the maximum and the
+// multiplies the row's results by. lo_off as for the gather. One CTA per row; the row is read once (a thread keeps its products in registers between the maximum and the
 // store) when inter <= 256 * 4 * ACT_KEEP.
 constexpr int ACT_KEEP = 2;
 // kind (MoeAct, src/gpu.rs:36-54; the arithmetic of the reference's moe_act, src/cuda.rs:300-316): 0 SiLU, 1 tanh GELU
@@ -197,21 +178,13 @@ __device__ __forceinline__ float gated_act(float g, float u, int kind, float lim
     return g / (1.0f + expf(-g)) * u;
 }
 
-__global__ void __launch_bounds__(256) moe_act_kernel(const float* __restrict__ g, const int* __restrict__ src, int inter, __half* __restrict__ a,
+__global__ void __launch_bounds__(256) moe_act_kernel(const float* __restrict__ g, int inter, __half* __restrict__ a,
                                                       float* __restrict__ unscale, size_t lo_off, int kind, float limit) {
     __shared__ float red[8];
     pdl_launch_dependents();  // a dependent launch: the kernel behind may set itself up; nothing is read or written before the wait
     pdl_wait();
     const size_t row = blockIdx.x;
     __half* ar = a + row * inter;
-    if (src && src[row] < 0) {  // a padding row of an expert's last tile: its products are zero, nothing to read
-        for (int c = threadIdx.x * 4; c < inter; c += 256 * 4) {
-            *(uint2*)(ar + c) = make_uint2(0u, 0u);
-            if (lo_off) *(uint2*)(ar + lo_off + c) = make_uint2(0u, 0u);
-        }
-        if (threadIdx.x == 0) unscale[row] = 1.0f;
-        return;
-    }
     const float* gr = g + row * 2 * (size_t)inter;
     const bool keep = inter <= 256 * 4 * ACT_KEEP;  // inter is a multiple of 256: whole float4 per thread
     auto act4 = [&](int c) {
@@ -258,7 +231,7 @@ __global__ void __launch_bounds__(256) moe_act_kernel(const float* __restrict__ 
 
 // The same with a warp per row (eight rows per CTA): inter = 128 * VPL, a lane keeps its VPL float4 of products.
 template <int VPL>
-__global__ void __launch_bounds__(256) moe_act_warp_kernel(const float* __restrict__ g, const int* __restrict__ src, int rows, __half* __restrict__ a,
+__global__ void __launch_bounds__(256) moe_act_warp_kernel(const float* __restrict__ g, int rows, __half* __restrict__ a,
                                                            float* __restrict__ unscale, size_t lo_off, int kind, float limit) {
     constexpr int INTER = 128 * VPL;
     pdl_launch_dependents();  // a dependent launch: the kernel behind may set itself up; nothing is read or written before the wait
@@ -266,16 +239,6 @@ __global__ void __launch_bounds__(256) moe_act_warp_kernel(const float* __restri
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
     __half* ar = a + (size_t)row * INTER;
-    if (src && src[row] < 0) {
-#pragma unroll
-        for (int j = 0; j < VPL; j++) {
-            const int c = (j * 32 + lane) * 4;
-            *(uint2*)(ar + c) = make_uint2(0u, 0u);
-            if (lo_off) *(uint2*)(ar + lo_off + c) = make_uint2(0u, 0u);
-        }
-        if (lane == 0) unscale[row] = 1.0f;
-        return;
-    }
     const float* gr = g + (size_t)row * 2 * INTER;
     float4 v[VPL];
     float mx = 0.0f;
@@ -396,16 +359,16 @@ cudaError_t launch_moe_gather(const float* x, const int* src, size_t rows, size_
     }
 }
 
-cudaError_t launch_moe_act(const float* g, const int* src, size_t rows, size_t inter, void* a, float* unscale, size_t lo_row0, cudaStream_t st,
+cudaError_t launch_moe_act(const float* g, size_t rows, size_t inter, void* a, float* unscale, size_t lo_row0, cudaStream_t st,
                            int kind, float limit) {
     if (inter % 256) return cudaErrorInvalidValue;
     if (rows == 0) return cudaSuccess;
     const unsigned wgrid = (unsigned)((rows + 7) / 8);
     switch (rows >= 1024 ? inter / 128 : 0) {  // many rows of a common width: a warp per row
-        case 4: return launch_k(moe_act_warp_kernel<4>, dim3(wgrid), dim3(256), 0, st, true, g, src, (int)rows, (__half*)a, unscale, lo_row0 * inter, kind, limit);
-        case 6: return launch_k(moe_act_warp_kernel<6>, dim3(wgrid), dim3(256), 0, st, true, g, src, (int)rows, (__half*)a, unscale, lo_row0 * inter, kind, limit);
-        case 8: return launch_k(moe_act_warp_kernel<8>, dim3(wgrid), dim3(256), 0, st, true, g, src, (int)rows, (__half*)a, unscale, lo_row0 * inter, kind, limit);
-        default: return launch_k(moe_act_kernel, dim3((unsigned)rows), dim3(256), 0, st, true, g, src, (int)inter, (__half*)a, unscale, lo_row0 * inter, kind, limit);
+        case 4: return launch_k(moe_act_warp_kernel<4>, dim3(wgrid), dim3(256), 0, st, true, g, (int)rows, (__half*)a, unscale, lo_row0 * inter, kind, limit);
+        case 6: return launch_k(moe_act_warp_kernel<6>, dim3(wgrid), dim3(256), 0, st, true, g, (int)rows, (__half*)a, unscale, lo_row0 * inter, kind, limit);
+        case 8: return launch_k(moe_act_warp_kernel<8>, dim3(wgrid), dim3(256), 0, st, true, g, (int)rows, (__half*)a, unscale, lo_row0 * inter, kind, limit);
+        default: return launch_k(moe_act_kernel, dim3((unsigned)rows), dim3(256), 0, st, true, g, (int)inter, (__half*)a, unscale, lo_row0 * inter, kind, limit);
     }
 }
 

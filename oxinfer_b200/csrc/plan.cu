@@ -965,7 +965,7 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
             char msg[256] = {0};
             GemmPeerY py;
             py.ld = y_ld;
-            cudaError_t e = gemm_tc_plan_create(w, x16_, t, y, B2_F32, &gp, msg, sizeof msg, 1, nullptr, 0, 0, 1, y_ld != w.n_out ? &py : nullptr);
+            cudaError_t e = gemm_tc_plan_create(w, x16_, t, y, B2_F32, &gp, msg, sizeof msg, 0, 0, 1, y_ld != w.n_out ? &py : nullptr);
             if (e != cudaSuccess) {
                 err = fmt("[b200qmm: prefill: %s]", msg);
                 return e;

@@ -1,0 +1,63 @@
+"""Products of 9 to 128 tokens and the routed experts' segments: weights in tensor memory, tokens on the instruction's N side."""
+import numpy as np
+import pytest
+import torch
+
+import oxinfer_b200 as ob
+from oxinfer_b200 import synth
+
+from util import make_pair, oracle_matrix, row_err
+
+pytestmark = pytest.mark.gpu
+
+
+# token counts around the steps of 16 and the change of the accumulator's width at 64; row counts around the tiles of 128; one super-block,
+# an odd number of them, the first K that is divided (2 parts), 4 parts and 8 unequal ones
+@pytest.mark.parametrize("fmt", ["mlx4", "q4_k", "q6_k", "q8_0", "f8_e4m3"])
+@pytest.mark.parametrize("shape", [(127, 256, 9), (128, 768, 16), (130, 2816, 17), (260, 3072, 64), (384, 6400, 65), (1001, 12544, 37), (257, 12288, 128)])
+def test_products_of_up_to_128_tokens(backend, fmt, shape):
+    """f16 operands with f32 sums: 1e-3 of a row (tests/test_gemm_gpu.py). A row shard has the bits of its rows, and a token of a smaller
+    batch the bits of the larger one's, f32 in place of the strided or bf16 results of the other entry points included."""
+    n_out, n_in, t = shape
+    ref, m = make_pair(fmt, n_out, n_in, 900 + t)
+    dev = backend.upload(ref, n_out, n_in)
+    x = synth.activations(t, n_in, 901)
+    y = np.full((t, n_out), np.nan, np.float32)
+    assert backend.matmul(x, [ob.Job(dev, y)])
+    assert row_err(y, m.matmul_f64(x)) < 1e-3
+    if n_out > 128:
+        shard = backend.shard_rows(dev, 128, n_out)
+        ys = np.zeros((t, n_out - 128), np.float32)
+        assert backend.matmul(x, [ob.Job(shard, ys)])
+        assert np.array_equal(ys, y[:, 128:])
+    y9 = np.zeros((9, n_out), np.float32)
+    assert backend.matmul(x[t - 9 :], [ob.Job(dev, y9)])
+    assert np.array_equal(y9, y[t - 9 :])
+    xd, yd = torch.from_numpy(x).cuda(), torch.zeros((t, n_out), device="cuda", dtype=torch.bfloat16)
+    assert backend.matmul_dev(dev, xd, yd)
+    torch.cuda.synchronize()
+    backend.check_status()
+    assert torch.equal(yd.cpu(), torch.from_numpy(y).bfloat16())
+
+
+# pairs per expert: none, one, a tile of 16 and one more, 128 and one more (two tiles of 80 and 49 rows), three tiles
+@pytest.mark.parametrize("fmt", ["mlx4", "q4_k"])
+@pytest.mark.parametrize("counts,h,inter", [([1, 16, 0, 17, 128, 129, 300, 64], 256, 512), ([70], 2048, 768)])
+def test_segments_of_every_length(backend, fmt, counts, h, inter):
+    n = len(counts)
+    refs = [(synth.make(fmt, 2 * inter, h, 920 + 2 * e), synth.make(fmt, h, inter, 921 + 2 * e)) for e in range(n)]
+    moe = backend.upload_moe([backend.upload(g, 2 * inter, h) for g, _ in refs], [backend.upload(d, h, inter) for _, d in refs], h, inter)
+    flat = np.random.default_rng(922).permutation(np.repeat(np.arange(n, dtype=np.int32), counts))
+    x = synth.activations(len(flat), h, 923)
+    y = torch.zeros((len(flat), h), device="cuda")
+    assert backend.moe_dev(torch.from_numpy(x).cuda(), flat.reshape(-1, 1), np.ones((len(flat), 1), np.float32), moe, y)
+    torch.cuda.synchronize()
+    backend.check_status()
+    for e, (g, d) in enumerate(refs):
+        rows = np.flatnonzero(flat == e)
+        if len(rows) == 0:
+            continue
+        gu = oracle_matrix(g, 2 * inter, h).matmul_f64(x[rows])
+        a = gu[:, :inter] / (1.0 + np.exp(-gu[:, :inter])) * gu[:, inter:]
+        want = a @ oracle_matrix(d, h, inter).dequantize_rows().astype(np.float64).T
+        assert row_err(y[torch.from_numpy(rows).cuda()].cpu().numpy(), want) < 1e-3, e
