@@ -80,23 +80,15 @@ __device__ __forceinline__ bool bar_try(uint64_t* bar, uint32_t parity) {
                  : "memory");
     return ok != 0;
 }
-// The same test with acquire semantics at cluster scope: for barriers that the peer CTA's threads, copies or instructions complete.
-__device__ __forceinline__ bool bar_try_cluster(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(s32(bar)), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
 // The address, in the cluster's shared window, of CTA `cta`'s copy of a shared-memory object of this CTA.
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t cta) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(s32(p)), "r"(cta));
     return r;
 }
+// (what it announces, reads of tensor memory, is ordered by the tcgen05 fence ahead of it)
 __device__ __forceinline__ void bar_arrive_cluster(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -106,14 +98,17 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync_all() {  // every thread of both CTAs
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-template <bool CLUSTER = false>
+__device__ __forceinline__ bool elect() {  // true in one lane of a whole warp (tcgen05.cuh says why not lane 0)
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, F8Shared* sh, GemmStatus* status, uint32_t where, uint32_t iter,
                                          bool heed_abort = true) {
-    auto test = [&] { return CLUSTER ? bar_try_cluster(bar, parity) : bar_try(bar, parity); };
-    if (test()) return true;
+    if (bar_try(bar, parity)) return true;
     const long long t0 = clock64();
     for (uint32_t spin = 1;; spin++) {
-        if (test()) return true;
+        if (bar_try(bar, parity)) return true;
         if ((spin & 255) == 0) {
             if (heed_abort && sh->abort_flag) return false;
             if (clock64() - t0 > F8_WAIT_LIMIT) {
@@ -266,7 +261,7 @@ gemm_f8_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     if (warp < 4) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 40;" ::: "memory");
       if (warp == 0) {
-        if (lane == 0) {
+        {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
             asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -278,7 +273,9 @@ gemm_f8_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 for (int b = 0; b < nb; b++, it++) {
                     const int s = it % F8_STAGES;
                     const uint32_t ph = (uint32_t)((it / F8_STAGES) & 1);
-                    if (!bar_wait<PAIR>(&sh->empty[s], ph ^ 1u, sh, status, 1, (uint32_t)it)) { ok = false; break; }
+                    ok = __all_sync(0xffffffffu, bar_wait(&sh->empty[s], ph ^ 1u, sh, status, 1, (uint32_t)it));
+                    if (!ok) break;
+                    if (!elect()) continue;
                     if constexpr (PAIR) {
                         // both CTAs' tiles are counted on the even CTA's barrier, which expects the bytes of both
                         const uint32_t bar0 = cluster_addr(&sh->full[s], 0);
@@ -292,14 +289,15 @@ gemm_f8_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     }
                 }
             }
+            __syncwarp();
             // let the copies still in flight land before the shared memory is released (pair form: the odd CTA's copies are
             // counted on the even CTA's barriers, and both CTAs meet at the cluster barrier of the teardown after these waits)
             if (sh->abort_flag && rank == 0)
                 for (int j = max(0, it - F8_STAGES); j < it; j++)
-                    bar_wait<PAIR>(&sh->full[j % F8_STAGES], (uint32_t)((j / F8_STAGES) & 1), sh, status, 2, (uint32_t)j, false);
+                    bar_wait(&sh->full[j % F8_STAGES], (uint32_t)((j / F8_STAGES) & 1), sh, status, 2, (uint32_t)j, false);
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             // D f32 (bit 4), A and B e4m3 (format code 0), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
             const uint32_t idesc = (1u << 4) | ((uint32_t)(F8_TN >> 3) << 17) | ((uint32_t)((PAIR ? 2 * F8_TM : F8_TM) >> 4) << 24);
             const uint64_t a_base = desc_sw128(s32(a_tiles)), b_base = desc_sw128(s32(b_tiles));
@@ -309,10 +307,12 @@ gemm_f8_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             const int n_it = n_mine * nb;
             for (int it = 0; it < n_it && ok; it++) {
                 const int s = it % F8_STAGES, buf = it & 1;
-                if (!bar_wait<PAIR>(&sh->full[s], (uint32_t)((it / F8_STAGES) & 1), sh, status, 3, (uint32_t)it)) { ok = false; break; }
-                // the partial accumulator `buf` was last used by block it - 2: wait until its promotion has read it
-                if (it >= 2 && !bar_wait<PAIR>(&sh->pfree[buf], (uint32_t)(((it >> 1) - 1) & 1), sh, status, 4, (uint32_t)it)) { ok = false; break; }
+                // (the partial accumulator `buf` was last used by block it - 2: its promotion has to have read it)
+                ok = __all_sync(0xffffffffu, bar_wait(&sh->full[s], (uint32_t)((it / F8_STAGES) & 1), sh, status, 3, (uint32_t)it) &&
+                                                 (it < 2 || bar_wait(&sh->pfree[buf], (uint32_t)(((it >> 1) - 1) & 1), sh, status, 4, (uint32_t)it)));
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (!elect()) continue;
                 const uint64_t ad = a_base + (uint64_t)((uint32_t)s * (F8_A_BYTES >> 4));
                 const uint64_t bd = b_base + (uint64_t)((uint32_t)s * (F8_B_BYTES >> 4));
 #pragma unroll
@@ -361,7 +361,7 @@ gemm_f8_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 const int buf = it & 1;
                 const float c = c_next;
                 if (b + 1 < nb) c_next = __ldg(sx_row + b + 1) * (sw_row ? __ldg(sw_row + b + 1) : 1.0f);
-                if (!bar_wait<PAIR>(&sh->pfull[buf], (uint32_t)((it >> 1) & 1), sh, status, 5, (uint32_t)it)) { ok = false; break; }
+                if (!bar_wait(&sh->pfull[buf], (uint32_t)((it >> 1) & 1), sh, status, 5, (uint32_t)it)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * F8_TN + chalf * 128);
                 // two loads in flight: the next 32 columns travel while this chunk's multiply-adds issue
@@ -515,11 +515,11 @@ cudaError_t launch_gemm_f8(const WeightDev& w, const uint8_t* qx, const float* s
         snprintf(err, errlen, "cuTensorMapEncodeTiled is not available from the driver");
         return cudaErrorNotSupported;
     }
-    // B2_F8_PAIR=1 selects the CTA-pair form for more than one 128-token tile. Off by default: with two partial accumulators
-    // the MMA -> promotion -> MMA chain of a block crosses SMs twice in that form, and it measures 6.8 ms against 3.2 ms at
-    // 8192 x 12288 x 28672 (bit-identical results).
+    // The CTA-pair form for more than one 128-token tile (B2_F8_PAIR=0: never): a CTA keeps half of the weight tile, so shared memory moves
+    // 32 KB a block of 128 k instead of 48. 8192 x 12288 x 28672: 3.27 ms against 3.59 for single CTAs; 512 x 4096 x 14336: 47.5 us
+    // against 50.9 (bit-identical results).
     const char* pe = getenv("B2_F8_PAIR");
-    const bool pair = t > (size_t)F8_TM && pe && atoi(pe) != 0;
+    const bool pair = t > (size_t)F8_TM && !(pe && atoi(pe) == 0);
     CUtensorMap tx, tw;
     cuuint32_t estr[2] = {1, 1};
     {
