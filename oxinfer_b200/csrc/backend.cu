@@ -883,12 +883,19 @@ class Backend {
 
     // One grouped GEMM: the rows of xg (f16, expert by expert, the second terms lo_row0 rows below) times the stacked matrices.
     int grouped_gemm(int fmt, const void* stacked, size_t experts, size_t n_out, size_t n_in, const void* xg, size_t rows, size_t longest, const WtTile* tiles,
-                     size_t n_tiles, float* out_dev, const float* row_unscale, size_t lo_row0) {
+                     size_t n_tiles, float* out_dev, const float* row_unscale, size_t lo_row0, bool pairs) {
         WeightDev w{};
         w.fmt = fmt;
         w.n_out = n_out;
         w.n_in = n_in;
         w.p0 = (const uint8_t*)stacked;
+        if (pairs) {
+            GemmWp g;
+            if (!gemm_wp_encode(&g, w, experts, xg, rows)) return fail(B2_ERR_CUDA, "[b200qmm: the tensor maps of a grouped product could not be made]");
+            cudaError_t e = launch_gemm_wp(g, w, rows, tiles, (int)n_tiles, out_dev, B2_F32, n_out, nullptr, 0, gemm_status, sm_count, row_unscale, stream);
+            launches++;
+            return e == cudaSuccess ? B2_OK : cuda_fail(e, "grouped gemm (pairs)");
+        }
         GemmWt g;
         if (!gemm_wt_encode(&g, w, experts, xg, lo_row0 ? lo_row0 + rows : rows, longest, lo_row0 ? 2 : 1, lo_row0, lo_row0 && fmt == B2_FMT_Q4_K, true))
             return fail(B2_ERR_CUDA, "[b200qmm: the tensor maps of a grouped product could not be made]");
@@ -1023,12 +1030,14 @@ class Backend {
         // layer above 1e-3 per output row (MLX-4 stays near 3e-4 with one term).
         const bool two_term = m.fmt == B2_FMT_Q4_K || exact;
         const size_t rows = t * k, terms = two_term ? 2 : 1, lo_row0 = two_term ? rows : 0;
+        const bool pairs = !two_term;  // the CTA-pair form, for one-term operands
+        const size_t most = pairs ? WP_MOST_ROWS : 128;
         std::vector<size_t> at(m.experts, 0);
         std::vector<WtTile> tiles;
         size_t longest = 0;
         for (size_t e = 0, row = 0; e < m.experts; e++) {
             at[e] = row;
-            const size_t n = (count[e] + 127) / 128, size = n ? ((count[e] + n - 1) / n + 15) / 16 * 16 : 0;
+            const size_t n = (count[e] + most - 1) / most, size = n ? ((count[e] + n - 1) / n + 15) / 16 * 16 : 0;
             for (size_t c = 0; c < count[e]; c += size)
                 tiles.push_back(WtTile{(int)e, (int)(row + c), (int)std::min(size, count[e] - c), 0});
             longest = std::max(longest, std::min(size, count[e]));
@@ -1063,11 +1072,11 @@ class Backend {
         e = launch_moe_gather(x_dev_, d_src, rows, m.h, moe_xg.p, x_unscale, lo_row0, stream);
         launches++;
         if (e != cudaSuccess) return cuda_fail(e, "moe_gather");
-        if ((rc = grouped_gemm(m.fmt, m.gate_up, m.experts, 2 * m.inter, m.h, moe_xg.p, rows, longest, d_tiles, tiles.size(), (float*)moe_g.p, x_unscale, lo_row0))) return rc;
+        if ((rc = grouped_gemm(m.fmt, m.gate_up, m.experts, 2 * m.inter, m.h, moe_xg.p, rows, longest, d_tiles, tiles.size(), (float*)moe_g.p, x_unscale, lo_row0, pairs))) return rc;
         e = launch_moe_act((const float*)moe_g.p, rows, m.inter, moe_a.p, a_unscale, lo_row0, stream, m.act, m.act_limit);
         launches++;
         if (e != cudaSuccess) return cuda_fail(e, "moe_act");
-        if ((rc = grouped_gemm(m.fmt, m.down, m.experts, m.h, m.inter, moe_a.p, rows, longest, d_tiles, tiles.size(), (float*)moe_o.p, a_unscale, lo_row0))) return rc;
+        if ((rc = grouped_gemm(m.fmt, m.down, m.experts, m.h, m.inter, moe_a.p, rows, longest, d_tiles, tiles.size(), (float*)moe_o.p, a_unscale, lo_row0, pairs))) return rc;
         e = launch_moe_combine((const float*)moe_o.p, d_slots, d_w, t, k, m.h, y_dev_, stream);
         launches++;
         if (e != cudaSuccess) return cuda_fail(e, "moe_combine");

@@ -830,8 +830,9 @@ TensorMapEncodeFn tensor_map_encode() {
 
 struct GemmPlan {
     CUtensorMap tmap_x, tmap_w, tmap_y;
-    bool wt_form = false;  // weights in tensor memory (gemm_wt.cu); only `wt` below and the shapes are then in use
+    int wt_form = 0;  // weights in tensor memory: 1 gemm_wt.cu, 2 its pair form gemm_wp.cu; only these and the shapes are then in use
     GemmWt wt;
+    GemmWp wp;
     const void* x16;
     const void* wptr;
     const void* y;
@@ -947,14 +948,15 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
     if (w_terms == 2 && w.fmt != B2_FMT_Q4_K) w_terms = 1;  // the other formats' weights round to f16 far below the bound
     p->w_terms = w_terms;
     if (w_terms == 1 && t <= WT_MOST && split_k_asked() == 1 && ((uintptr_t)w.p2 & 7) == 0) {
-        p->wt_form = true;
+        p->wt_form = t <= WT_MOST ? 1 : 2;
         p->split_asked = 1;
         p->pair_asked = pair_form_enabled();
         p->y_ld = gathered ? peer_y->ld : 0;
         p->n_more = gathered ? peer_y->n_more : 0;
         for (int d = 0; d < p->n_more; d++) p->more_ptr[d] = peer_y->more[d];
-        if (!gemm_wt_encode(&p->wt, w, 1, x16, a_lo_row0 ? a_lo_row0 + t : t, t, a_lo_row0 ? 2 : 1, a_lo_row0, false, false)) {
-            snprintf(err, errlen, "the tensor maps of a product of up to 128 tokens could not be made");
+        if (!(p->wt_form == 1 ? gemm_wt_encode(&p->wt, w, 1, x16, a_lo_row0 ? a_lo_row0 + t : t, t, a_lo_row0 ? 2 : 1, a_lo_row0, false, false)
+                              : gemm_wp_encode(&p->wp, w, 1, x16, t))) {
+            snprintf(err, errlen, "the tensor maps of a product could not be made");
             delete p;
             return cudaErrorInvalidValue;
         }
@@ -1106,8 +1108,10 @@ bool gemm_tc_plan_matches(const GemmPlan* p, const WeightDev& w, const void* x16
            p->split_asked == split_k_asked() && p->pair_asked == pair_form_enabled();
 }
 
-cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, int y_dtype, GemmStatus* status_dev, int /*sm_count*/,
+cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, int y_dtype, GemmStatus* status_dev, int sm_count,
                            cudaStream_t st, const float* row_unscale) {
+    if (p->wt_form == 2)
+        return launch_gemm_wp(p->wp, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, p->more_ptr, p->n_more, status_dev, sm_count, row_unscale, st);
     if (p->wt_form)
         return launch_gemm_wt(p->wt, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, p->more_ptr, p->n_more, status_dev, row_unscale, st);
     const bool split = p->k_splits > 1;

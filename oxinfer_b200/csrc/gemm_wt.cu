@@ -21,12 +21,12 @@
 // Tensor memory: a CTA takes 256 of the 512 columns and at least 77 KB of shared memory, so that no more than two CTAs of these kernels fit
 // an SM and an allocation never waits for a CTA that itself waits for another CTA of its cluster.
 #include <cuda.h>
-#include <cuda_fp8.h>
 
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 
+#include "expand.cuh"
 #include "gemm_wt.h"
 #include "tcgen05.cuh"
 
@@ -76,22 +76,6 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uin
         "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ bool elect_one() {  // true in one lane of a whole warp
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, "
-        "%21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
-        "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]),
-        "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ __half2 as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
@@ -106,74 +90,16 @@ __device__ __forceinline__ void store_y(const WtArgs& a, size_t at, float v) {
     for (int d = 0; d < a.n_more; d++) a.more[d][at] = v;
 }
 
-// 64 weights of a 4-bit block: 32 bytes, low nibbles = elements 0..31, high nibbles = 32..63 (see gemm_tc.cu for the arithmetic).
-// hdr: the block's 16 bytes in front; j: which of its four groups of 64. LO (Q4_K): the second term, the exact f32 weight minus the
-// first term.
-template <int FMT, bool LO>
-__device__ __forceinline__ void expand_4bit(const uint4& hdr, const uint32_t (&qw)[8], int j, uint32_t (&o)[32]) {
-    __half2 dmul, c1lo, c2lo, c1hi, c2hi, addlo, addhi;
-    uint32_t sc0 = 0, mn0 = 0, sc1 = 0, mn1 = 0;
-    if constexpr (FMT == B2_FMT_MLX4) {
-        const uint32_t sw = (j & 2) ? hdr.y : hdr.x, bw = (j & 2) ? hdr.w : hdr.z;
-        dmul = __half2half2(__ushort_as_half((unsigned short)((sw >> (16 * (j & 1))) & 0xffffu)));
-        c1lo = __float2half2_rn(1.0f);
-        c2lo = __float2half2_rn(-1032.0f);
-        c1hi = __float2half2_rn(0.0625f);
-        c2hi = __float2half2_rn(-72.0f);
-        addlo = addhi = __float2half2_rn(bf16_bits_to_f32((bw >> (16 * (j & 1))) & 0xffffu));
-    } else {
-        q4k_scale_min(2 * j, hdr.y, hdr.z, hdr.w, sc0, mn0);
-        q4k_scale_min(2 * j + 1, hdr.y, hdr.z, hdr.w, sc1, mn1);
-        const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
-        dmul = __half2half2(__ushort_as_half((unsigned short)(hdr.x & 0xffff)));
-        c1lo = __float2half2_rn((float)sc0);
-        c2lo = __float2half2_rn(-1024.0f * (float)sc0);
-        c1hi = __float2half2_rn(0.0625f * (float)sc1);
-        c2hi = __float2half2_rn(-64.0f * (float)sc1);
-        addlo = __float2half2_rn(-(dmin * (float)mn0));
-        addhi = __float2half2_rn(-(dmin * (float)mn1));
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const uint32_t p0 = __byte_perm(qw[i], 0, 0x4140), p1 = __byte_perm(qw[i], 0, 0x4342);
-        o[2 * i] = h2_bits(__hfma2(__hfma2(as_h2((p0 & 0x000F000Fu) | 0x64006400u), c1lo, c2lo), dmul, addlo));
-        o[2 * i + 1] = h2_bits(__hfma2(__hfma2(as_h2((p1 & 0x000F000Fu) | 0x64006400u), c1lo, c2lo), dmul, addlo));
-        o[16 + 2 * i] = h2_bits(__hfma2(__hfma2(as_h2((p0 & 0x00F000F0u) | 0x64006400u), c1hi, c2hi), dmul, addhi));
-        o[16 + 2 * i + 1] = h2_bits(__hfma2(__hfma2(as_h2((p1 & 0x00F000F0u) | 0x64006400u), c1hi, c2hi), dmul, addhi));
-    }
-    if constexpr (LO) {
-        const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffff)));
-        const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
-        const float d1l = __fmul_rn(d, (float)sc0), m1l = __fmul_rn(dmin, (float)mn0);
-        const float d1h = __fmul_rn(d, (float)sc1), m1h = __fmul_rn(dmin, (float)mn1);
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const uint32_t b0 = (qw[i] >> (16 * e)) & 0xffu, b1 = (qw[i] >> (16 * e + 8)) & 0xffu;
-                const float2 hl = __half22float2(as_h2(o[2 * i + e])), hh = __half22float2(as_h2(o[16 + 2 * i + e]));
-                const float vl0 = __fsub_rn(__fmul_rn(d1l, __uint_as_float(0x4B000000u | (b0 & 15u)) - 8388608.0f), m1l);
-                const float vl1 = __fsub_rn(__fmul_rn(d1l, __uint_as_float(0x4B000000u | (b1 & 15u)) - 8388608.0f), m1l);
-                const float vh0 = __fsub_rn(__fmul_rn(d1h, __uint_as_float(0x4B000000u | (b0 >> 4)) - 8388608.0f), m1h);
-                const float vh1 = __fsub_rn(__fmul_rn(d1h, __uint_as_float(0x4B000000u | (b1 >> 4)) - 8388608.0f), m1h);
-                o[2 * i + e] = h2_bits(__floats2half2_rn(vl0 - hl.x, vl1 - hl.y));
-                o[16 + 2 * i + e] = h2_bits(__floats2half2_rn(vh0 - hh.x, vh1 - hh.y));
-            }
-        }
-    }
-}
-
 // W2 (Q4_K): every weight as two f16 terms; set 0 expands the first terms of every stage, set 1 the second.
 template <int FMT, bool W2>
 __global__ void __launch_bounds__(WT_THREADS, 2)
-gemm_wt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2,
+gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2,
                const __grid_constant__ WtArgs a) {
     // A dependent launch: the weights, their expansion and the set-up run under the kernel ahead; the activations, the row factors and y
     // wait for it.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr bool BYTE_ROWS = FMT == B2_FMT_F8E4M3 || FMT == B2_FMT_Q8_0;
     constexpr bool PRE_SCALED = BYTE_ROWS || FMT == B2_FMT_Q6_K;
-    constexpr float PRE = 256.0f;                       // power of two in the f16 weights of these formats
     constexpr int SB_K = BYTE_ROWS ? 128 : 256;         // a super-block, what a part of K is a whole number of
     constexpr int SB_G = SB_K / 64;                     // groups of 64 k in a super-block
     constexpr int RAW_SLOT = BYTE_ROWS ? WT_ROWS * 64 : WT_ROWS * (FMT == B2_FMT_Q6_K ? 192 : 144);
@@ -228,28 +154,23 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
 
     if (warp == 8) {
         // ---------------- activations ----------------
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+        {
+            const CUtensorMap* tmap_x = &maps.m[n / 16 - 1];
+            asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_x) : "memory");
             const uint32_t bytes = (uint32_t)(n * 128 * a.x_terms * a.groups);
             asm volatile("griddepcontrol.wait;" ::: "memory");
             int issued = 0;
             for (int ks = 0, s = 0; ks < nks; ks++) {
                 const int old = ks - a.n_b;  // the stage whose slot this one takes
-                if (old >= 0 && !mbar_wait(&sh->done[old & 3], (uint32_t)((old >> 2) & 1), sh, a.status, 21, (uint32_t)ks)) break;
-                mbar_arrive_expect_tx(&sh->b_full[s], bytes);
-                uint8_t* dst = b_tiles + (size_t)s * b_stage;  // [group][term][n][64]
-                for (int i = 0; i < a.groups * a.x_terms; i++, dst += (size_t)n * 128) {
-                    const int term = a.x_terms == 2 ? i & 1 : 0, g = a.x_terms == 2 ? i >> 1 : i;
-                    const int kx = (sb0 * SB_G + ks * a.groups + g) * 64, y = x_row0 + term * a.lo_row0;
-                    if (!a.tiles) {
-                        tma_load_2d(dst, &tmap_x, &sh->b_full[s], kx, y);
-                        continue;
-                    }
-                    int r = 0;  // grouped: whole boxes of 64 tokens, then of 16
-                    for (; r + 64 <= n; r += 64) tma_load_2d(dst + (size_t)r * 128, &tmap_w2, &sh->b_full[s], kx, y + r);
-                    for (; r < n; r += 16) tma_load_2d(dst + (size_t)r * 128, &tmap_x, &sh->b_full[s], kx, y + r);
-                }
+                if (old >= 0 && !__all_sync(0xffffffffu, mbar_wait(&sh->done[old & 3], (uint32_t)((old >> 2) & 1), sh, a.status, 21, (uint32_t)ks))) break;
                 issued = ks + 1;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&sh->b_full[s], bytes);
+                    uint8_t* dst = b_tiles + (size_t)s * b_stage;  // [term][group][n][64]
+                    for (int term = 0; term < a.x_terms; term++, dst += (size_t)n * 128 * a.groups)
+                        tma_load_3d(dst, tmap_x, &sh->b_full[s], 0, x_row0 + term * a.lo_row0, sb0 * SB_G + ks * a.groups);
+                }
+                __syncwarp();
                 if (++s == a.n_b) s = 0;
             }
             if (sh->abort_flag)  // copies in flight land before the shared memory goes away
@@ -258,23 +179,26 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         }
     } else if (warp == 10) {
         // ---------------- packed weights ----------------
-        if (lane == 0) {
+        {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
             const int copies = BYTE_ROWS ? 2 * nsb : nsb;
             int issued = 0;
             for (int c = 0, s = 0, ph = 0; c < copies; c++) {
-                if (!mbar_wait(&sh->raw_empty[s], (uint32_t)(ph ^ 1), sh, a.status, 23, (uint32_t)c)) break;
-                mbar_arrive_expect_tx(&sh->raw_full[s], (uint32_t)RAW_SLOT);
-                uint8_t* dst = raw + (size_t)s * RAW_SLOT;
-                if constexpr (FMT == B2_FMT_Q6_K) {  // [128][128] low nibbles, then [128][64] high bit pairs
-                    tma_load_2d(dst, &tmap_w, &sh->raw_full[s], (sb0 + c) * 128, w_row0 + n0);
-                    tma_load_2d(dst + WT_ROWS * 128, &tmap_w2, &sh->raw_full[s], (sb0 + c) * 64, w_row0 + n0);
-                } else if constexpr (BYTE_ROWS) {
-                    tma_load_2d(dst, &tmap_w, &sh->raw_full[s], (sb0 * 2 + c) * 64, w_row0 + n0);
-                } else {
-                    tma_load_2d(dst, &tmap_w, &sh->raw_full[s], (sb0 + c) * 144, w_row0 + n0);
-                }
+                if (!__all_sync(0xffffffffu, mbar_wait(&sh->raw_empty[s], (uint32_t)(ph ^ 1), sh, a.status, 23, (uint32_t)c))) break;
                 issued = c + 1;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&sh->raw_full[s], (uint32_t)RAW_SLOT);
+                    uint8_t* dst = raw + (size_t)s * RAW_SLOT;
+                    if constexpr (FMT == B2_FMT_Q6_K) {  // [128][128] low nibbles, then [128][64] high bit pairs
+                        tma_load_2d(dst, &tmap_w, &sh->raw_full[s], (sb0 + c) * 128, w_row0 + n0);
+                        tma_load_2d(dst + WT_ROWS * 128, &tmap_w2, &sh->raw_full[s], (sb0 + c) * 64, w_row0 + n0);
+                    } else if constexpr (BYTE_ROWS) {
+                        tma_load_2d(dst, &tmap_w, &sh->raw_full[s], (sb0 * 2 + c) * 64, w_row0 + n0);
+                    } else {
+                        tma_load_2d(dst, &tmap_w, &sh->raw_full[s], (sb0 + c) * 144, w_row0 + n0);
+                    }
+                }
+                __syncwarp();
                 if (++s == a.n_raw) s = 0, ph ^= 1;
             }
             if (sh->abort_flag)
@@ -283,15 +207,12 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         }
     } else if (warp == 9) {
         // ---------------- instructions ----------------
-        // The warp stays together: every lane waits, one elected lane issues (in a branch of one lane the four instructions and the
-        // commit of 64 k take 550 cycles, this way 250).
         const uint32_t idesc = (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
         const uint64_t bdesc0 = smem_desc_sw128(smem_u32(b_tiles));
-        const uint32_t lo = (uint32_t)(n * 128) >> 4;  // the second term's tile, in descriptor units
+        const uint32_t tile = (uint32_t)(n * 128) >> 4, lo = tile * (uint32_t)a.groups;  // a group's tile, the second terms: in descriptor units
         bool ok = true;
         for (int ks = 0, sa = 0, pa = 0, s = 0, ph = 0; ks < nks; ks++) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&sh->b_full[s], (uint32_t)ph, sh, a.status, 25, (uint32_t)ks) &&
-                                             mbar_wait(&sh->a_full[sa], (uint32_t)pa, sh, a.status, 26, (uint32_t)ks));
+            ok = __all_sync(0xffffffffu, mbar_wait_both(&sh->b_full[s], (uint32_t)ph, &sh->a_full[sa], (uint32_t)pa, sh, a.status, 25, (uint32_t)ks));
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) {
@@ -306,7 +227,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     }
                 };
                 group(at, bdesc, ks == 0);
-                if (a.groups == 2) group(at + 32, bdesc + lo * (uint32_t)a.x_terms, false);
+                if (a.groups == 2) group(at + 32, bdesc + tile, false);
                 mma_commit(&sh->done[ks & 3]);
             }
             __syncwarp();
@@ -369,34 +290,10 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 slot += 2;
                 if (slot >= a.n_raw) slot -= a.n_raw, ph ^= 1;
                 uint32_t o[32];
-                if constexpr (FMT == B2_FMT_Q8_0) {
-                    const __half2 m0 = __float2half2_rn(__half2float(__ushort_as_half((unsigned short)(sc & 0xffffu))) * PRE);
-                    const __half2 m1 = __float2half2_rn(__half2float(__ushort_as_half((unsigned short)(sc >> 16))) * PRE);
-                    const __half2 bias = __float2half2_rn(1152.0f);  // 1024 under the exponent byte 0x64, and 128
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const uint32_t wds[4] = {q[c].x, q[c].y, q[c].z, q[c].w};
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const uint32_t u = wds[i] ^ 0x80808080u;
-                            o[8 * c + 2 * i] = h2_bits(__hmul2(__hsub2(as_h2(__byte_perm(u, 0x64646464u, 0x4140)), bias), c < 2 ? m0 : m1));
-                            o[8 * c + 2 * i + 1] = h2_bits(__hmul2(__hsub2(as_h2(__byte_perm(u, 0x64646464u, 0x4342)), bias), c < 2 ? m0 : m1));
-                        }
-                    }
-                } else {
-                    const __half2 sc2 = __float2half2_rn((a.s ? __uint_as_float(sc) : 1.0f) * PRE);
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const uint32_t wds[4] = {q[c].x, q[c].y, q[c].z, q[c].w};
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            __half2_raw h01 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(wds[i] & 0xffff), __NV_E4M3);
-                            __half2_raw h23 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(wds[i] >> 16), __NV_E4M3);
-                            o[8 * c + 2 * i] = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&h01), sc2));
-                            o[8 * c + 2 * i + 1] = h2_bits(__hmul2(*reinterpret_cast<__half2*>(&h23), sc2));
-                        }
-                    }
-                }
+                if constexpr (FMT == B2_FMT_Q8_0)
+                    expand_q8_0(q, sc, o);
+                else
+                    expand_f8(q, a.s ? __uint_as_float(sc) : 1.0f, o);
                 put(g, o);
                 if (!ok) break;
             }
@@ -427,25 +324,10 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 for (int c = 0; c < 2; c++) qh4[c] = my_qh[((uint32_t)(2 * set + c)) ^ swh];
                 release_raw(&sh->raw_empty[slot], ql4[0].x | ql4[1].x | ql4[2].x | ql4[3].x | qh4[0].x | qh4[1].x, a.zero, lane);
                 if (++slot == a.n_raw) slot = 0, ph ^= 1;
-                const uint32_t qlw[16] = {ql4[0].x, ql4[0].y, ql4[0].z, ql4[0].w, ql4[1].x, ql4[1].y, ql4[1].z, ql4[1].w,
-                                          ql4[2].x, ql4[2].y, ql4[2].z, ql4[2].w, ql4[3].x, ql4[3].y, ql4[3].z, ql4[3].w};
-                const uint32_t qhw[8] = {qh4[0].x, qh4[0].y, qh4[0].z, qh4[0].w, qh4[1].x, qh4[1].y, qh4[1].z, qh4[1].w};
-                const __half2 bias = __float2half2_rn(1056.0f);  // 1024 under the exponent byte 0x64, and 32
 #pragma unroll
                 for (int odd = 0; odd < 2; odd++) {
-                    __half2 mul[4];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) mul[i] = __float2half2_rn(d * (float)(int8_t)(sc8[odd] >> (8 * i)) * PRE);
                     uint32_t o[32];
-#pragma unroll
-                    for (int i = 0; i < 16; i++) {  // word i: elements 4 i .. 4 i + 3 of the group
-                        const uint32_t nib = odd ? (qlw[i] >> 4) & 0x0F0F0F0Fu : qlw[i] & 0x0F0F0F0Fu;
-                        const int at = 4 * odd + 2 * (i >> 3);  // the bit pair's place in its byte; it goes to bits 4 and 5
-                        const uint32_t hb = (at < 4 ? qhw[i & 7] << (4 - at) : qhw[i & 7] >> (at - 4)) & 0x30303030u;
-                        const uint32_t q4 = nib | hb;
-                        o[2 * i] = h2_bits(__hmul2(__hsub2(as_h2(__byte_perm(q4, 0x64646464u, 0x4140)), bias), mul[i >> 2]));
-                        o[2 * i + 1] = h2_bits(__hmul2(__hsub2(as_h2(__byte_perm(q4, 0x64646464u, 0x4342)), bias), mul[i >> 2]));
-                    }
+                    expand_q6k(ql4, qh4, d, sc8[odd], odd, o);
                     put(sb * 4 + 2 * set + odd, o);
                     if (!ok) break;
                 }
@@ -500,7 +382,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 float f[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++)
-                    f[i] = (PRE_SCALED ? 1.0f / PRE : 1.0f) * (a.row_unscale && c + i < count ? __ldg(a.row_unscale + x_row0 + c + i) : 1.0f);
+                    f[i] = (PRE_SCALED ? 1.0f / WT_PRE : 1.0f) * (a.row_unscale && c + i < count ? __ldg(a.row_unscale + x_row0 + c + i) : 1.0f);
                 if (live) {
                     const size_t at = (size_t)(x_row0 + c) * a.y_ld + n0 + r;
                     if (plain) {
@@ -528,7 +410,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             const bool vec = !a.y_bf16 && a.n_more == 0 && (a.y_ld & 3) == 0 && ((uintptr_t)a.y & 15) == 0 && row + 4 <= a.n_out;
             for (int tok = part * 8 + warp; tok < count; tok += 8 * a.splits) {
                 const uint32_t at = sums + (uint32_t)(tok * WT_ROWS + 4 * lane) * 4u;
-                const float f = (PRE_SCALED ? 1.0f / PRE : 1.0f) * (a.row_unscale ? __ldg(a.row_unscale + x_row0 + tok) : 1.0f);
+                const float f = (PRE_SCALED ? 1.0f / WT_PRE : 1.0f) * (a.row_unscale ? __ldg(a.row_unscale + x_row0 + tok) : 1.0f);
                 float4 u[8];
 #pragma unroll
                 for (int p = 0; p < 8; p++) {
@@ -592,22 +474,31 @@ int wt_splits(size_t K) {
     return s;
 }
 
+bool gemm_x_maps(XMaps* x, int first, int last, const void* x16, size_t rows, size_t n_in, int groups) {
+    TensorMapEncodeFn enc = tensor_map_encode();
+    cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(n_in / 64)};
+    cuuint64_t strides[2] = {(cuuint64_t)n_in * 2, 128};
+    cuuint32_t estr[3] = {1, 1, 1};
+    for (int i = first; enc && i <= last; i++) {
+        cuuint32_t box[3] = {64, (cuuint32_t)(16 * (i + 1)), (cuuint32_t)groups};
+        if (enc(&x->m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void*)x16, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    }
+    return enc != nullptr;
+}
+
 bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x16, size_t x_rows, size_t tokens, int x_terms, size_t lo_row0, bool two_term_w, bool grouped) {
     TensorMapEncodeFn enc = tensor_map_encode();
     if (!enc) return false;
-    if (grouped && w.fmt != B2_FMT_MLX4 && w.fmt != B2_FMT_Q4_K) return false;  // (w2 is then the longer box of x)
     g->n_max = (int)std::min<size_t>(128, (tokens + 15) / 16 * 16);
     g->splits = grouped ? 1 : wt_splits(w.n_in);
     g->x_terms = x_terms;
     g->lo_row0 = (int)lo_row0;
     g->two_term_w = two_term_w;
-    auto x_map = [&](CUtensorMap* m, int box) {
-        return encode_2d(enc, m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x16, w.n_in, x_rows, w.n_in * 2, 64, (uint32_t)box, CU_TENSOR_MAP_SWIZZLE_128B);
-    };
-    CUresult r = x_map(&g->x, grouped ? 16 : g->n_max);
+    CUresult r;
     const size_t rows = w.n_out * experts;
     const CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
-    if (r != CUDA_SUCCESS) return false;
     if (w.fmt == B2_FMT_Q6_K) {
         r = encode_2d(enc, &g->w, u8, w.p0, w.n_in / 2, rows, w.n_in / 2, 128, WT_ROWS, CU_TENSOR_MAP_SWIZZLE_128B);
         if (r == CUDA_SUCCESS) r = encode_2d(enc, &g->w2, u8, w.p1, w.n_in / 4, rows, w.n_in / 4, 64, WT_ROWS, CU_TENSOR_MAP_SWIZZLE_64B);
@@ -618,7 +509,6 @@ bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x
         const size_t row = w.n_in / 256 * 144;
         r = encode_2d(enc, &g->w, u8, w.p0, row, rows, row, 144, WT_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE);
         g->w2 = g->w;
-        if (r == CUDA_SUCCESS && grouped) r = x_map(&g->w2, 64);
     }
     if (r != CUDA_SUCCESS) return false;
     // The rings in what two CTAs per SM leave: stages of 128 k (a stage costs the issuing warp about 400 cycles besides its instructions)
@@ -627,6 +517,7 @@ bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x
     const size_t slot = raw_slot_bytes(w.fmt), tile = (size_t)g->n_max * 128 * x_terms, room = WT_SMEM_MAX - sizeof(WtShared) - 128 - 1024;
     const int least = bytes ? 4 : 2, most = bytes ? WT_MAX_RING : 5;
     g->groups = two_term_w || 4 * tile + (size_t)least * slot > room ? 1 : 2;
+    if (!gemm_x_maps(&g->x, grouped ? 0 : g->n_max / 16 - 1, g->n_max / 16 - 1, x16, x_rows, w.n_in, g->groups)) return false;
     g->n_a = g->n_max <= 64 ? 3 : 2;
     g->n_b = (int)std::min<size_t>(4, (room - (size_t)least * slot) / (tile * g->groups));
     if (g->n_b < 2) return false;
@@ -638,7 +529,7 @@ bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x
 
 cudaError_t launch_gemm_wt(const GemmWt& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
                            GemmStatus* status, const float* row_unscale, cudaStream_t st) {
-    using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, WtArgs);
+    using Kern = void (*)(XMaps, CUtensorMap, CUtensorMap, WtArgs);
     Kern kern = w.fmt == B2_FMT_Q6_K     ? gemm_wt_kernel<B2_FMT_Q6_K, false>
                 : w.fmt == B2_FMT_Q8_0   ? gemm_wt_kernel<B2_FMT_Q8_0, false>
                 : w.fmt == B2_FMT_MLX4   ? gemm_wt_kernel<B2_FMT_MLX4, false>

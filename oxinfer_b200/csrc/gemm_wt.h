@@ -1,4 +1,4 @@
-// Host side of gemm_wt.cu: dequant-GEMM with the weights in tensor memory and the tokens on the instruction's N side.
+// Host side of gemm_wt.cu and gemm_wp.cu: dequant-GEMM with the weights in tensor memory and the tokens on the instruction's N side.
 #pragma once
 #include <cuda.h>
 
@@ -10,8 +10,14 @@ typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint3
                                       const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 TensorMapEncodeFn tensor_map_encode();  // cuTensorMapEncodeTiled, or null (gemm_tc.cu)
 
+// Maps of f16 activations [rows][n_in] as [n_in / 64][rows][64]: map i copies 16 (i + 1) rows of one or two groups of 64 k, group by group.
+// (One copy a stage: the copying warp issues one in about 100 cycles.)
+struct XMaps {
+    CUtensorMap m[8];
+};
 struct GemmWt {
-    CUtensorMap x, w, w2;
+    XMaps x;
+    CUtensorMap w, w2;  // (w2: Q6_K's second plane)
     int n_max = 0, splits = 1, x_terms = 1, lo_row0 = 0, n_raw = 0, n_b = 0, n_a = 0, groups = 1;
     bool two_term_w = false;
     size_t smem = 0;
@@ -25,5 +31,17 @@ bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x
 // copies of an f32 y.
 cudaError_t launch_gemm_wt(const GemmWt& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
                            GemmStatus* status, const float* row_unscale, cudaStream_t st);
+// Maps first .. last of a set, `groups` of 64 k a copy.
+bool gemm_x_maps(XMaps* x, int first, int last, const void* x16, size_t rows, size_t n_in, int groups);
+
+// The CTA-pair form (gemm_wp.cu), one-term operands. A grouped launch's tiles hold up to WP_MOST_ROWS rows.
+constexpr int WP_MOST_ROWS = 160;
+struct GemmWp {
+    XMaps x;
+    CUtensorMap w, w2;
+};
+bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, const void* x16, size_t x_rows);
+cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
+                           GemmStatus* status, int sm_count, const float* row_unscale, cudaStream_t st);
 
 }  // namespace b2

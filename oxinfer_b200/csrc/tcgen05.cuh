@@ -86,6 +86,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, Shared
     }
 }
 
+// Both barriers (a warp's wait for two operands: the two tests overlap).
+template <typename Shared>
+__device__ __forceinline__ bool mbar_wait_both(uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1, Shared* sh, GemmStatus* status, uint32_t where, uint32_t iter) {
+    const bool r0 = mbar_try_wait(bar0, parity0), r1 = mbar_try_wait(bar1, parity1);
+    return (r0 || mbar_wait(bar0, parity0, sh, status, where, iter)) && (r1 || mbar_wait(bar1, parity1, sh, status, where + 1, iter));
+}
+
+// True in one lane of a whole warp. A warp that issues copies or instructions stays together: every lane waits, one elected lane issues.
+// (In a branch of one lane, `if (lane == 0)`, four instructions and a commit took 550 cycles, behind elect.sync 250.)
+__device__ __forceinline__ bool elect_one() {  // true in one lane of a whole warp
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -103,6 +117,19 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
         "l"(map), "r"(cluster_bar), "r"(x), "r"(y)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(cluster_bar), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
 
