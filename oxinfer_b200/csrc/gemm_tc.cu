@@ -910,6 +910,18 @@ static CUresult encode_q6k_qh(TensorMapEncodeFn enc, CUtensorMap* m, const Weigh
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
+// Whether more than 128 one-term tokens take gemm_wp.cu. Both forms are estimated in cycles; here a CTA takes 64 k of 256 tokens in about 1130
+// cycles (more where the expansion is longer) whatever its width, and the last wave counts whole. Measured, us, here / there: Q4_K 14336 x
+// 4096, 200 tokens 47 / 35, 256: 49 / 38, 512: 54 / 59 (one whole wave here), 2048: 213 / 197; 4096 x 14336, 700 tokens 132 / 90; 8192 x
+// 4096, 1000 tokens 59 / 64; Q6_K 4096 x 4096, 4000 tokens 162 / 143; FP8 there 129 / 132; Q8_0 8192 x 1024, 4000 tokens 81 / 94 (the sums
+// of a segment leave as slowly after 8 stages as after 32). The bits are the same.
+static bool pairs_are_faster(GemmWp* g, const WeightDev& w, size_t t, int sm_count) {
+    const int m_tiles = (int)((t + 255) / 256), tile_n = pick_tile_n(w.n_out, m_tiles, sm_count, w.n_in, w.fmt == B2_FMT_Q6_K ? Q6K_MAX_TILE_N : MAX_TILE_N);
+    const size_t tiles = (w.n_out + tile_n - 1) / tile_n * (size_t)m_tiles, waves = (tiles + sm_count - 1) / sm_count;
+    const double stage = w.fmt == B2_FMT_Q6_K ? 1400.0 : w.fmt == B2_FMT_F8E4M3 ? 1080.0 : 1130.0;
+    return gemm_wp_share(g, w.n_out, t, w.n_in, sm_count) + 6000.0 < waves * (w.n_in / 64) * stage + 8000.0;
+}
+
 cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, void* y, int y_dtype, GemmPlan** out, char* err,
                                 size_t errlen, int force_m_halves, size_t a_lo_row0, int w_terms,
                                 const GemmPeerY* peer_y) {
@@ -947,15 +959,20 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (w_terms == 2 && w.fmt != B2_FMT_Q4_K) w_terms = 1;  // the other formats' weights round to f16 far below the bound
     p->w_terms = w_terms;
-    if (w_terms == 1 && t <= WT_MOST && split_k_asked() == 1 && ((uintptr_t)w.p2 & 7) == 0) {
-        p->wt_form = t <= WT_MOST ? 1 : 2;
+    if (w_terms == 1 && split_k_asked() == 1 && ((uintptr_t)w.p2 & 7) == 0) {
+        if (t <= WT_MOST)
+            p->wt_form = 1;
+        else if (!a_lo_row0 && !pair_form_enabled() && pairs_are_faster(&p->wp, w, t, sm_count))
+            p->wt_form = 2;
+    }
+    if (p->wt_form) {
         p->split_asked = 1;
         p->pair_asked = pair_form_enabled();
         p->y_ld = gathered ? peer_y->ld : 0;
         p->n_more = gathered ? peer_y->n_more : 0;
         for (int d = 0; d < p->n_more; d++) p->more_ptr[d] = peer_y->more[d];
         if (!(p->wt_form == 1 ? gemm_wt_encode(&p->wt, w, 1, x16, a_lo_row0 ? a_lo_row0 + t : t, t, a_lo_row0 ? 2 : 1, a_lo_row0, false, false)
-                              : gemm_wp_encode(&p->wp, w, 1, x16, t))) {
+                              : gemm_wp_encode(&p->wp, w, 1, false, x16, t, sm_count, y, y_dtype, p->y_ld ? p->y_ld : w.n_out))) {
             snprintf(err, errlen, "the tensor maps of a product could not be made");
             delete p;
             return cudaErrorInvalidValue;
@@ -1108,10 +1125,10 @@ bool gemm_tc_plan_matches(const GemmPlan* p, const WeightDev& w, const void* x16
            p->split_asked == split_k_asked() && p->pair_asked == pair_form_enabled();
 }
 
-cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, int y_dtype, GemmStatus* status_dev, int sm_count,
+cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, int y_dtype, GemmStatus* status_dev, int /*sm_count*/,
                            cudaStream_t st, const float* row_unscale) {
     if (p->wt_form == 2)
-        return launch_gemm_wp(p->wp, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, p->more_ptr, p->n_more, status_dev, sm_count, row_unscale, st);
+        return launch_gemm_wp(p->wp, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, p->more_ptr, p->n_more, status_dev, row_unscale, st);
     if (p->wt_form)
         return launch_gemm_wt(p->wt, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, p->more_ptr, p->n_more, status_dev, row_unscale, st);
     const bool split = p->k_splits > 1;

@@ -2,16 +2,17 @@
 //
 //   y[t][n_out] = x[t][K] * W^T      (one-term f16 operands, f32 sums; the operands and the order of the sums of gemm_wt.cu)
 //
-// A pair of CTAs (tcgen05 cta_group::2, M = 256) multiplies 256 weight rows by a segment of up to 160 tokens over the whole K: each CTA
-// expands 128 of the rows into its own tensor memory (the A operand) and copies half of the segment's tokens into its shared memory
-// (half of the B operand). The pairs are persistent and share the work out evenly:
-// the units (row block, 32 tokens) are one list of which every pair takes an equal run, cut into segments at the ends of row blocks.
+// A pair of CTAs (tcgen05 cta_group::2, M = 256) multiplies 256 weight rows by a segment of up to 256 tokens over the whole K: each CTA
+// expands 128 of the rows into its own tensor memory (the A operand, a ring of slots of 128 k) and copies half of the segment's
+// tokens into its shared memory (half of the B operand). The pairs are persistent; Segments says what each of them takes.
 //   warps 0..15  : dequantizers, four sets of four warps, a thread per weight row; set s takes every fourth group of 64 k.
-//   warps 16..19 : epilogue. The accumulator is double (2 x 160 columns), so a segment's sums leave while the next one is multiplied.
+//   warps 16..19 : epilogue, through staging tiles and the copy engine.
 //   warp 20      : copies the activations; warp 21 of the even CTA issues the instructions; warp 22 copies the packed weights.
-// What bounds it: the form it replaces (tokens on M, expanded weights through shared memory) used 1250 cycles of shared memory a stage of
-// 64 k for 830 cycles of tensor cores, in tiles that leave half of a last wave idle (14336 x 512 tokens: 138 CTAs of 148). Here
-// shared memory works two thirds as long as the tensor cores.
+// What bounds it: a stage of 128 k takes the tensor cores 4 cycles a token and the dequantizers about 780 cycles whatever the tokens, and the
+// sums of a segment leave at the rate of the L2 (8000 cycles for 256 tokens when all CTAs store at once). Two layouts of tensor memory: two
+// accumulators of 160 tokens, whose sums leave while the next segment is multiplied (grouped launches: many short segments), or one of 256
+// (in halves, for short segments in turn), bound by the tensor cores until its sums leave (dense launches).
+// (The form with tokens on M, gemm_tc.cu, needs 1250 cycles of shared memory for 830 of tensor cores.)
 //
 // A CTA takes all 512 columns of tensor memory and more than half of the shared memory, so it has its SM to itself.
 #include <cuda.h>
@@ -27,30 +28,36 @@ namespace b2 {
 namespace {
 
 constexpr int WP_THREADS = 736, WP_ROWS = 128, WP_SEG = WP_MOST_ROWS, WP_UNIT = 32;
-constexpr int WP_NB = 4;                                        // activation stages of 128 k x 80 tokens
-constexpr uint32_t WP_B_STAGE = WP_SEG / 2 * 256;
-constexpr uint32_t WP_A_COL = 2 * WP_SEG, WP_SLOT_COLS = 64;    // two accumulators, then the A slots of 128 k
-constexpr int WP_NA = (512 - 2 * WP_SEG) / 64;
+constexpr uint32_t WP_SLOT_COLS = 64;                           // an A slot of 128 k; the slots are tensor memory's last columns
+constexpr int WP_TWO = WP_TILE_ROWS;                            // longest segment of the layout with two accumulators
+// The two layouts: A slots, activation stages of 128 k, and what the epilogue stages its results in (two tiles of 32 tokens x 32 rows a warp).
+__host__ __device__ constexpr int wp_n_a(bool two) { return two ? 3 : 4; }
+__host__ __device__ constexpr int wp_n_b(bool two) { return two ? 4 : 3; }
+__host__ __device__ constexpr uint32_t wp_b_stage(bool two) { return (two ? WP_TWO : WP_SEG) / 2 * 256; }
+__host__ __device__ constexpr uint32_t wp_staging(bool two) { return two ? 0 : 4 * 2 * 4096; }
 __host__ __device__ constexpr int wp_raw_slot(int fmt) { return WP_ROWS * (fmt == B2_FMT_F8E4M3 || fmt == B2_FMT_Q8_0 ? 64 : fmt == B2_FMT_Q6_K ? 192 : 144); }
-__host__ __device__ constexpr int wp_n_raw(int fmt) { return fmt == B2_FMT_F8E4M3 || fmt == B2_FMT_Q8_0 ? 16 : 6; }
+__host__ __device__ constexpr int wp_n_raw(int fmt, bool two) { return two ? 8 : fmt == B2_FMT_F8E4M3 || fmt == B2_FMT_Q8_0 ? 12 : fmt == B2_FMT_Q6_K ? 4 : 5; }
 
 struct __align__(8) WpShared {
-    uint64_t a_full[WP_NA];        // even CTA: both CTAs' dequantizers
-    uint64_t b_full[WP_NB];        // even CTA: both CTAs' copies
+    uint64_t a_full[4];            // even CTA: both CTAs' dequantizers
+    uint64_t b_full[4];            // even CTA: both CTAs' copies
     uint64_t done[4];              // each CTA: the instructions of stage i (mod 4) have completed
     uint64_t raw_full[16], raw_empty[16];
-    uint64_t acc_full[2];          // each CTA
-    uint64_t acc_empty[2];         // even CTA: both CTAs' epilogues
+    uint64_t acc_full[2];          // each CTA, [half]: the sums of the segment that starts there
+    uint64_t acc_empty[2];         // even CTA, [half]: both CTAs' epilogues have read it
     uint32_t tmem_base;
     volatile uint32_t abort_flag;
 };
-constexpr size_t wp_smem(int fmt) { return 1024 + (size_t)WP_NB * WP_B_STAGE + (size_t)wp_n_raw(fmt) * wp_raw_slot(fmt); }
-static_assert(wp_smem(B2_FMT_Q4_K) + sizeof(WpShared) <= 227 * 1024 && wp_smem(B2_FMT_Q6_K) + sizeof(WpShared) <= 227 * 1024 &&
-              wp_smem(B2_FMT_Q8_0) + sizeof(WpShared) <= 227 * 1024, "shared memory budget");
+constexpr size_t wp_smem(int fmt, bool two) {
+    return 1024 + (size_t)wp_n_b(two) * wp_b_stage(two) + (size_t)wp_n_raw(fmt, two) * wp_raw_slot(fmt) + wp_staging(two);
+}
+static_assert(wp_smem(B2_FMT_Q4_K, false) + sizeof(WpShared) <= 227 * 1024 && wp_smem(B2_FMT_Q6_K, false) + sizeof(WpShared) <= 227 * 1024 &&
+              wp_smem(B2_FMT_Q8_0, false) + sizeof(WpShared) <= 227 * 1024 && wp_smem(B2_FMT_MLX4, true) + sizeof(WpShared) <= 227 * 1024, "shared memory budget");
 
 struct WpArgs {
     int K, n_out, t;
-    int y_bf16, zero;
+    int pieces, snap;     // dense: how the work is shared out (Segments)
+    int y_bf16, zero, staged;  // staged: results leave through tmap_y
     size_t y_ld;
     void* y;
     GemmStatus* status;
@@ -64,49 +71,85 @@ struct WpArgs {
     float* more[7];
 };
 
-// The segments of a pair, the same for every role of both CTAs.
+// The segments of a pair, the same for every role of both CTAs. Grouped launches: every tile with every row block, dealt out in turn.
+// Dense: per row block of 256, `pieces` equal segments dealt out in turn, or (pieces 0) one list of units of 32 tokens of which every pair
+// takes an equal run, cut at the ends of row blocks; a run's end within `snap` units of a row block's end is moved there.
 struct Segments {
-    int pos, end, per_block, blocks;
+    int pos, end, step, per_block, blocks, pieces;
     int row, w_row, x_row0, n, count;  // first of the 256 rows in its matrix / in the stack; tokens: first, padded to 32, real
-    __device__ __forceinline__ Segments(const WpArgs& a) {
-        const int c = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-        blocks = (a.n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
-        per_block = (a.t + WP_UNIT - 1) / WP_UNIT;
-        if (a.tiles) {
-            pos = c;
-            end = a.n_tiles * blocks;
-        } else {
-            // (a run that would end or start within a unit or two of a row block's end is moved there: a segment of 32 tokens takes as
-            // long as one of 128)
-            const long long units = (long long)blocks * per_block;
-            auto bound = [&](int i) {
-                const int p = (int)(units * i / pairs), u = p % per_block;
-                return per_block < 8 ? p : u <= 2 ? p - u : per_block - u <= 2 ? p - u + per_block : p;
-            };
-            pos = bound(c);
-            end = bound(c + 1);
+    __host__ __device__ __forceinline__ Segments(int n_out, int t, int n_tiles, int pieces_, int snap, int c, int pairs) : pieces(pieces_) {
+        blocks = (n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
+        per_block = (t + WP_UNIT - 1) / WP_UNIT;
+        pos = c;
+        step = pairs;
+        end = n_tiles ? n_tiles * blocks : pieces * blocks;
+        if (!n_tiles && !pieces) {
+            pos = bound(c, pairs, snap);
+            end = bound(c + 1, pairs, snap);
         }
     }
-    __device__ __forceinline__ bool next(const WpArgs& a) {
+    __host__ __device__ __forceinline__ int bound(int i, int pairs, int snap) const {
+        const int p = (int)((long long)blocks * per_block * i / pairs), u = p % per_block;
+        return u <= snap ? p - u : per_block - u <= snap ? p - u + per_block : p;
+    }
+    __host__ __device__ __forceinline__ bool next(const WtTile* tiles, int n_out, int t) {
         if (pos >= end) return false;
-        if (a.tiles) {
-            const WtTile tile = a.tiles[pos / blocks];
+        if (tiles) {
+            const WtTile tile = tiles[pos / blocks];
             row = pos % blocks * (2 * WP_ROWS);
-            w_row = tile.expert * a.n_out + row;
+            w_row = tile.expert * n_out + row;
             x_row0 = tile.row0;
             count = tile.count;
             n = (count + WP_UNIT - 1) / WP_UNIT * WP_UNIT;
-            pos += gridDim.x >> 1;
+            pos += step;
+            return true;
+        }
+        int u, take;
+        if (pieces) {
+            const int p = pos % pieces;
+            row = pos / pieces * (2 * WP_ROWS);
+            u = per_block * p / pieces;
+            take = per_block * (p + 1) / pieces - u;
+            pos += step;
         } else {
-            const int u = pos % per_block, left = min(per_block - u, end - pos);
-            const int pieces = (left + WP_SEG / WP_UNIT - 1) / (WP_SEG / WP_UNIT), take = (left + pieces - 1) / pieces;
-            row = w_row = pos / per_block * (2 * WP_ROWS);
-            x_row0 = u * WP_UNIT;
-            n = take * WP_UNIT;
-            count = min(n, a.t - x_row0);
+            constexpr int most = WP_SEG / WP_UNIT;
+            u = pos % per_block;
+            const int left = per_block - u < end - pos ? per_block - u : end - pos, parts = (left + most - 1) / most;
+            take = (left + parts - 1) / parts;
+            row = pos / per_block * (2 * WP_ROWS);
             pos += take;
         }
+        w_row = row;
+        x_row0 = u * WP_UNIT;
+        n = take * WP_UNIT;
+        count = n < t - x_row0 ? n : t - x_row0;
         return true;
+    }
+};
+
+// The accumulators of a pair's segments, the same for the issuing warp and the epilogues. Two: in turn. One: segments of up to 128 tokens take
+// its halves in turn, longer ones both (`both`).
+template <bool TWO>
+struct Halves {
+    int turn = 0, uses[2] = {0, 0}, sums[2] = {0, 0};
+    int half;
+    uint32_t col;  // first column
+    bool both;
+    uint32_t empty_parity[2], full_parity;
+    __device__ __forceinline__ void next(int n) {
+        both = !TWO && n > 128;
+        half = both ? 0 : turn;
+        turn = both ? 0 : turn ^ 1;
+        col = half ? (TWO ? (uint32_t)WP_TWO : 128u) : 0u;
+        empty_parity[0] = (uint32_t)(uses[0] & 1) ^ 1u;
+        empty_parity[1] = (uint32_t)(uses[1] & 1) ^ 1u;
+        full_parity = (uint32_t)((half ? sums[1] : sums[0]) & 1);
+        if (both || half == 0) uses[0]++;
+        if (both || half == 1) uses[1]++;
+        if (half)
+            sums[1]++;
+        else
+            sums[0]++;
     }
 };
 
@@ -124,19 +167,21 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 
-template <int FMT>
+// TWO: the layout with two accumulators, for grouped launches; the other for dense ones.
+template <int FMT, bool TWO>
 __global__ void __launch_bounds__(WP_THREADS, 1)
 gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUtensorMap tmap_w,
-               const __grid_constant__ CUtensorMap tmap_w2, const __grid_constant__ WpArgs a) {
+               const __grid_constant__ CUtensorMap tmap_w2, const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ WpArgs a) {
     // A dependent launch: see gemm_wt.cu.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr bool BYTE_ROWS = FMT == B2_FMT_F8E4M3 || FMT == B2_FMT_Q8_0;
     constexpr bool PRE_SCALED = BYTE_ROWS || FMT == B2_FMT_Q6_K;
-    constexpr int NRAW = wp_n_raw(FMT), RAW_SLOT = wp_raw_slot(FMT);
+    constexpr int NRAW = wp_n_raw(FMT, TWO), RAW_SLOT = wp_raw_slot(FMT), NA = wp_n_a(TWO), NB = wp_n_b(TWO);
+    constexpr uint32_t B_STAGE = wp_b_stage(TWO);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* b_tiles = smem;
-    uint8_t* raw = smem + (size_t)WP_NB * WP_B_STAGE;
+    uint8_t* raw = smem + NB * B_STAGE;
     __shared__ WpShared shared;
     WpShared* sh = &shared;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -148,7 +193,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             mbar_init(&sh->acc_full[s], 1);
             mbar_init(&sh->acc_empty[s], 8);
         }
-        for (int s = 0; s < WP_NA; s++) mbar_init(&sh->a_full[s], 16);
+        for (int s = 0; s < 4; s++) mbar_init(&sh->a_full[s], 16);
         for (int s = 0; s < 4; s++) {
             mbar_init(&sh->b_full[s], 1);
             mbar_init(&sh->done[s], 1);
@@ -168,30 +213,30 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
     __syncthreads();
     cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
-    const uint32_t tmem = sh->tmem_base;
-    Segments seg(a);
+    const uint32_t tmem = sh->tmem_base, a_cols = tmem + 512u - NA * WP_SLOT_COLS;
+    Segments seg(a.n_out, a.t, a.tiles ? a.n_tiles : 0, a.pieces, a.snap, blockIdx.x >> 1, gridDim.x >> 1);
 
     if (warp == 20) {
         // ---------------- activations: this CTA's half of the segment's tokens ----------------
         {
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            int it = 0;
+            int it = 0, s = 0;
             bool ok = true;
-            while (ok && seg.next(a)) {
+            while (ok && seg.next(a.tiles, a.n_out, a.t)) {
                 const int half = seg.n / 2, y0 = seg.x_row0 + (int)rank * half;
                 const CUtensorMap* tmap_x = &maps.m[half / 16 - 1];
-                for (int ks = 0; ks < stages; ks++, it++) {
-                    const int old = it - WP_NB, s = it & (WP_NB - 1);
+                for (int ks = 0; ks < stages; ks++, it++, s = s + 1 == NB ? 0 : s + 1) {
+                    const int old = it - NB;
                     if (old >= 0) ok = __all_sync(0xffffffffu, mbar_wait(&sh->done[old & 3], (uint32_t)((old >> 2) & 1), sh, a.status, 41, (uint32_t)it));
                     if (!ok) break;
                     if (!elect_one()) continue;
                     if (rank == 0) mbar_arrive_expect_tx(&sh->b_full[s], (uint32_t)(seg.n * 256));
-                    tma_load_3d_pair(b_tiles + (size_t)s * WP_B_STAGE, tmap_x, cluster_addr(&sh->b_full[s], 0), 0, y0, 2 * ks);  // [group][tokens][64]
+                    tma_load_3d_pair(b_tiles + (size_t)s * B_STAGE, tmap_x, cluster_addr(&sh->b_full[s], 0), 0, y0, 2 * ks);  // [group][tokens][64]
                 }
             }
             __syncwarp();
             if (sh->abort_flag && rank == 0)  // (the odd CTA's copies are counted here too; the CTAs meet before the shared memory goes away)
-                for (int i = max(0, it - WP_NB); i < it; i++) mbar_wait(&sh->b_full[i & (WP_NB - 1)], (uint32_t)((i / WP_NB) & 1), sh, a.status, 42, (uint32_t)i, false);
+                for (int i = max(0, it - NB); i < it; i++) mbar_wait(&sh->b_full[i % NB], (uint32_t)((i / NB) & 1), sh, a.status, 42, (uint32_t)i, false);
         }
     } else if (warp == 22) {
         // ---------------- packed weights: this CTA's 128 rows ----------------
@@ -200,7 +245,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             const int copies = BYTE_ROWS ? groups : groups / 4;
             int issued = 0, s = 0, ph = 0;
             bool ok = true;
-            while (ok && seg.next(a)) {
+            while (ok && seg.next(a.tiles, a.n_out, a.t)) {
                 const int w_row = seg.w_row + (int)rank * WP_ROWS;
                 for (int c = 0; c < copies; c++, issued++) {
                     ok = __all_sync(0xffffffffu, mbar_wait(&sh->raw_empty[s], (uint32_t)(ph ^ 1), sh, a.status, 43, (uint32_t)issued));
@@ -229,24 +274,25 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             const uint64_t bdesc0 = smem_desc_sw128(smem_u32(b_tiles));
             const uint32_t done_of[2] = {cluster_addr(&sh->done[0], 0), cluster_addr(&sh->done[0], 1)};
             bool ok = true;
-            int it = 0, si = 0;
-            for (; ok && seg.next(a); si++) {
-                const int buf = si & 1;
-                const uint32_t acc = tmem + (uint32_t)(buf * WP_SEG);
+            int it = 0, sa = 0, pa = 0, s = 0, ph = 0;
+            Halves<TWO> acc_of;
+            while (ok && seg.next(a.tiles, a.n_out, a.t)) {
+                acc_of.next(seg.n);
+                const uint32_t acc = tmem + acc_of.col;
                 const uint32_t idesc = (1u << 4) | ((uint32_t)(seg.n >> 3) << 17) | ((256u >> 4) << 24);
                 const uint32_t group_b = (uint32_t)(seg.n / 2 * 128) >> 4;
-                ok = __all_sync(0xffffffffu, mbar_wait(&sh->acc_empty[buf], (uint32_t)(((si >> 1) & 1) ^ 1), sh, a.status, 45, (uint32_t)si));
+                ok = __all_sync(0xffffffffu, (!(acc_of.both || acc_of.half == 0) || mbar_wait(&sh->acc_empty[0], acc_of.empty_parity[0], sh, a.status, 45, (uint32_t)it)) &&
+                                                 (!(acc_of.both || acc_of.half == 1) || mbar_wait(&sh->acc_empty[1], acc_of.empty_parity[1], sh, a.status, 45, (uint32_t)it)));
                 if (!ok) break;
                 tc_fence_after();
                 for (int ks = 0; ks < stages; ks++, it++) {
-                    const int s = it & (WP_NB - 1), sa = it % WP_NA;
-                    ok = __all_sync(0xffffffffu, mbar_wait_both(&sh->b_full[s], (uint32_t)((it / WP_NB) & 1), &sh->a_full[sa], (uint32_t)((it / WP_NA) & 1), sh,
+                    ok = __all_sync(0xffffffffu, mbar_wait_both(&sh->b_full[s], (uint32_t)ph, &sh->a_full[sa], (uint32_t)pa, sh,
                                                                     a.status, 46, (uint32_t)it));
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
-                        const uint64_t bd = bdesc0 + (uint64_t)(((uint32_t)s * WP_B_STAGE) >> 4);
-                        const uint32_t at = tmem + WP_A_COL + (uint32_t)sa * WP_SLOT_COLS;
+                        const uint64_t bd = bdesc0 + (uint64_t)(((uint32_t)s * B_STAGE) >> 4);
+                        const uint32_t at = a_cols + (uint32_t)sa * WP_SLOT_COLS;
 #pragma unroll
                         for (int g = 0; g < 2; g++)
 #pragma unroll
@@ -255,11 +301,13 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                         mma_commit_pair(done_of[0] + (uint32_t)(it & 3) * 8u);
                         mma_commit_pair(done_of[1] + (uint32_t)(it & 3) * 8u);
                         if (ks == stages - 1) {
-                            mma_commit_pair(cluster_addr(&sh->acc_full[buf], 0));
-                            mma_commit_pair(cluster_addr(&sh->acc_full[buf], 1));
+                            mma_commit_pair(cluster_addr(&sh->acc_full[acc_of.half], 0));
+                            mma_commit_pair(cluster_addr(&sh->acc_full[acc_of.half], 1));
                         }
                     }
                     __syncwarp();
+                    if (++sa == NA) sa = 0, pa ^= 1;
+                    if (++s == NB) s = 0, ph ^= 1;
                 }
             }
             if (!ok && it > 0) mbar_wait(&sh->done[(it - 1) & 3], (uint32_t)(((it - 1) >> 2) & 1), sh, a.status, 48, 0, false);  // what was issued completes
@@ -270,13 +318,17 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
         const uint32_t acc_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const uint32_t empty_even = cluster_addr(&sh->acc_empty[0], 0);
         const bool plain = !a.y_bf16 && a.n_more == 0;
-        for (int si = 0; seg.next(a); si++) {
-            const int buf = si & 1, row = seg.row + (int)rank * WP_ROWS + (warp & 3) * 32 + lane;
+        uint8_t* staging = raw + (size_t)NRAW * RAW_SLOT + (size_t)(warp & 3) * 8192;
+        Halves<TWO> acc_of;
+        int tile = 0;
+        while (seg.next(a.tiles, a.n_out, a.t)) {
+            acc_of.next(seg.n);
+            const int row0 = seg.row + (int)rank * WP_ROWS + (warp & 3) * 32, row = row0 + lane;
             auto factor = [&](int c) {  // of token c + lane
                 return (PRE_SCALED ? 1.0f / WT_PRE : 1.0f) * (a.row_unscale && c + lane < seg.count ? __ldg(a.row_unscale + seg.x_row0 + c + lane) : 1.0f);
             };
             float next = factor(0);
-            if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_full[buf], (uint32_t)((si >> 1) & 1), sh, a.status, 49, (uint32_t)si) && !sh->abort_flag)) break;
+            if (!__all_sync(0xffffffffu, mbar_wait(&sh->acc_full[acc_of.half], acc_of.full_parity, sh, a.status, 49, (uint32_t)tile) && !sh->abort_flag)) break;
             tc_fence_after();
             // (a loop of one chunk: unrolled over the segment it is 24 KB of code that runs once a segment, at the rate of its instruction
             // fetches, 15000 cycles)
@@ -285,22 +337,51 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                 const float f = next;
                 next = factor(c + 32);
                 uint32_t v[32];
-                tmem_ld32(acc_lane + (uint32_t)(buf * WP_SEG + c), v);
+                tmem_ld32(acc_lane + acc_of.col + (uint32_t)c, v);
+                if (c == 96 && acc_of.both) {  // the first half is free
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_remote(empty_even);
+                }
+                const int live = seg.count - c;  // tokens to store
+                if (!TWO && a.staged) {  // (the copy engine leaves out what lies past t and n_out)
+                    uint8_t* buf = staging + (tile++ & 1) * 4096;
+                    if (elect_one()) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the store before the last has read this tile
+                    __syncwarp();
+                    if (a.y_bf16) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            ((__nv_bfloat16*)buf)[j * 32 + lane] = __float2bfloat16_rn(__uint_as_float(v[j]) * __shfl_sync(0xffffffffu, f, j));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) ((float*)buf)[j * 32 + lane] = __uint_as_float(v[j]) * __shfl_sync(0xffffffffu, f, j);
+                    }
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (elect_one()) {
+                        asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&tmap_y), "r"(smem_u32(buf)),
+                                     "r"(row0), "r"(seg.x_row0 + c)
+                                     : "memory");
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                    __syncwarp();
+                    continue;
+                }
                 const size_t at = (size_t)(seg.x_row0 + c) * a.y_ld + row;
-                const int live = row < a.n_out ? seg.count - c : 0;  // tokens to store
-                if (plain) {
+                const int rows = row < a.n_out ? live : 0;
+                if (TWO || plain) {
                     float* o = (float*)a.y + at;
 #pragma unroll
                     for (int j = 0; j < 32; j++, o += a.y_ld) {
                         const float w = __uint_as_float(v[j]) * __shfl_sync(0xffffffffu, f, j);
-                        if (j < live) *o = w;
+                        if (j < rows) *o = w;
                     }
                 } else {
 #pragma unroll
                     for (int j = 0; j < 32; j++) {
                         const float w = __uint_as_float(v[j]) * __shfl_sync(0xffffffffu, f, j);
                         const size_t o = at + (size_t)j * a.y_ld;
-                        if (j < live) {
+                        if (j < rows) {
                             if (a.y_bf16)
                                 ((__nv_bfloat16*)a.y)[o] = __float2bfloat16_rn(w);
                             else
@@ -312,18 +393,22 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_remote(empty_even + (uint32_t)buf * 8u);
+            if (lane == 0) mbar_arrive_remote(empty_even + (acc_of.both || acc_of.half == 1 ? 8u : 0u));
         }
+        if (elect_one()) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // the staging tiles have been read and written out
+        __syncwarp();
     } else {
         // ---------------- dequantizers ----------------
         const int set = warp >> 2, r = (warp & 3) * 32 + lane;
         const uint32_t swz = (uint32_t)(r & 7), swh = (uint32_t)((r >> 1) & 3);
-        const uint32_t a_lane = tmem + WP_A_COL + ((uint32_t)((warp & 3) * 32) << 16);
+        const uint32_t a_lane = a_cols + ((uint32_t)((warp & 3) * 32) << 16);
         const uint32_t full_even = cluster_addr(&sh->a_full[0], 0);
         bool ok = true;
         // 64 expanded weights, group g of the segment whose first stage is it0, to this lane of tensor memory
+        int stage_a = 0, sa = 0;  // (a set's groups come in ascending order)
         auto put = [&](int it0, int g, const uint32_t(&o)[32]) {
-            const int it = it0 + (g >> 1), old = it - WP_NA, sa = it % WP_NA;
+            const int it = it0 + (g >> 1), old = it - NA;
+            for (; stage_a < it; stage_a++) sa = sa + 1 == NA ? 0 : sa + 1;
             if (old >= 0) ok = __all_sync(0xffffffffu, mbar_wait(&sh->done[old & 3], (uint32_t)((old >> 2) & 1), sh, a.status, 50, (uint32_t)it));
             if (!ok) return;
             tc_fence_after();
@@ -337,7 +422,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             return ok;
         };
         int it0 = 0, slot = 0, ph = 0, base = 0;
-        for (; ok && seg.next(a); it0 += stages) {
+        for (; ok && seg.next(a.tiles, a.n_out, a.t); it0 += stages) {
             const int row = seg.row + (int)rank * WP_ROWS + r;
             const bool live = row < a.n_out;
             const size_t wrow = live ? (size_t)row : 0;
@@ -429,28 +514,81 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
 
 }  // namespace
 
-bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, const void* x16, size_t x_rows) {
+// How a dense launch is shared out, and what its slowest pair takes in cycles: a stage of 128 k max(780, 4 tokens), the sums of a segment
+// of more than 128 tokens 7500 (nothing is multiplied meanwhile).
+double gemm_wp_share(GemmWp* g, size_t n_out_, size_t t_, size_t n_in, int sm_count) {
+    const int n_out = (int)n_out_, t = (int)t_, stages = (int)(n_in / 128), units = (t + WP_UNIT - 1) / WP_UNIT, blocks = (n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
+    const int pairs = (int)std::min<long long>(std::max(1, sm_count / 2), (long long)blocks * units), most = WP_SEG / WP_UNIT, least = (units + most - 1) / most;
+    auto segment = [&](int n) { return stages * std::max(780.0, 4.0 * n) + (n > 128 ? 7500.0 : 500.0); };
+    double best = 1e30;
+    auto take = [&](int pieces, int snap) {
+        double cost = 0.0;
+        for (int c = 0; c < pairs && cost < best; c++) {
+            double sum = 0.0;
+            for (Segments s(n_out, t, 0, pieces, snap, c, pairs); s.next(nullptr, n_out, t);) sum += segment(s.n);
+            cost = std::max(cost, sum);
+        }
+        if (cost < best) {
+            best = cost;
+            g->pieces = pieces;
+            g->snap = snap;
+        }
+    };
+    g->pairs = pairs;
+    const long long run = (long long)blocks * units / pairs;
+    if (run <= 16) {
+        take(0, std::min(3, (units - 1) / 2));
+        take(0, 0);
+        take(least, 0);
+        if (least < units) take(least + 1, 0);
+    } else {  // (long runs are even enough, and the count of their segments would take long)
+        g->pieces = 0;
+        g->snap = std::min(3, (units - 1) / 2);
+        const long long segs = (run + 2 + most - 1) / most + (run < units ? 0 : run / units);
+        best = segs * segment((int)((run + segs) / segs) * WP_UNIT);
+    }
+    return best;
+}
+
+bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, bool grouped, const void* x16, size_t x_rows, int sm_count, void* y, int y_dtype, size_t y_ld) {
     GemmWt m;  // the weights' maps are gemm_wt.cu's (boxes of 128 rows)
     if (!gemm_wt_encode(&m, w, experts, x16, x_rows, 16, 1, 0, false, false)) return false;
     g->w = m.w;
     g->w2 = m.w2;
+    g->y = m.w;
+    const size_t esize = y_dtype == B2_BF16 ? 2 : 4;
+    g->staged = !grouped && y_ld * esize % 16 == 0 && ((uintptr_t)y & 15) == 0;
+    if (g->staged) {
+        cuuint64_t dims[2] = {(cuuint64_t)w.n_out, (cuuint64_t)x_rows};
+        cuuint64_t strides[1] = {(cuuint64_t)(y_ld * esize)};
+        cuuint32_t box[2] = {32, 32}, estr[2] = {1, 1};
+        if (tensor_map_encode()(&g->y, esize == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, y, dims, strides, box, estr,
+                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    }
+    if (grouped) g->pairs = std::max(1, sm_count / 2);
     return gemm_x_maps(&g->x, 0, WP_SEG / 32 - 1, x16, x_rows, w.n_in, 2);
 }
 
 cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
-                           GemmStatus* status, int sm_count, const float* row_unscale, cudaStream_t st) {
-    using Kern = void (*)(XMaps, CUtensorMap, CUtensorMap, WpArgs);
-    Kern kern = w.fmt == B2_FMT_Q6_K     ? gemm_wp_kernel<B2_FMT_Q6_K>
-                : w.fmt == B2_FMT_Q8_0   ? gemm_wp_kernel<B2_FMT_Q8_0>
-                : w.fmt == B2_FMT_MLX4   ? gemm_wp_kernel<B2_FMT_MLX4>
-                : w.fmt == B2_FMT_F8E4M3 ? gemm_wp_kernel<B2_FMT_F8E4M3>
-                                         : gemm_wp_kernel<B2_FMT_Q4_K>;
-    const size_t smem = wp_smem(w.fmt);
+                           GemmStatus* status, const float* row_unscale, cudaStream_t st) {
+    using Kern = void (*)(XMaps, CUtensorMap, CUtensorMap, CUtensorMap, WpArgs);
+    if (tiles && w.fmt != B2_FMT_MLX4) return cudaErrorInvalidValue;  // (Q4_K experts take two-term operands: gemm_wt.cu)
+    Kern kern = tiles                    ? gemm_wp_kernel<B2_FMT_MLX4, true>
+                : w.fmt == B2_FMT_Q6_K   ? gemm_wp_kernel<B2_FMT_Q6_K, false>
+                : w.fmt == B2_FMT_Q8_0   ? gemm_wp_kernel<B2_FMT_Q8_0, false>
+                : w.fmt == B2_FMT_MLX4   ? gemm_wp_kernel<B2_FMT_MLX4, false>
+                : w.fmt == B2_FMT_F8E4M3 ? gemm_wp_kernel<B2_FMT_F8E4M3, false>
+                                         : gemm_wp_kernel<B2_FMT_Q4_K, false>;
+    const size_t smem = wp_smem(w.fmt, tiles != nullptr);
     if (cudaError_t e = ensure_dynamic_smem((const void*)kern, smem, 0); e != cudaSuccess) return e;
     WpArgs a{};
     a.K = (int)w.n_in;
     a.n_out = (int)w.n_out;
     a.t = (int)t;
+    a.pieces = g.pieces;
+    a.snap = g.snap;
+    a.staged = g.staged && n_more == 0;
     a.y_bf16 = y_dtype == B2_BF16;
     a.y_ld = y_ld;
     a.y = y;
@@ -466,9 +604,8 @@ cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const 
     a.n_more = n_more;
     for (int i = 0; i < n_more; i++) a.more[i] = more[i];
     const size_t blocks = (w.n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
-    const size_t units = tiles ? blocks * (size_t)n_tiles : blocks * ((t + WP_UNIT - 1) / WP_UNIT);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(2 * std::min<size_t>(units, (size_t)std::max(1, sm_count / 2))));
+    cfg.gridDim = dim3((unsigned)(2 * (tiles ? std::min<size_t>(blocks * (size_t)n_tiles, (size_t)g.pairs) : (size_t)g.pairs)));
     cfg.blockDim = dim3(WP_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -480,7 +617,7 @@ cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const 
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, kern, g.x, g.w, g.w2, a);
+    return cudaLaunchKernelEx(&cfg, kern, g.x, g.w, g.w2, g.y, a);
 }
 
 }  // namespace b2

@@ -1,4 +1,4 @@
-"""Products of 9 to 128 tokens and the routed experts' segments: weights in tensor memory, tokens on the instruction's N side."""
+"""Products of more than eight tokens and the routed experts' segments: weights in tensor memory, tokens on the instruction's N side."""
 import numpy as np
 import pytest
 import torch
@@ -33,6 +33,31 @@ def test_products_of_up_to_128_tokens(backend, fmt, shape):
     y9 = np.zeros((9, n_out), np.float32)
     assert backend.matmul(x[t - 9 :], [ob.Job(dev, y9)])
     assert np.array_equal(y9, y[t - 9 :])
+    xd, yd = torch.from_numpy(x).cuda(), torch.zeros((t, n_out), device="cuda", dtype=torch.bfloat16)
+    assert backend.matmul_dev(dev, xd, yd)
+    torch.cuda.synchronize()
+    backend.check_status()
+    assert torch.equal(yd.cpu(), torch.from_numpy(y).bfloat16())
+
+
+# one token and one unit of 32 past what the smaller kernel takes, segments of 160, 256 and around them, rows that end inside a pair's 256 and
+# inside a CTA's 128, an odd number of super-blocks
+@pytest.mark.parametrize("fmt", ["mlx4", "q4_k", "q6_k", "q8_0", "f8_e4m3"])
+@pytest.mark.parametrize("shape", [(200, 256, 129), (333, 768, 161), (1000, 512, 257), (2100, 1280, 300), (512, 2048, 700)])
+def test_products_of_more_tokens(backend, fmt, shape):
+    """f16 operands with f32 sums: 1e-3 of a row (tests/test_gemm_gpu.py). A row shard, which may run in other segments or on the form with
+    tokens on M, has the bits of its rows, and a bf16 result is the f32 one rounded."""
+    n_out, n_in, t = shape
+    ref, m = make_pair(fmt, n_out, n_in, 940 + t)
+    dev = backend.upload(ref, n_out, n_in)
+    x = synth.activations(t, n_in, 941)
+    y = np.full((t, n_out), np.nan, np.float32)
+    assert backend.matmul(x, [ob.Job(dev, y)])
+    assert row_err(y, m.matmul_f64(x)) < 1e-3
+    shard = backend.shard_rows(dev, 128, n_out)
+    ys = np.zeros((t, n_out - 128), np.float32)
+    assert backend.matmul(x, [ob.Job(shard, ys)])
+    assert np.array_equal(ys, y[:, 128:])
     xd, yd = torch.from_numpy(x).cuda(), torch.zeros((t, n_out), device="cuda", dtype=torch.bfloat16)
     assert backend.matmul_dev(dev, xd, yd)
     torch.cuda.synchronize()
