@@ -906,9 +906,8 @@ class Backend {
     }
 
     // ---- Backend::moe (src/gpu.rs:232-248, src/cuda.rs:798-966): y[i] += sum_j w_ij down_e(act(gate_e x_i) * up_e x_i).
-    // The host builds the per-expert segments as the reference does (src/cuda.rs:810-857), padded to the
-    // GEMM's 128-row token tile; x_dev / y_dev are device f32 [t][h].
-    // A few (token, route) pairs (decode): the 128-row tiles of the tensor-core GEMM would be almost empty. Three launches
+    // The host builds the per-expert segments as the reference does (src/cuda.rs:810-857); x_dev / y_dev are device f32 [t][h].
+    // A few (token, route) pairs (decode): the tiles of the tensor-core GEMM would be almost empty. Three launches
     // instead: the fused gate / up product and the down product of gemv_mma.cu over groups of up to eight pairs of one expert, and the
     // ordered combine (src/moe.rs:625-828 does the same per expert on the CPU; f32-like arithmetic, no f16 operands). The routes travel as
     // kernel arguments: no copy, no synchronization.
@@ -1023,7 +1022,7 @@ class Backend {
         // (the clamped SiLU has no fused pair mode in the matrix-vector kernels: those layers take the GEMM path at any batch)
         if (std::max(t * k, layer_pairs) <= GEMV_GROUP_ROWS && m.act != B2_ACT_SILU_CLAMP && !getenv("B2_MOE_NO_GEMV"))
             return moe_small(m, x_dev_, t, ids, rw, k, y_dev_, count);
-        // The pairs' rows lie expert by expert without padding; a token tile is up to 128 rows of one expert, and an expert's tiles are
+        // The pairs' rows lie expert by expert without padding; a token tile is up to 128 rows of one expert (160 on CTA pairs), and an expert's tiles are
         // about equally long. Long tiles come first: the short ones then fill the gaps that they leave at the end of the launch.
         // Two-term operands (activations of both projections as two f16 terms, Q4_K weights as two f16 terms): Q4_K experts always
         // take them. Q4_K values round harder to f16 than MLX-4's, and one-term operands through two chained projections leave that

@@ -1,4 +1,5 @@
-// Prefill dequant-GEMM for Q4_K weights on the 5th-generation tensor cores (tcgen05 + TMEM).
+// Prefill dequant-GEMM on the 5th-generation tensor cores (tcgen05 + TMEM), the form with tokens on M: more than 128 tokens where gemm_wp.cu is
+// not faster, and the exact switch. It also holds the plans of all three forms (gemm_tc_plan_create).
 //
 //   y[t][n_out] = x[t][K] * W^T,  W in GGUF Q4_K super-blocks (src/ggml.rs:750-773).
 //

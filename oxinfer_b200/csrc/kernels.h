@@ -131,7 +131,7 @@ struct GemmStatus {   // written by the kernel when a bounded wait gives up
     uint32_t t[8];    // cycle stamps of one CTA (diagnostics, B2_GEMM_DEBUG & 32768)
 };
 bool gemm_tc_supports(const WeightDev& w, size_t t);
-// A token tile of a grouped launch (gemm_wt.cu): `count` rows (1 .. 128) from row0, all of one expert.
+// A token tile of a grouped launch (gemm_wt.cu, gemm_wp.cu): `count` rows (1 .. 128, 1 .. 160) from row0, all of one expert.
 struct WtTile {
     int expert, row0, count, pad;
 };
