@@ -891,7 +891,7 @@ class Backend {
         w.p0 = (const uint8_t*)stacked;
         if (pairs) {
             GemmWp g;
-            if (!gemm_wp_encode(&g, w, experts, true, xg, rows, sm_count, out_dev, B2_F32, n_out)) return fail(B2_ERR_CUDA, "[b200qmm: the tensor maps of a grouped product could not be made]");
+            if (!gemm_wp_encode(&g, w, experts, true, xg, rows, sm_count, out_dev, B2_F32, n_out, lo_row0)) return fail(B2_ERR_CUDA, "[b200qmm: the tensor maps of a grouped product could not be made]");
             cudaError_t e = launch_gemm_wp(g, w, rows, tiles, (int)n_tiles, out_dev, B2_F32, n_out, nullptr, 0, gemm_status, row_unscale, stream);
             launches++;
             return e == cudaSuccess ? B2_OK : cuda_fail(e, "grouped gemm (pairs)");
@@ -1029,8 +1029,8 @@ class Backend {
         // layer above 1e-3 per output row (MLX-4 stays near 3e-4 with one term).
         const bool two_term = m.fmt == B2_FMT_Q4_K || exact;
         const size_t rows = t * k, terms = two_term ? 2 : 1, lo_row0 = two_term ? rows : 0;
-        const bool pairs = !two_term;  // the CTA-pair form, for one-term operands
-        const size_t most = pairs ? WP_TILE_ROWS : 128;
+        const bool pairs = !two_term || m.fmt == B2_FMT_Q4_K;  // (two-term activations on one-term weights, the exact switch on MLX-4: gemm_wt.cu)
+        const size_t most = pairs && !two_term ? WP_TILE_ROWS : 128;
         std::vector<size_t> at(m.experts, 0);
         std::vector<WtTile> tiles;
         size_t longest = 0;

@@ -29,6 +29,32 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ __half2 as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
+// The second terms of Q4_K weights in the place of their first: the exact f32 weight of the reference's decode, d1 * q - m1 with both
+// roundings (src/ggml.rs:750-773), minus the first term.
+__device__ __forceinline__ void expand_4bit_rest(const uint4& hdr, const uint32_t (&qw)[8], int j, uint32_t (&o)[32]) {
+    uint32_t sc0, mn0, sc1, mn1;
+    q4k_scale_min(2 * j, hdr.y, hdr.z, hdr.w, sc0, mn0);
+    q4k_scale_min(2 * j + 1, hdr.y, hdr.z, hdr.w, sc1, mn1);
+    const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffff)));
+    const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
+    const float d1l = __fmul_rn(d, (float)sc0), m1l = __fmul_rn(dmin, (float)mn0);
+    const float d1h = __fmul_rn(d, (float)sc1), m1h = __fmul_rn(dmin, (float)mn1);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const uint32_t b0 = (qw[i] >> (16 * e)) & 0xffu, b1 = (qw[i] >> (16 * e + 8)) & 0xffu;
+            const float2 hl = __half22float2(as_h2(o[2 * i + e])), hh = __half22float2(as_h2(o[16 + 2 * i + e]));
+            const float vl0 = __fsub_rn(__fmul_rn(d1l, __uint_as_float(0x4B000000u | (b0 & 15u)) - 8388608.0f), m1l);
+            const float vl1 = __fsub_rn(__fmul_rn(d1l, __uint_as_float(0x4B000000u | (b1 & 15u)) - 8388608.0f), m1l);
+            const float vh0 = __fsub_rn(__fmul_rn(d1h, __uint_as_float(0x4B000000u | (b0 >> 4)) - 8388608.0f), m1h);
+            const float vh1 = __fsub_rn(__fmul_rn(d1h, __uint_as_float(0x4B000000u | (b1 >> 4)) - 8388608.0f), m1h);
+            o[2 * i + e] = h2_bits(__floats2half2_rn(vl0 - hl.x, vl1 - hl.y));
+            o[16 + 2 * i + e] = h2_bits(__floats2half2_rn(vh0 - hh.x, vh1 - hh.y));
+        }
+    }
+}
+
 // 64 weights of a 4-bit block: 32 bytes, low nibbles = elements 0..31, high nibbles = 32..63 (see gemm_tc.cu for the arithmetic).
 // hdr: the block's 16 bytes in front; j: which of its four groups of 64. LO (Q4_K): the second term, the exact f32 weight minus the
 // first term.
@@ -64,26 +90,7 @@ __device__ __forceinline__ void expand_4bit(const uint4& hdr, const uint32_t (&q
         o[16 + 2 * i] = h2_bits(__hfma2(__hfma2(as_h2((p0 & 0x00F000F0u) | 0x64006400u), c1hi, c2hi), dmul, addhi));
         o[16 + 2 * i + 1] = h2_bits(__hfma2(__hfma2(as_h2((p1 & 0x00F000F0u) | 0x64006400u), c1hi, c2hi), dmul, addhi));
     }
-    if constexpr (LO) {
-        const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xffff)));
-        const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
-        const float d1l = __fmul_rn(d, (float)sc0), m1l = __fmul_rn(dmin, (float)mn0);
-        const float d1h = __fmul_rn(d, (float)sc1), m1h = __fmul_rn(dmin, (float)mn1);
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const uint32_t b0 = (qw[i] >> (16 * e)) & 0xffu, b1 = (qw[i] >> (16 * e + 8)) & 0xffu;
-                const float2 hl = __half22float2(as_h2(o[2 * i + e])), hh = __half22float2(as_h2(o[16 + 2 * i + e]));
-                const float vl0 = __fsub_rn(__fmul_rn(d1l, __uint_as_float(0x4B000000u | (b0 & 15u)) - 8388608.0f), m1l);
-                const float vl1 = __fsub_rn(__fmul_rn(d1l, __uint_as_float(0x4B000000u | (b1 & 15u)) - 8388608.0f), m1l);
-                const float vh0 = __fsub_rn(__fmul_rn(d1h, __uint_as_float(0x4B000000u | (b0 >> 4)) - 8388608.0f), m1h);
-                const float vh1 = __fsub_rn(__fmul_rn(d1h, __uint_as_float(0x4B000000u | (b1 >> 4)) - 8388608.0f), m1h);
-                o[2 * i + e] = h2_bits(__floats2half2_rn(vl0 - hl.x, vl1 - hl.y));
-                o[16 + 2 * i + e] = h2_bits(__floats2half2_rn(vh0 - hh.x, vh1 - hh.y));
-            }
-        }
-    }
+    if constexpr (LO) expand_4bit_rest(hdr, qw, j, o);
 }
 
 constexpr float WT_PRE = 256.0f;  // power of two in the f16 weights of Q6_K, Q8_0 and FP8: small scales stay out of f16's subnormals

@@ -63,6 +63,7 @@ struct WpArgs {
     GemmStatus* status;
     const WtTile* tiles;  // grouped launches; null: dense
     int n_tiles;
+    int lo_row0;          // two-term operands: the activations' second terms lie this many rows below the first
     const float* row_unscale;
     const float* s;       // scales beside the packed rows, as in gemm_tc.cu
     const void* s2;
@@ -129,7 +130,7 @@ struct Segments {
 
 // The accumulators of a pair's segments, the same for the issuing warp and the epilogues. Two: in turn. One: segments of up to 128 tokens take
 // its halves in turn, longer ones both (`both`).
-template <bool TWO>
+template <int SECOND>  // first column of the second accumulator; 0: one
 struct Halves {
     int turn = 0, uses[2] = {0, 0}, sums[2] = {0, 0};
     int half;
@@ -137,10 +138,10 @@ struct Halves {
     bool both;
     uint32_t empty_parity[2], full_parity;
     __device__ __forceinline__ void next(int n) {
-        both = !TWO && n > 128;
+        both = !SECOND && n > 128;
         half = both ? 0 : turn;
         turn = both ? 0 : turn ^ 1;
-        col = half ? (TWO ? (uint32_t)WP_TWO : 128u) : 0u;
+        col = half ? (SECOND ? (uint32_t)SECOND : 128u) : 0u;
         empty_parity[0] = (uint32_t)(uses[0] & 1) ^ 1u;
         empty_parity[1] = (uint32_t)(uses[1] & 1) ^ 1u;
         full_parity = (uint32_t)((half ? sums[1] : sums[0]) & 1);
@@ -167,8 +168,9 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 
-// TWO: the layout with two accumulators, for grouped launches; the other for dense ones.
-template <int FMT, bool TWO>
+// TWO: the layout with two accumulators, for grouped launches; the other for dense ones. W2 (grouped, Q4_K): weights and activations as two f16
+// terms; a stage is then 64 k, its slots hold both terms, the accumulators are 128 columns and the A slots four.
+template <int FMT, bool TWO, bool W2 = false>
 __global__ void __launch_bounds__(WP_THREADS, 1)
 gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUtensorMap tmap_w,
                const __grid_constant__ CUtensorMap tmap_w2, const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ WpArgs a) {
@@ -176,7 +178,9 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr bool BYTE_ROWS = FMT == B2_FMT_F8E4M3 || FMT == B2_FMT_Q8_0;
     constexpr bool PRE_SCALED = BYTE_ROWS || FMT == B2_FMT_Q6_K;
-    constexpr int NRAW = wp_n_raw(FMT, TWO), RAW_SLOT = wp_raw_slot(FMT), NA = wp_n_a(TWO), NB = wp_n_b(TWO);
+    constexpr int NRAW = wp_n_raw(FMT, TWO), RAW_SLOT = wp_raw_slot(FMT), NA = W2 ? 4 : wp_n_a(TWO), NB = wp_n_b(TWO);
+    constexpr int GROUPS = W2 ? 1 : 2;                  // groups of 64 k in a stage
+    constexpr int SECOND = !TWO ? 0 : W2 ? 128 : WP_TWO;
     constexpr uint32_t B_STAGE = wp_b_stage(TWO);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -186,14 +190,14 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
     WpShared* sh = &shared;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
-    const int groups = a.K / 64, stages = groups / 2;  // of a segment
+    const int groups = a.K / 64, stages = groups / GROUPS;  // of a segment
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; s++) {
             mbar_init(&sh->acc_full[s], 1);
             mbar_init(&sh->acc_empty[s], 8);
         }
-        for (int s = 0; s < 4; s++) mbar_init(&sh->a_full[s], 16);
+        for (int s = 0; s < 4; s++) mbar_init(&sh->a_full[s], 8 * GROUPS);
         for (int s = 0; s < 4; s++) {
             mbar_init(&sh->b_full[s], 1);
             mbar_init(&sh->done[s], 1);
@@ -231,7 +235,8 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                     if (!ok) break;
                     if (!elect_one()) continue;
                     if (rank == 0) mbar_arrive_expect_tx(&sh->b_full[s], (uint32_t)(seg.n * 256));
-                    tma_load_3d_pair(b_tiles + (size_t)s * B_STAGE, tmap_x, cluster_addr(&sh->b_full[s], 0), 0, y0, 2 * ks);  // [group][tokens][64]
+                    tma_load_3d_pair(b_tiles + (size_t)s * B_STAGE, tmap_x, cluster_addr(&sh->b_full[s], 0), 0, y0, GROUPS * ks);  // [group or term][tokens][64]
+                    if (W2) tma_load_3d_pair(b_tiles + (size_t)s * B_STAGE + (size_t)half * 128, tmap_x, cluster_addr(&sh->b_full[s], 0), 0, a.lo_row0 + y0, ks);
                 }
             }
             __syncwarp();
@@ -275,7 +280,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             const uint32_t done_of[2] = {cluster_addr(&sh->done[0], 0), cluster_addr(&sh->done[0], 1)};
             bool ok = true;
             int it = 0, sa = 0, pa = 0, s = 0, ph = 0;
-            Halves<TWO> acc_of;
+            Halves<SECOND> acc_of;
             while (ok && seg.next(a.tiles, a.n_out, a.t)) {
                 acc_of.next(seg.n);
                 const uint32_t acc = tmem + acc_of.col;
@@ -294,10 +299,15 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                         const uint64_t bd = bdesc0 + (uint64_t)(((uint32_t)s * B_STAGE) >> 4);
                         const uint32_t at = a_cols + (uint32_t)sa * WP_SLOT_COLS;
 #pragma unroll
-                        for (int g = 0; g < 2; g++)
+                        for (int g = 0; g < GROUPS; g++)
 #pragma unroll
-                            for (int kk = 0; kk < 4; kk++)
+                            for (int kk = 0; kk < 4; kk++) {
                                 mma_f16_ts_pair(acc, at + 32 * g + 8 * kk, bd + g * group_b + 2 * kk, idesc, ks > 0 || g > 0 || kk > 0 ? 1u : 0u);
+                                if (W2) {  // (second terms of both: below f32's rounding)
+                                    mma_f16_ts_pair(acc, at + 8 * kk, bd + group_b + 2 * kk, idesc, 1u);
+                                    mma_f16_ts_pair(acc, at + 32 + 8 * kk, bd + 2 * kk, idesc, 1u);
+                                }
+                            }
                         mma_commit_pair(done_of[0] + (uint32_t)(it & 3) * 8u);
                         mma_commit_pair(done_of[1] + (uint32_t)(it & 3) * 8u);
                         if (ks == stages - 1) {
@@ -319,7 +329,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
         const uint32_t empty_even = cluster_addr(&sh->acc_empty[0], 0);
         const bool plain = !a.y_bf16 && a.n_more == 0;
         uint8_t* staging = raw + (size_t)NRAW * RAW_SLOT + (size_t)(warp & 3) * 8192;
-        Halves<TWO> acc_of;
+        Halves<SECOND> acc_of;
         int tile = 0;
         while (seg.next(a.tiles, a.n_out, a.t)) {
             acc_of.next(seg.n);
@@ -404,15 +414,16 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
         const uint32_t a_lane = a_cols + ((uint32_t)((warp & 3) * 32) << 16);
         const uint32_t full_even = cluster_addr(&sh->a_full[0], 0);
         bool ok = true;
-        // 64 expanded weights, group g of the segment whose first stage is it0, to this lane of tensor memory
+        // 64 expanded weights, group g of the segment whose first stage is it0, to this lane of tensor memory. W2: `term` 0, then 1.
         int stage_a = 0, sa = 0;  // (a set's groups come in ascending order)
-        auto put = [&](int it0, int g, const uint32_t(&o)[32]) {
-            const int it = it0 + (g >> 1), old = it - NA;
+        auto put = [&](int it0, int g, const uint32_t(&o)[32], int term = 0) {
+            const int it = it0 + g / GROUPS, old = it - NA;
             for (; stage_a < it; stage_a++) sa = sa + 1 == NA ? 0 : sa + 1;
-            if (old >= 0) ok = __all_sync(0xffffffffu, mbar_wait(&sh->done[old & 3], (uint32_t)((old >> 2) & 1), sh, a.status, 50, (uint32_t)it));
+            if (old >= 0 && term == 0) ok = __all_sync(0xffffffffu, mbar_wait(&sh->done[old & 3], (uint32_t)((old >> 2) & 1), sh, a.status, 50, (uint32_t)it));
             if (!ok) return;
             tc_fence_after();
-            tmem_st32(a_lane + (uint32_t)sa * WP_SLOT_COLS + (uint32_t)(g & 1) * 32u, o);
+            tmem_st32(a_lane + (uint32_t)sa * WP_SLOT_COLS + (uint32_t)(W2 ? term : g & 1) * 32u, o);
+            if (W2 && term == 0) return;
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(full_even + (uint32_t)sa * 8u);
@@ -497,6 +508,10 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                     uint32_t o[32];
                     expand_4bit<FMT, false>(hdr, qw, set, o);
                     put(it0, sb * 4 + set, o);
+                    if (W2 && ok) {
+                        expand_4bit_rest(hdr, qw, set, o);
+                        put(it0, sb * 4 + set, o, 1);
+                    }
                     if (!ok) break;
                 }
             }
@@ -550,7 +565,7 @@ double gemm_wp_share(GemmWp* g, size_t n_out_, size_t t_, size_t n_in, int sm_co
     return best;
 }
 
-bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, bool grouped, const void* x16, size_t x_rows, int sm_count, void* y, int y_dtype, size_t y_ld) {
+bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, bool grouped, const void* x16, size_t x_rows, int sm_count, void* y, int y_dtype, size_t y_ld, size_t lo_row0) {
     GemmWt m;  // the weights' maps are gemm_wt.cu's (boxes of 128 rows)
     if (!gemm_wt_encode(&m, w, experts, x16, x_rows, 16, 1, 0, false, false)) return false;
     g->w = m.w;
@@ -567,14 +582,16 @@ bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, bool grouped,
             return false;
     }
     if (grouped) g->pairs = std::max(1, sm_count / 2);
-    return gemm_x_maps(&g->x, 0, WP_SEG / 32 - 1, x16, x_rows, w.n_in, 2);
+    g->lo_row0 = (int)lo_row0;
+    return gemm_x_maps(&g->x, 0, WP_SEG / 32 - 1, x16, lo_row0 + x_rows, w.n_in, lo_row0 ? 1 : 2);
 }
 
 cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
                            GemmStatus* status, const float* row_unscale, cudaStream_t st) {
     using Kern = void (*)(XMaps, CUtensorMap, CUtensorMap, CUtensorMap, WpArgs);
-    if (tiles && w.fmt != B2_FMT_MLX4) return cudaErrorInvalidValue;  // (Q4_K experts take two-term operands: gemm_wt.cu)
-    Kern kern = tiles                    ? gemm_wp_kernel<B2_FMT_MLX4, true>
+    if (tiles && w.fmt != (g.lo_row0 ? B2_FMT_Q4_K : B2_FMT_MLX4)) return cudaErrorInvalidValue;
+    Kern kern = tiles && g.lo_row0       ? gemm_wp_kernel<B2_FMT_Q4_K, true, true>
+                : tiles                  ? gemm_wp_kernel<B2_FMT_MLX4, true>
                 : w.fmt == B2_FMT_Q6_K   ? gemm_wp_kernel<B2_FMT_Q6_K, false>
                 : w.fmt == B2_FMT_Q8_0   ? gemm_wp_kernel<B2_FMT_Q8_0, false>
                 : w.fmt == B2_FMT_MLX4   ? gemm_wp_kernel<B2_FMT_MLX4, false>
@@ -595,6 +612,7 @@ cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const 
     a.status = status;
     a.tiles = tiles;
     a.n_tiles = n_tiles;
+    a.lo_row0 = g.lo_row0;
     a.row_unscale = row_unscale;
     a.s = (const float*)(w.fmt == B2_FMT_Q6_K ? w.p2 : w.p1);
     a.s2 = w.p3;

@@ -34,18 +34,21 @@ cudaError_t launch_gemm_wt(const GemmWt& g, const WeightDev& w, size_t t, const 
 // Maps first .. last of a set, `groups` of 64 k a copy.
 bool gemm_x_maps(XMaps* x, int first, int last, const void* x16, size_t rows, size_t n_in, int groups);
 
-// The CTA-pair form (gemm_wp.cu), one-term operands. A grouped launch's tiles hold up to WP_TILE_ROWS rows.
+// The CTA-pair form (gemm_wp.cu), one-term operands, or grouped Q4_K with two-term ones. A grouped launch's tiles hold up to WP_TILE_ROWS rows
+// (two-term: 128).
 constexpr int WP_MOST_ROWS = 256, WP_TILE_ROWS = 160;
 struct GemmWp {
     XMaps x;
     CUtensorMap w, w2, y;
     int pairs = 0, pieces = 0, snap = 0;  // how a dense launch is shared out
+    int lo_row0 = 0;                      // grouped Q4_K launches with two-term operands: the activations' second terms, rows below the first
     bool staged = false;                  // the results can leave through the copy engine
 };
 // Fills in how a dense launch is shared out and returns an estimate of its time in cycles.
 double gemm_wp_share(GemmWp* g, size_t n_out, size_t t, size_t n_in, int sm_count);
 // x_rows: the tokens (grouped: the rows of all segments). Dense: after gemm_wp_share.
-bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, bool grouped, const void* x16, size_t x_rows, int sm_count, void* y, int y_dtype, size_t y_ld);
+bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, bool grouped, const void* x16, size_t x_rows, int sm_count, void* y, int y_dtype, size_t y_ld,
+                    size_t lo_row0 = 0);
 cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
                            GemmStatus* status, const float* row_unscale, cudaStream_t st);
 
