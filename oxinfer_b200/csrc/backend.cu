@@ -897,7 +897,7 @@ class Backend {
             return e == cudaSuccess ? B2_OK : cuda_fail(e, "grouped gemm (pairs)");
         }
         GemmWt g;
-        if (!gemm_wt_encode(&g, w, experts, xg, lo_row0 ? lo_row0 + rows : rows, longest, lo_row0 ? 2 : 1, lo_row0, lo_row0 && fmt == B2_FMT_Q4_K, true))
+        if (!gemm_wt_encode(&g, w, experts, xg, lo_row0 ? lo_row0 + rows : rows, longest, lo_row0 ? 2 : 1, lo_row0, true))
             return fail(B2_ERR_CUDA, "[b200qmm: the tensor maps of a grouped product could not be made]");
         cudaError_t e = launch_gemm_wt(g, w, rows, tiles, (int)n_tiles, out_dev, B2_F32, n_out, nullptr, 0, gemm_status, row_unscale, stream);
         launches++;

@@ -56,9 +56,8 @@ __device__ __forceinline__ void expand_4bit_rest(const uint4& hdr, const uint32_
 }
 
 // 64 weights of a 4-bit block: 32 bytes, low nibbles = elements 0..31, high nibbles = 32..63 (see gemm_tc.cu for the arithmetic).
-// hdr: the block's 16 bytes in front; j: which of its four groups of 64. LO (Q4_K): the second term, the exact f32 weight minus the
-// first term.
-template <int FMT, bool LO>
+// hdr: the block's 16 bytes in front; j: which of its four groups of 64.
+template <int FMT>
 __device__ __forceinline__ void expand_4bit(const uint4& hdr, const uint32_t (&qw)[8], int j, uint32_t (&o)[32]) {
     __half2 dmul, c1lo, c2lo, c1hi, c2hi, addlo, addhi;
     uint32_t sc0 = 0, mn0 = 0, sc1 = 0, mn1 = 0;
@@ -90,7 +89,6 @@ __device__ __forceinline__ void expand_4bit(const uint4& hdr, const uint32_t (&q
         o[16 + 2 * i] = h2_bits(__hfma2(__hfma2(as_h2((p0 & 0x00F000F0u) | 0x64006400u), c1hi, c2hi), dmul, addhi));
         o[16 + 2 * i + 1] = h2_bits(__hfma2(__hfma2(as_h2((p1 & 0x00F000F0u) | 0x64006400u), c1hi, c2hi), dmul, addhi));
     }
-    if constexpr (LO) expand_4bit_rest(hdr, qw, j, o);
 }
 
 constexpr float WT_PRE = 256.0f;  // power of two in the f16 weights of Q6_K, Q8_0 and FP8: small scales stay out of f16's subnormals

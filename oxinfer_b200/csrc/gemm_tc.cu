@@ -972,7 +972,7 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
         p->y_ld = gathered ? peer_y->ld : 0;
         p->n_more = gathered ? peer_y->n_more : 0;
         for (int d = 0; d < p->n_more; d++) p->more_ptr[d] = peer_y->more[d];
-        if (!(p->wt_form == 1 ? gemm_wt_encode(&p->wt, w, 1, x16, a_lo_row0 ? a_lo_row0 + t : t, t, a_lo_row0 ? 2 : 1, a_lo_row0, false, false)
+        if (!(p->wt_form == 1 ? gemm_wt_encode(&p->wt, w, 1, x16, a_lo_row0 ? a_lo_row0 + t : t, t, a_lo_row0 ? 2 : 1, a_lo_row0, false)
                               : gemm_wp_encode(&p->wp, w, 1, false, x16, t, sm_count, y, y_dtype, p->y_ld ? p->y_ld : w.n_out))) {
             snprintf(err, errlen, "the tensor maps of a product could not be made");
             delete p;

@@ -506,7 +506,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                     if (++slot == NRAW) slot = 0, ph ^= 1;
                     const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
                     uint32_t o[32];
-                    expand_4bit<FMT, false>(hdr, qw, set, o);
+                    expand_4bit<FMT>(hdr, qw, set, o);
                     put(it0, sb * 4 + set, o);
                     if (W2 && ok) {
                         expand_4bit_rest(hdr, qw, set, o);
@@ -567,7 +567,7 @@ double gemm_wp_share(GemmWp* g, size_t n_out_, size_t t_, size_t n_in, int sm_co
 
 bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, bool grouped, const void* x16, size_t x_rows, int sm_count, void* y, int y_dtype, size_t y_ld, size_t lo_row0) {
     GemmWt m;  // the weights' maps are gemm_wt.cu's (boxes of 128 rows)
-    if (!gemm_wt_encode(&m, w, experts, x16, x_rows, 16, 1, 0, false, false)) return false;
+    if (!gemm_wt_encode(&m, w, experts, x16, x_rows, 16, 1, 0, false)) return false;
     g->w = m.w;
     g->w2 = m.w2;
     g->y = m.w;

@@ -52,7 +52,7 @@ struct __align__(8) WtShared {
 struct WtArgs {
     int K, n_out, t;
     int n_raw, n_b, n_a;  // slots of the two rings in shared memory and of the one in tensor memory
-    int groups;           // 64-k groups of a stage: 1 or 2 (two-term weights: 1)
+    int groups;           // 64-k groups of a stage: 1 or 2
     int splits;           // parts of K = CTAs of a cluster
     int n_max;            // the B ring's stage holds this many tokens
     int x_terms, lo_row0; // 2: activations as two f16 terms, the second lo_row0 rows below the first
@@ -90,8 +90,7 @@ __device__ __forceinline__ void store_y(const WtArgs& a, size_t at, float v) {
     for (int d = 0; d < a.n_more; d++) a.more[d][at] = v;
 }
 
-// W2 (Q4_K): every weight as two f16 terms; set 0 expands the first terms of every stage, set 1 the second.
-template <int FMT, bool W2>
+template <int FMT>
 __global__ void __launch_bounds__(WT_THREADS, 2)
 gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2,
                const __grid_constant__ WtArgs a) {
@@ -131,7 +130,7 @@ gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < 4; s++) {
-            mbar_init(&sh->a_full[s], W2 ? 8 : 4 * a.groups);
+            mbar_init(&sh->a_full[s], 4 * a.groups);
             mbar_init(&sh->b_full[s], 1);
             mbar_init(&sh->done[s], 1);
         }
@@ -223,7 +222,6 @@ gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                     for (int kk = 0; kk < 4; kk++) {
                         mma_f16_ts(tmem, ag + 8 * kk, bg + 2 * kk, idesc, first && kk == 0 ? 0u : 1u);
                         if (a.x_terms == 2) mma_f16_ts(tmem, ag + 8 * kk, bg + lo + 2 * kk, idesc, 1u);
-                        if (W2) mma_f16_ts(tmem, ag + 32 + 8 * kk, bg + 2 * kk, idesc, 1u);  // (second terms of both: below f32's rounding)
                     }
                 };
                 group(at, bdesc, ks == 0);
@@ -254,7 +252,7 @@ gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             if (old >= 0) ok = __all_sync(0xffffffffu, mbar_wait(&sh->done[old & 3], (uint32_t)((old >> 2) & 1), sh, a.status, 28, (uint32_t)ks));
             if (!ok) return;
             tc_fence_after();
-            tmem_st32(a_lane + (uint32_t)slot_a * WT_SLOT_COLS + ((W2 ? set : g - ks * a.groups) ? 32u : 0u), o);
+            tmem_st32(a_lane + (uint32_t)slot_a * WT_SLOT_COLS + (g - ks * a.groups ? 32u : 0u), o);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh->a_full[slot_a]);
@@ -333,8 +331,8 @@ gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                 }
             }
         } else {
-            // one-term: set s expands groups s and s + 2 of every super-block; two-term: both sets all four groups
-            constexpr int GROUPS = W2 ? 4 : 2;
+            // set s expands groups s and s + 2 of every super-block
+            constexpr int GROUPS = 2;
             int slot = 0, ph = 0;
             for (int sb = 0; sb < nsb && ok; sb++) {
                 if (!raw_ready(slot, ph, sb)) break;
@@ -344,7 +342,7 @@ gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                 uint32_t words = hdr.x;
 #pragma unroll
                 for (int i = 0; i < 2 * GROUPS; i++) {
-                    q[i] = my[1 + (W2 ? i : 2 * set + 4 * (i >> 1) + (i & 1))];
+                    q[i] = my[1 + 2 * set + 4 * (i >> 1) + (i & 1)];
                     words |= q[i].x;
                 }
                 release_raw(&sh->raw_empty[slot], words, a.zero, lane);
@@ -354,11 +352,8 @@ gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                     const uint32_t qw[8] = {q[2 * jj].x,     q[2 * jj].y,     q[2 * jj].z,     q[2 * jj].w,
                                             q[2 * jj + 1].x, q[2 * jj + 1].y, q[2 * jj + 1].z, q[2 * jj + 1].w};
                     uint32_t o[32];
-                    if (W2 && set)
-                        expand_4bit<FMT, W2>(hdr, qw, jj, o);
-                    else
-                        expand_4bit<FMT, false>(hdr, qw, W2 ? jj : 2 * jj + set, o);
-                    put(sb * 4 + (W2 ? jj : 2 * jj + set), o);
+                    expand_4bit<FMT>(hdr, qw, 2 * jj + set, o);
+                    put(sb * 4 + 2 * jj + set, o);
                     if (!ok) break;
                 }
             }
@@ -488,14 +483,13 @@ bool gemm_x_maps(XMaps* x, int first, int last, const void* x16, size_t rows, si
     return enc != nullptr;
 }
 
-bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x16, size_t x_rows, size_t tokens, int x_terms, size_t lo_row0, bool two_term_w, bool grouped) {
+bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x16, size_t x_rows, size_t tokens, int x_terms, size_t lo_row0, bool grouped) {
     TensorMapEncodeFn enc = tensor_map_encode();
     if (!enc) return false;
     g->n_max = (int)std::min<size_t>(128, (tokens + 15) / 16 * 16);
     g->splits = grouped ? 1 : wt_splits(w.n_in);
     g->x_terms = x_terms;
     g->lo_row0 = (int)lo_row0;
-    g->two_term_w = two_term_w;
     CUresult r;
     const size_t rows = w.n_out * experts;
     const CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
@@ -516,7 +510,7 @@ bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x
     const bool bytes = w.fmt == B2_FMT_F8E4M3 || w.fmt == B2_FMT_Q8_0;
     const size_t slot = raw_slot_bytes(w.fmt), tile = (size_t)g->n_max * 128 * x_terms, room = WT_SMEM_MAX - sizeof(WtShared) - 128 - 1024;
     const int least = bytes ? 4 : 2, most = bytes ? WT_MAX_RING : 5;
-    g->groups = two_term_w || 4 * tile + (size_t)least * slot > room ? 1 : 2;
+    g->groups = 4 * tile + (size_t)least * slot > room ? 1 : 2;
     if (!gemm_x_maps(&g->x, grouped ? 0 : g->n_max / 16 - 1, g->n_max / 16 - 1, x16, x_rows, w.n_in, g->groups)) return false;
     g->n_a = g->n_max <= 64 ? 3 : 2;
     g->n_b = (int)std::min<size_t>(4, (room - (size_t)least * slot) / (tile * g->groups));
@@ -530,12 +524,11 @@ bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x
 cudaError_t launch_gemm_wt(const GemmWt& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
                            GemmStatus* status, const float* row_unscale, cudaStream_t st) {
     using Kern = void (*)(XMaps, CUtensorMap, CUtensorMap, WtArgs);
-    Kern kern = w.fmt == B2_FMT_Q6_K     ? gemm_wt_kernel<B2_FMT_Q6_K, false>
-                : w.fmt == B2_FMT_Q8_0   ? gemm_wt_kernel<B2_FMT_Q8_0, false>
-                : w.fmt == B2_FMT_MLX4   ? gemm_wt_kernel<B2_FMT_MLX4, false>
-                : w.fmt == B2_FMT_F8E4M3 ? gemm_wt_kernel<B2_FMT_F8E4M3, false>
-                : g.two_term_w           ? gemm_wt_kernel<B2_FMT_Q4_K, true>
-                                         : gemm_wt_kernel<B2_FMT_Q4_K, false>;
+    Kern kern = w.fmt == B2_FMT_Q6_K     ? gemm_wt_kernel<B2_FMT_Q6_K>
+                : w.fmt == B2_FMT_Q8_0   ? gemm_wt_kernel<B2_FMT_Q8_0>
+                : w.fmt == B2_FMT_MLX4   ? gemm_wt_kernel<B2_FMT_MLX4>
+                : w.fmt == B2_FMT_F8E4M3 ? gemm_wt_kernel<B2_FMT_F8E4M3>
+                                         : gemm_wt_kernel<B2_FMT_Q4_K>;
     if (cudaError_t e = ensure_dynamic_smem((const void*)kern, g.smem, 0); e != cudaSuccess) return e;
     WtArgs a{};
     a.K = (int)w.n_in;

@@ -19,14 +19,13 @@ struct GemmWt {
     XMaps x;
     CUtensorMap w, w2;  // (w2: Q6_K's second plane)
     int n_max = 0, splits = 1, x_terms = 1, lo_row0 = 0, n_raw = 0, n_b = 0, n_a = 0, groups = 1;
-    bool two_term_w = false;
     size_t smem = 0;
 };
 // Parts of K of a dense product.
 int wt_splits(size_t K);
 // x16: f16 [x_rows][n_in], `tokens` of them in the longest tile (at most 128 a tile). x_terms 2: the second terms lo_row0 rows below.
 // grouped: w.p0 stacks `experts` matrices of n_out rows (MLX-4, Q4_K). false: no tensor map could be made.
-bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x16, size_t x_rows, size_t tokens, int x_terms, size_t lo_row0, bool two_term_w, bool grouped);
+bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x16, size_t x_rows, size_t tokens, int x_terms, size_t lo_row0, bool grouped);
 // tiles (device; grouped launches): n_tiles of them; null: `t` tokens in order. y rows y_ld elements apart; more[0 .. n_more): other ranks'
 // copies of an f32 y.
 cudaError_t launch_gemm_wt(const GemmWt& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
