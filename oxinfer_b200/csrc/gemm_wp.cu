@@ -446,8 +446,12 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                 auto scales_of = [&](int g) {
                     return live && g < groups && sc_row ? __ldg((const uint32_t*)(sc_row + (size_t)(FMT == B2_FMT_Q8_0 ? g : g >> 1) * 4)) : 0u;
                 };
-                uint32_t next = scales_of(set);
-                for (int g = set; g < groups; g += 4) {
+                // The staging slots run on over the segments, and a slot stays with one set: its waits then come in the order of the slot's
+                // phases also where a segment has no whole number of four groups (K a multiple of 128 and not of 256).
+                static_assert(!BYTE_ROWS || NRAW % 4 == 0, "a slot has one owner");
+                const int first = (set - base) & 3;
+                uint32_t next = scales_of(first);
+                for (int g = first; g < groups; g += 4) {
                     const uint32_t sc = next;
                     next = scales_of(g + 4);
                     const int c = base + g, s = c % NRAW;

@@ -1,4 +1,6 @@
 """Products of more than eight tokens and the routed experts' segments: weights in tensor memory, tokens on the instruction's N side."""
+import os
+
 import numpy as np
 import pytest
 import torch
@@ -63,6 +65,33 @@ def test_products_of_more_tokens(backend, fmt, shape):
     torch.cuda.synchronize()
     backend.check_status()
     assert torch.equal(yd.cpu(), torch.from_numpy(y).bfloat16())
+
+
+def with_tokens_on_m(backend, x, dev, n_out):
+    """The same product on gemm_tc.cu's form (any B2_GEMM_SPLIT_K but 1; 0 divides nothing)."""
+    y = np.full((len(x), n_out), np.nan, np.float32)
+    os.environ["B2_GEMM_SPLIT_K"] = "0"
+    try:
+        assert backend.matmul(x, [ob.Job(dev, y)])
+    finally:
+        del os.environ["B2_GEMM_SPLIT_K"]
+    return y
+
+
+# several segments a pair whose 10 or 22 groups of 64 k are not whole fours: the sets of dequantizers and the 12 staging slots go on over them
+@pytest.mark.parametrize("fmt", ["q8_0", "f8_e4m3"])
+@pytest.mark.parametrize("shape", [(20000, 640, 300), (3000, 1408, 3108)])
+def test_byte_rows_that_end_inside_a_round_of_the_sets(backend, fmt, shape):
+    """The bits of the form with tokens on M, and 1e-3 of a row (tests/test_gemm_gpu.py) on a sample of the tokens."""
+    n_out, n_in, t = shape
+    ref, m = make_pair(fmt, n_out, n_in, 960 + t)
+    dev = backend.upload(ref, n_out, n_in)
+    x = synth.activations(t, n_in, 961)
+    y = np.full((t, n_out), np.nan, np.float32)
+    assert backend.matmul(x, [ob.Job(dev, y)])
+    rows = np.arange(0, t, 97)
+    assert row_err(y[rows], m.matmul_f64(x[rows])) < 1e-3
+    assert np.array_equal(y, with_tokens_on_m(backend, x, dev, n_out))
 
 
 # pairs per expert: none, one, a tile of 16 and one more, 128 and one more (two tiles of 80 and 49 rows), three tiles
