@@ -27,7 +27,7 @@ namespace b2 {
 
 namespace {
 
-constexpr int WP_THREADS = 736, WP_ROWS = 128, WP_SEG = WP_MOST_ROWS, WP_UNIT = 32;
+constexpr int WP_THREADS = 736, WP_ROWS = 128, WP_SEG = WP_MOST_ROWS, WP_UNIT = 32, WP_PANEL = 8;
 constexpr uint32_t WP_SLOT_COLS = 64;                           // an A slot of 128 k; the slots are tensor memory's last columns
 constexpr int WP_TWO = WP_TILE_ROWS;                            // longest segment of the layout with two accumulators
 // The two layouts: A slots, activation stages of 128 k, and what the epilogue stages its results in (two tiles of 32 tokens x 32 rows a warp).
@@ -56,7 +56,7 @@ static_assert(wp_smem(B2_FMT_Q4_K, false) + sizeof(WpShared) <= 227 * 1024 && wp
 
 struct WpArgs {
     int K, n_out, t;
-    int pieces, snap;     // dense: how the work is shared out (Segments)
+    WpShare share;        // dense: how the work is shared out (Segments)
     int y_bf16, zero, staged;  // staged: results leave through tmap_y
     size_t y_ld;
     void* y;
@@ -72,28 +72,31 @@ struct WpArgs {
     float* more[7];
 };
 
-// The segments of a pair, the same for every role of both CTAs. Grouped launches: every tile with every row block, dealt out in turn.
-// Dense: per row block of 256, `pieces` equal segments dealt out in turn, or (pieces 0) one list of units of 32 tokens of which every pair
-// takes an equal run, cut at the ends of row blocks; a run's end within `snap` units of a row block's end is moved there.
+// The segments of a pair, the same for every role of both CTAs. Grouped launches: every tile with every row block, dealt out in turn. Dense, one of
+// - pieces > 0: every row block of 256 in `pieces` equal segments, dealt out in turn, of `split` parts each from number `whole` on (the last wave).
+//   They go in panels of WP_PANEL token ranges, a panel's row blocks before the next panel, its token ranges fastest: pairs that run together share
+//   8 token ranges and about 9 row blocks, which fit L2 over a long stretch of K.
+// - pieces 0: one list of units of 32 tokens, row block by row block, of which every pair takes an equal run, cut at the ends of row blocks; a
+//   run's end within `snap` units of a row block's end is moved there. Pairs stand at unrelated tokens: for launches whose operands fit L2.
 struct Segments {
-    int pos, end, step, per_block, blocks, pieces;
+    int pos, end, step, per_block, blocks;
     int row, w_row, x_row0, n, count;  // first of the 256 rows in its matrix / in the stack; tokens: first, padded to 32, real
-    __host__ __device__ __forceinline__ Segments(int n_out, int t, int n_tiles, int pieces_, int snap, int c, int pairs) : pieces(pieces_) {
+    __host__ __device__ __forceinline__ Segments(int n_out, int t, int n_tiles, const WpShare& share, int c, int pairs) {
         blocks = (n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
         per_block = (t + WP_UNIT - 1) / WP_UNIT;
         pos = c;
         step = pairs;
-        end = n_tiles ? n_tiles * blocks : pieces * blocks;
-        if (!n_tiles && !pieces) {
-            pos = bound(c, pairs, snap);
-            end = bound(c + 1, pairs, snap);
+        end = n_tiles ? n_tiles * blocks : share.whole + (share.pieces * blocks - share.whole) * share.split;
+        if (!n_tiles && !share.pieces) {
+            pos = bound(c, pairs, share.snap);
+            end = bound(c + 1, pairs, share.snap);
         }
     }
     __host__ __device__ __forceinline__ int bound(int i, int pairs, int snap) const {
         const int p = (int)((long long)blocks * per_block * i / pairs), u = p % per_block;
         return u <= snap ? p - u : per_block - u <= snap ? p - u + per_block : p;
     }
-    __host__ __device__ __forceinline__ bool next(const WtTile* tiles, int n_out, int t) {
+    __host__ __device__ __forceinline__ bool next(const WtTile* tiles, int n_out, int t, const WpShare& share) {
         if (pos >= end) return false;
         if (tiles) {
             const WtTile tile = tiles[pos / blocks];
@@ -106,11 +109,16 @@ struct Segments {
             return true;
         }
         int u, take;
-        if (pieces) {
-            const int p = pos % pieces;
-            row = pos / pieces * (2 * WP_ROWS);
-            u = per_block * p / pieces;
-            take = per_block * (p + 1) / pieces - u;
+        if (share.pieces) {
+            const int over = pos - share.whole, tile = over < 0 ? pos : share.whole + over / share.split, part = over < 0 ? 0 : over % share.split;
+            const int panel = tile / (WP_PANEL * blocks), in = tile - panel * (WP_PANEL * blocks), left = share.pieces - panel * WP_PANEL;
+            const int wide = left < WP_PANEL ? left : WP_PANEL, p = panel * WP_PANEL + in % wide, parts = over < 0 ? 1 : share.split;
+            row = in / wide * (2 * WP_ROWS);
+            u = (int)((long long)per_block * p / share.pieces);
+            take = (int)((long long)per_block * (p + 1) / share.pieces) - u;
+            const int from = take * part / parts;
+            take = take * (part + 1) / parts - from;
+            u += from;
             pos += step;
         } else {
             constexpr int most = WP_SEG / WP_UNIT;
@@ -218,7 +226,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
     cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base, a_cols = tmem + 512u - NA * WP_SLOT_COLS;
-    Segments seg(a.n_out, a.t, a.tiles ? a.n_tiles : 0, a.pieces, a.snap, blockIdx.x >> 1, gridDim.x >> 1);
+    Segments seg(a.n_out, a.t, a.tiles ? a.n_tiles : 0, a.share, blockIdx.x >> 1, gridDim.x >> 1);
 
     if (warp == 20) {
         // ---------------- activations: this CTA's half of the segment's tokens ----------------
@@ -226,7 +234,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             asm volatile("griddepcontrol.wait;" ::: "memory");
             int it = 0, s = 0;
             bool ok = true;
-            while (ok && seg.next(a.tiles, a.n_out, a.t)) {
+            while (ok && seg.next(a.tiles, a.n_out, a.t, a.share)) {
                 const int half = seg.n / 2, y0 = seg.x_row0 + (int)rank * half;
                 const CUtensorMap* tmap_x = &maps.m[half / 16 - 1];
                 for (int ks = 0; ks < stages; ks++, it++, s = s + 1 == NB ? 0 : s + 1) {
@@ -250,7 +258,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             const int copies = BYTE_ROWS ? groups : groups / 4;
             int issued = 0, s = 0, ph = 0;
             bool ok = true;
-            while (ok && seg.next(a.tiles, a.n_out, a.t)) {
+            while (ok && seg.next(a.tiles, a.n_out, a.t, a.share)) {
                 const int w_row = seg.w_row + (int)rank * WP_ROWS;
                 for (int c = 0; c < copies; c++, issued++) {
                     ok = __all_sync(0xffffffffu, mbar_wait(&sh->raw_empty[s], (uint32_t)(ph ^ 1), sh, a.status, 43, (uint32_t)issued));
@@ -281,7 +289,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             bool ok = true;
             int it = 0, sa = 0, pa = 0, s = 0, ph = 0;
             Halves<SECOND> acc_of;
-            while (ok && seg.next(a.tiles, a.n_out, a.t)) {
+            while (ok && seg.next(a.tiles, a.n_out, a.t, a.share)) {
                 acc_of.next(seg.n);
                 const uint32_t acc = tmem + acc_of.col;
                 const uint32_t idesc = (1u << 4) | ((uint32_t)(seg.n >> 3) << 17) | ((256u >> 4) << 24);
@@ -331,7 +339,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
         uint8_t* staging = raw + (size_t)NRAW * RAW_SLOT + (size_t)(warp & 3) * 8192;
         Halves<SECOND> acc_of;
         int tile = 0;
-        while (seg.next(a.tiles, a.n_out, a.t)) {
+        while (seg.next(a.tiles, a.n_out, a.t, a.share)) {
             acc_of.next(seg.n);
             const int row0 = seg.row + (int)rank * WP_ROWS + (warp & 3) * 32, row = row0 + lane;
             auto factor = [&](int c) {  // of token c + lane
@@ -433,7 +441,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             return ok;
         };
         int it0 = 0, slot = 0, ph = 0, base = 0;
-        for (; ok && seg.next(a.tiles, a.n_out, a.t); it0 += stages) {
+        for (; ok && seg.next(a.tiles, a.n_out, a.t, a.share); it0 += stages) {
             const int row = seg.row + (int)rank * WP_ROWS + r;
             const bool live = row < a.n_out;
             const size_t wrow = live ? (size_t)row : 0;
@@ -534,37 +542,42 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
 }  // namespace
 
 // How a dense launch is shared out, and what its slowest pair takes in cycles: a stage of 128 k max(780, 4 tokens), the sums of a segment
-// of more than 128 tokens 7500 (nothing is multiplied meanwhile).
+// of more than 128 tokens 7500 (nothing is multiplied meanwhile). Runs of up to 16 units come as equal runs or as whole segments, whichever ends first;
+// longer ones, whose launches' operands may not fit L2, in panels: FP8 28672 x 12288, 8192 tokens, read 24.9 GB from DRAM in equal runs (5.36 ms)
+// and reads 6.8 in panels (4.27); Q4_K 4096 x 14336, 8192 tokens, 2.07 GB (732 us) and 0.72 (654).
 double gemm_wp_share(GemmWp* g, size_t n_out_, size_t t_, size_t n_in, int sm_count) {
     const int n_out = (int)n_out_, t = (int)t_, stages = (int)(n_in / 128), units = (t + WP_UNIT - 1) / WP_UNIT, blocks = (n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
     const int pairs = (int)std::min<long long>(std::max(1, sm_count / 2), (long long)blocks * units), most = WP_SEG / WP_UNIT, least = (units + most - 1) / most;
     auto segment = [&](int n) { return stages * std::max(780.0, 4.0 * n) + (n > 128 ? 7500.0 : 500.0); };
     double best = 1e30;
-    auto take = [&](int pieces, int snap) {
+    auto take = [&](double cost, const WpShare& share) {
+        if (cost >= best) return;
+        best = cost;
+        g->share = share;
+    };
+    auto run = [&](int snap) {
+        const WpShare share{0, snap, 0, 1};
         double cost = 0.0;
         for (int c = 0; c < pairs && cost < best; c++) {
             double sum = 0.0;
-            for (Segments s(n_out, t, 0, pieces, snap, c, pairs); s.next(nullptr, n_out, t);) sum += segment(s.n);
+            for (Segments s(n_out, t, 0, share, c, pairs); s.next(nullptr, n_out, t, share);) sum += segment(s.n);
             cost = std::max(cost, sum);
         }
-        if (cost < best) {
-            best = cost;
-            g->pieces = pieces;
-            g->snap = snap;
-        }
+        take(cost, share);
+    };
+    auto deal = [&](int pieces, int most_parts) {  // whole waves of whole segments, and the rest in as many parts as cost least
+        const int tiles = pieces * blocks, rest = tiles % pairs, longest = (units + pieces - 1) / pieces;
+        for (int split = 1; split <= most_parts; split++)
+            take(tiles / pairs * segment(longest * WP_UNIT) + (rest * split + pairs - 1) / pairs * segment((longest + split - 1) / split * WP_UNIT), WpShare{pieces, 0, tiles - rest, split});
     };
     g->pairs = pairs;
-    const long long run = (long long)blocks * units / pairs;
-    if (run <= 16) {
-        take(0, std::min(3, (units - 1) / 2));
-        take(0, 0);
-        take(least, 0);
-        if (least < units) take(least + 1, 0);
-    } else {  // (long runs are even enough, and the count of their segments would take long)
-        g->pieces = 0;
-        g->snap = std::min(3, (units - 1) / 2);
-        const long long segs = (run + 2 + most - 1) / most + (run < units ? 0 : run / units);
-        best = segs * segment((int)((run + segs) / segs) * WP_UNIT);
+    if ((long long)blocks * units / pairs <= 16) {
+        run(std::min(3, (units - 1) / 2));
+        run(0);
+        deal(least, 1);
+        if (least < units) deal(least + 1, 1);
+    } else {
+        deal(least, units / least);
     }
     return best;
 }
@@ -607,8 +620,7 @@ cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const 
     a.K = (int)w.n_in;
     a.n_out = (int)w.n_out;
     a.t = (int)t;
-    a.pieces = g.pieces;
-    a.snap = g.snap;
+    a.share = g.share;
     a.staged = g.staged && n_more == 0;
     a.y_bf16 = y_dtype == B2_BF16;
     a.y_ld = y_ld;

@@ -36,10 +36,14 @@ bool gemm_x_maps(XMaps* x, int first, int last, const void* x16, size_t rows, si
 // The CTA-pair form (gemm_wp.cu), one-term operands, or grouped Q4_K with two-term ones. A grouped launch's tiles hold up to WP_TILE_ROWS rows
 // (two-term: 128).
 constexpr int WP_MOST_ROWS = 256, WP_TILE_ROWS = 160;
+struct WpShare {  // how a dense launch is shared out (Segments in gemm_wp.cu)
+    int pieces, snap, whole, split;
+};
 struct GemmWp {
     XMaps x;
     CUtensorMap w, w2, y;
-    int pairs = 0, pieces = 0, snap = 0;  // how a dense launch is shared out
+    int pairs = 0;
+    WpShare share = {};
     int lo_row0 = 0;                      // grouped Q4_K launches with two-term operands: the activations' second terms, rows below the first
     bool staged = false;                  // the results can leave through the copy engine
 };

@@ -94,6 +94,23 @@ def test_byte_rows_that_end_inside_a_round_of_the_sets(backend, fmt, shape):
     assert np.array_equal(y, with_tokens_on_m(backend, x, dev, n_out))
 
 
+# equal runs of three segments of 64 to 256 tokens; 15 token ranges (a panel of eight and the rest) by 11 row blocks, the last 17 of 165 segments in
+# four parts each; rows that end inside a pair's 256
+@pytest.mark.parametrize("fmt", ["mlx4", "q4_k", "q6_k", "q8_0", "f8_e4m3"])
+@pytest.mark.parametrize("shape", [(3000, 1536, 3108), (2600, 768, 3350)])
+def test_several_segments_a_pair(backend, fmt, shape):
+    """The bits of the form with tokens on M, and 1e-3 of a row (tests/test_gemm_gpu.py) on a sample of the tokens."""
+    n_out, n_in, t = shape
+    ref, m = make_pair(fmt, n_out, n_in, 970 + t)
+    dev = backend.upload(ref, n_out, n_in)
+    x = synth.activations(t, n_in, 971)
+    y = np.full((t, n_out), np.nan, np.float32)
+    assert backend.matmul(x, [ob.Job(dev, y)])
+    rows = np.arange(0, t, 97)
+    assert row_err(y[rows], m.matmul_f64(x[rows])) < 1e-3
+    assert np.array_equal(y, with_tokens_on_m(backend, x, dev, n_out))
+
+
 # pairs per expert: none, one, a tile of 16 and one more, 128 and one more (two tiles of 80 and 49 rows), three tiles
 @pytest.mark.parametrize("fmt", ["mlx4", "q4_k"])
 @pytest.mark.parametrize("counts,h,inter", [([1, 16, 0, 17, 128, 129, 300, 64], 256, 512), ([70], 2048, 768)])
