@@ -911,16 +911,18 @@ static CUresult encode_q6k_qh(TensorMapEncodeFn enc, CUtensorMap* m, const Weigh
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
-// Whether more than 128 one-term tokens take gemm_wp.cu. Both forms are estimated in cycles; here a CTA takes 64 k of 256 tokens in about 1130
-// cycles (more where the expansion is longer) whatever its width, and the last wave counts whole. Measured, us, here / there: Q4_K 14336 x
-// 4096, 200 tokens 47 / 35, 256: 49 / 38, 512: 54 / 59 (one whole wave here), 2048: 213 / 197; 4096 x 14336, 700 tokens 132 / 90; 8192 x
-// 4096, 1000 tokens 59 / 64; Q6_K 4096 x 4096, 4000 tokens 162 / 143; FP8 there 129 / 132; Q8_0 8192 x 1024, 4000 tokens 81 / 94 (the sums
-// of a segment leave as slowly after 8 stages as after 32). The bits are the same.
+// Whether more than 128 one-term tokens take gemm_wp.cu. Both forms are estimated in cycles: here a wave of CTAs takes 64 k of 256 tokens in 1130 and
+// stores in 60 a row of its tiles, and the last wave counts whole; there gemm_wp_share, and for the pairs' start and their last sums 11000, or 7000
+// where the launch leaves a quarter of the SMs to the one behind it. (Fitted to the ratios of 5000 launches of the five formats, 512 .. 28672 rows, K 512 ..
+// 28672, 129 .. 8192 tokens: the choice is 0.2 % slower than the faster form of each, always taking the pairs 0.8 %.) Measured, us, here / there:
+// Q4_K 14336 x 4096, 200 tokens 47 / 35, 512: 54 / 59 (one whole wave here), 2048: 213 / 197; 4096 x 14336, 700 tokens 132 / 90; Q6_K 4096 x 4096,
+// 4000 tokens 162 / 143; of short K: Q6_K 4096 x 1024, 512 tokens 11.9 / 14.4, Q4_K 4096 x 512, 768 tokens 14.3 / 18.2; 512 x 512, 200: 12.1 / 8.0.
+// The bits are the same.
 static bool pairs_are_faster(GemmWp* g, const WeightDev& w, size_t t, int sm_count) {
     const int m_tiles = (int)((t + 255) / 256), tile_n = pick_tile_n(w.n_out, m_tiles, sm_count, w.n_in, w.fmt == B2_FMT_Q6_K ? Q6K_MAX_TILE_N : MAX_TILE_N);
     const size_t tiles = (w.n_out + tile_n - 1) / tile_n * (size_t)m_tiles, waves = (tiles + sm_count - 1) / sm_count;
-    const double stage = w.fmt == B2_FMT_Q6_K ? 1400.0 : w.fmt == B2_FMT_F8E4M3 ? 1080.0 : 1130.0;
-    return gemm_wp_share(g, w.n_out, t, w.n_in, sm_count) + 6000.0 < waves * (w.n_in / 64) * stage + 8000.0;
+    const double there = gemm_wp_share(g, w.n_out, t, w.n_in, sm_count) + (8 * g->busy <= 3 * sm_count ? 7000.0 : 11000.0);
+    return there < waves * (w.n_in / 64 * 1130.0 + 60.0 * tile_n);
 }
 
 cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, void* y, int y_dtype, GemmPlan** out, char* err,

@@ -550,25 +550,29 @@ double gemm_wp_share(GemmWp* g, size_t n_out_, size_t t_, size_t n_in, int sm_co
     const int pairs = (int)std::min<long long>(std::max(1, sm_count / 2), (long long)blocks * units), most = WP_SEG / WP_UNIT, least = (units + most - 1) / most;
     auto segment = [&](int n) { return stages * std::max(780.0, 4.0 * n) + (n > 128 ? 7500.0 : 500.0); };
     double best = 1e30;
-    auto take = [&](double cost, const WpShare& share) {
+    auto take = [&](double cost, int busy, const WpShare& share) {
         if (cost >= best) return;
         best = cost;
+        g->busy = std::min(busy, pairs);
         g->share = share;
     };
     auto run = [&](int snap) {
         const WpShare share{0, snap, 0, 1};
         double cost = 0.0;
+        int busy = 0;
         for (int c = 0; c < pairs && cost < best; c++) {
             double sum = 0.0;
             for (Segments s(n_out, t, 0, share, c, pairs); s.next(nullptr, n_out, t, share);) sum += segment(s.n);
             cost = std::max(cost, sum);
+            busy += sum > 0.0;
         }
-        take(cost, share);
+        take(cost, busy, share);
     };
     auto deal = [&](int pieces, int most_parts) {  // whole waves of whole segments, and the rest in as many parts as cost least
         const int tiles = pieces * blocks, rest = tiles % pairs, longest = (units + pieces - 1) / pieces;
         for (int split = 1; split <= most_parts; split++)
-            take(tiles / pairs * segment(longest * WP_UNIT) + (rest * split + pairs - 1) / pairs * segment((longest + split - 1) / split * WP_UNIT), WpShare{pieces, 0, tiles - rest, split});
+            take(tiles / pairs * segment(longest * WP_UNIT) + (rest * split + pairs - 1) / pairs * segment((longest + split - 1) / split * WP_UNIT),
+                 tiles - rest + rest * split, WpShare{pieces, 0, tiles - rest, split});
     };
     g->pairs = pairs;
     if ((long long)blocks * units / pairs <= 16) {

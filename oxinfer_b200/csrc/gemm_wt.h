@@ -43,6 +43,7 @@ struct GemmWp {
     XMaps x;
     CUtensorMap w, w2, y;
     int pairs = 0;
+    int busy = 0;                         // a dense launch's pairs that have segments
     WpShare share = {};
     int lo_row0 = 0;                      // grouped Q4_K launches with two-term operands: the activations' second terms, rows below the first
     bool staged = false;                  // the results can leave through the copy engine
