@@ -515,11 +515,17 @@ cudaError_t launch_gemm_f8(const WeightDev& w, const uint8_t* qx, const float* s
         snprintf(err, errlen, "cuTensorMapEncodeTiled is not available from the driver");
         return cudaErrorNotSupported;
     }
-    // The CTA-pair form for more than one 128-token tile (B2_F8_PAIR=0: never): a CTA keeps half of the weight tile, so shared memory moves
-    // 32 KB a block of 128 k instead of 48. 8192 x 12288 x 28672: 3.27 ms against 3.59 for single CTAs; 512 x 4096 x 14336: 47.5 us
-    // against 50.9 (bit-identical results).
+    const int n_tiles = (int)((w.n_out + F8_TN - 1) / F8_TN);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int m_tiles = (int)((t + F8_TM - 1) / F8_TM), pm_tiles = (m_tiles + 1) / 2;
+    // The CTA-pair form: a CTA keeps half of the weight tile, so shared memory moves 32 KB a block of 128 k instead of 48, and a block takes 0.92 of the
+    // time; a launch starts later by 1.3 blocks; and an odd count of 128-token tiles is rounded up, which can cost a wave: 384 tokens of 12288 rows, K =
+    // 4096, 28 us on single CTAs (one wave), 48 on pairs (two); with as many waves either way 0.92 .. 0.96 from K = 4096 on (8192 x 12288 x
+    // 28672: 3.27 ms against 3.59), 1.03 at one wave of K = 1024. B2_F8_PAIR: 0 never, 1 always above 128 tokens. The bits are the same.
     const char* pe = getenv("B2_F8_PAIR");
-    const bool pair = t > (size_t)F8_TM && !(pe && atoi(pe) == 0);
+    const size_t nb = w.n_in / F8_BK, waves = ((size_t)m_tiles * n_tiles + sms - 1) / sms, pair_waves = ((size_t)pm_tiles * n_tiles + sms / 2 - 1) / (sms / 2);
+    const bool pair = m_tiles > 1 && (pe ? atoi(pe) != 0 : 0.92 * (double)(pair_waves * nb) + 1.3 < (double)(waves * nb));
     CUtensorMap tx, tw;
     cuuint32_t estr[2] = {1, 1};
     {
@@ -544,31 +550,28 @@ cudaError_t launch_gemm_f8(const WeightDev& w, const uint8_t* qx, const float* s
             return cudaErrorInvalidValue;
         }
     }
-    const int n_tiles = (int)((w.n_out + F8_TN - 1) / F8_TN);
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (pair) {
         auto kern = gemm_f8_tc_kernel<true>;
         if (cudaError_t e = ensure_dynamic_smem((const void*)kern, F8_PAIR_SMEM, 0); e != cudaSuccess) return e;
-        const int pm_tiles = (int)((t + 2 * F8_TM - 1) / (2 * F8_TM));
         const int pairs = std::min(pm_tiles * n_tiles, sms / 2);  // persistent: one CTA per SM, two SMs per pair
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(2 * pairs));
         cfg.blockDim = dim3(F8_THREADS);
         cfg.dynamicSmemBytes = F8_PAIR_SMEM;
         cfg.stream = st;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;  // a CTA pair is formed along x
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
+        cudaLaunchAttribute attr[2] = {};
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2;  // a CTA pair is formed along x
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (as the other form: see the top of the kernel)
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
         return cudaLaunchKernelEx(&cfg, kern, tx, tw, (int)w.n_in, (int)w.n_out, (int)t, pm_tiles, n_tiles, sx, (const float*)w.p1, (int)w.bs_ncb,
                                   (int)w.bs_row0, y, y_dtype, status_dev);
     }
     if (cudaError_t e = ensure_dynamic_smem((const void*)gemm_f8_tc_kernel<false>, F8_SMEM, 0); e != cudaSuccess) return e;
-    const int m_tiles = (int)((t + F8_TM - 1) / F8_TM);
     const int grid = m_tiles * n_tiles < sms ? m_tiles * n_tiles : sms;  // persistent: one CTA per SM
     return launch_k(gemm_f8_tc_kernel<false>, dim3((unsigned)grid), dim3(F8_THREADS), F8_SMEM, st, true, tx, tw, (int)w.n_in, (int)w.n_out, (int)t, m_tiles,
                     n_tiles, sx, (const float*)w.p1, (int)w.bs_ncb, (int)w.bs_row0, y, y_dtype, status_dev);

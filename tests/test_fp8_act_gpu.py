@@ -88,27 +88,29 @@ def test_default_keeps_the_reference_definition(backend):
     assert row_err(y, m.matmul_f64(x)) < 2e-3
 
 
-@pytest.mark.parametrize("shape", [(1000, 2048, 700), (2304, 4096, 1024), (256, 256, 129)])
+# ragged counts of tokens and rows, an odd count of 128-token tiles, and more tiles than there are pairs (148 of 256 x 256 for 74)
+@pytest.mark.parametrize("shape", [(1000, 2048, 700), (2304, 4096, 1024), (256, 256, 129), (600, 512, 300), (9400, 512, 1000)])
 def test_fp8_cta_pair_form_equals_the_single_cta_form(fp8_backend, shape):
-    """B2_F8_PAIR=1: more than 128 tokens run as pairs of CTAs that share each weight tile (M = 256 instructions, tcgen05
-    cta_group::2). Each output is the same sequence of 128-k partial sums promoted in the same order: the results must be
-    equal to the single-CTA form's bit for bit, ragged token and row counts included."""
+    """More than 128 tokens run on single CTAs (B2_F8_PAIR=0), as pairs of CTAs that share each weight tile (1: M = 256 instructions, tcgen05
+    cta_group::2), or on the form that the launch's counts of tiles make faster (unset). Each output is the same sequence of 128-k partial
+    sums promoted in the same order: the results must be equal bit for bit."""
     import os
 
     n_out, n_in, t = shape
     ref, m = make_pair("f8_e4m3", n_out, n_in, 520 + t)
     dev = fp8_backend.upload(ref, n_out, n_in)
     x = synth.activations(t, n_in, 521)
-    y1 = np.full((t, n_out), np.nan, np.float32)
-    assert fp8_backend.matmul(x, [ob.Job(dev, y1)])
-    os.environ["B2_F8_PAIR"] = "1"
-    try:
-        y = np.full((t, n_out), np.nan, np.float32)
-        assert fp8_backend.matmul(x, [ob.Job(dev, y)])
-    finally:
-        del os.environ["B2_F8_PAIR"]
-    assert np.isfinite(y).all()
-    assert np.array_equal(y, y1)
+    y = {}
+    for form in ("0", "1", None):
+        if form:
+            os.environ["B2_F8_PAIR"] = form
+        try:
+            y[form] = np.full((t, n_out), np.nan, np.float32)
+            assert fp8_backend.matmul(x, [ob.Job(dev, y[form])])
+        finally:
+            os.environ.pop("B2_F8_PAIR", None)
+    assert np.isfinite(y["0"]).all()
+    assert np.array_equal(y["1"], y["0"]) and np.array_equal(y[None], y["0"])
     rows = np.unique(np.concatenate([np.arange(0, t, 53), [t - 1, 127, 128]]))
     want, _ = oracle_fp8_act(m, x[rows])
-    assert row_err(y[rows], want) < 1e-5
+    assert row_err(y["0"][rows], want) < 1e-5
