@@ -892,7 +892,7 @@ class Backend {
         if (pairs) {
             GemmWp g;
             if (!gemm_wp_encode(&g, w, experts, true, xg, rows, sm_count, out_dev, B2_F32, n_out, lo_row0)) return fail(B2_ERR_CUDA, "[b200qmm: the tensor maps of a grouped product could not be made]");
-            cudaError_t e = launch_gemm_wp(g, w, rows, tiles, (int)n_tiles, out_dev, B2_F32, n_out, nullptr, 0, gemm_status, row_unscale, stream);
+            cudaError_t e = launch_gemm_wp(g, w, rows, tiles, (int)n_tiles, out_dev, B2_F32, n_out, gemm_status, row_unscale, stream);
             launches++;
             return e == cudaSuccess ? B2_OK : cuda_fail(e, "grouped gemm (pairs)");
         }

@@ -917,7 +917,7 @@ static CUresult encode_q6k_qh(TensorMapEncodeFn enc, CUtensorMap* m, const Weigh
 // 28672, 129 .. 8192 tokens: the choice is 0.2 % slower than the faster form of each, always taking the pairs 0.8 %.) Measured, us, here / there:
 // Q4_K 14336 x 4096, 200 tokens 47 / 35, 512: 54 / 59 (one whole wave here), 2048: 213 / 197; 4096 x 14336, 700 tokens 132 / 90; Q6_K 4096 x 4096,
 // 4000 tokens 162 / 143; of short K: Q6_K 4096 x 1024, 512 tokens 11.9 / 14.4, Q4_K 4096 x 512, 768 tokens 14.3 / 18.2; 512 x 512, 200: 12.1 / 8.0.
-// The bits are the same.
+// The bits are the same. (Results that go to peers too keep the form with tokens on M, whose tiles leave through the copy engine, once per destination.)
 static bool pairs_are_faster(GemmWp* g, const WeightDev& w, size_t t, int sm_count) {
     const int m_tiles = (int)((t + 255) / 256), tile_n = pick_tile_n(w.n_out, m_tiles, sm_count, w.n_in, w.fmt == B2_FMT_Q6_K ? Q6K_MAX_TILE_N : MAX_TILE_N);
     const size_t tiles = (w.n_out + tile_n - 1) / tile_n * (size_t)m_tiles, waves = (tiles + sm_count - 1) / sm_count;
@@ -935,6 +935,11 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
         snprintf(err, errlen, "a gathered product needs a dense f32 result with 16-byte aligned column blocks");
         return cudaErrorInvalidValue;
     }
+    for (int d = 0; gathered && d < peer_y->n_more; d++)
+        if ((uintptr_t)peer_y->more[d] & 15) {
+            snprintf(err, errlen, "a gathered product needs 16-byte aligned column blocks of the peers' results");
+            return cudaErrorInvalidValue;
+        }
 
     if (!enc) {
         snprintf(err, errlen, "cuTensorMapEncodeTiled is not available from the driver");
@@ -965,7 +970,7 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
     if (w_terms == 1 && split_k_asked() == 1 && ((uintptr_t)w.p2 & 7) == 0) {
         if (t <= WT_MOST)
             p->wt_form = 1;
-        else if (!a_lo_row0 && !pair_form_enabled() && pairs_are_faster(&p->wp, w, t, sm_count))
+        else if (!a_lo_row0 && !pair_form_enabled() && !(gathered && peer_y->n_more > 0) && pairs_are_faster(&p->wp, w, t, sm_count))
             p->wt_form = 2;
     }
     if (p->wt_form) {
@@ -1073,7 +1078,6 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
         if (gathered && peer_y->n_more > 0) {
             CUtensorMap maps[8];
             for (int d = 0; d < peer_y->n_more; d++) {
-                if (((uintptr_t)peer_y->more[d] & 15) != 0) r = CUDA_ERROR_INVALID_VALUE;
                 if (r == CUDA_SUCCESS)
                     r = enc(&maps[d], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, peer_y->more[d], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1131,7 +1135,7 @@ bool gemm_tc_plan_matches(const GemmPlan* p, const WeightDev& w, const void* x16
 cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, int y_dtype, GemmStatus* status_dev, int /*sm_count*/,
                            cudaStream_t st, const float* row_unscale) {
     if (p->wt_form == 2)
-        return launch_gemm_wp(p->wp, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, p->more_ptr, p->n_more, status_dev, row_unscale, st);
+        return launch_gemm_wp(p->wp, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, status_dev, row_unscale, st);
     if (p->wt_form)
         return launch_gemm_wt(p->wt, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, p->more_ptr, p->n_more, status_dev, row_unscale, st);
     const bool split = p->k_splits > 1;

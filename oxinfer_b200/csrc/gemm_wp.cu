@@ -68,8 +68,6 @@ struct WpArgs {
     const float* s;       // scales beside the packed rows, as in gemm_tc.cu
     const void* s2;
     int f8_rows, f8_ncb, f8_row0;
-    int n_more;           // other ranks' copies of y
-    float* more[7];
 };
 
 // The segments of a pair, the same for every role of both CTAs. Grouped launches: every tile with every row block, dealt out in turn. Dense, one of
@@ -335,7 +333,6 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
         asm volatile("griddepcontrol.wait;" ::: "memory");
         const uint32_t acc_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const uint32_t empty_even = cluster_addr(&sh->acc_empty[0], 0);
-        const bool plain = !a.y_bf16 && a.n_more == 0;
         uint8_t* staging = raw + (size_t)NRAW * RAW_SLOT + (size_t)(warp & 3) * 8192;
         Halves<SECOND> acc_of;
         int tile = 0;
@@ -387,7 +384,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                 }
                 const size_t at = (size_t)(seg.x_row0 + c) * a.y_ld + row;
                 const int rows = row < a.n_out ? live : 0;
-                if (TWO || plain) {
+                if (TWO || !a.y_bf16) {
                     float* o = (float*)a.y + at;
 #pragma unroll
                     for (int j = 0; j < 32; j++, o += a.y_ld) {
@@ -398,14 +395,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
 #pragma unroll
                     for (int j = 0; j < 32; j++) {
                         const float w = __uint_as_float(v[j]) * __shfl_sync(0xffffffffu, f, j);
-                        const size_t o = at + (size_t)j * a.y_ld;
-                        if (j < rows) {
-                            if (a.y_bf16)
-                                ((__nv_bfloat16*)a.y)[o] = __float2bfloat16_rn(w);
-                            else
-                                ((float*)a.y)[o] = w;
-                            for (int d = 0; d < a.n_more; d++) a.more[d][o] = w;
-                        }
+                        if (j < rows) ((__nv_bfloat16*)a.y)[at + (size_t)j * a.y_ld] = __float2bfloat16_rn(w);
                     }
                 }
             }
@@ -607,7 +597,7 @@ bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, bool grouped,
     return gemm_x_maps(&g->x, 0, WP_SEG / 32 - 1, x16, lo_row0 + x_rows, w.n_in, lo_row0 ? 1 : 2);
 }
 
-cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
+cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld,
                            GemmStatus* status, const float* row_unscale, cudaStream_t st) {
     using Kern = void (*)(XMaps, CUtensorMap, CUtensorMap, CUtensorMap, WpArgs);
     if (tiles && w.fmt != (g.lo_row0 ? B2_FMT_Q4_K : B2_FMT_MLX4)) return cudaErrorInvalidValue;
@@ -625,7 +615,7 @@ cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const 
     a.n_out = (int)w.n_out;
     a.t = (int)t;
     a.share = g.share;
-    a.staged = g.staged && n_more == 0;
+    a.staged = g.staged;
     a.y_bf16 = y_dtype == B2_BF16;
     a.y_ld = y_ld;
     a.y = y;
@@ -639,8 +629,6 @@ cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const 
     a.f8_rows = w.fmt == B2_FMT_F8E4M3 ? (int)w.bs_rows : 1;
     a.f8_ncb = w.fmt == B2_FMT_Q8_0 ? (int)(w.n_in / 32) : (int)w.bs_ncb;
     a.f8_row0 = (int)w.bs_row0;
-    a.n_more = n_more;
-    for (int i = 0; i < n_more; i++) a.more[i] = more[i];
     const size_t blocks = (w.n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(2 * (tiles ? std::min<size_t>(blocks * (size_t)n_tiles, (size_t)g.pairs) : (size_t)g.pairs)));

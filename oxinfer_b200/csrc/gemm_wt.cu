@@ -402,7 +402,7 @@ gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
         if (warp < 8 && !sh->abort_flag) {
             const uint32_t sums = smem_u32(smem);
             const int row = n0 + 4 * lane;
-            const bool vec = !a.y_bf16 && a.n_more == 0 && (a.y_ld & 3) == 0 && ((uintptr_t)a.y & 15) == 0 && row + 4 <= a.n_out;
+            const bool vec = !a.y_bf16 && (a.y_ld & 3) == 0 && ((uintptr_t)a.y & 15) == 0 && row + 4 <= a.n_out;  // (other ranks' copies are aligned as y)
             for (int tok = part * 8 + warp; tok < count; tok += 8 * a.splits) {
                 const uint32_t at = sums + (uint32_t)(tok * WT_ROWS + 4 * lane) * 4u;
                 const float f = (PRE_SCALED ? 1.0f / WT_PRE : 1.0f) * (a.row_unscale ? __ldg(a.row_unscale + x_row0 + tok) : 1.0f);
@@ -425,7 +425,9 @@ gemm_wt_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
                 }
                 const size_t o = (size_t)(x_row0 + tok) * a.y_ld + row;
                 if (vec) {
-                    *(float4*)((float*)a.y + o) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+                    const float4 w = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+                    *(float4*)((float*)a.y + o) = w;
+                    for (int d = 0; d < a.n_more; d++) *(float4*)(a.more[d] + o) = w;
                 } else {
                     const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll

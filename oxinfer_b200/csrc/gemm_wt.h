@@ -53,7 +53,7 @@ double gemm_wp_share(GemmWp* g, size_t n_out, size_t t, size_t n_in, int sm_coun
 // x_rows: the tokens (grouped: the rows of all segments). Dense: after gemm_wp_share.
 bool gemm_wp_encode(GemmWp* g, const WeightDev& w, size_t experts, bool grouped, const void* x16, size_t x_rows, int sm_count, void* y, int y_dtype, size_t y_ld,
                     size_t lo_row0 = 0);
-cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld, float* const* more, int n_more,
+cudaError_t launch_gemm_wp(const GemmWp& g, const WeightDev& w, size_t t, const WtTile* tiles, int n_tiles, void* y, int y_dtype, size_t y_ld,
                            GemmStatus* status, const float* row_unscale, cudaStream_t st);
 
 }  // namespace b2

@@ -144,8 +144,9 @@ struct GemmPlan;
 // value to about 22 bits; tiles are then at most 112 rows wide.
 // Where a row-sharded product's f32 result goes when every rank is to end up with the whole y [t][ld]: this rank's columns
 // of its own y (`y` of the call, already offset to them) and of n_more peers' copies (device pointers mapped from the
-// peers, offset the same way). The GEMM's epilogue then issues each staging tile's bulk store once per destination, so the
-// all-gather happens tile by tile from the kernel that computes the tiles.
+// peers, offset the same way). The GEMM's epilogue then stores its results once per destination (more than 128 tokens: each staging
+// tile by the copy engine; up to 128: gemm_wt.cu's threads, 16 bytes at a time where K is divided), so the all-gather happens tile by
+// tile from the kernel that computes the tiles.
 struct GemmPeerY {
     size_t ld = 0;        // row stride of the destinations in elements (0: not a gathered product, the stride is n_out)
     int n_more = 0;       // peers' destinations
