@@ -853,8 +853,13 @@ struct GemmPlan {
     int split_asked = 1;  // B2_GEMM_SPLIT_K when the plan was made (a cached plan is reused only under the same setting)
 };
 
-// Dense products of up to this many tokens take gemm_wt.cu.
-static constexpr size_t WT_MOST = 128;
+// Dense products of up to this many tokens take gemm_wt.cu: 128, fewer where K is short (and not divided: the bits are the same) and the tokens
+// are many, so that 64-row tiles here end before 128-row ones there. us, here / there: 4096 x 256, Q4_K, 112 tokens 5.2 / 6.1, 96: 5.3 / 5.5; Q6_K, 128
+// tokens, 4096 x 512 7.1 / 8.0, 14336 x 1024 13.4 / 14.1, 4096 x 1536 14.2 / 14.3, 32064 x 512 (two waves here) 17.5 / 10.5.
+static size_t wt_most(const WeightDev& w, int sm_count) {
+    if (w.n_in <= 256) return 96;
+    return w.fmt == B2_FMT_Q6_K && w.n_in <= 1024 && w.n_out <= (size_t)Q6K_MAX_TILE_N * sm_count ? 112 : 128;
+}
 
 bool gemm_tc_supports(const WeightDev& w, size_t t) {
     if (w.fmt == B2_FMT_F8E4M3) return w.n_in % 128 == 0 && t >= 1 && ((uintptr_t)w.p0 & 15) == 0 && (w.p1 == nullptr || w.bs_cols == 128);
@@ -968,8 +973,8 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
     if (w_terms == 2 && w.fmt != B2_FMT_Q4_K) w_terms = 1;  // the other formats' weights round to f16 far below the bound
     p->w_terms = w_terms;
     if (w_terms == 1 && split_k_asked() == 1 && ((uintptr_t)w.p2 & 7) == 0) {
-        if (t <= WT_MOST)
-            p->wt_form = 1;
+        if (t <= 128)
+            p->wt_form = t <= wt_most(w, sm_count) ? 1 : 0;
         else if (!a_lo_row0 && !pair_form_enabled() && !(gathered && peer_y->n_more > 0) && pairs_are_faster(&p->wp, w, t, sm_count))
             p->wt_form = 2;
     }
