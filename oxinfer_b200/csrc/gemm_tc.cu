@@ -97,7 +97,7 @@ static_assert(PAIR_SMEM <= 227 * 1024, "shared memory budget (pair form)");
 template <int FMT, bool SPLIT, bool TT, bool PAIR = false>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
-                   const __grid_constant__ CUtensorMap tmap_y, int K, int n_out, int t,
+                   const __grid_constant__ CUtensorMap tmap_w2, const __grid_constant__ CUtensorMap tmap_y, int K, int n_out, int t,
                    int tile_n, int m_halves, void* __restrict__ y, int y_dtype_arg, GemmStatus* __restrict__ status, int dbg_arg, int zero,
                    F8Scales f8, int k_splits, const float* __restrict__ row_unscale, int a_lo_row_arg, int w_terms,
                    const CUtensorMap* __restrict__ y_more, int n_more) {
@@ -120,7 +120,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     // A "raw block" is a row's part of the packed weights that are expanded in one round: a 144-byte 4-bit block (256 k, four pipeline
     // stages) or 128 e4m3 bytes (128 k = one column of FP8 scale blocks, two stages), which come in two copies.
     // Q8_0 rows are 128 int8 like the FP8 rows; a Q6_K copy brings a row's 128 bytes of low nibbles and, through a
-    // second tensor map (y_more[n_more]), its 64 bytes of high bit pairs (the planes of formats.cuh), 256 k = four stages.
+    // second tensor map (tmap_w2), its 64 bytes of high bit pairs (the planes of formats.cuh), 256 k = four stages.
     constexpr bool BYTE_ROWS = FMT == B2_FMT_F8E4M3 || FMT == B2_FMT_Q8_0;
     constexpr bool PRE_SCALED = BYTE_ROWS || FMT == B2_FMT_Q6_K;  // the f16 weights carry the factor f8.pre, the epilogue takes it out
     constexpr int RAW_ROW = BYTE_ROWS ? 128 : (FMT == B2_FMT_Q6_K ? 192 : 144);
@@ -264,7 +264,7 @@ gemm_q4k_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 mbar_arrive_expect_tx(&sh->raw_full[rb], w_bytes);
                 if constexpr (FMT == B2_FMT_Q6_K) {  // [rows][128] low nibbles, then [rows][64] high bit pairs
                     tma_load_2d(raw, &tmap_w, &sh->raw_full[rb], (sb0 + c) * 128, n0);
-                    tma_load_2d(raw + (size_t)my_rows * 128, y_more + n_more, &sh->raw_full[rb], (sb0 + c) * 64, n0);
+                    tma_load_2d(raw + (size_t)my_rows * 128, &tmap_w2, &sh->raw_full[rb], (sb0 + c) * 64, n0);
                     w_issued = c + 1;
                     continue;
                 }
@@ -830,7 +830,7 @@ TensorMapEncodeFn tensor_map_encode() {
 }
 
 struct GemmPlan {
-    CUtensorMap tmap_x, tmap_w, tmap_y;
+    CUtensorMap tmap_x, tmap_w, tmap_w2, tmap_y;  // (tmap_w2: Q6_K's second plane)
     int wt_form = 0;  // weights in tensor memory: 1 gemm_wt.cu, 2 its pair form gemm_wp.cu; only these and the shapes are then in use
     GemmWt wt;
     GemmWp wp;
@@ -1063,6 +1063,13 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
             return cudaErrorInvalidValue;
         }
     }
+    p->tmap_w2 = p->tmap_w;
+    if (w.fmt == B2_FMT_Q6_K)
+        if (CUresult r = encode_q6k_qh(enc, &p->tmap_w2, w, p->tile_n); r != CUDA_SUCCESS) {
+            snprintf(err, errlen, "the tensor map of the Q6_K high-bit plane could not be made (CUresult %d)", (int)r);
+            delete p;
+            return cudaErrorInvalidValue;
+        }
     p->tmap_y = p->tmap_x;  // placeholder when the epilogue stores directly (bf16 output)
     p->y_direct = y_dtype == B2_F32 && !gathered && (w.n_out % 4 != 0 || ((uintptr_t)y & 15) != 0);
     if (y_dtype == B2_F32 && !p->y_direct) {
@@ -1088,10 +1095,8 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
                 p->more_ptr[d] = peer_y->more[d];
             }
-            const int extra = w.fmt == B2_FMT_Q6_K ? 1 : 0;  // the qh plane's map goes behind the peers'
-            if (extra && r == CUDA_SUCCESS) r = encode_q6k_qh(enc, &maps[peer_y->n_more], w, p->tile_n);
-            cudaError_t ce = r == CUDA_SUCCESS ? cudaMalloc((void**)&p->y_more, sizeof(CUtensorMap) * (peer_y->n_more + extra)) : cudaErrorInvalidValue;
-            if (ce == cudaSuccess) ce = cudaMemcpy(p->y_more, maps, sizeof(CUtensorMap) * (peer_y->n_more + extra), cudaMemcpyHostToDevice);
+            cudaError_t ce = r == CUDA_SUCCESS ? cudaMalloc((void**)&p->y_more, sizeof(CUtensorMap) * peer_y->n_more) : cudaErrorInvalidValue;
+            if (ce == cudaSuccess) ce = cudaMemcpy(p->y_more, maps, sizeof(CUtensorMap) * peer_y->n_more, cudaMemcpyHostToDevice);
             if (ce != cudaSuccess) {
                 snprintf(err, errlen, "tensor maps of the peers' y could not be made (CUresult %d, %s)", (int)r, cudaGetErrorString(ce));
                 if (p->y_more) cudaFree(p->y_more);
@@ -1101,18 +1106,6 @@ cudaError_t gemm_tc_plan_create(const WeightDev& w, const void* x16, size_t t, v
             p->n_more = peer_y->n_more;
         }
         p->y_ld = gathered ? ld : 0;
-    }
-    if (w.fmt == B2_FMT_Q6_K && !p->y_more) {  // the second weight plane's tensor map, read from global memory by the kernel
-        CUtensorMap m;
-        CUresult r = encode_q6k_qh(enc, &m, w, p->tile_n);
-        cudaError_t ce = r == CUDA_SUCCESS ? cudaMalloc((void**)&p->y_more, sizeof(CUtensorMap)) : cudaErrorInvalidValue;
-        if (ce == cudaSuccess) ce = cudaMemcpy(p->y_more, &m, sizeof m, cudaMemcpyHostToDevice);
-        if (ce != cudaSuccess) {
-            snprintf(err, errlen, "the tensor map of the Q6_K high-bit plane could not be made (CUresult %d, %s)", (int)r, cudaGetErrorString(ce));
-            if (p->y_more) cudaFree(p->y_more);
-            delete p;
-            return cudaErrorInvalidValue;
-        }
     }
     *out = p;
     return cudaSuccess;
@@ -1145,7 +1138,7 @@ cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, i
         return launch_gemm_wt(p->wt, w, t, nullptr, 0, y, y_dtype, p->y_ld ? p->y_ld : w.n_out, p->more_ptr, p->n_more, status_dev, row_unscale, st);
     const bool split = p->k_splits > 1;
     const bool tt = p->a_lo_row0 > 0 || p->w_terms == 2;
-    using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, int, int, int, int, int, void*, int, GemmStatus*, int, int, F8Scales, int, const float*,
+    using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, int, int, int, int, int, void*, int, GemmStatus*, int, int, F8Scales, int, const float*,
                           int, int, const CUtensorMap*, int);
     Kern kern;
     if (tt)  // two-term operands never come with a K split
@@ -1177,7 +1170,7 @@ cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, i
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 2;
-        cudaError_t le = cudaLaunchKernelEx(&cfg, kern, p->tmap_x, p->tmap_w, p->tmap_y, (int)w.n_in, (int)w.n_out, (int)t, p->tile_n, p->m_halves, y,
+        cudaError_t le = cudaLaunchKernelEx(&cfg, kern, p->tmap_x, p->tmap_w, p->tmap_w2, p->tmap_y, (int)w.n_in, (int)w.n_out, (int)t, p->tile_n, p->m_halves, y,
                                   y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), 0, f8, 1, row_unscale, 0, 1, (const CUtensorMap*)nullptr, 0);
         return le;
     }
@@ -1188,7 +1181,7 @@ cudaError_t launch_gemm_tc(GemmPlan* p, const WeightDev& w, size_t t, void* y, i
         if (e != cudaSuccess) return e;
     }
     // (a dependent launch: see the top of the kernel)
-    return launch_k(kern, grid, dim3(GEMM_THREADS), GEMM_SMEM, st, true, p->tmap_x, p->tmap_w, p->tmap_y, (int)w.n_in, (int)w.n_out, (int)t, p->tile_n, p->m_halves, y,
+    return launch_k(kern, grid, dim3(GEMM_THREADS), GEMM_SMEM, st, true, p->tmap_x, p->tmap_w, p->tmap_w2, p->tmap_y, (int)w.n_in, (int)w.n_out, (int)t, p->tile_n, p->m_halves, y,
                     y_dtype | (p->y_direct ? 0x100 : 0), status_dev, debug_switches(), 0, f8, p->k_splits, row_unscale, (int)p->a_lo_row0, p->w_terms,
                     (const CUtensorMap*)p->y_more, p->n_more);
 }

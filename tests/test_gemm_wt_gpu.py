@@ -134,3 +134,27 @@ def test_segments_of_every_length(backend, fmt, counts, h, inter):
         a = gu[:, :inter] / (1.0 + np.exp(-gu[:, :inter])) * gu[:, inter:]
         want = a @ oracle_matrix(d, h, inter).dequantize_rows().astype(np.float64).T
         assert row_err(y[torch.from_numpy(rows).cuda()].cpu().numpy(), want) < 1e-3, e
+
+
+def test_a_first_q6_k_product_inside_a_capture(backend):
+    """A product with tokens on M allocates and copies nothing when its weights and buffers come up for the first time: it can be captured."""
+    n_out, n_in, t = 300, 1024, 128
+    devs = [backend.upload(make_pair("q6_k", n_out, n_in, 990 + i)[0], n_out, n_in) for i in range(2)]
+    x = torch.from_numpy(synth.activations(t, n_in, 992)).cuda()
+    y, want = torch.zeros((2, t, n_out), device="cuda"), torch.zeros((t, n_out), device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    backend.set_stream(stream.cuda_stream)
+    try:
+        assert backend.matmul_dev(devs[0], x, y[0])  # (scratch for this batch)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            assert backend.matmul_dev(devs[1], x, y[1])
+        graph.replay()
+        assert backend.matmul_dev(devs[1], x, want)
+        torch.cuda.synchronize()
+        backend.check_status()
+    finally:
+        backend.set_stream(0)
+    assert torch.equal(y[1], want) and not torch.equal(y[0], want)
