@@ -1,6 +1,6 @@
 // Dequant-GEMM with the weights in tensor memory, CTA-pair form: more than 128 tokens, and routed experts with long segments.
 //
-//   y[t][n_out] = x[t][K] * W^T      (one-term f16 operands, f32 sums; the operands and the order of the sums of gemm_wt.cu)
+//   y[t][n_out] = x[t][K] * W^T      (one-term f16 operands, two-term ones for Q4_K experts; f32 sums; the order of the sums of gemm_wt.cu)
 //
 // A pair of CTAs (tcgen05 cta_group::2, M = 256) multiplies 256 weight rows by a segment of up to 256 tokens over the whole K: each CTA
 // expands 128 of the rows into its own tensor memory (the A operand, a ring of slots of 128 k) and copies half of the segment's
@@ -77,25 +77,24 @@ struct WpArgs {
 // - pieces 0: one list of units of 32 tokens, row block by row block, of which every pair takes an equal run, cut at the ends of row blocks; a
 //   run's end within `snap` units of a row block's end is moved there. Pairs stand at unrelated tokens: for launches whose operands fit L2.
 struct Segments {
-    int pos, end, step, per_block, blocks;
+    int pos, end;
     int row, w_row, x_row0, n, count;  // first of the 256 rows in its matrix / in the stack; tokens: first, padded to 32, real
     __host__ __device__ __forceinline__ Segments(int n_out, int t, int n_tiles, const WpShare& share, int c, int pairs) {
-        blocks = (n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
-        per_block = (t + WP_UNIT - 1) / WP_UNIT;
+        const int blocks = (n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
         pos = c;
-        step = pairs;
         end = n_tiles ? n_tiles * blocks : share.whole + (share.pieces * blocks - share.whole) * share.split;
         if (!n_tiles && !share.pieces) {
-            pos = bound(c, pairs, share.snap);
-            end = bound(c + 1, pairs, share.snap);
+            pos = bound(blocks, (t + WP_UNIT - 1) / WP_UNIT, c, pairs, share.snap);
+            end = bound(blocks, (t + WP_UNIT - 1) / WP_UNIT, c + 1, pairs, share.snap);
         }
     }
-    __host__ __device__ __forceinline__ int bound(int i, int pairs, int snap) const {
+    __host__ __device__ __forceinline__ static int bound(int blocks, int per_block, int i, int pairs, int snap) {
         const int p = (int)((long long)blocks * per_block * i / pairs), u = p % per_block;
         return u <= snap ? p - u : per_block - u <= snap ? p - u + per_block : p;
     }
-    __host__ __device__ __forceinline__ bool next(const WtTile* tiles, int n_out, int t, const WpShare& share) {
+    __host__ __device__ __forceinline__ bool next(const WtTile* tiles, int n_out, int t, const WpShare& share, int pairs) {
         if (pos >= end) return false;
+        const int blocks = (n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
         if (tiles) {
             const WtTile tile = tiles[pos / blocks];
             row = pos % blocks * (2 * WP_ROWS);
@@ -103,23 +102,39 @@ struct Segments {
             x_row0 = tile.row0;
             count = tile.count;
             n = (count + WP_UNIT - 1) / WP_UNIT * WP_UNIT;
-            pos += step;
+            pos += pairs;
             return true;
         }
         int u, take;
         if (share.pieces) {
-            const int over = pos - share.whole, tile = over < 0 ? pos : share.whole + over / share.split, part = over < 0 ? 0 : over % share.split;
-            const int panel = tile / (WP_PANEL * blocks), in = tile - panel * (WP_PANEL * blocks), left = share.pieces - panel * WP_PANEL;
-            const int wide = left < WP_PANEL ? left : WP_PANEL, p = panel * WP_PANEL + in % wide, parts = over < 0 ? 1 : share.split;
-            row = in / wide * (2 * WP_ROWS);
-            u = (int)((long long)per_block * p / share.pieces);
-            take = (int)((long long)per_block * (p + 1) / share.pieces) - u;
-            const int from = take * part / parts;
-            take = take * (part + 1) / parts - from;
-            u += from;
-            pos += step;
+            // (no 64-bit division: the first segment's place is on the way to a launch's first weights. With two of them 2816 x 1024, 300 tokens,
+            // took 8.9 us instead of 8.4.)
+            const int over = pos - share.whole;
+            int tile = pos, part = 0, panel = 0, wide = share.pieces;
+            if (over >= 0 && share.split > 1) {
+                tile = share.whole + over / share.split;
+                part = over % share.split;
+            }
+            int in = tile;
+            if (share.pieces > WP_PANEL) {
+                panel = tile / (WP_PANEL * blocks);
+                in -= panel * (WP_PANEL * blocks);
+                const int left = share.pieces - panel * WP_PANEL;
+                wide = left < WP_PANEL ? left : WP_PANEL;
+            }
+            const int block = in / wide, p = panel * WP_PANEL + in - block * wide;
+            row = block * (2 * WP_ROWS);
+            u = share.units * p + (p < share.longer ? p : share.longer);
+            take = share.units + (p < share.longer ? 1 : 0);
+            if (over >= 0 && share.split > 1) {
+                const int from = take * part / share.split;
+                take = take * (part + 1) / share.split - from;
+                u += from;
+            }
+            pos += pairs;
         } else {
             constexpr int most = WP_SEG / WP_UNIT;
+            const int per_block = (t + WP_UNIT - 1) / WP_UNIT;
             u = pos % per_block;
             const int left = per_block - u < end - pos ? per_block - u : end - pos, parts = (left + most - 1) / most;
             take = (left + parts - 1) / parts;
@@ -232,7 +247,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             asm volatile("griddepcontrol.wait;" ::: "memory");
             int it = 0, s = 0;
             bool ok = true;
-            while (ok && seg.next(a.tiles, a.n_out, a.t, a.share)) {
+            while (ok && seg.next(a.tiles, a.n_out, a.t, a.share, gridDim.x >> 1)) {
                 const int half = seg.n / 2, y0 = seg.x_row0 + (int)rank * half;
                 const CUtensorMap* tmap_x = &maps.m[half / 16 - 1];
                 for (int ks = 0; ks < stages; ks++, it++, s = s + 1 == NB ? 0 : s + 1) {
@@ -256,7 +271,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             const int copies = BYTE_ROWS ? groups : groups / 4;
             int issued = 0, s = 0, ph = 0;
             bool ok = true;
-            while (ok && seg.next(a.tiles, a.n_out, a.t, a.share)) {
+            while (ok && seg.next(a.tiles, a.n_out, a.t, a.share, gridDim.x >> 1)) {
                 const int w_row = seg.w_row + (int)rank * WP_ROWS;
                 for (int c = 0; c < copies; c++, issued++) {
                     ok = __all_sync(0xffffffffu, mbar_wait(&sh->raw_empty[s], (uint32_t)(ph ^ 1), sh, a.status, 43, (uint32_t)issued));
@@ -287,7 +302,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             bool ok = true;
             int it = 0, sa = 0, pa = 0, s = 0, ph = 0;
             Halves<SECOND> acc_of;
-            while (ok && seg.next(a.tiles, a.n_out, a.t, a.share)) {
+            while (ok && seg.next(a.tiles, a.n_out, a.t, a.share, gridDim.x >> 1)) {
                 acc_of.next(seg.n);
                 const uint32_t acc = tmem + acc_of.col;
                 const uint32_t idesc = (1u << 4) | ((uint32_t)(seg.n >> 3) << 17) | ((256u >> 4) << 24);
@@ -336,7 +351,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
         uint8_t* staging = raw + (size_t)NRAW * RAW_SLOT + (size_t)(warp & 3) * 8192;
         Halves<SECOND> acc_of;
         int tile = 0;
-        while (seg.next(a.tiles, a.n_out, a.t, a.share)) {
+        while (seg.next(a.tiles, a.n_out, a.t, a.share, gridDim.x >> 1)) {
             acc_of.next(seg.n);
             const int row0 = seg.row + (int)rank * WP_ROWS + (warp & 3) * 32, row = row0 + lane;
             auto factor = [&](int c) {  // of token c + lane
@@ -431,7 +446,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
             return ok;
         };
         int it0 = 0, slot = 0, ph = 0, base = 0;
-        for (; ok && seg.next(a.tiles, a.n_out, a.t, a.share); it0 += stages) {
+        for (; ok && seg.next(a.tiles, a.n_out, a.t, a.share, gridDim.x >> 1); it0 += stages) {
             const int row = seg.row + (int)rank * WP_ROWS + r;
             const bool live = row < a.n_out;
             const size_t wrow = live ? (size_t)row : 0;
@@ -547,12 +562,12 @@ double gemm_wp_share(GemmWp* g, size_t n_out_, size_t t_, size_t n_in, int sm_co
         g->share = share;
     };
     auto run = [&](int snap) {
-        const WpShare share{0, snap, 0, 1};
+        const WpShare share{0, snap, 0, 1, 0, 0};
         double cost = 0.0;
         int busy = 0;
         for (int c = 0; c < pairs && cost < best; c++) {
             double sum = 0.0;
-            for (Segments s(n_out, t, 0, share, c, pairs); s.next(nullptr, n_out, t, share);) sum += segment(s.n);
+            for (Segments s(n_out, t, 0, share, c, pairs); s.next(nullptr, n_out, t, share, pairs);) sum += segment(s.n);
             cost = std::max(cost, sum);
             busy += sum > 0.0;
         }
@@ -562,7 +577,7 @@ double gemm_wp_share(GemmWp* g, size_t n_out_, size_t t_, size_t n_in, int sm_co
         const int tiles = pieces * blocks, rest = tiles % pairs, longest = (units + pieces - 1) / pieces;
         for (int split = 1; split <= most_parts; split++)
             take(tiles / pairs * segment(longest * WP_UNIT) + (rest * split + pairs - 1) / pairs * segment((longest + split - 1) / split * WP_UNIT),
-                 tiles - rest + rest * split, WpShare{pieces, 0, tiles - rest, split});
+                 tiles - rest + rest * split, WpShare{pieces, 0, tiles - rest, split, units / pieces, units % pieces});
     };
     g->pairs = pairs;
     if ((long long)blocks * units / pairs <= 16) {

@@ -24,7 +24,7 @@ struct GemmWt {
 // Parts of K of a dense product.
 int wt_splits(size_t K);
 // x16: f16 [x_rows][n_in], `tokens` of them in the longest tile (at most 128 a tile). x_terms 2: the second terms lo_row0 rows below.
-// grouped: w.p0 stacks `experts` matrices of n_out rows (MLX-4, Q4_K). false: no tensor map could be made.
+// grouped: w.p0 stacks `experts` matrices of n_out rows. false: no tensor map could be made.
 bool gemm_wt_encode(GemmWt* g, const WeightDev& w, size_t experts, const void* x16, size_t x_rows, size_t tokens, int x_terms, size_t lo_row0, bool grouped);
 // tiles (device; grouped launches): n_tiles of them; null: `t` tokens in order. y rows y_ld elements apart; more[0 .. n_more): other ranks'
 // copies of an f32 y.
@@ -38,6 +38,7 @@ bool gemm_x_maps(XMaps* x, int first, int last, const void* x16, size_t rows, si
 constexpr int WP_MOST_ROWS = 256, WP_TILE_ROWS = 160;
 struct WpShare {  // how a dense launch is shared out (Segments in gemm_wp.cu)
     int pieces, snap, whole, split;
+    int units, longer;  // a piece's units of 32 tokens, and how many of the first pieces have one more
 };
 struct GemmWp {
     XMaps x;
