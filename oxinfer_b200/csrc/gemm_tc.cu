@@ -855,10 +855,11 @@ struct GemmPlan {
 
 // Dense products of up to this many tokens take gemm_wt.cu: 128, fewer where K is short (and not divided: the bits are the same) and the tokens
 // are many, so that 64-row tiles here end before 128-row ones there. us, here / there: 4096 x 256, Q4_K, 112 tokens 5.2 / 6.1, 96: 5.3 / 5.5; Q6_K, 128
-// tokens, 4096 x 512 7.1 / 8.0, 14336 x 1024 13.4 / 14.1, 4096 x 1536 14.2 / 14.3, 32064 x 512 (two waves here) 17.5 / 10.5.
+// tokens, 4096 x 512 7.1 / 8.0, 14336 x 1024 13.4 / 14.1, 4096 x 1536 14.2 / 14.3; more than a wave here: 32064 x 512 17.5 / 10.5, x 256 12.9 / 8.5.
 static size_t wt_most(const WeightDev& w, int sm_count) {
+    if (w.n_out > (size_t)(w.fmt == B2_FMT_Q6_K ? Q6K_MAX_TILE_N : MAX_TILE_N) * sm_count) return 128;  // more than a wave here
     if (w.n_in <= 256) return 96;
-    return w.fmt == B2_FMT_Q6_K && w.n_in <= 1024 && w.n_out <= (size_t)Q6K_MAX_TILE_N * sm_count ? 112 : 128;
+    return w.fmt == B2_FMT_Q6_K && w.n_in <= 1024 ? 112 : 128;
 }
 
 bool gemm_tc_supports(const WeightDev& w, size_t t) {

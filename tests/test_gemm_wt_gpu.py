@@ -15,10 +15,10 @@ pytestmark = pytest.mark.gpu
 
 # token counts around the steps of 16 and the change of the accumulator's width at 64; row counts around the tiles of 128; one super-block,
 # an odd number of them, the first K that is divided (2 parts), 4 parts and 8 unequal ones; short K whose larger batch runs with tokens on M (all
-# formats, Q6_K)
+# formats, Q6_K, all but Q6_K)
 @pytest.mark.parametrize("fmt", ["mlx4", "q4_k", "q6_k", "q8_0", "f8_e4m3"])
 @pytest.mark.parametrize("shape", [(127, 256, 9), (128, 768, 16), (130, 2816, 17), (260, 3072, 64), (384, 6400, 65), (1001, 12544, 37), (257, 12288, 128),
-                                   (130, 256, 100), (300, 1024, 128)])
+                                   (130, 256, 100), (300, 1024, 128), (31000, 256, 113)])
 def test_products_of_up_to_128_tokens(backend, fmt, shape):
     """f16 operands with f32 sums: 1e-3 of a row (tests/test_gemm_gpu.py). A row shard has the bits of its rows, and a token of a smaller
     batch the bits of the larger one's, f32 in place of the strided or bf16 results of the other entry points included."""
