@@ -76,14 +76,15 @@ struct WpArgs {
 //   8 token ranges and about 9 row blocks, which fit L2 over a long stretch of K.
 // - pieces 0: one list of units of 32 tokens, row block by row block, of which every pair takes an equal run, cut at the ends of row blocks; a
 //   run's end within `snap` units of a row block's end is moved there. Pairs stand at unrelated tokens: for launches whose operands fit L2.
+template <bool GROUPED>
 struct Segments {
     int pos, end;
     int row, w_row, x_row0, n, count;  // first of the 256 rows in its matrix / in the stack; tokens: first, padded to 32, real
     __host__ __device__ __forceinline__ Segments(int n_out, int t, int n_tiles, const WpShare& share, int c, int pairs) {
         const int blocks = (n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
         pos = c;
-        end = n_tiles ? n_tiles * blocks : share.whole + (share.pieces * blocks - share.whole) * share.split;
-        if (!n_tiles && !share.pieces) {
+        end = GROUPED ? n_tiles * blocks : share.whole + (share.pieces * blocks - share.whole) * share.split;
+        if (!GROUPED && !share.pieces) {
             pos = bound(blocks, (t + WP_UNIT - 1) / WP_UNIT, c, pairs, share.snap);
             end = bound(blocks, (t + WP_UNIT - 1) / WP_UNIT, c + 1, pairs, share.snap);
         }
@@ -95,7 +96,7 @@ struct Segments {
     __host__ __device__ __forceinline__ bool next(const WtTile* tiles, int n_out, int t, const WpShare& share, int pairs) {
         if (pos >= end) return false;
         const int blocks = (n_out + 2 * WP_ROWS - 1) / (2 * WP_ROWS);
-        if (tiles) {
+        if constexpr (GROUPED) {
             const WtTile tile = tiles[pos / blocks];
             row = pos % blocks * (2 * WP_ROWS);
             w_row = tile.expert * n_out + row;
@@ -239,7 +240,7 @@ gemm_wp_kernel(const __grid_constant__ XMaps maps, const __grid_constant__ CUten
     cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base, a_cols = tmem + 512u - NA * WP_SLOT_COLS;
-    Segments seg(a.n_out, a.t, a.tiles ? a.n_tiles : 0, a.share, blockIdx.x >> 1, gridDim.x >> 1);
+    Segments<TWO> seg(a.n_out, a.t, a.n_tiles, a.share, blockIdx.x >> 1, gridDim.x >> 1);
 
     if (warp == 20) {
         // ---------------- activations: this CTA's half of the segment's tokens ----------------
@@ -567,7 +568,7 @@ double gemm_wp_share(GemmWp* g, size_t n_out_, size_t t_, size_t n_in, int sm_co
         int busy = 0;
         for (int c = 0; c < pairs && cost < best; c++) {
             double sum = 0.0;
-            for (Segments s(n_out, t, 0, share, c, pairs); s.next(nullptr, n_out, t, share, pairs);) sum += segment(s.n);
+            for (Segments<false> s(n_out, t, 0, share, c, pairs); s.next(nullptr, n_out, t, share, pairs);) sum += segment(s.n);
             cost = std::max(cost, sum);
             busy += sum > 0.0;
         }
