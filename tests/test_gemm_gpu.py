@@ -286,7 +286,11 @@ def test_cta_pair_form_equals_the_single_cta_form(backend, fmt, shape):
     dev = backend.upload(ref, n_out, n_in)
     x = synth.activations(t, n_in, 471)
     y1 = np.full((t, n_out), np.nan, np.float32)
-    assert backend.matmul(x, [ob.Job(dev, y1)])
+    os.environ["B2_GEMM_SPLIT_K"] = "0"  # (tokens on M; unset, the launch may run on the CTA pairs of gemm_wp.cu)
+    try:
+        assert backend.matmul(x, [ob.Job(dev, y1)])
+    finally:
+        del os.environ["B2_GEMM_SPLIT_K"]
     os.environ["B2_GEMM_PAIR"] = "1"
     try:
         y = np.full((t, n_out), np.nan, np.float32)

@@ -44,8 +44,8 @@ def test_products_of_up_to_128_tokens(backend, fmt, shape):
     assert torch.equal(yd.cpu(), torch.from_numpy(y).bfloat16())
 
 
-# one token and one unit of 32 past what the smaller kernel takes, segments of 160, 256 and around them, rows that end inside a pair's 256 and
-# inside a CTA's 128, an odd number of super-blocks
+# one token and one unit of 32 past what the smaller kernel takes, one segment of 32 to 128 tokens a pair (longer ones and several a pair:
+# test_several_segments_a_pair; the smallest shape runs with tokens on M), rows that end inside a pair's 256 and inside a CTA's 128, an odd number of super-blocks
 @pytest.mark.parametrize("fmt", ["mlx4", "q4_k", "q6_k", "q8_0", "f8_e4m3"])
 @pytest.mark.parametrize("shape", [(200, 256, 129), (333, 768, 161), (1000, 512, 257), (2100, 1280, 300), (512, 2048, 700)])
 def test_products_of_more_tokens(backend, fmt, shape):
@@ -96,10 +96,10 @@ def test_byte_rows_that_end_inside_a_round_of_the_sets(backend, fmt, shape):
     assert np.array_equal(y, with_tokens_on_m(backend, x, dev, n_out))
 
 
-# equal runs of three segments of 64 to 256 tokens; 15 token ranges (a panel of eight and the rest) by 11 row blocks, the last 17 of 165 segments in
-# four parts each; rows that end inside a pair's 256
+# equal runs of three segments of 64 to 256 tokens; 12 token ranges (a panel of eight and the rest) by 14 row blocks, the last 20 of 168 segments in
+# two parts each; rows that end inside a pair's 256
 @pytest.mark.parametrize("fmt", ["mlx4", "q4_k", "q6_k", "q8_0", "f8_e4m3"])
-@pytest.mark.parametrize("shape", [(3000, 1536, 3108), (2600, 768, 3350)])
+@pytest.mark.parametrize("shape", [(3000, 1536, 3108), (3400, 768, 2850)])
 def test_several_segments_a_pair(backend, fmt, shape):
     """The bits of the form with tokens on M, and 1e-3 of a row (tests/test_gemm_gpu.py) on a sample of the tokens."""
     n_out, n_in, t = shape
@@ -113,10 +113,13 @@ def test_several_segments_a_pair(backend, fmt, shape):
     assert np.array_equal(y, with_tokens_on_m(backend, x, dev, n_out))
 
 
-# pairs per expert: none, one, a tile of 16 and one more, 128 and one more (two tiles of 80 and 49 rows), three tiles
-@pytest.mark.parametrize("fmt", ["mlx4", "q4_k"])
-@pytest.mark.parametrize("counts,h,inter", [([1, 16, 0, 17, 128, 129, 300, 64], 256, 512), ([70], 2048, 768)])
-def test_segments_of_every_length(backend, fmt, counts, h, inter):
+# pairs per expert: none, one, a tile of 16 and one more, 128 and one more (two tiles of 80 and 49 rows), three tiles; 45 experts in 51 tiles
+# (MLX-4: 44), so that a pair of CTAs takes two or three segments of the gate / up projection (204) and one or two of the down projection (102) in turn
+COUNTS = [([1, 16, 0, 17, 128, 129, 300, 64], 256, 512), ([70], 2048, 768), ([29 * i % 150 for i in range(45)], 512, 512)]
+
+
+def expert_rows(backend, fmt, counts, h, inter):
+    """(result, f64 result) of the pairs of each expert that has some."""
     n = len(counts)
     refs = [(synth.make(fmt, 2 * inter, h, 920 + 2 * e), synth.make(fmt, h, inter, 921 + 2 * e)) for e in range(n)]
     moe = backend.upload_moe([backend.upload(g, 2 * inter, h) for g, _ in refs], [backend.upload(d, h, inter) for _, d in refs], h, inter)
@@ -132,8 +135,26 @@ def test_segments_of_every_length(backend, fmt, counts, h, inter):
             continue
         gu = oracle_matrix(g, 2 * inter, h).matmul_f64(x[rows])
         a = gu[:, :inter] / (1.0 + np.exp(-gu[:, :inter])) * gu[:, inter:]
-        want = a @ oracle_matrix(d, h, inter).dequantize_rows().astype(np.float64).T
-        assert row_err(y[torch.from_numpy(rows).cuda()].cpu().numpy(), want) < 1e-3, e
+        yield y[torch.from_numpy(rows).cuda()].cpu().numpy(), a @ oracle_matrix(d, h, inter).dequantize_rows().astype(np.float64).T
+
+
+@pytest.mark.parametrize("fmt", ["mlx4", "q4_k"])
+@pytest.mark.parametrize("counts,h,inter", COUNTS)
+def test_segments_of_every_length(backend, fmt, counts, h, inter):
+    for got, want in expert_rows(backend, fmt, counts, h, inter):
+        assert row_err(got, want) < 1e-3
+
+
+@pytest.mark.parametrize("counts,h,inter", COUNTS)
+def test_exact_segments_of_mlx4(backend, counts, h, inter):
+    """Two-term activations on one-term weights run on gemm_wt.cu, tiles of up to 128 rows of an expert: the exact switch's 1e-4
+    (tests/test_gemm_gpu.py), which one-term activations miss (2.8e-4 and more on these layers)."""
+    backend.set_exact(True)
+    try:
+        for got, want in expert_rows(backend, "mlx4", counts, h, inter):
+            assert row_err(got, want) < 1e-4
+    finally:
+        backend.set_exact(False)
 
 
 def test_a_first_q6_k_product_inside_a_capture(backend):

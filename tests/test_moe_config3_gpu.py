@@ -2,8 +2,8 @@
 intermediate 768, MLX affine 4-bit weights (group 64), at token batches of 512 and 4096 with a skewed load
 (router logits N(0,1) plus a per-expert bias N(0,1)).
 
-At these sizes the grouped tensor-core GEMM runs with its large-batch launch shapes (256-row token tiles, the
-tile width chosen by the wave model), which the small cases of test_moe_gpu.py never reach. The oracle
+At these sizes the grouped tensor-core GEMM runs with several segments of up to 160 rows of an expert per CTA pair and tens of
+thousands of rows, which the small cases of test_moe_gpu.py never reach. The oracle
 (f64 products over the bit-exact dequantized weights, the reference's own CUDA test bar at
 src/cuda.rs:2178-2186) is evaluated on a sample of token rows, since a token's result depends only on its own
 row and routes. Bound: 1e-3 max relative error per output row.
