@@ -1,5 +1,5 @@
-// Dequant-GEMM with the weights in tensor memory and the tokens on the instruction's N side (tcgen05): dense batches of up to 128 tokens,
-// and the routed experts' segments of any length.
+// Dequant-GEMM with the weights in tensor memory and the tokens on the instruction's N side (tcgen05): dense batches of up to 128 tokens, and
+// MLX-4 experts under the exact switch (two-term activations; all other experts' segments run on gemm_wp.cu).
 //
 //   y[t][n_out] = x[t][K] * W^T
 //
