@@ -200,7 +200,7 @@ cudaError_t launch_moe_combine(const float* o, const int* slots, const float* w,
 cudaError_t launch_gather_rows(const float* x, const int* idx, size_t rows, size_t h, float* out, cudaStream_t st);
 cudaError_t launch_scatter_blocks(const float* gathered, size_t world, size_t t, size_t n_local, float* y, cudaStream_t st);
 
-// ---- decode_ops.cu: the non-matmul ops of one decode token -------------------------------------------
+// ---- decode_ops.cu, attend.cu: the non-matmul ops of one decode token -------------------------------------------
 // Every kernel reads the step words `sp` on the device: sp[0] position of the token, sp[1] position of row 0
 // of the RoPE table, sp[2] tokens generated so far (the argmax kernel advances [0] and [2]).
 struct DecNorm {
@@ -233,27 +233,25 @@ cudaError_t launch_norm(const float* x, float* out, const float* w, const DecNor
 cudaError_t launch_qk_rope(const float* qkv, float* qo, void* kc, void* vc, int kv_f16, const float* qn, const float* kn, const float* cs_table,
                            const uint32_t* sp, const DecRope& p, cudaStream_t st, bool pdl = false);
 bool attend_supports(uint32_t nh, uint32_t nkv, uint32_t hd);
-size_t attend_part_floats(uint32_t nh, uint32_t hd);  // scratch for the per-split partials
-// Attention that prepares its own inputs: with qkv set, the kernel applies RoPE to the token's query heads as it stages
-// them (`q` is not read), and the CTA whose keys end at the token's position rotates the token's key, appends key and value
-// to the caches and puts them into its tile; the arithmetic of launch_qk_rope, which is then not launched. Per-head norms
+// Attention that prepares its own inputs: with qkv set, the kernel applies RoPE to the tokens' query heads as it stages
+// them (`q` is not read), and the CTA that has the tile of a token's position rotates the token's key, appends key and value
+// to the caches and keeps them for itself; the arithmetic of launch_qk_rope, which is then not launched. Per-head norms
 // are not taken (r.* as for launch_qk_rope; qkv == nullptr: plain attention over q and the caches).
 struct FusedRope {
     const float* qkv;
     const float* cs_table;
     DecRope r;
 };
-// Several tokens of a step in one launch (only without FusedRope: every token's key and value must be in the caches
-// already): token i's queries / outputs act_stride floats behind token 0's, its partials
-// part_stride floats, its counters nkv words, its step words 4 words.
+// Several tokens of a step in one launch, at positions sp[0], sp[0] + 1, ..: token i's queries / outputs (and qkv) act_stride floats
+// behind token 0's.
+constexpr int ATT_STEP_TOKENS = 4;  // at most
 struct AttnTokens {
     int n;  // 0 or 1: one token
-    size_t act_stride, part_stride;
+    size_t act_stride;
 };
-// counters: nkv zeroed words (left zero by every launch); status: set to 1 if a bounded wait gave up.
-cudaError_t launch_attend(const float* q, void* kc, void* vc, int kv_f16, float* out, float* part, uint32_t* counters,
-                          const uint32_t* sp, const DecAttn& p, uint32_t* status, cudaStream_t st, bool pdl = false,
-                          const FusedRope* fr = nullptr, const AttnTokens* tokens = nullptr);
+// status: set to 1 if a bounded wait gave up.
+cudaError_t launch_attend(const float* q, void* kc, void* vc, int kv_f16, float* out, const uint32_t* sp, const DecAttn& p, uint32_t* status,
+                          cudaStream_t st, bool pdl = false, const FusedRope* fr = nullptr, const AttnTokens* tokens = nullptr);
 // Host-order rows [n][nkv][hd] f32 <-> cache rows pos0 .. pos0 + n - 1.
 cudaError_t launch_kv_rows(float* rows, void* cache, int kv_f16, bool to_cache, uint32_t nkv, uint32_t hd, uint32_t max_len, uint32_t pos0,
                            uint32_t n, cudaStream_t st);

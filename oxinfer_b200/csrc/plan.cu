@@ -126,7 +126,7 @@ DecodePlanImpl::~DecodePlanImpl() {
     for (void* m : peer_maps_) cudaIpcCloseMemHandle(m);
     for (auto& kv : gemm_plans_)
         for (GemmPlan* gp : kv.second) gemm_tc_plan_destroy(gp);
-    void* frees[] = {kv16_, x16_, unscale_, tmp_a_, tmp_b_, gemm_status_, xflags_, bufs_, records_, consts_, part_, words_, rope_table_, argmax_val_, argmax_idx_, token_, out_tokens_, stage_};
+    void* frees[] = {kv16_, x16_, unscale_, tmp_a_, tmp_b_, gemm_status_, xflags_, bufs_, records_, consts_, words_, rope_table_, argmax_val_, argmax_idx_, token_, out_tokens_, stage_};
     for (void* p : frees)
         if (p) cudaFree(p);
 }
@@ -207,7 +207,6 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
 
     // ---- KV caches --------------------------------------------------------------------------------
     const size_t esz = p->kv_f16_ ? 2 : 4;
-    uint32_t max_nh = 0, max_hd = 0, max_nkv = 0;
     size_t max_row = 0;
     for (uint32_t i = 0; i < g->n_kv; i++) {
         Kv k;
@@ -219,7 +218,6 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
         PLAN_CUDA(cudaMalloc(&p->kv_.back().v, bytes), "cudaMalloc(V cache)");
         PLAN_CUDA(cudaMemset(p->kv_.back().k, 0, bytes), "cudaMemset(K cache)");
         PLAN_CUDA(cudaMemset(p->kv_.back().v, 0, bytes), "cudaMemset(V cache)");
-        max_nkv = std::max(max_nkv, k.nkv);
         max_row = std::max(max_row, (size_t)k.nkv * k.hd);
     }
 
@@ -395,8 +393,6 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
                 op.y = view(o.y, (size_t)o.nh * o.hd);
                 op.kv = o.kv;
                 op.attn = DecAttn{o.nh, o.nkv, o.hd, g->max_len, o.window, o.scale};
-                max_nh = std::max(max_nh, o.nh);
-                max_hd = std::max(max_hd, o.hd);
                 touch(o.y.buf);
                 break;
             }
@@ -605,9 +601,7 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
     }
 
     // ---- scratch ------------------------------------------------------------------------------------
-    p->part_stride_ = max_nh ? attend_part_floats(max_nh, max_hd) : 0;
-    if (max_nh) PLAN_CUDA(cudaMalloc((void**)&p->part_, (prefill ? 1 : T) * p->part_stride_ * sizeof(float)), "cudaMalloc(attention partials)");
-    size_t n_words = 8 + T * std::max<uint32_t>(max_nkv, 1) + 4 * T;  // (a prefill plan's T counters are unused: a few KB)
+    const size_t n_words = 8 + 4 * T;
     PLAN_CUDA(cudaMalloc((void**)&p->words_, n_words * 4), "cudaMalloc(step words)");
     PLAN_CUDA(cudaMemset(p->words_, 0, n_words * 4), "cudaMemset(step words)");
     if (p->has_exchange_) {
@@ -617,9 +611,7 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
     p->sp_ = p->words_;
     p->status_ = p->words_ + 4;
     p->argmax_counter_ = p->words_ + 5;
-    p->att_counters_ = p->words_ + 8;
-    p->n_counters_ = T * std::max<uint32_t>(max_nkv, 1);
-    p->sp_multi_ = p->words_ + 8 + p->n_counters_;
+    p->sp_multi_ = p->words_ + 8;
     size_t table = (size_t)std::max<uint32_t>(p->cs_stride_, 1) * g->max_len;
     PLAN_CUDA(cudaMalloc((void**)&p->rope_table_, table * sizeof(float)), "cudaMalloc(rope table)");
     PLAN_CUDA(cudaMemset(p->rope_table_, 0, table * sizeof(float)), "cudaMemset(rope table)");
@@ -731,9 +723,9 @@ int DecodePlanImpl::run_ops(cudaStream_t st, std::string& err, bool chained, boo
                 if (o.fr.qkv) {
                     FusedRope fr = o.fr;
                     fr.cs_table = rope_table_;
-                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, part_, att_counters_, sp_, o.attn, status_, st, pdl, &fr);
+                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, sp_, o.attn, status_, st, pdl, &fr);
                 } else {
-                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, part_, att_counters_, sp_, o.attn, status_, st, pdl);
+                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, sp_, o.attn, status_, st, pdl);
                 }
                 break;
             case B2_OP_GLU: e = launch_glu(o.x, o.z, o.y, o.n, o.gelu, st, pdl); break;
@@ -752,8 +744,6 @@ int DecodePlanImpl::run_ops(cudaStream_t st, std::string& err, bool chained, boo
 
 // The ops for nt tokens at once, op by op: a product reads its weights once for all tokens (each token's sums are its one-token sums),
 // every other op runs once per token on that token's blocks (activations, records, step words) or has the token as a grid dimension.
-// Attention and RoPE are ordinary launches, not dependent ones: token i's attention reads the keys the launches just ahead of it
-// appended, and its first key tile is fetched before the dependency wait.
 int DecodePlanImpl::run_ops_multi(cudaStream_t st, int nt, std::string& err, bool chained) {
     auto A = [&](const float* p, int tk) -> float* { return p ? const_cast<float*>(p) + (size_t)tk * block_floats_ : nullptr; };
     bool first = true;
@@ -800,19 +790,14 @@ int DecodePlanImpl::run_ops_multi(cudaStream_t st, int nt, std::string& err, boo
                 count++;
                 break;
             case B2_OP_ATTEND: {
-                // Where the one-token plan rotates and appends inside the attention kernel, the tokens' keys and values go into
-                // the caches first (the same arithmetic in a kernel of its own); then one launch attends for all tokens.
-                if (o.fr.qkv) {
-                    e = launch_qk_rope_rows(o.fr.qkv, o.x, block_floats_, (uint32_t)nt, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, nullptr, nullptr, rope_table_,
-                                            sp_multi_, o.fr.r, st);
-                    count++;
-                }
-                const AttnTokens at{nt, block_floats_, part_stride_};
-                if (e == cudaSuccess)
-                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, part_, att_counters_, sp_multi_, o.attn, status_, st, false, nullptr,
-                                      &at);
-                first = false;
-                count++;
+                // One launch attends for all tokens, and rotates and appends where the one-token plan's does. Otherwise it is an
+                // ordinary launch: all tokens' rows of the caches come from the launch just ahead of it.
+                const AttnTokens at{nt, block_floats_};
+                FusedRope fr = o.fr;
+                fr.cs_table = rope_table_;
+                const bool dependent = pdl();
+                e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, sp_multi_, o.attn, status_, st, dependent && o.fr.qkv, o.fr.qkv ? &fr : nullptr,
+                                  &at);
                 break;
             }
             case B2_OP_GLU:
@@ -860,7 +845,6 @@ int DecodePlanImpl::check_status(std::string& err) {
     PLAN_CUDA(cudaMemcpy(&s, status_, 4, cudaMemcpyDeviceToHost), "cudaMemcpy(status)");
     if (s) {
         cudaMemset(status_, 0, 4);
-        cudaMemset(att_counters_, 0, 4 * n_counters_);  // a CTA that gave up never counted itself
         err = s == 4 ? "[b200qmm: plan: a peer did not arrive at an exchange within the time limit]"
                      : "[b200qmm: plan: an attention kernel's wait on its copy ran into the time limit]";
         return B2_ERR_TIMEOUT;
@@ -1059,8 +1043,7 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
             case B2_OP_ATTEND:
                 if (loop_attend_) {
                     for (size_t tk = 0; tk < t && e == cudaSuccess; tk++, count++)
-                        e = launch_attend(o.x + tk * ld, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y + tk * ld, part_, att_counters_, sp_multi_ + 4 * tk, o.attn,
-                                          status_, st, false, nullptr);
+                        e = launch_attend(o.x + tk * ld, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y + tk * ld, sp_multi_ + 4 * tk, o.attn, status_, st);
                 } else {
                     e = launch_attend_rows(o.x, o.y, ld, rows, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, kv16_, (uint32_t)(pos + t), sp_, o.attn, st);
                     count += kv_f16_ ? 1 : 3;

@@ -92,8 +92,6 @@ class DecodePlanImpl {
     std::vector<uint32_t> cs_off_;        // start of each RoPE table's values inside a row of the device table
     cudaGraphExec_t multi_exec_[5] = {};  // [nt], nt = 2 .. tokens
     uint64_t multi_launches_[5] = {};     // kernels of a step of nt tokens
-    size_t part_stride_ = 0;              // floats of attention partials per token
-    size_t n_counters_ = 0;               // attention counter words (KV heads x tokens)
     // prefill plans
     bool prefill_ = false;
     bool loop_attend_ = false;       // B2_PREFILL_ATTEND=loop: the one-token attention kernel token by token (for comparisons)
@@ -130,12 +128,10 @@ class DecodePlanImpl {
     std::vector<Kv> kv_;
     uint32_t max_len_ = 0;
     int kv_f16_ = 0;
-    float* part_ = nullptr;       // attention partials
     uint32_t* words_ = nullptr;   // sp[4] | status | argmax counter | attention counters[...]
     uint32_t* sp_ = nullptr;
     uint32_t* status_ = nullptr;
     uint32_t* argmax_counter_ = nullptr;
-    uint32_t* att_counters_ = nullptr;
     float* rope_table_ = nullptr;  // [max_len][cs_stride]
     uint32_t cs_stride_ = 0;
     float* argmax_val_ = nullptr;
