@@ -266,12 +266,12 @@ cudaError_t launch_argmax(const float* logits, uint32_t n, float* pval, int* pid
 cudaError_t launch_qk_rope_rows(const float* qkv, float* qo, size_t stride, uint32_t rows, void* kc, void* vc, int kv_f16, const float* qn,
                                 const float* kn, const float* cs_table, const uint32_t* sp, const DecRope& p, cudaStream_t st);
 bool attend_rows_supports(uint32_t nh, uint32_t nkv, uint32_t hd);
-// Causal attention of `rows` query tokens over the cache (which already holds their keys and values): tensor-core products
-// over f16 roundings of q, k, v and the probabilities, f32 sums. `len`: positions the cache holds now (sp[0] + rows, as the
-// host knows it). f32 caches: `scratch` (attend_rows_scratch_bytes) receives an f16 copy of those rows first.
+// attend_rows.cu: causal attention of `tokens` query tokens over the cache (which already holds their keys and values): tensor-core products
+// over f16 roundings of q, k, v and the probabilities, f32 sums. `len`: positions the cache holds now, the tokens' own the last of them.
+// f32 caches: `scratch` (attend_rows_scratch_bytes) receives an f16 copy of those rows first.
 size_t attend_rows_scratch_bytes(uint32_t nkv, uint32_t max_len, uint32_t hd, int kv_f16);
-cudaError_t launch_attend_rows(const float* q, float* out, size_t stride, uint32_t rows, const void* kc, const void* vc, int kv_f16, void* scratch,
-                               uint32_t len, const uint32_t* sp, const DecAttn& p, cudaStream_t st);
+cudaError_t launch_attend_rows(const float* q, float* out, size_t stride, uint32_t tokens, const void* kc, const void* vc, int kv_f16, void* scratch,
+                               uint32_t len, const DecAttn& p, GemmStatus* status, int sm_count, cudaStream_t st);
 // RMS norm of `rows` rows (p.n values each, p.pre / p.eps / p.add as for launch_norm; the strides here replace p's). With
 // x16 / unscale the rows also leave as the f16 operands launch_to_f16 would make of the result (rows of p.n halves).
 bool norm_rows_supports(uint32_t n, const float* x, const float* out, const float* w, size_t x_stride, size_t out_stride);

@@ -1045,8 +1045,8 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
                     for (size_t tk = 0; tk < t && e == cudaSuccess; tk++, count++)
                         e = launch_attend(o.x + tk * ld, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y + tk * ld, sp_multi_ + 4 * tk, o.attn, status_, st);
                 } else {
-                    e = launch_attend_rows(o.x, o.y, ld, rows, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, kv16_, (uint32_t)(pos + t), sp_, o.attn, st);
-                    count += kv_f16_ ? 1 : 3;
+                    e = launch_attend_rows(o.x, o.y, ld, rows, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, kv16_, (uint32_t)(pos + t), o.attn, gemm_status_, sm_count_, st);
+                    count += kv_f16_ ? 1 : 2;
                 }
                 if (overlaps_f(o.y, (size_t)o.attn.nh * o.attn.hd, x16_src, x16_k)) x16_src = nullptr;
                 break;
