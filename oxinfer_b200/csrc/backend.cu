@@ -88,6 +88,7 @@ class Backend {
     uint8_t* host_stage = nullptr;
     bool stage_busy = false;  // a call that failed half-way may have left a copy from it in flight
     GemmStatus* gemm_status = nullptr;  // device
+    uint32_t* wait_status = nullptr;    // page-locked: the products of a few tokens write it when a bounded wait gives up
     // cached tensor maps of the tensor-core GEMM (see matmul_dev)
     std::vector<GemmPlan*> plans;
     // cumulative times, like Backend::stats (src/cuda.rs:403-409)
@@ -486,6 +487,7 @@ class Backend {
             GemvIn in;
             in.x = x_dev_;
             in.fast = fast_planes && !exact;
+            in.status = wait_status;
             e = launch_gemv_mma(w->dev, u ? &u->dev : nullptr, in, 1, y_dev_, 0, mode, gate, 0, sm_count, stream, true);
         } else {
             e = launch_gemv_f8_float(w->dev, u ? &u->dev : nullptr, x_dev_, y_dev_, mode, gate, sm_count, stream, true);
@@ -510,15 +512,24 @@ class Backend {
     // Q4_K 14336 x 4096 42 and 30 us, 28672 x 4096 136 and 47; Q8_0 48 and 32, 83 and 51. (4096 x 14336 has fewer tiles than that: one launch, 41 and 42 us.)
     // The second launch waits for the first, so a matrix whose tiles fill no more than half of the SMs gains nothing by it: Q8_0
     // 1024 x 2048 10.1 us in two launches, 7.8 in one; FP8 512 x 4096 11.5 and 10.1. Seven or eight tokens of Q6_K do (512 x 4096 12.7
-    // and 13.8), and the 4-bit formats keep a launch per four rows there, as their callers count them (1024 x 4096 12.3 and 12.2).
-    int small_products(const WeightDev& w, const WeightDev* up, const uint8_t* rec, size_t t, float* y, int mode) {
+    // and 13.8). Matrices whose CTAs split only the part of K that they multiply (gemv_tc.cu) need no records (null), x instead, and take eight
+    // tokens a launch (4096 x 4096 7.9 us, in two launches 12.4); from records four, as the callers with host buffers count them.
+    int small_products(const WeightDev& w, const WeightDev* up, const uint8_t* rec, const float* x, size_t t, float* y, int mode) {
         const size_t stride = record_stride(w.n_in, gemv_mma_halves(w)), tiles = (w.n_out + 15) / 16;
-        const bool narrow = 2 * tiles <= (size_t)sm_count && (w.fmt == B2_FMT_Q4_K || w.fmt == B2_FMT_MLX4 || (w.fmt == B2_FMT_Q6_K && t > 6));
-        const size_t per = narrow || (tiles > 2 * (size_t)sm_count && w.n_in > GEMV_WHOLE_8) ? 4 : 8;
+        const bool narrow = 2 * tiles <= (size_t)sm_count && w.fmt == B2_FMT_Q6_K && t > 6;
+        const bool tc = gemv_tc_supports(w);
+        const size_t per = narrow || (tc && rec) || (!tc && tiles > 2 * (size_t)sm_count && w.n_in > GEMV_WHOLE_8) ? 4 : 8;
         for (size_t i = 0; i < t; i += per) {
             GemvIn in;
-            in.rec = rec + i * stride;
-            in.rec_stride = stride;
+            if (!rec) {
+                in.x = x + i * w.n_in;
+                in.x_stride = w.n_in;
+                in.fast = fast_planes && !exact;
+            } else {
+                in.rec = rec + i * stride;
+                in.rec_stride = stride;
+            }
+            in.status = wait_status;
             cudaError_t e = launch_gemv_mma(w, up, in, (int)std::min(per, t - i), y + i * w.n_out, w.n_out, mode, nullptr, 0, sm_count, stream, true);
             launches++;
             if (e != cudaSuccess) return cuda_fail(e, "gemv (several rows)");
@@ -540,7 +551,8 @@ class Backend {
     // t tokens on the device through the tensor-core GEMM (or token by token through the GEMV).
     // peer_y (matmul_sharded_peer): the result goes, tile by tile from the GEMM's epilogue, to this rank's columns of its own y and
     // of the peers' copies; only the tensor-core GEMM takes it, every other route declines.
-    int matmul_dev(uint64_t h, const void* x, int x_dtype, size_t t, void* y, int y_dtype, const GemmPeerY* peer_y = nullptr) {
+    // records: up to eight rows are split by a launch of their own (host calls: the launches that they report).
+    int matmul_dev(uint64_t h, const void* x, int x_dtype, size_t t, void* y, int y_dtype, const GemmPeerY* peer_y = nullptr, bool records = false) {
         Weight* w = find(h);
         if (!w) return fail(B2_ERR_ARG, "[b200qmm: matmul: unknown weight]");
         if (t == 0) return B2_OK;
@@ -574,11 +586,16 @@ class Backend {
                 for (size_t i = 0; i < t && !rc; i++) rc = matvec_dev(h, 0, xf + i * K, (float*)y + i * w->dev.n_out, B2_MODE_STORE, nullptr);
                 return rc;
             }
+            if (gemv_tc_supports(w->dev) && !records) {
+                const float* xf = (const float*)x;
+                if (int rc = apart(xf, t * K, (const float*)y, t * w->dev.n_out)) return rc;
+                return small_products(w->dev, nullptr, nullptr, xf, t, (float*)y, B2_MODE_STORE);
+            }
             const bool halves = gemv_mma_halves(w->dev);
             cudaError_t e = xrec.reserve(t * record_stride(K, halves));
             if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(records)");
             int rc = make_records((const float*)x, t, K, halves, (uint8_t*)xrec.p);
-            return rc ? rc : small_products(w->dev, nullptr, (const uint8_t*)xrec.p, t, (float*)y, B2_MODE_STORE);
+            return rc ? rc : small_products(w->dev, nullptr, (const uint8_t*)xrec.p, nullptr, t, (float*)y, B2_MODE_STORE);
         }
         if (fp8_act && !exact && gemm_f8_supports(w->dev, t)) {
             // FP8 on both sides: the activations are quantized per token and per 128 k to e4m3, and the tensor cores multiply
@@ -646,8 +663,15 @@ class Backend {
         return B2_OK;
     }
 
-    // Reads the status word the GEMM writes when a bounded wait gives up (after a synchronize).
+    // The word of the products of a few tokens (after a synchronize).
+    int check_wait_status() {
+        if (!*(volatile uint32_t*)wait_status) return B2_OK;
+        *(volatile uint32_t*)wait_status = 0;
+        return fail(B2_ERR_TIMEOUT, "[b200qmm: matvec: a device wait gave up]");
+    }
+    // Reads the status words that the kernels write when a bounded wait gives up (after a synchronize).
     int check_gemm_status() {
+        if (int rc = check_wait_status()) return rc;
         if (!gemm_status) return B2_OK;
         GemmStatus s{};
         cudaError_t e = cudaMemcpy(&s, gemm_status, sizeof s, cudaMemcpyDeviceToHost);
@@ -694,7 +718,7 @@ class Backend {
             e = cudaMemcpyAsync(jobs[j].y, (uint8_t*)y_dev.p + y_off[j], t * jobs[j].n_out * 4, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e == cudaSuccess) stage_busy = false;
-        for (size_t j = 0; j < n_jobs && staged && e == cudaSuccess; j++) std::memcpy(jobs[j].y, host_stage + HOST_STAGE + y_off[j], t * jobs[j].n_out * 4);
+        for (size_t j = 0; j < n_jobs && staged && e == cudaSuccess && !*(volatile uint32_t*)wait_status; j++) std::memcpy(jobs[j].y, host_stage + HOST_STAGE + y_off[j], t * jobs[j].n_out * 4);
         return e;
     }
 
@@ -727,7 +751,7 @@ class Backend {
         ns_in += since(t0);
         auto t1 = clk::now();
         for (size_t j = 0; j < n_jobs; j++) {
-            int rc = matmul_dev(jobs[j].w, x_dev.p, B2_F32, t, (uint8_t*)y_dev.p + y_off[j], B2_F32);
+            int rc = matmul_dev(jobs[j].w, x_dev.p, B2_F32, t, (uint8_t*)y_dev.p + y_off[j], B2_F32, nullptr, true);
             if (rc) {
                 cudaStreamSynchronize(stream);
                 return rc;
@@ -793,9 +817,11 @@ class Backend {
             if (t > 1 && gemv_mma_supports(w->dev)) {  // one launch reads the weights once for all rows
                 const bool halves = gemv_mma_halves(w->dev);
                 uint8_t* rec = (uint8_t*)xrec.p + (halves ? digits : 0);
-                if (!made[halves]) rc = make_records((const float*)x_dev.p, t, n_in, halves, rec);
-                made[halves] = true;
-                if (!rc) rc = small_products(w->dev, u ? &u->dev : nullptr, rec, t, yj, mode);
+                if (!made[halves] && !gemv_tc_supports(w->dev)) {
+                    rc = make_records((const float*)x_dev.p, t, n_in, halves, rec);
+                    made[halves] = true;
+                }
+                if (!rc) rc = small_products(w->dev, u ? &u->dev : nullptr, gemv_tc_supports(w->dev) ? nullptr : rec, (const float*)x_dev.p, t, yj, mode);
             } else {
                 for (size_t i = 0; i < t && !rc; i++)
                     rc = matvec_dev(jobs[j].w, jobs[j].up, (const float*)x_dev.p + i * n_in, yj + i * jobs[j].n_out, mode, nullptr);
@@ -805,11 +831,16 @@ class Backend {
                 return rc;
             }
         }
-        // Every launch was accepted (a refused one returned above, before any y is touched): the results follow the kernels on
-        // the stream and the call synchronizes once. (The matrix-vector kernels have no status word to consult in between; a
-        // product of a few microseconds would otherwise pay two host round trips.) The kernels' and the copies' time are
-        // booked together as kernel time.
+        // Every launch was accepted (a refused one returned above, before any y is touched): small results follow the kernels on
+        // the stream to page-locked memory and the call synchronizes once (a product of a few microseconds would otherwise pay two
+        // host round trips); large ones are copied when the kernels' waits are known to have ended. The kernels' and the copies'
+        // time are booked together as kernel time.
+        if (y_total > HOST_STAGE || !stage_host()) {
+            if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(e, "matvec_rows kernels");
+            if (int rc = check_wait_status()) return rc;
+        }
         e = copy_out(jobs, n_jobs, t, y_off, y_total);
+        if (int rc = check_wait_status()) return rc;
         if (e != cudaSuccess) return cuda_fail(e, "matvec_rows kernels / copy-out");
         ns_gpu += since(t1);
         calls++;
@@ -1504,6 +1535,8 @@ class Backend {
         xrec.release();
         if (gemm_status) cudaFree(gemm_status);
         gemm_status = nullptr;
+        if (wait_status) cudaFreeHost(wait_status);
+        wait_status = nullptr;
         for (GemmPlan* p : plans) gemm_tc_plan_destroy(p);
         plans.clear();
     }
@@ -1558,7 +1591,15 @@ B2_EXPORT int b2_open(int ordinal, b2_ctx** out) {
         g_open_error = "[b200qmm: cudaSetDevice failed]";
         return B2_ERR_CUDA;
     }
+    uint32_t* word = nullptr;
+    if (cudaHostAlloc((void**)&word, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        g_open_error = "[b200qmm: cudaHostAlloc failed]";
+        cudaGetLastError();
+        return B2_ERR_NOMEM;
+    }
+    *word = 0;
     b2_ctx* c = new b2_ctx();
+    c->be.wait_status = word;
     c->be.device = ordinal;
     c->be.sm_count = prop.multiProcessorCount;
     *out = c;

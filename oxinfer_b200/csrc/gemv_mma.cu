@@ -72,6 +72,7 @@ bool gemv_mma_halves(const WeightDev& w) { return w.fmt == B2_FMT_F8E4M3; }
 cudaError_t launch_gemv_mma(const WeightDev& w, const WeightDev* up, const GemvIn& in, int T, float* y, size_t y_stride, int mode, const float* gate,
                             size_t gate_stride, int sm_count, cudaStream_t st, bool pdl) {
     if (!gemv_mma_supports(w) || T < 1 || T > 8) return cudaErrorInvalidValue;
+    if (in.status && gemv_tc_supports(w)) return launch_gemv_tc(w, up, in, T, y, y_stride, mode, gate, gate_stride, sm_count, st, pdl);
     const bool pair = mode == B2_MODE_SILU_PAIR || mode == B2_MODE_GELU_PAIR;
     Args a{};
     a.w = w;

@@ -81,6 +81,7 @@ struct GemvIn {
     const uint8_t* rec = nullptr;  // token i at rec + i * rec_stride
     size_t rec_stride = 0;
     int fast = 0;  // 18 bits of every value (split.cuh)
+    uint32_t* status = nullptr;  // set to 2 if a bounded wait gives up; products that have one may take gemv_tc.cu
 };
 bool gemv_mma_supports(const WeightDev& w);
 constexpr size_t GEMV_WHOLE_8 = 2048;  // rows of up to this many values are held whole by a launch of eight tokens, whatever the format
@@ -91,6 +92,10 @@ bool gemv_mma_halves(const WeightDev& w);  // the form of split this format's pr
 // for bit, from records or not.
 cudaError_t launch_gemv_mma(const WeightDev& w, const WeightDev* up, const GemvIn& in, int T, float* y, size_t y_stride, int mode, const float* gate,
                             size_t gate_stride, int sm_count, cudaStream_t st, bool pdl);
+// gemv_tc.cu: the same for 4-bit matrices on tcgen05 (launch_gemv_mma calls it where `status` is set).
+bool gemv_tc_supports(const WeightDev& w);
+cudaError_t launch_gemv_tc(const WeightDev& w, const WeightDev* up, const GemvIn& in, int T, float* y, size_t y_stride, int mode, const float* gate,
+                           size_t gate_stride, int sm_count, cudaStream_t st, bool pdl);
 // Products over a stack of equally shaped 4-bit matrices (the routed experts of a batch; w describes matrix 0, the others w_stride bytes
 // apart): group g multiplies matrix expert[g] by rows row0[g] .. + count[g] - 1 (at most `most`, 1 .. 8) of the pairs' list. Row i reads the
 // vector of x's row src[i] (gather) or i and writes row i of y. The table travels as a kernel argument: no copy, no synchronization.

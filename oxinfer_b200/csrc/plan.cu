@@ -539,8 +539,11 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
             stale = stale || writes(o, s.sx, s.n);
         }
         s.self = ok;
+        s.parts = ok;
+        for (size_t b : users) s.parts = s.parts && gemv_tc_supports(p->ops_[b].w);
         for (size_t b : users) {
             Op& o = p->ops_[b];
+            o.parts = s.parts;
             o.sx = s.sx;
             o.nw = s.nw;
             o.npre = s.npre;
@@ -696,6 +699,7 @@ GemvIn DecodePlanImpl::product_in(const Op& o, bool self) const {
     in.norm = o.normed;
     in.eps = o.neps;
     in.fast = fast_;
+    in.status = status_;
     return in;
 }
 
@@ -754,10 +758,10 @@ int DecodePlanImpl::run_ops_multi(cudaStream_t st, int nt, std::string& err, boo
         count++;
         return v;
     };
-    // A vector's record is made in a launch of its own where the products would have more than `self_blocks` blocks of 256 values per
-    // warp to split, every CTA all of them.
+    // A vector's record is made in a launch of its own where the products' CTAs would split all of it, more than `self_blocks` blocks of 256
+    // values per warp.
     constexpr size_t self_blocks = 2;
-    auto self = [&](const Op& o, size_t n) { return o.self && split_blocks_of(n) * (size_t)nt <= 16 * self_blocks; };
+    auto self = [&](const Op& o, size_t n) { return o.parts || (o.self && split_blocks_of(n) * (size_t)nt <= 16 * self_blocks); };
     for (size_t i = 0; i < ops_.size(); i++) {
         const Op& o = ops_[i];
         cudaError_t e = cudaSuccess;
@@ -846,6 +850,7 @@ int DecodePlanImpl::check_status(std::string& err) {
     if (s) {
         cudaMemset(status_, 0, 4);
         err = s == 4 ? "[b200qmm: plan: a peer did not arrive at an exchange within the time limit]"
+              : s == 2 ? "[b200qmm: plan: a product's wait ran into the time limit]"
                      : "[b200qmm: plan: an attention kernel's wait on its copy ran into the time limit]";
         return B2_ERR_TIMEOUT;
     }

@@ -70,6 +70,7 @@ class DecodePlanImpl {
         int region = -1;
         size_t rec_at = 0;
         bool halves = false, self = false;
+        bool parts = false;  // self, and a CTA splits only the part of K it multiplies (gemv_tc.cu)
         bool x16_only = false;  // prefill: the op's f32 result is read by nobody but products that take its f16 rows
         FusedRope fr{};   // ATTEND: RoPE and the cache append done by the attention kernel (the QK_ROPE op ahead of it is dropped)
     };
