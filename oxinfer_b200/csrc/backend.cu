@@ -88,7 +88,7 @@ class Backend {
     uint8_t* host_stage = nullptr;
     bool stage_busy = false;  // a call that failed half-way may have left a copy from it in flight
     GemmStatus* gemm_status = nullptr;  // device
-    uint32_t* wait_status = nullptr;    // page-locked: the products of a few tokens write it when a bounded wait gives up
+    uint32_t* wait_status = nullptr;    // page-locked: the products of a few tokens write it when a bounded wait gives up; 64 bytes on, a copy of *gemm_status
     // cached tensor maps of the tensor-core GEMM (see matmul_dev)
     std::vector<GemmPlan*> plans;
     // cumulative times, like Backend::stats (src/cuda.rs:403-409)
@@ -676,6 +676,9 @@ class Backend {
         GemmStatus s{};
         cudaError_t e = cudaMemcpy(&s, gemm_status, sizeof s, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(e, "status read");
+        return gemm_status_of(s);
+    }
+    int gemm_status_of(const GemmStatus& s) {
 #ifdef B2_DEBUG
         if (getenv("B2_GEMM_DEBUG") && (atoi(getenv("B2_GEMM_DEBUG")) & 32768)) fprintf(stderr, "[gemm debug] mma loop cycles %u over %u stages; stamps: loop start %u, loop end %u, acc seen %u, epilogue done %u, all done %u; mma thread waited %u on activations, %u on weights\n", s.where, s.iter, s.t[0], s.t[1], s.t[2], s.t[3], s.t[4], s.t[5], s.t[6]);
 #endif
@@ -689,37 +692,51 @@ class Backend {
     using clk = std::chrono::steady_clock;
     static double since(clk::time_point t0) { return std::chrono::duration<double, std::nano>(clk::now() - t0).count(); }
 
-    // Host vectors to x_dev, and the jobs' results back with the stream synchronized. Small ones go through page-locked memory, the
-    // results in one copy: a copy to pageable memory is a round trip of its own (the q / k / v products of
-    // one token: 67 us with four of them, 44 this way). Above a few hundred KB the bytes count, and a second
-    // copy on the host loses.
+    // Host vectors to x_dev, and the jobs' results back with the stream synchronized. Small ones go through page-locked memory, by
+    // kernels that read and write it there: a copy to pageable memory is a round trip of its own, and each copy of the copy engine is two
+    // hand-overs between it and the kernels (the q / k / v products of one token: 67 us with pageable copies, 44 with two by the
+    // engine, 32 this way and with one launch for the three). Products of gemv_tc.cu store rows of 128 bytes, there directly. Above a few
+    // hundred KB the bytes count, and a second copy on the host loses.
     bool stage_host() {
-        if (!host_stage && cudaHostAlloc((void**)&host_stage, 2 * HOST_STAGE, cudaHostAllocDefault) != cudaSuccess) {
+        if (!host_stage && cudaHostAlloc((void**)&host_stage, 2 * HOST_STAGE, cudaHostAllocMapped) != cudaSuccess) {
             cudaGetLastError();
             host_stage = nullptr;
         }
         return host_stage != nullptr;
     }
+    bool staged(size_t y_total) { return y_total <= HOST_STAGE && stage_host(); }
     cudaError_t copy_in(const float* x, size_t bytes) {
-        const void* src = x;
-        if (bytes <= HOST_STAGE && stage_host()) {
-            if (stage_busy) cudaDeviceSynchronize();
-            src = std::memcpy(host_stage, x, bytes);
-            stage_busy = true;
-        }
-        return cudaMemcpyAsync(x_dev.p, src, bytes, cudaMemcpyHostToDevice, stream);
+        if (bytes > HOST_STAGE || bytes % 16 != 0 || !stage_host()) return cudaMemcpyAsync(x_dev.p, x, bytes, cudaMemcpyHostToDevice, stream);
+        if (stage_busy) cudaDeviceSynchronize();
+        std::memcpy(host_stage, x, bytes);
+        stage_busy = true;
+        return launch_copy16(x_dev.p, host_stage, bytes, nullptr, nullptr, 0, stream, false);
     }
     template <typename Job>
-    cudaError_t copy_out(const Job* jobs, size_t n_jobs, size_t t, const std::vector<size_t>& y_off, size_t y_total) {
-        const bool staged = y_total <= HOST_STAGE && stage_host();
+    cudaError_t copy_out(const Job* jobs, size_t n_jobs, size_t t, const std::vector<size_t>& y_off) {
         cudaError_t e = cudaSuccess;
-        if (staged) e = cudaMemcpyAsync(host_stage + HOST_STAGE, y_dev.p, y_total, cudaMemcpyDeviceToHost, stream);
-        for (size_t j = 0; j < n_jobs && !staged && e == cudaSuccess; j++)
+        for (size_t j = 0; j < n_jobs && e == cudaSuccess; j++)
             e = cudaMemcpyAsync(jobs[j].y, (uint8_t*)y_dev.p + y_off[j], t * jobs[j].n_out * 4, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e == cudaSuccess) stage_busy = false;
-        for (size_t j = 0; j < n_jobs && staged && e == cudaSuccess && !*(volatile uint32_t*)wait_status; j++) std::memcpy(jobs[j].y, host_stage + HOST_STAGE + y_off[j], t * jobs[j].n_out * 4);
         return e;
+    }
+    // The staged results and the status words in one launch and one synchronize; y is written when every wait is known to have ended.
+    // in_place: the products have stored to the stage.
+    template <typename Job>
+    int staged_out(const Job* jobs, size_t n_jobs, size_t t, const std::vector<size_t>& y_off, size_t y_total, bool in_place, const char* what) {
+        uint8_t* const ys = host_stage + HOST_STAGE;
+        GemmStatus* const gs = (GemmStatus*)(wait_status + 16);
+        cudaError_t e = cudaSuccess;
+        if (!in_place) e = launch_copy16(ys, y_dev.p, y_total, gs, gemm_status, gemm_status ? sizeof(GemmStatus) : 0, stream, true);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) return cuda_fail(e, what);
+        stage_busy = false;
+        if (int rc = check_wait_status()) return rc;
+        if (!in_place && gemm_status)
+            if (int rc = gemm_status_of(*gs)) return rc;
+        for (size_t j = 0; j < n_jobs; j++) std::memcpy(jobs[j].y, ys + y_off[j], t * jobs[j].n_out * 4);
+        return B2_OK;
     }
 
     // ---- Backend::matmul (src/cuda.rs:1428-1493)
@@ -757,12 +774,18 @@ class Backend {
                 return rc;
             }
         }
+        if (staged(y_total)) {
+            if (int rc = staged_out(jobs, n_jobs, t, y_off, y_total, false, "matmul kernels / copy-out")) return rc;
+            ns_gpu += since(t1);  // (with the results' way back)
+            calls++;
+            return B2_OK;
+        }
         e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return cuda_fail(e, "matmul kernels");
         if (int rc = check_gemm_status()) return rc;
         ns_gpu += since(t1);
         auto t2 = clk::now();
-        e = copy_out(jobs, n_jobs, t, y_off, y_total);
+        e = copy_out(jobs, n_jobs, t, y_off);
         if (e != cudaSuccess) return cuda_fail(e, "copy-out");
         ns_out += since(t2);
         calls++;
@@ -790,8 +813,16 @@ class Backend {
             y_total += (t * jobs[j].n_out * 4 + 255) / 256 * 256;
         }
         auto t0 = clk::now();
+        // Matrices of one format that have the form with several jobs go in one launch, which stores to page-locked memory. (Launches that
+        // do so by turns wait for their stores: three of them 49 us, by way of the device 41.)
+        bool one = n_jobs <= (size_t)GEMV_TC_JOBS;
+        for (size_t j = 0; j < n_jobs; j++) {
+            const WeightDev& w = find(jobs[j].w)->dev;
+            one = one && gemv_tc_supports(w) && w.fmt == find(jobs[0].w)->dev.fmt && (n_jobs == 1 || !jobs[j].up);
+        }
+        const bool in_place = one && staged(y_total);
         cudaError_t e = x_dev.reserve(t * n_in * 4);
-        if (e == cudaSuccess) e = y_dev.reserve(y_total);  // all jobs run before any result goes back to the host
+        if (e == cudaSuccess && !in_place) e = y_dev.reserve(y_total);  // all jobs run before any result goes back to the host
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(staging)");
         e = copy_in(x, t * n_in * 4);
         if (e != cudaSuccess) return cuda_fail(e, "copy-in");
@@ -802,10 +833,22 @@ class Backend {
         const size_t digits = t * record_stride(n_in, false);
         bool made[2] = {false, false};
         if (t > 1 && (e = xrec.reserve(digits + t * record_stride(n_in, true))) != cudaSuccess) return cuda_fail(e, "cudaMalloc(records)");
-        for (size_t j = 0; j < n_jobs; j++) {
+        if (one && n_jobs > 1) {
+            GemvTcJob all[GEMV_TC_JOBS];
+            for (size_t j = 0; j < n_jobs; j++) all[j] = {&find(jobs[j].w)->dev, (float*)((in_place ? host_stage + HOST_STAGE : (uint8_t*)y_dev.p) + y_off[j])};
+            GemvIn in;
+            in.x = (const float*)x_dev.p;
+            in.x_stride = n_in;
+            in.fast = fast_planes && !exact;
+            in.status = wait_status;
+            e = launch_gemv_tc_jobs(all, (int)n_jobs, in, (int)t, sm_count, stream, true);
+            launches++;
+            if (e != cudaSuccess) return cuda_fail(e, "gemv (jobs)");
+        }
+        for (size_t j = 0; j < n_jobs && !(one && n_jobs > 1); j++) {
             Weight* w = find(jobs[j].w);
             Weight* u = jobs[j].up ? find(jobs[j].up) : nullptr;
-            float* yj = (float*)((uint8_t*)y_dev.p + y_off[j]);
+            float* yj = (float*)((in_place ? host_stage + HOST_STAGE : (uint8_t*)y_dev.p) + y_off[j]);
             const int mode = jobs[j].up ? B2_MODE_SILU_PAIR : B2_MODE_STORE;
             if (fmt_is_other(w->dev.fmt)) {
                 e = launch_gemv_other(w->dev, u ? &u->dev : nullptr, (const float*)x_dev.p, n_in, yj, jobs[j].n_out, (int)t, mode, nullptr, sm_count, stream);
@@ -832,16 +875,15 @@ class Backend {
             }
         }
         // Every launch was accepted (a refused one returned above, before any y is touched): small results follow the kernels on
-        // the stream to page-locked memory and the call synchronizes once (a product of a few microseconds would otherwise pay two
-        // host round trips); large ones are copied when the kernels' waits are known to have ended. The kernels' and the copies'
-        // time are booked together as kernel time.
-        if (y_total > HOST_STAGE || !stage_host()) {
+        // the stream to page-locked memory and the call synchronizes once; large ones are copied when the kernels' waits are known to
+        // have ended. The kernels' and the copies' time are booked together as kernel time.
+        if (staged(y_total)) {
+            if (int rc = staged_out(jobs, n_jobs, t, y_off, y_total, in_place, "matvec_rows kernels / copy-out")) return rc;
+        } else {
             if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(e, "matvec_rows kernels");
             if (int rc = check_wait_status()) return rc;
+            if ((e = copy_out(jobs, n_jobs, t, y_off)) != cudaSuccess) return cuda_fail(e, "copy-out");
         }
-        e = copy_out(jobs, n_jobs, t, y_off, y_total);
-        if (int rc = check_wait_status()) return rc;
-        if (e != cudaSuccess) return cuda_fail(e, "matvec_rows kernels / copy-out");
         ns_gpu += since(t1);
         calls++;
         return B2_OK;
@@ -1592,7 +1634,7 @@ B2_EXPORT int b2_open(int ordinal, b2_ctx** out) {
         return B2_ERR_CUDA;
     }
     uint32_t* word = nullptr;
-    if (cudaHostAlloc((void**)&word, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    if (cudaHostAlloc((void**)&word, 64 + sizeof(b2::GemmStatus), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
         g_open_error = "[b200qmm: cudaHostAlloc failed]";
         cudaGetLastError();
         return B2_ERR_NOMEM;

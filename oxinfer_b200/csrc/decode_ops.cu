@@ -196,6 +196,16 @@ __global__ void __launch_bounds__(256) kv_rows_kernel(float* rows, T* cache, uin
     else rows[i] = (float)cache[at];
 }
 
+// Two runs of 16-byte words, one of them to or from page-locked memory of the host (read past the caches). Latency bounds it: a word a
+// thread, all in flight at once.
+__global__ void __launch_bounds__(256) copy16_kernel(uint4* d0, const uint4* s0, uint32_t n0, uint4* d1, const uint4* s1, uint32_t n1) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n0) d0[i] = __ldcv(s0 + i);
+    else if (i - n0 < n1) d1[i - n0] = __ldcv(s1 + (i - n0));
+}
+
 __global__ void set_step_kernel(uint32_t* sp, uint32_t pos, uint32_t table_pos0, uint32_t count, int* token, int tok) {
     sp[0] = pos;
     sp[1] = table_pos0;
@@ -318,6 +328,12 @@ cudaError_t launch_glu(const float* g, const float* u, float* out, uint32_t n, i
 cudaError_t launch_argmax(const float* logits, uint32_t n, float* pval, int* pidx, uint32_t* counter, int* token, int* out_tokens, uint32_t* sp,
                           cudaStream_t st, bool pdl) {
     return launch_k(argmax_kernel, dim3(ARGMAX_CTAS), dim3(256), 0, st, pdl, logits, n, pval, pidx, counter, token, out_tokens, sp);
+}
+
+cudaError_t launch_copy16(void* d0, const void* s0, size_t bytes0, void* d1, const void* s1, size_t bytes1, cudaStream_t st, bool pdl) {
+    const uint32_t n0 = (uint32_t)(bytes0 / 16), n1 = (uint32_t)(bytes1 / 16);
+    if (n0 + n1 == 0) return cudaSuccess;
+    return launch_k(copy16_kernel, dim3((n0 + n1 + 255) / 256), dim3(256), 0, st, pdl, (uint4*)d0, (const uint4*)s0, n0, (uint4*)d1, (const uint4*)s1, n1);
 }
 
 }  // namespace b2

@@ -30,6 +30,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <climits>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -43,7 +44,7 @@ namespace b2 {
 namespace {
 
 constexpr int GT_CTAS = 4, GT_ROWS = 128, GT_SETS = 4, GT_WARPS = 2 + 4 * GT_SETS, GT_THREADS = GT_WARPS * 32;
-constexpr int GT_MOST_SLOTS = 8, GT_TOKENS = 4;
+constexpr int GT_MOST_SLOTS = 8, GT_TOKENS = 4, GT_MOST_JOBS = GEMV_TC_JOBS;
 constexpr uint32_t GT_RAW = GT_ROWS * 144;                 // a slot: a block of 256 k of 128 rows
 constexpr uint32_t GT_TMEM_COLS = 512, GT_SET_COLS = 128;  // of a set: 64 of weights, 64 of sums
 constexpr uint32_t GT_AM = 0, GT_DM = 16, GT_D = 64;       // (the minimums and their sums lie where weights were)
@@ -65,6 +66,19 @@ struct GtArgs {
     size_t n_out;
     uint32_t b_off, min_off, sum_off, xs_off;  // shared memory
     uint32_t* status;
+};
+
+// The matrices: one, a pair, or up to GT_MOST_JOBS with results of their own (JOBS), whose tiles follow one another.
+template <bool JOBS>
+struct GtMats {
+    CUtensorMap m[2];
+};
+template <>
+struct GtMats<true> {
+    CUtensorMap m[GT_MOST_JOBS];
+    float* y[GT_MOST_JOBS];
+    size_t n_out[GT_MOST_JOBS];
+    int first[GT_MOST_JOBS];  // tile; behind the last matrix: no tile
 };
 
 template <int TP>
@@ -148,9 +162,9 @@ __device__ __forceinline__ uint32_t gt_at(uint32_t n, uint32_t k) { return (n >>
 __device__ __forceinline__ float gt_silu(float a) { return a / (1.0f + __expf(-a)); }
 __device__ __forceinline__ float gt_gelu(float a) { return 0.5f * a * (1.0f + tanhf(0.7978845608f * (a + 0.044715f * a * a * a))); }
 
-template <bool MLX, bool PAIR, int TP>
+template <bool MLX, bool PAIR, int TP, bool JOBS>
 __global__ void __launch_bounds__(GT_THREADS, 1)
-gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_u, const __grid_constant__ GtArgs a) {
+gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant__ GtArgs a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* const smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -166,8 +180,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     const int total = my_tiles * nbq;  // blocks to copy
     constexpr uint32_t IN_BYTES = GT_SETS * GT_CTAS * 32 * TP * 4;
     if (warp == 0) {
-        if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-        if (PAIR && lane == 1) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_u) : "memory");
+        if (lane < (JOBS ? GT_MOST_JOBS : PAIR ? 2 : 1)) asm volatile("prefetch.tensormap [%0];" ::"l"(&mats.m[lane]) : "memory");
         if (lane < a.slots) {
             mbar_init(&sh->raw_full[lane], 1);
             mbar_init(&sh->raw_empty[lane], 4);
@@ -186,6 +199,13 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         tc_fence_before();
     }
+    auto job_of = [&](int tile) {
+        int j = 0;
+        if constexpr (JOBS)
+#pragma unroll
+            for (int k = 1; k < GT_MOST_JOBS; k++) j += tile >= mats.first[k];
+        return j;
+    };
     // warp 0: the next block goes to slot c_slot: block c_blk of tile c_tile
     int c_slot = 0, c_blk = 0, c_tile = cluster;
     auto copy = [&] {
@@ -194,10 +214,13 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             uint8_t* dst = smem + (size_t)c_slot * GT_RAW;
             mbar_arrive_expect_tx(&sh->raw_full[c_slot], GT_RAW);
             if constexpr (PAIR) {  // 64 rows of either matrix
-                tma_load_2d(dst, &tmap_w, &sh->raw_full[c_slot], x, c_tile * 64);
-                tma_load_2d(dst + 64 * 144, &tmap_u, &sh->raw_full[c_slot], x, c_tile * 64);
+                tma_load_2d(dst, &mats.m[0], &sh->raw_full[c_slot], x, c_tile * 64);
+                tma_load_2d(dst + 64 * 144, &mats.m[1], &sh->raw_full[c_slot], x, c_tile * 64);
+            } else if constexpr (JOBS) {
+                const int j = job_of(c_tile);
+                tma_load_2d(dst, &mats.m[j], &sh->raw_full[c_slot], x, (c_tile - mats.first[j]) * GT_ROWS);
             } else {
-                tma_load_2d(dst, &tmap_w, &sh->raw_full[c_slot], x, c_tile * GT_ROWS);
+                tma_load_2d(dst, &mats.m[0], &sh->raw_full[c_slot], x, c_tile * GT_ROWS);
             }
         }
         __syncwarp();
@@ -483,13 +506,23 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         }
 #pragma unroll 1
         for (int i = -1; i < my_tiles && ok; i++) {  // (the first pass fetches the code and stores nothing)
-            const int buf = i & 1, tile = cluster + i * clusters;
-            const size_t row = i < 0 ? a.n_out : PAIR ? (size_t)tile * 64 + 16 * rank + (lane & 15) : (size_t)tile * GT_ROWS + 32 * rank + lane;
+            const int buf = i & 1;
+            int tile = cluster + i * clusters;
+            float* y = a.y;
+            size_t n_out = a.n_out;
+            if constexpr (JOBS) {
+                const int j = job_of(max(tile, 0));
+                y = mats.y[j];
+                n_out = mats.n_out[j];
+                tile -= mats.first[j];
+            }
+            const size_t y_stride = JOBS ? n_out : a.y_stride;
+            const size_t row = i < 0 ? n_out : PAIR ? (size_t)tile * 64 + 16 * rank + (lane & 15) : (size_t)tile * GT_ROWS + 32 * rank + lane;
             float old[TP], times[TP];  // what the results are added to, read while the products run
             if (!PAIR) {
 #pragma unroll
                 for (int t = 0; t < TP; t++) {
-                    old[t] = a.mode != B2_MODE_STORE && t < T && row < a.n_out ? a.y[(size_t)(t0 + t) * a.y_stride + row] : 0.0f;
+                    old[t] = a.mode != B2_MODE_STORE && t < T && row < n_out ? y[(size_t)(t0 + t) * y_stride + row] : 0.0f;
                     times[t] = a.mode != B2_MODE_STORE && a.mode != B2_MODE_ADD && t < T ? 1.0f / (1.0f + __expf(-a.gate[(size_t)(t0 + t) * a.gate_stride])) : 1.0f;
                 }
             }
@@ -518,8 +551,8 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 #pragma unroll
             for (int t = 0; t < TP; t++) {
                 const float up = PAIR ? __shfl_xor_sync(0xffffffffu, v[t], 16) : 0.0f;
-                if (t >= T || row >= a.n_out || (PAIR && lane >= 16)) continue;
-                float* o = a.y + (size_t)(t0 + t) * a.y_stride + row;
+                if (t >= T || row >= n_out || (PAIR && lane >= 16)) continue;
+                float* o = y + (size_t)(t0 + t) * y_stride + row;
                 if (PAIR) *o = (a.mode == B2_MODE_SILU_PAIR ? gt_silu(v[t]) : gt_gelu(v[t])) * up;
                 else *o = a.mode == B2_MODE_STORE ? v[t] : old[t] + v[t] * times[t];
             }
@@ -550,14 +583,22 @@ size_t gt_fixed(size_t K) {  // shared memory beside the ring
     return 1024 + nbq * 4096 + (nbq + 3) / 4 * 2048 + nbq * GT_TOKENS * 4 * 6;
 }
 
-template <bool MLX, bool PAIR, int TP>
-cudaError_t gt_launch(const WeightDev& w, const WeightDev* up, GtArgs a, int sm_count, cudaStream_t st, bool pdl) {
-    CUtensorMap mw, mu;
-    if (!gt_map(&mw, w, PAIR ? 64 : GT_ROWS)) return cudaErrorInvalidValue;
-    if (PAIR) {
-        if (!gt_map(&mu, *up, 64)) return cudaErrorInvalidValue;
+template <bool MLX, bool PAIR, int TP, bool JOBS>
+cudaError_t gt_launch(const WeightDev& w, const WeightDev* up, const GemvTcJob* jobs, int n_jobs, GtArgs a, int sm_count, cudaStream_t st, bool pdl) {
+    GtMats<JOBS> mats;
+    if constexpr (JOBS) {
+        a.tiles = 0;
+        for (int j = 0; j < GT_MOST_JOBS; j++) {
+            const GemvTcJob& job = jobs[std::min(j, n_jobs - 1)];
+            if (!gt_map(&mats.m[j], *job.w, GT_ROWS)) return cudaErrorInvalidValue;
+            mats.y[j] = job.y;
+            mats.n_out[j] = job.w->n_out;
+            mats.first[j] = j < n_jobs ? a.tiles : INT_MAX;
+            if (j < n_jobs) a.tiles += (int)((job.w->n_out + GT_ROWS - 1) / GT_ROWS);
+        }
     } else {
-        mu = mw;
+        if (!gt_map(&mats.m[0], w, PAIR ? 64 : GT_ROWS) || !gt_map(&mats.m[1], PAIR ? *up : w, PAIR ? 64 : GT_ROWS)) return cudaErrorInvalidValue;
+        a.tiles = (int)((w.n_out + (PAIR ? 63 : 127)) / (PAIR ? 64 : 128));
     }
     const size_t nbq = (w.n_in / 256 + GT_CTAS - 1) / GT_CTAS, fixed = gt_fixed(w.n_in);
     a.slots = (int)std::min<size_t>(GT_MOST_SLOTS, (GT_SMEM - fixed) / GT_RAW);
@@ -565,9 +606,8 @@ cudaError_t gt_launch(const WeightDev& w, const WeightDev* up, GtArgs a, int sm_
     a.min_off = a.b_off + (uint32_t)nbq * 4096;
     a.sum_off = a.min_off + (uint32_t)((nbq + 3) / 4 * 2048);
     a.xs_off = a.sum_off + (uint32_t)(nbq * TP * 16);
-    a.tiles = (int)((w.n_out + (PAIR ? 63 : 127)) / (PAIR ? 64 : 128));
     const size_t smem = fixed + (size_t)a.slots * GT_RAW;
-    auto kern = gemv_tc_kernel<MLX, PAIR, TP>;
+    auto kern = gemv_tc_kernel<MLX, PAIR, TP, JOBS>;
     if (cudaError_t e = ensure_dynamic_smem((const void*)kern, smem, 0); e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GT_THREADS);
@@ -603,14 +643,32 @@ cudaError_t gt_launch(const WeightDev& w, const WeightDev* up, GtArgs a, int sm_
     a.rounds = (a.tiles + most - 1) / most;
     cfg.gridDim = dim3((unsigned)((a.tiles + a.rounds - 1) / a.rounds * GT_CTAS << a.two));
     cfg.numAttrs = pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kern, mw, mu, a);
+    return cudaLaunchKernelEx(&cfg, kern, mats, a);
 }
 
-template <bool MLX, bool PAIR>
-cudaError_t gt_tokens(const WeightDev& w, const WeightDev* up, const GtArgs& a, int sm_count, cudaStream_t st, bool pdl) {
-    if (a.T == 1) return gt_launch<MLX, PAIR, 1>(w, up, a, sm_count, st, pdl);
-    if (a.T == 2) return gt_launch<MLX, PAIR, 2>(w, up, a, sm_count, st, pdl);
-    return gt_launch<MLX, PAIR, 4>(w, up, a, sm_count, st, pdl);
+template <bool MLX, bool PAIR, bool JOBS = false>
+cudaError_t gt_tokens(const WeightDev& w, const WeightDev* up, const GtArgs& a, int sm_count, cudaStream_t st, bool pdl, const GemvTcJob* jobs = nullptr, int n_jobs = 0) {
+    if (a.T == 1) return gt_launch<MLX, PAIR, 1, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
+    if (a.T == 2) return gt_launch<MLX, PAIR, 2, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
+    return gt_launch<MLX, PAIR, 4, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
+}
+
+GtArgs gt_args(const WeightDev& w, const GemvIn& in, int T) {
+    GtArgs a{};
+    a.x = in.x;
+    a.x_stride = in.x_stride;
+    a.nw = in.norm_w;
+    a.pre = in.pre;
+    a.norm = in.norm;
+    a.eps = in.eps;
+    a.rec = in.rec;
+    a.rec_stride = in.rec_stride;
+    a.fast = in.fast;
+    a.T = T;
+    a.two = T > GT_TOKENS;
+    a.n_in = (int)w.n_in;
+    a.status = in.status;
+    return a;
 }
 
 }  // namespace
@@ -625,32 +683,31 @@ cudaError_t launch_gemv_tc(const WeightDev& w, const WeightDev* up, const GemvIn
     if (!gemv_tc_supports(w) || !in.status || T < 1) return cudaErrorInvalidValue;
     const bool pair = mode == B2_MODE_SILU_PAIR || mode == B2_MODE_GELU_PAIR;
     for (int t = 0; t < T; t += 2 * GT_TOKENS) {
-        GtArgs a{};
-        a.x = in.x ? in.x + (size_t)t * in.x_stride : nullptr;
-        a.x_stride = in.x_stride;
-        a.nw = in.norm_w;
-        a.pre = in.pre;
-        a.norm = in.norm;
-        a.eps = in.eps;
-        a.rec = in.rec ? in.rec + (size_t)t * in.rec_stride : nullptr;
-        a.rec_stride = in.rec_stride;
-        a.fast = in.fast;
+        GemvIn at = in;
+        if (in.x) at.x = in.x + (size_t)t * in.x_stride;
+        if (in.rec) at.rec = in.rec + (size_t)t * in.rec_stride;
+        GtArgs a = gt_args(w, at, std::min(T - t, 2 * GT_TOKENS));
         a.y = y + (size_t)t * y_stride;
         a.y_stride = y_stride;
         a.gate = gate ? gate + (size_t)t * gate_stride : nullptr;
         a.gate_stride = gate_stride;
         a.mode = mode;
-        a.T = std::min(T - t, 2 * GT_TOKENS);
-        a.two = a.T > GT_TOKENS;
-        a.n_in = (int)w.n_in;
         a.n_out = w.n_out;
-        a.status = in.status;
         cudaError_t e;
         if (w.fmt == B2_FMT_MLX4) e = pair ? gt_tokens<true, true>(w, up, a, sm_count, st, pdl) : gt_tokens<true, false>(w, up, a, sm_count, st, pdl);
         else e = pair ? gt_tokens<false, true>(w, up, a, sm_count, st, pdl) : gt_tokens<false, false>(w, up, a, sm_count, st, pdl);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+cudaError_t launch_gemv_tc_jobs(const GemvTcJob* jobs, int n_jobs, const GemvIn& in, int T, int sm_count, cudaStream_t st, bool pdl) {
+    if (n_jobs < 1 || n_jobs > GEMV_TC_JOBS || !in.status || T < 1 || T > 2 * GT_TOKENS) return cudaErrorInvalidValue;
+    const WeightDev& w = *jobs[0].w;
+    for (int j = 0; j < n_jobs; j++)
+        if (!gemv_tc_supports(*jobs[j].w) || jobs[j].w->fmt != w.fmt || jobs[j].w->n_in != w.n_in) return cudaErrorInvalidValue;
+    const GtArgs a = gt_args(w, in, T);
+    return w.fmt == B2_FMT_MLX4 ? gt_tokens<true, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs) : gt_tokens<false, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs);
 }
 
 }  // namespace b2

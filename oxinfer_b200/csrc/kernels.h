@@ -96,6 +96,13 @@ cudaError_t launch_gemv_mma(const WeightDev& w, const WeightDev* up, const GemvI
 bool gemv_tc_supports(const WeightDev& w);
 cudaError_t launch_gemv_tc(const WeightDev& w, const WeightDev* up, const GemvIn& in, int T, float* y, size_t y_stride, int mode, const float* gate,
                            size_t gate_stride, int sm_count, cudaStream_t st, bool pdl);
+// Up to four matrices of one format and K by the same T (1 .. 8) rows, in one launch; results one after another, [T][n_out] each.
+constexpr int GEMV_TC_JOBS = 4;
+struct GemvTcJob {
+    const WeightDev* w;
+    float* y;
+};
+cudaError_t launch_gemv_tc_jobs(const GemvTcJob* jobs, int n_jobs, const GemvIn& in, int T, int sm_count, cudaStream_t st, bool pdl);
 // Products over a stack of equally shaped 4-bit matrices (the routed experts of a batch; w describes matrix 0, the others w_stride bytes
 // apart): group g multiplies matrix expert[g] by rows row0[g] .. + count[g] - 1 (at most `most`, 1 .. 8) of the pairs' list. Row i reads the
 // vector of x's row src[i] (gather) or i and writes row i of y. The table travels as a kernel argument: no copy, no synchronization.
@@ -110,6 +117,8 @@ struct GemvGroups {
 int gemv_groups_most(size_t K);  // 8, 4, 1, or 0: not even one row of K values fits
 cudaError_t launch_gemv_groups(const WeightDev& w, const WeightDev* up, const float* x, size_t x_stride, const GemvGroups& groups, int most, float* y,
                                size_t y_stride, int mode, bool fast, int sm_count, cudaStream_t st);
+// decode_ops.cu: two runs of whole 16-byte words (the second may be empty), not overlapping; page-locked host memory on either side.
+cudaError_t launch_copy16(void* d0, const void* s0, size_t bytes0, void* d1, const void* s1, size_t bytes1, cudaStream_t st, bool pdl);
 // Records (split.cuh, split_bytes each) of `tokens` vectors of x * pre * norm_w.
 cudaError_t launch_split(const float* x, size_t x_stride, const float* norm_w, float pre, size_t K, int tokens, uint8_t* rec, size_t rec_stride, bool halves,
                          bool fast, cudaStream_t st, bool pdl);

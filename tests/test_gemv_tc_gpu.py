@@ -66,3 +66,31 @@ def test_device_rows_and_row_shards_have_the_whole_matrix_bits(backend, fmt):
         assert np.array_equal(ys.cpu().numpy(), ones[:4])
     finally:
         backend.set_stream(0)
+
+
+@pytest.mark.parametrize("fmt", ["q4_k", "mlx4"])
+@pytest.mark.parametrize("t", [1, 2, 3, 4])
+def test_matrices_of_one_call_share_a_launch_and_keep_their_bits(backend, fmt, t):
+    """Row counts at the edges of the tiles; more than four matrices, a pair or another format among them take launches of their own; results that do
+    not fit the page-locked stage (256 KB)."""
+    n_in = 1280
+    outs = [1, 128, 129, 300, 33000]
+    devs = [backend.upload(make_pair(fmt, n, n_in, 700 + n % 89)[0], n, n_in) for n in outs]
+    other = backend.upload(make_pair("q8_0", 96, n_in, 790)[0], 96, n_in)
+    x = synth.activations(t, n_in, 701)
+
+    def run(ds, ns, ups=None):
+        ys = [np.full((t, n), np.nan, np.float32) for n in ns]
+        before = backend.launch_count()
+        assert backend.matvec_rows(x, [ob.RowsJob(d, y, up=u) for d, y, u in zip(ds, ys, ups or [None] * len(ds))])
+        return ys, backend.launch_count() - before
+
+    alone = [run([d], [n])[0][0] for d, n in zip(devs, outs)]
+    for pick, launches in (((0, 1), 1), ((3, 0, 2), 1), ((2, 4, 1, 0), 1), ((0, 1, 2, 3, 4), 5)):
+        ys, count = run([devs[k] for k in pick], [outs[k] for k in pick])
+        assert count == launches
+        for k, y in zip(pick, ys):
+            assert np.array_equal(y, alone[k]), (pick, k)
+    pair = run([devs[1]], [128], [devs[1]])[0][0]
+    ys, _ = run([devs[1], devs[2], other], [128, 129, 96], [devs[1], None, None])
+    assert np.array_equal(ys[0], pair) and np.array_equal(ys[1], alone[2]) and np.isfinite(ys[2]).all()
