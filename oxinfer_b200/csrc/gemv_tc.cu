@@ -85,7 +85,9 @@ template <int TP>
 struct __align__(16) GtShared {
     float in[2][GT_SETS * GT_CTAS][32][TP];   // tiles in turn: a set's sums of this CTA's 32 rows
     float ssq_in[GT_CTAS][GT_TOKENS];   // the parts' sums of squares
-    uint64_t raw_full[GT_MOST_SLOTS], raw_empty[GT_MOST_SLOTS];
+    // A set's copies have barriers of their own, in the order of its blocks: a slot passes from set to set, and one that waited on a slot's barrier
+    // could be two uses ahead of it, where a parity says nothing. (At most GT_MOST_SLOTS blocks are in flight, so eight are enough.)
+    uint64_t raw_full[GT_SETS][GT_MOST_SLOTS], raw_empty[GT_MOST_SLOTS];
     uint64_t d_full[GT_SETS];
     uint64_t in_full[2], in_free[GT_CTAS][2], ssq_full;  // in_free: CTA w's places are free again
     uint32_t tmem_base;
@@ -181,10 +183,8 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
     constexpr uint32_t IN_BYTES = GT_SETS * GT_CTAS * 32 * TP * 4;
     if (warp == 0) {
         if (lane < (JOBS ? GT_MOST_JOBS : PAIR ? 2 : 1)) asm volatile("prefetch.tensormap [%0];" ::"l"(&mats.m[lane]) : "memory");
-        if (lane < a.slots) {
-            mbar_init(&sh->raw_full[lane], 1);
-            mbar_init(&sh->raw_empty[lane], 4);
-        }
+        mbar_init(&sh->raw_full[lane / GT_MOST_SLOTS][lane % GT_MOST_SLOTS], 1);
+        if (lane < GT_MOST_SLOTS) mbar_init(&sh->raw_empty[lane], 4);
         if (lane < GT_SETS) mbar_init(&sh->d_full[lane], 1);
         if (lane < 2 * GT_CTAS) mbar_init(&sh->in_free[lane >> 1][lane & 1], 1);
         if (lane < 2) mbar_init(&sh->in_full[lane], 1);
@@ -207,20 +207,22 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
         return j;
     };
     // warp 0: the next block goes to slot c_slot: block c_blk of tile c_tile
-    int c_slot = 0, c_blk = 0, c_tile = cluster;
+    int c_slot = 0, c_blk = 0, c_tile = cluster, c_round = 0;
+    auto place_of = [&](int round, int blk) { return round * ((nbq - (blk & 3) + 3) >> 2) + (blk >> 2); };  // among the blocks of its set
     auto copy = [&] {
         if (elect_one()) {
             const int x = (b0 + c_blk) * 144;
             uint8_t* dst = smem + (size_t)c_slot * GT_RAW;
-            mbar_arrive_expect_tx(&sh->raw_full[c_slot], GT_RAW);
+            uint64_t* const full = &sh->raw_full[c_blk & 3][place_of(c_round, c_blk) & (GT_MOST_SLOTS - 1)];
+            mbar_arrive_expect_tx(full, GT_RAW);
             if constexpr (PAIR) {  // 64 rows of either matrix
-                tma_load_2d(dst, &mats.m[0], &sh->raw_full[c_slot], x, c_tile * 64);
-                tma_load_2d(dst + 64 * 144, &mats.m[1], &sh->raw_full[c_slot], x, c_tile * 64);
+                tma_load_2d(dst, &mats.m[0], full, x, c_tile * 64);
+                tma_load_2d(dst + 64 * 144, &mats.m[1], full, x, c_tile * 64);
             } else if constexpr (JOBS) {
                 const int j = job_of(c_tile);
-                tma_load_2d(dst, &mats.m[j], &sh->raw_full[c_slot], x, (c_tile - mats.first[j]) * GT_ROWS);
+                tma_load_2d(dst, &mats.m[j], full, x, (c_tile - mats.first[j]) * GT_ROWS);
             } else {
-                tma_load_2d(dst, &mats.m[0], &sh->raw_full[c_slot], x, c_tile * GT_ROWS);
+                tma_load_2d(dst, &mats.m[0], full, x, c_tile * GT_ROWS);
             }
         }
         __syncwarp();
@@ -228,6 +230,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
         if (++c_blk == nbq) {
             c_blk = 0;
             c_tile += clusters;
+            c_round++;
         }
     };
     const int first = min(total, a.slots);
@@ -306,8 +309,8 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
         const uint32_t at = tmem + ((uint32_t)(32 * w) << 16) + set * GT_SET_COLS;
         const uint32_t base = tmem + set * GT_SET_COLS;
         const uint64_t bd = smem_desc_sw128(smem_u32(b_s)), md = smem_desc_sw128(smem_u32(min_s));
-        uint32_t phase = 0, raw_phase = 0;
-        int s = 0, at_n = 0;  // the slot of block at_n
+        uint32_t phase = 0;
+        int s = 0, at_n = 0, place = 0;  // the slot of block at_n; the next block among this set's
         bool ok = true;
         for (int i = 0; i < my_tiles && ok; i++) {
             float acc[TP], low[TP];  // the third digit's share, the others'
@@ -315,8 +318,9 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
             for (int t = 0; t < TP; t++) acc[t] = low[t] = 0.0f;
             for (int lb = set; lb < nbq && ok; lb += GT_SETS) {
                 const int n = i * nbq + lb;
-                for (s += n - at_n, at_n = n; s >= a.slots; s -= a.slots) raw_phase ^= 1;
-                ok = __all_sync(0xffffffffu, gt_wait(&sh->raw_full[s], raw_phase, sh, a.status));
+                for (s += n - at_n, at_n = n; s >= a.slots;) s -= a.slots;
+                ok = __all_sync(0xffffffffu, gt_wait(&sh->raw_full[set][place & (GT_MOST_SLOTS - 1)], (uint32_t)((place / GT_MOST_SLOTS) & 1), sh, a.status));
+                place++;
                 if (!ok) break;
                 const uint4* my = (const uint4*)(smem + (size_t)s * GT_RAW + (size_t)r * 144);
                 const uint4 hd = my[0];
@@ -465,10 +469,10 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
             // To the CTA that has the row: 32 of them each; of a pair, 16 of either matrix (rows 0 .. 63 of the tile are the first one's).
 #pragma unroll
             for (int t = 0; t < TP; t++) acc[t] += low[t];
-            const int buf = i & 1, to = PAIR ? 2 * (w & 1) + (lane >> 4) : w, place = PAIR ? 16 * (w >> 1) + (lane & 15) : lane;
+            const int buf = i & 1, to = PAIR ? 2 * (w & 1) + (lane >> 4) : w, row = PAIR ? 16 * (w >> 1) + (lane & 15) : lane;
             if (i >= 2) ok = __all_sync(0xffffffffu, gt_wait(&sh->in_free[to][buf], (uint32_t)(((i >> 1) - 1) & 1), sh, a.status));
             if (!ok) break;
-            gt_send(cluster_addr(&sh->in[buf][GT_SETS * rank + set][place][0], to), acc, cluster_addr(&sh->in_full[buf], to));
+            gt_send(cluster_addr(&sh->in[buf][GT_SETS * rank + set][row][0], to), acc, cluster_addr(&sh->in_full[buf], to));
         }
     } else if (warp == 0) {
         // ---------------- packed weights ----------------
@@ -481,7 +485,10 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
             copy();
         }
         if (sh->abort_flag)  // copies in flight land before the shared memory goes away
-            for (int n = max(0, issued - a.slots); n < issued; n++) gt_wait(&sh->raw_full[n % a.slots], (uint32_t)((n / a.slots) & 1), sh, a.status, false);
+            for (int n = max(0, issued - a.slots); n < issued; n++) {
+                const int round_n = n / nbq, blk = n - round_n * nbq, at = place_of(round_n, blk);
+                gt_wait(&sh->raw_full[blk & 3][at & (GT_MOST_SLOTS - 1)], (uint32_t)((at / GT_MOST_SLOTS) & 1), sh, a.status, false);
+            }
     } else if (warp == 1) {
         // ---------------- results ----------------
         float factor[TP];

@@ -13,7 +13,7 @@ from util import row_err
 pytestmark = pytest.mark.gpu
 
 # rows, K: parts without a block (one and two blocks), with unequal numbers, more blocks than sets; one row, tiles' edges, several tiles a cluster
-SHAPES = [(1, 256), (129, 512), (65, 768), (127, 1280), (64, 1024), (300, 5120), (128, 16640), (5000, 1024)]
+SHAPES = [(1, 256), (129, 512), (65, 768), (127, 1280), (64, 1024), (300, 5120), (128, 16640), (5000, 1024), (9300, 2560)]
 
 
 @pytest.mark.parametrize("fmt", ["q4_k", "mlx4"])
