@@ -508,17 +508,17 @@ class Backend {
     }
     // t tokens of one matrix from their records, up to eight per launch (the weights are read once per launch). A matrix that has more
     // tiles than the SMs have groups of warps goes four at a time, unless the activations of eight fit whole: the parts of K pass over
-    // several tiles each, and their sums through shared memory, one part at a time for eight. Eight tokens in one launch and in two:
-    // Q4_K 14336 x 4096 42 and 30 us, 28672 x 4096 136 and 47; Q8_0 48 and 32, 83 and 51. (4096 x 14336 has fewer tiles than that: one launch, 41 and 42 us.)
-    // The second launch waits for the first, so a matrix whose tiles fill no more than half of the SMs gains nothing by it: Q8_0
-    // 1024 x 2048 10.1 us in two launches, 7.8 in one; FP8 512 x 4096 11.5 and 10.1. Seven or eight tokens of Q6_K do (512 x 4096 12.7
+    // several tiles each, and their sums through shared memory, one part at a time for eight. Eight tokens in one launch and in two (FP8,
+    // Q6_K; the forms that gemv_tc.cu took over behaved alike): 14336 x 4096 48 and 32 us, 28672 x 4096 83 and 51.
+    // The second launch waits for the first, so a matrix whose tiles fill no more than half of the SMs gains nothing by it:
+    // FP8 512 x 4096 10.1 us in one launch, 11.5 in two. Seven or eight tokens of Q6_K do (512 x 4096 12.7
     // and 13.8). Matrices whose CTAs split only the part of K that they multiply (gemv_tc.cu) need no records (null), x instead, and take eight
-    // tokens a launch (4096 x 4096 7.9 us, in two launches 12.4); from records four, as the callers with host buffers count them.
+    // tokens a launch (Q4_K 4096 x 4096 7.9 us, in two launches 12.4); 4-bit ones from records four, as the callers with host buffers count them.
     int small_products(const WeightDev& w, const WeightDev* up, const uint8_t* rec, const float* x, size_t t, float* y, int mode) {
         const size_t stride = record_stride(w.n_in, gemv_mma_halves(w)), tiles = (w.n_out + 15) / 16;
         const bool narrow = 2 * tiles <= (size_t)sm_count && w.fmt == B2_FMT_Q6_K && t > 6;
         const bool tc = gemv_tc_supports(w);
-        const size_t per = narrow || (tc && rec) || (!tc && tiles > 2 * (size_t)sm_count && w.n_in > GEMV_WHOLE_8) ? 4 : 8;
+        const size_t per = narrow || (tc && rec && w.fmt != B2_FMT_Q8_0) || (!tc && tiles > 2 * (size_t)sm_count && w.n_in > GEMV_WHOLE_8) ? 4 : 8;
         for (size_t i = 0; i < t; i += per) {
             GemvIn in;
             if (!rec) {
@@ -818,7 +818,7 @@ class Backend {
         bool one = n_jobs <= (size_t)GEMV_TC_JOBS;
         for (size_t j = 0; j < n_jobs; j++) {
             const WeightDev& w = find(jobs[j].w)->dev;
-            one = one && gemv_tc_supports(w) && w.fmt == find(jobs[0].w)->dev.fmt && (n_jobs == 1 || !jobs[j].up);
+            one = one && gemv_tc_supports(w) && w.fmt == find(jobs[0].w)->dev.fmt && (n_jobs == 1 || (!jobs[j].up && w.fmt != B2_FMT_Q8_0));
         }
         const bool in_place = one && staged(y_total);
         cudaError_t e = x_dev.reserve(t * n_in * 4);

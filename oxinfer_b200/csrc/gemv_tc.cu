@@ -1,4 +1,4 @@
-// Products of one to eight tokens of 4-bit matrices (Q4_K, the repacked MLX-4) on the fifth-generation tensor cores: the role of dmv_* and dmvk_*
+// Products of one to eight tokens of 4-bit matrices (Q4_K, the repacked MLX-4) and Q8_0 on the fifth-generation tensor cores: the role of dmv_* and dmvk_*
 // in the reference (src/cuda_decode.cu:139-232). The arithmetic is that of gemv_mma.cuh: the packed integers of the weights times
 // signed digits of the activations (split.cuh: 23 to 24 bits of every value), summed exactly, scaled by 32 values in integers (Q4_K) or by
 // 64 in f32 (MLX-4). Here tcgen05.mma.kind::i8 makes the sums: A = 128 weight rows, a byte a weight, in tensor memory; B = the digits in
@@ -12,6 +12,8 @@
 //   warp 1        : adds the sixteen sums of its rows in pairs, applies the norm's factor and the output mode, and stores.
 // All but warp 0 split the CTA's part of the activations first (an RMS norm's weights multiply before the split, its factor the results).
 // Five to eight tokens: every other cluster has those from the fifth on, and the second reading of the weights comes from L2.
+// Q8_0 rows are bytes already: the instructions read them where the copies put them (two swizzled tiles of 128 k and the rows' scales), and a set's warps
+// only scale the sums (f32, per 32). Eight tokens are 32 columns then: read twice, the bytes would pass at L2's rate.
 //
 // What bounds it: HBM on large matrices, the start on small ones. The form on mma.sync (gemv_mma.cu) issued 276 warp instructions for 4096 weights (one
 // token; 367: four) and was bound by that; this one about 110 (four: 150). Of the 4.7 us of 4096 x 4096, 0.5 pass before the first copy is issued, 1.5 until
@@ -24,9 +26,13 @@
 //   MLX-4 4096 x 4096    4.9 / 8.6 / 9.8 / 14.9    5.2 / 5.5 / 6.0 / 7.7
 //         4096 x 14336  11.7 / 20.3 / 23.8 / 36.9  9.5 / 11.3 / 13.5 / 18.3
 //         32064 x 4096  15.9 / 22.8 / 24.9 / 45.6  15.9 / 16.7 / 18.5 / 31.8
+//   Q8_0  4096 x 4096    6.3 / 8.7 / 9.6 / 16.9    5.2 / 5.6 / 8.0 / 9.2
+//         4096 x 14336  15.0 / 24.3 / 28.4 / 42.1  13.0 / 14.6 / 16.2 / 24.5
+//         32064 x 4096  23.9 / 27.0 / 28.1 / 54.5  23.3 / 24.6 / 24.6 / 28.0
 // (6144 x 4096, MLX-4, one token: 5.9 and 6.3: its 48 tiles take two rounds of 24 clusters. In a graph 4096 x 4096 takes 4.5 and 4.4.)
 // Largest error of a result against 64 bits, in parts of the row's norm, N(0, 1) activations, K = 1024 / 4096 / 14336:
-// Q4_K 1.60 / 1.70 / 1.71e-7 on mma.sync, 1.60 / 1.65 / 1.66e-7 here; MLX-4 1.78 / 2.07 / 2.39e-7 and 1.57 / 1.65 / 1.59e-7.
+// Q4_K 1.60 / 1.70 / 1.71e-7 on mma.sync, 1.60 / 1.65 / 1.66e-7 here; MLX-4 1.78 / 2.07 / 2.39e-7 and 1.57 / 1.65 / 1.59e-7;
+// Q8_0 1.67 / 1.72 / 1.79e-7 and 1.67 / 1.69 / 1.73e-7.
 #include <cuda.h>
 
 #include <algorithm>
@@ -45,7 +51,7 @@ namespace {
 
 constexpr int GT_CTAS = 4, GT_ROWS = 128, GT_SETS = 4, GT_WARPS = 2 + 4 * GT_SETS, GT_THREADS = GT_WARPS * 32;
 constexpr int GT_MOST_SLOTS = 8, GT_TOKENS = 4, GT_MOST_JOBS = GEMV_TC_JOBS;
-constexpr uint32_t GT_RAW = GT_ROWS * 144;                 // a slot: a block of 256 k of 128 rows
+__host__ __device__ constexpr uint32_t gt_raw(int fmt) { return GT_ROWS * (fmt == B2_FMT_Q8_0 ? 272 : 144); }  // a slot: a block of 256 k of 128 rows
 constexpr uint32_t GT_TMEM_COLS = 512, GT_SET_COLS = 128;  // of a set: 64 of weights, 64 of sums
 constexpr uint32_t GT_AM = 0, GT_DM = 16, GT_D = 64;       // (the minimums and their sums lie where weights were)
 
@@ -69,12 +75,12 @@ struct GtArgs {
 };
 
 // The matrices: one, a pair, or up to GT_MOST_JOBS with results of their own (JOBS), whose tiles follow one another.
-template <bool JOBS>
+template <bool JOBS, bool Q8>
 struct GtMats {
-    CUtensorMap m[2];
+    CUtensorMap m[Q8 ? 4 : 2];  // (Q8_0: of bytes, then of scales)
 };
 template <>
-struct GtMats<true> {
+struct GtMats<true, false> {
     CUtensorMap m[GT_MOST_JOBS];
     float* y[GT_MOST_JOBS];
     size_t n_out[GT_MOST_JOBS];
@@ -84,7 +90,7 @@ struct GtMats<true> {
 template <int TP>
 struct __align__(16) GtShared {
     float in[2][GT_SETS * GT_CTAS][32][TP];   // tiles in turn: a set's sums of this CTA's 32 rows
-    float ssq_in[GT_CTAS][GT_TOKENS];   // the parts' sums of squares
+    float ssq_in[GT_CTAS][TP == 8 ? 8 : GT_TOKENS];  // the parts' sums of squares
     // A set's copies have barriers of their own, in the order of its blocks: a slot passes from set to set, and one that waited on a slot's barrier
     // could be two uses ahead of it, where a parity says nothing. (At most GT_MOST_SLOTS blocks are in flight, so eight are enough.)
     uint64_t raw_full[GT_SETS][GT_MOST_SLOTS], raw_empty[GT_MOST_SLOTS];
@@ -118,6 +124,13 @@ __device__ __forceinline__ void gt_mma(uint32_t d, uint32_t a, uint64_t bdesc, u
         "r"(a), "l"(bdesc), "r"(idesc), "r"(add)
         : "memory");
 }
+__device__ __forceinline__ void gt_mma_ss(uint32_t d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(0)
+        : "memory");
+}
 __device__ __forceinline__ void gt_st32(uint32_t taddr, const uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, "
@@ -146,6 +159,10 @@ __device__ __forceinline__ void gt_ld(uint32_t taddr, int (&v)[16]) {
                    "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                  : "r"(taddr));
 }
+__device__ __forceinline__ void gt_ld(uint32_t taddr, int (&v)[24]) {
+    gt_ld(taddr, *(int(*)[16]) & v[0]);
+    gt_ld(taddr + 16, *(int(*)[8]) & v[16]);
+}
 // Into a CTA of the cluster, counted on its barrier.
 __device__ __forceinline__ void gt_send(uint32_t a, const float (&v)[1], uint32_t bar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(a), "f"(v[0]), "r"(bar) : "memory");
@@ -157,6 +174,11 @@ __device__ __forceinline__ void gt_send(uint32_t a, const float (&v)[4], uint32_
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar)
                  : "memory");
 }
+__device__ __forceinline__ void gt_send(uint32_t a, const float (&v)[8], uint32_t bar) {
+    const float lo[4] = {v[0], v[1], v[2], v[3]}, hi[4] = {v[4], v[5], v[6], v[7]};
+    gt_send(a, lo, bar);
+    gt_send(a + 16, hi, bar);
+}
 __device__ __forceinline__ void gt_arrive(uint32_t cluster_bar) { asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory"); }
 __device__ __forceinline__ float gt_half(uint32_t w, int hi) { return __half2float(__ushort_as_half((unsigned short)(hi ? w >> 16 : w & 0xffffu))); }
 // Byte k of row n in a 128-byte swizzled tile of 16 rows.
@@ -164,9 +186,13 @@ __device__ __forceinline__ uint32_t gt_at(uint32_t n, uint32_t k) { return (n >>
 __device__ __forceinline__ float gt_silu(float a) { return a / (1.0f + __expf(-a)); }
 __device__ __forceinline__ float gt_gelu(float a) { return 0.5f * a * (1.0f + tanhf(0.7978845608f * (a + 0.044715f * a * a * a))); }
 
-template <bool MLX, bool PAIR, int TP, bool JOBS>
+template <int FMT, bool PAIR, int TP, bool JOBS>
 __global__ void __launch_bounds__(GT_THREADS, 1)
-gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant__ GtArgs a) {
+gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, const __grid_constant__ GtArgs a) {
+    constexpr bool MLX = FMT == B2_FMT_MLX4, Q8 = FMT == B2_FMT_Q8_0;
+    constexpr int MOST = TP == 8 ? 8 : GT_TOKENS;     // tokens of a cluster
+    constexpr uint32_t NB = TP == 8 ? 32 : 16;        // columns of an instruction
+    constexpr uint32_t RAW = gt_raw(FMT);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* const smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -176,13 +202,13 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
     // (five to eight tokens: every other cluster has those from the fifth on)
     const int rank = (int)cluster_rank(), t0 = a.two ? (int)(blockIdx.x / GT_CTAS & 1) * GT_TOKENS : 0;
     const int cluster = (int)(blockIdx.x / GT_CTAS) >> a.two, clusters = (int)(gridDim.x / GT_CTAS) >> a.two;
-    const int T = min(a.T - t0, GT_TOKENS);
+    const int T = min(a.T - t0, MOST);
     const int nb = a.n_in / 256, b0 = rank * nb / GT_CTAS, nbq = (rank + 1) * nb / GT_CTAS - b0;  // this CTA's blocks of K
     const int my_tiles = a.rounds - (cluster + (a.rounds - 1) * clusters >= a.tiles);  // (no divisions here and below: they are a third of the time to the first copy)
     const int total = my_tiles * nbq;  // blocks to copy
     constexpr uint32_t IN_BYTES = GT_SETS * GT_CTAS * 32 * TP * 4;
     if (warp == 0) {
-        if (lane < (JOBS ? GT_MOST_JOBS : PAIR ? 2 : 1)) asm volatile("prefetch.tensormap [%0];" ::"l"(&mats.m[lane]) : "memory");
+        if (lane < (JOBS ? GT_MOST_JOBS : Q8 ? 4 : PAIR ? 2 : 1)) asm volatile("prefetch.tensormap [%0];" ::"l"(&mats.m[lane]) : "memory");
         mbar_init(&sh->raw_full[lane / GT_MOST_SLOTS][lane % GT_MOST_SLOTS], 1);
         if (lane < GT_MOST_SLOTS) mbar_init(&sh->raw_empty[lane], 4);
         if (lane < GT_SETS) mbar_init(&sh->d_full[lane], 1);
@@ -192,7 +218,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
         if (lane == 3) sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (lane < 2) mbar_arrive_expect_tx(&sh->in_full[lane], IN_BYTES);
-        if (lane == 2) mbar_arrive_expect_tx(&sh->ssq_full, GT_CTAS * GT_TOKENS * 4);
+        if (lane == 2) mbar_arrive_expect_tx(&sh->ssq_full, GT_CTAS * MOST * 4);
         __syncwarp();
     } else if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem_base)), "r"(GT_TMEM_COLS) : "memory");
@@ -211,11 +237,19 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
     auto place_of = [&](int round, int blk) { return round * ((nbq - (blk & 3) + 3) >> 2) + (blk >> 2); };  // among the blocks of its set
     auto copy = [&] {
         if (elect_one()) {
-            const int x = (b0 + c_blk) * 144;
-            uint8_t* dst = smem + (size_t)c_slot * GT_RAW;
+            const int x = (b0 + c_blk) * (Q8 ? 256 : 144);
+            uint8_t* dst = smem + (size_t)c_slot * RAW;
             uint64_t* const full = &sh->raw_full[c_blk & 3][place_of(c_round, c_blk) & (GT_MOST_SLOTS - 1)];
-            mbar_arrive_expect_tx(full, GT_RAW);
-            if constexpr (PAIR) {  // 64 rows of either matrix
+            mbar_arrive_expect_tx(full, RAW);
+            if constexpr (Q8) {  // two swizzled tiles of 128 k and the rows' eight scales; a pair's matrices 64 rows each
+#pragma unroll
+                for (int u = 0; u < (PAIR ? 2 : 1); u++) {
+                    const int y = c_tile * (PAIR ? 64 : GT_ROWS);
+                    tma_load_2d(dst + u * 64 * 128, &mats.m[u], full, x, y);
+                    tma_load_2d(dst + GT_ROWS * 128 + u * 64 * 128, &mats.m[u], full, x + 128, y);
+                    tma_load_2d(dst + GT_ROWS * 256 + u * 64 * 16, &mats.m[2 + u], full, (b0 + c_blk) * 8, y);
+                }
+            } else if constexpr (PAIR) {  // 64 rows of either matrix
                 tma_load_2d(dst, &mats.m[0], full, x, c_tile * 64);
                 tma_load_2d(dst + 64 * 144, &mats.m[1], full, x, c_tile * 64);
             } else if constexpr (JOBS) {
@@ -246,7 +280,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
     float* const xs_s = (float*)(smem + a.xs_off);    // [block][TP]
     float* const ssq_s = xs_s + nbq * TP;
     const int items = nbq * T;
-    auto block_of = [&](int i) { return TP == 1 ? i : TP == 2 ? i >> 1 : T == 4 ? i >> 2 : T == 3 ? (i * 21846) >> 16 : T == 2 ? i >> 1 : i; };  // i / T
+    auto block_of = [&](int i) { return TP == 1 ? i : TP == 2 ? i >> 1 : T == 4 ? i >> 2 : T == 3 ? (i * 21846) >> 16 : T == 2 ? i >> 1 : T == 1 ? i : T == 8 ? i >> 3 : T == 7 ? (i * 9363) >> 16 : T == 6 ? (i * 10923) >> 16 : (i * 13108) >> 16; };  // i / T
     auto load = [&](int i) {
         const int lb = block_of(i), tk = i - lb * T, blk = b0 + lb;
         return split_load(a.x + (size_t)(t0 + tk) * a.x_stride + (size_t)blk * 256, a.nw ? a.nw + (size_t)blk * 256 : nullptr, 256, lane);
@@ -282,8 +316,9 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
 #pragma unroll
         for (int h = 0; h < 2; h++)
 #pragma unroll
-            for (int p = 0; p < 3; p++) *(uint32_t*)(b_s + lb * 4096 + h * 2048 + gt_at(3 * tk + p, 4 * lane)) = d.d[h][p];
-        if constexpr (MLX) {
+            for (int p = 0; p < 3; p++) *(uint32_t*)(b_s + lb * (NB * 256) + h * (NB * 128) + gt_at(3 * tk + p, 4 * lane)) = d.d[h][p];
+        if constexpr (Q8) {  // (no offsets: the sums are not needed)
+        } else if constexpr (MLX) {
             const int o = __shfl_xor_sync(0xffffffffu, s, 1);
             if (lane < 8 && (lane & 1) == 0) sum_s[(lb * TP + tk) * 4 + (lane >> 1)] = d.xs * (float)(s + o);
         } else {  // four signed digits (|s| < 2^28), eight bytes of a block's 32; the others are zeros
@@ -304,7 +339,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
 
     if (warp > 1) {
         // ---------------- bytes in, sums out ----------------
-        constexpr uint32_t idesc = (2u << 4) | (MLX ? 1u << 7 : 0u) | (1u << 10) | ((16u >> 3) << 17) | ((128u >> 4) << 24);  // s32 = u8 or s8 x s8, 128 x 16
+        constexpr uint32_t idesc = (2u << 4) | (MLX || Q8 ? 1u << 7 : 0u) | (1u << 10) | ((NB >> 3) << 17) | ((128u >> 4) << 24);  // s32 = u8 or s8 x s8, 128 x 16 or 32
         const int set = (warp - 2) >> 2, w = warp & 3, r = 32 * w + lane;
         const uint32_t at = tmem + ((uint32_t)(32 * w) << 16) + set * GT_SET_COLS;
         const uint32_t base = tmem + set * GT_SET_COLS;
@@ -322,16 +357,18 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
                 ok = __all_sync(0xffffffffu, gt_wait(&sh->raw_full[set][place & (GT_MOST_SLOTS - 1)], (uint32_t)((place / GT_MOST_SLOTS) & 1), sh, a.status));
                 place++;
                 if (!ok) break;
-                const uint4* my = (const uint4*)(smem + (size_t)s * GT_RAW + (size_t)r * 144);
-                const uint4 hd = my[0];
+                const uint8_t* const slot = smem + (size_t)s * RAW;
+                const uint4 hd = *(const uint4*)(slot + (Q8 ? GT_ROWS * 256 + r * 16 : r * 144));  // (Q8_0: eight scales)
                 uint4 q[8];
-                uint32_t words = hd.x;
+                if constexpr (!Q8) {
+                    uint32_t words = hd.x;
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    q[k] = my[1 + k];
-                    words |= q[k].x;
+                    for (int k = 0; k < 8; k++) {
+                        q[k] = *(const uint4*)(slot + r * 144 + 16 + 16 * k);
+                        words |= q[k].x;
+                    }
+                    release_raw(&sh->raw_empty[s], words, a.zero, lane);
                 }
-                release_raw(&sh->raw_empty[s], words, a.zero, lane);
                 int p[TP][3];
                 float f[TP], fl[TP];
 #pragma unroll
@@ -362,7 +399,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
                     if (w == 0) {
                         tc_fence_after();
                         if (elect_one()) {
-                            issue(bd + (uint64_t)((lb * 4096) >> 4));
+                            issue(bd + (uint64_t)((lb * (NB * 256)) >> 4));
                             mma_commit(&sh->d_full[set]);
                         }
                         __syncwarp();
@@ -373,8 +410,41 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
                     phase ^= 1;
                     tc_fence_after();
                 };
-                constexpr int AT_ONCE = TP == 4 ? 2 : 4;  // sums of three digits a token that registers hold at once
-                if constexpr (MLX) {  // a sum per 64 values
+                constexpr int AT_ONCE = TP == 8 ? 1 : TP == 4 ? 2 : 4;  // sums of three digits a token that registers hold at once
+                constexpr int CW = TP == 8 ? 24 : 4 * TP;
+                if constexpr (Q8) {  // a sum per 32, the bytes from where they were copied; 128 columns of sums at a time
+                    constexpr int CHUNKS = NB == 16 ? 8 : 4;
+                    const uint64_t ad = smem_desc_sw128(smem_u32(slot));
+#pragma unroll
+                    for (int k0 = 0; k0 < 8; k0 += CHUNKS) {
+                        multiply([&](uint64_t b) {
+#pragma unroll
+                            for (int k = k0; k < k0 + CHUNKS; k++)
+                                gt_mma_ss(base + NB * (k - k0), ad + (k >> 2) * (GT_ROWS * 128 >> 4) + 2 * (k & 3), b + (k >> 2) * (NB * 128 >> 4) + 2 * (k & 3), idesc);
+                        });
+                        sums();
+                        if (!ok) break;
+                        if (k0 + CHUNKS == 8) release_raw(&sh->raw_empty[s], hd.x, a.zero, lane);
+#pragma unroll
+                        for (int k1 = 0; k1 < CHUNKS; k1 += AT_ONCE) {
+                            int c[AT_ONCE][CW];
+#pragma unroll
+                            for (int k = 0; k < AT_ONCE; k++) gt_ld(at + NB * (k1 + k), c[k]);
+                            gt_ld_wait();
+#pragma unroll
+                            for (int k = 0; k < AT_ONCE; k++) {
+                                const int g = k0 + k1 + k;
+                                const float d = gt_half(g < 2 ? hd.x : g < 4 ? hd.y : g < 6 ? hd.z : hd.w, g & 1);
+#pragma unroll
+                                for (int t = 0; t < TP; t++) {
+                                    f[t] = fmaf(d, (float)c[k][3 * t + 2], f[t]);
+                                    fl[t] = fmaf(d, (float)(256 * c[k][3 * t + 1] + c[k][3 * t]), fl[t]);
+                                }
+                            }
+                        }
+                    }
+                    if (!ok) break;
+                } else if constexpr (MLX) {  // a sum per 64 values
                     expand(0);
                     expand(1);
                     multiply([&](uint64_t b) {
@@ -385,7 +455,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
                     if (!ok) break;
 #pragma unroll
                     for (int g0 = 0; g0 < 4; g0 += AT_ONCE) {
-                        int c[AT_ONCE][4 * TP];
+                        int c[AT_ONCE][CW];
 #pragma unroll
                         for (int g = 0; g < AT_ONCE; g++) gt_ld(at + GT_D + 16 * (g0 + g), c[g]);
                         gt_ld_wait();
@@ -403,7 +473,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
                     auto scaled = [&](uint32_t sc) {
 #pragma unroll
                         for (int k0 = 0; k0 < 4; k0 += AT_ONCE) {
-                            int c[AT_ONCE][4 * TP];
+                            int c[AT_ONCE][CW];
 #pragma unroll
                             for (int k = 0; k < AT_ONCE; k++) gt_ld(at + GT_D + 16 * (k0 + k), c[k]);
                             gt_ld_wait();
@@ -437,7 +507,14 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
                     if (!ok) break;
                     scaled((hd.w & LOW) | ((hd.y >> 2) & 0x30303030u));
                 }
-                if constexpr (MLX) {  // w = (n - 8) d + off per 64: off times the sums of 64
+                if constexpr (Q8) {
+#pragma unroll
+                    for (int t = 0; t < TP; t++) {
+                        const float xs = xs_s[lb * TP + t];
+                        acc[t] = fmaf(xs * 65536.0f, f[t], acc[t]);
+                        low[t] = fmaf(xs, fl[t], low[t]);
+                    }
+                } else if constexpr (MLX) {  // w = (n - 8) d + off per 64: off times the sums of 64
 #pragma unroll
                     for (int t = 0; t < TP; t++) {
                         const float xs = 0.0625f * xs_s[lb * TP + t];
@@ -497,7 +574,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
         bool ok = true;
         if (a.norm) {
             if (lane < GT_CTAS) {  // this part's sums of squares, to every CTA
-                float q[GT_TOKENS] = {};
+                float q[MOST] = {};
 #pragma unroll
                 for (int t = 0; t < TP; t++)
                     for (int lb = 0; lb < nbq && t < T; lb++) q[t] += ssq_s[lb * TP + t];
@@ -574,25 +651,36 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS> mats, const __grid_constant_
     }
 }
 
-bool gt_map(CUtensorMap* m, const WeightDev& w, uint32_t rows) {
+bool gt_encode(CUtensorMap* m, CUtensorMapDataType type, const void* p, size_t width, size_t rows, size_t bytes, uint32_t bw, uint32_t bh, CUtensorMapSwizzle sw) {
     TensorMapEncodeFn enc = tensor_map_encode();
     if (!enc) return false;
-    const cuuint64_t row = w.n_in / 256 * 144;
-    cuuint64_t dims[2] = {row, w.n_out}, strides[1] = {row};
-    cuuint32_t box[2] = {144, rows}, estr[2] = {1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)w.p0, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    cuuint64_t dims[2] = {width, rows}, strides[1] = {bytes};
+    cuuint32_t box[2] = {bw, bh}, estr[2] = {1, 1};
+    return enc(m, type, 2, (void*)p, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool gt_map(CUtensorMap* m, const WeightDev& w, uint32_t rows) {
+    const size_t row = w.n_in / 256 * 144;
+    return gt_encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, w.p0, row, w.n_out, row, 144, rows, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+bool gt_map_bytes(CUtensorMap* m, const WeightDev& w, uint32_t rows) {
+    return gt_encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, w.p0, w.n_in, w.n_out, w.n_in, 128, rows, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+bool gt_map_scales(CUtensorMap* m, const WeightDev& w, uint32_t rows) {
+    return gt_encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, w.p1, w.n_in / 32, w.n_out, w.n_in / 16, 8, rows, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
-constexpr size_t GT_SMEM = 208 * 1024;  // of an SM (beside the static part)
-size_t gt_fixed(size_t K) {  // shared memory beside the ring
+constexpr size_t gt_smem(int tp) { return tp == 8 ? 190 * 1024 : 208 * 1024; }  // of an SM (beside the static part)
+size_t gt_fixed(int fmt, size_t K, int tp) {  // shared memory beside the ring
     const size_t nbq = (K / 256 + GT_CTAS - 1) / GT_CTAS;
-    return 1024 + nbq * 4096 + (nbq + 3) / 4 * 2048 + nbq * GT_TOKENS * 4 * 6;
+    return 1024 + nbq * (tp == 8 ? 8192 : 4096) + (fmt == B2_FMT_Q4_K ? (nbq + 3) / 4 * 2048 : 0) + nbq * (tp == 8 ? 8 : GT_TOKENS) * 4 * 6;
 }
 
-template <bool MLX, bool PAIR, int TP, bool JOBS>
+template <int FMT, bool PAIR, int TP, bool JOBS>
 cudaError_t gt_launch(const WeightDev& w, const WeightDev* up, const GemvTcJob* jobs, int n_jobs, GtArgs a, int sm_count, cudaStream_t st, bool pdl) {
-    GtMats<JOBS> mats;
+    constexpr bool Q8 = FMT == B2_FMT_Q8_0;
+    constexpr uint32_t ROWS = PAIR ? 64 : GT_ROWS;
+    GtMats<JOBS, Q8> mats;
     if constexpr (JOBS) {
         a.tiles = 0;
         for (int j = 0; j < GT_MOST_JOBS; j++) {
@@ -604,17 +692,24 @@ cudaError_t gt_launch(const WeightDev& w, const WeightDev* up, const GemvTcJob* 
             if (j < n_jobs) a.tiles += (int)((job.w->n_out + GT_ROWS - 1) / GT_ROWS);
         }
     } else {
-        if (!gt_map(&mats.m[0], w, PAIR ? 64 : GT_ROWS) || !gt_map(&mats.m[1], PAIR ? *up : w, PAIR ? 64 : GT_ROWS)) return cudaErrorInvalidValue;
-        a.tiles = (int)((w.n_out + (PAIR ? 63 : 127)) / (PAIR ? 64 : 128));
+        for (int u = 0; u < 2; u++) {
+            const WeightDev& m = u && PAIR ? *up : w;
+            if constexpr (Q8) {
+                if (!gt_map_bytes(&mats.m[u], m, ROWS) || !gt_map_scales(&mats.m[2 + u], m, ROWS)) return cudaErrorInvalidValue;
+            } else {
+                if (!gt_map(&mats.m[u], m, ROWS)) return cudaErrorInvalidValue;
+            }
+        }
+        a.tiles = (int)((w.n_out + ROWS - 1) / ROWS);
     }
-    const size_t nbq = (w.n_in / 256 + GT_CTAS - 1) / GT_CTAS, fixed = gt_fixed(w.n_in);
-    a.slots = (int)std::min<size_t>(GT_MOST_SLOTS, (GT_SMEM - fixed) / GT_RAW);
-    a.b_off = (uint32_t)a.slots * GT_RAW;
-    a.min_off = a.b_off + (uint32_t)nbq * 4096;
-    a.sum_off = a.min_off + (uint32_t)((nbq + 3) / 4 * 2048);
+    const size_t nbq = (w.n_in / 256 + GT_CTAS - 1) / GT_CTAS, fixed = gt_fixed(FMT, w.n_in, TP);
+    a.slots = (int)std::min<size_t>(GT_MOST_SLOTS, (gt_smem(TP) - fixed) / gt_raw(FMT));
+    a.b_off = (uint32_t)a.slots * gt_raw(FMT);
+    a.min_off = a.b_off + (uint32_t)nbq * (TP == 8 ? 8192 : 4096);
+    a.sum_off = a.min_off + (uint32_t)(FMT == B2_FMT_Q4_K ? (nbq + 3) / 4 * 2048 : 0);
     a.xs_off = a.sum_off + (uint32_t)(nbq * TP * 16);
-    const size_t smem = fixed + (size_t)a.slots * GT_RAW;
-    auto kern = gemv_tc_kernel<MLX, PAIR, TP, JOBS>;
+    const size_t smem = fixed + (size_t)a.slots * gt_raw(FMT);
+    auto kern = gemv_tc_kernel<FMT, PAIR, TP, JOBS>;
     if (cudaError_t e = ensure_dynamic_smem((const void*)kern, smem, 0); e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GT_THREADS);
@@ -653,11 +748,15 @@ cudaError_t gt_launch(const WeightDev& w, const WeightDev* up, const GemvTcJob* 
     return cudaLaunchKernelEx(&cfg, kern, mats, a);
 }
 
-template <bool MLX, bool PAIR, bool JOBS = false>
-cudaError_t gt_tokens(const WeightDev& w, const WeightDev* up, const GtArgs& a, int sm_count, cudaStream_t st, bool pdl, const GemvTcJob* jobs = nullptr, int n_jobs = 0) {
-    if (a.T == 1) return gt_launch<MLX, PAIR, 1, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
-    if (a.T == 2) return gt_launch<MLX, PAIR, 2, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
-    return gt_launch<MLX, PAIR, 4, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
+template <int FMT, bool PAIR, bool JOBS = false>
+cudaError_t gt_tokens(const WeightDev& w, const WeightDev* up, GtArgs a, int sm_count, cudaStream_t st, bool pdl, const GemvTcJob* jobs = nullptr, int n_jobs = 0) {
+    if constexpr (FMT == B2_FMT_Q8_0) {  // (twice the bytes: a second reading costs more than columns for eight tokens)
+        a.two = 0;
+        if (a.T > GT_TOKENS) return gt_launch<FMT, PAIR, 8, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
+    }
+    if (a.T == 1) return gt_launch<FMT, PAIR, 1, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
+    if (a.T == 2) return gt_launch<FMT, PAIR, 2, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
+    return gt_launch<FMT, PAIR, 4, JOBS>(w, up, jobs, n_jobs, a, sm_count, st, pdl);
 }
 
 GtArgs gt_args(const WeightDev& w, const GemvIn& in, int T) {
@@ -680,9 +779,12 @@ GtArgs gt_args(const WeightDev& w, const GemvIn& in, int T) {
 
 }  // namespace
 
-// By format and K alone: all of a matrix's rows, whatever shard or token they belong to, have to take the same form.
+// By format and K alone: all of a matrix's rows, whatever shard or token they belong to, have to take the same form. (Q8_0 up to 14336 values a row: two slots
+// beside the digits of eight tokens. Q4_K up to 36864, MLX-4 to 41984.)
 bool gemv_tc_supports(const WeightDev& w) {
-    return (w.fmt == B2_FMT_Q4_K || w.fmt == B2_FMT_MLX4) && ((uintptr_t)w.p0 & 15) == 0 && w.n_in % 256 == 0 && w.n_in > 0 && gt_fixed(w.n_in) + 2 * GT_RAW <= GT_SMEM;
+    const int tp = w.fmt == B2_FMT_Q8_0 ? 8 : GT_TOKENS;
+    return (w.fmt == B2_FMT_Q4_K || w.fmt == B2_FMT_MLX4 || (w.fmt == B2_FMT_Q8_0 && ((uintptr_t)w.p1 & 15) == 0)) && ((uintptr_t)w.p0 & 15) == 0 && w.n_in % 256 == 0 &&
+           w.n_in > 0 && gt_fixed(w.fmt, w.n_in, tp) + 2 * gt_raw(w.fmt) <= gt_smem(tp);
 }
 
 cudaError_t launch_gemv_tc(const WeightDev& w, const WeightDev* up, const GemvIn& in, int T, float* y, size_t y_stride, int mode, const float* gate,
@@ -701,8 +803,11 @@ cudaError_t launch_gemv_tc(const WeightDev& w, const WeightDev* up, const GemvIn
         a.mode = mode;
         a.n_out = w.n_out;
         cudaError_t e;
-        if (w.fmt == B2_FMT_MLX4) e = pair ? gt_tokens<true, true>(w, up, a, sm_count, st, pdl) : gt_tokens<true, false>(w, up, a, sm_count, st, pdl);
-        else e = pair ? gt_tokens<false, true>(w, up, a, sm_count, st, pdl) : gt_tokens<false, false>(w, up, a, sm_count, st, pdl);
+        switch (w.fmt) {
+            case B2_FMT_MLX4: e = pair ? gt_tokens<B2_FMT_MLX4, true>(w, up, a, sm_count, st, pdl) : gt_tokens<B2_FMT_MLX4, false>(w, up, a, sm_count, st, pdl); break;
+            case B2_FMT_Q4_K: e = pair ? gt_tokens<B2_FMT_Q4_K, true>(w, up, a, sm_count, st, pdl) : gt_tokens<B2_FMT_Q4_K, false>(w, up, a, sm_count, st, pdl); break;
+            default: e = pair ? gt_tokens<B2_FMT_Q8_0, true>(w, up, a, sm_count, st, pdl) : gt_tokens<B2_FMT_Q8_0, false>(w, up, a, sm_count, st, pdl); break;
+        }
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -712,9 +817,9 @@ cudaError_t launch_gemv_tc_jobs(const GemvTcJob* jobs, int n_jobs, const GemvIn&
     if (n_jobs < 1 || n_jobs > GEMV_TC_JOBS || !in.status || T < 1 || T > 2 * GT_TOKENS) return cudaErrorInvalidValue;
     const WeightDev& w = *jobs[0].w;
     for (int j = 0; j < n_jobs; j++)
-        if (!gemv_tc_supports(*jobs[j].w) || jobs[j].w->fmt != w.fmt || jobs[j].w->n_in != w.n_in) return cudaErrorInvalidValue;
+        if (!gemv_tc_supports(*jobs[j].w) || w.fmt == B2_FMT_Q8_0 || jobs[j].w->fmt != w.fmt || jobs[j].w->n_in != w.n_in) return cudaErrorInvalidValue;
     const GtArgs a = gt_args(w, in, T);
-    return w.fmt == B2_FMT_MLX4 ? gt_tokens<true, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs) : gt_tokens<false, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs);
+    return w.fmt == B2_FMT_MLX4 ? gt_tokens<B2_FMT_MLX4, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs) : gt_tokens<B2_FMT_Q4_K, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs);
 }
 
 }  // namespace b2

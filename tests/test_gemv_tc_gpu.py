@@ -1,4 +1,4 @@
-"""4-bit products of one to eight tokens on the tensor cores (`dmv_*`, `dmvk_*`, src/cuda_decode.cu:139-232) at the edges of their tiles (128 rows, 64 of
+"""4-bit and Q8_0 products of one to eight tokens on the tensor cores (`dmv_*`, `dmvk_*`, src/cuda_decode.cu:139-232) at the edges of their tiles (128 rows, 64 of
 a pair), of the four parts of K and the sets' blocks, and over several rounds of the clusters."""
 import numpy as np
 import pytest
@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(1, 256), (129, 512), (65, 768), (127, 1280), (64, 1024), (300, 5120), (128, 16640), (5000, 1024), (9300, 2560)]
 
 
-@pytest.mark.parametrize("fmt", ["q4_k", "mlx4"])
+@pytest.mark.parametrize("fmt", ["q4_k", "mlx4", "q8_0"])
 @pytest.mark.parametrize("n_out,n_in", SHAPES)
 def test_tiles_parts_and_tokens(backend, fmt, n_out, n_in):
     ref, m = make_pair(fmt, n_out, n_in, 500 + n_in % 97)
@@ -41,7 +41,7 @@ def test_tiles_parts_and_tokens(backend, fmt, n_out, n_in):
         assert np.array_equal(y, ones[:t]), t
 
 
-@pytest.mark.parametrize("fmt", ["q4_k", "mlx4"])
+@pytest.mark.parametrize("fmt", ["q4_k", "mlx4", "q8_0"])
 def test_device_rows_and_row_shards_have_the_whole_matrix_bits(backend, fmt):
     torch = pytest.importorskip("torch")
     n_out, n_in = 700, 2560
