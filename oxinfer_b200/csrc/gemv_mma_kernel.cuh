@@ -170,27 +170,20 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
         const int i_end = GROUPED ? min(my_tiles, max(0, ((seg + 1) * tiles - tile0 + tile_step - 1) / tile_step)) : my_tiles;
         const int b0 = PARTS ? p * (a.part_units * bpu / BPX) : 0, nb = PARTS ? min(xblocks, b0 + a.part_units * bpu / BPX) - b0 : xblocks;
         if ((PARTS || GROUPED) && p > 0) __syncthreads();  // every warp is done with the part before
+        auto block_of = [&](int i) { return TP == 1 ? i : i / T; };
         auto load = [&](int i) {
-            const int b = i / T, tk = i - b * T, k = (b0 + b) * 256;
+            const int b = block_of(i), tk = TP == 1 ? 0 : i - b * T, k = (b0 + b) * 256;
             size_t xr = (size_t)tk;
             if constexpr (GROUPED) xr = gt.gather ? gt.src[row0 + tk] : row0 + tk;
             return split_load(a.x + xr * a.x_stride + k, a.nw ? a.nw + k : nullptr, (int)a.w.n_in - k, lane);
         };
         SplitIn next;
         if (!a.rec && wq < nb * T) next = load(wq);
-        for (int i = wq; i < nb * T; i += WARPS) {
-            const int b = i / T, tk = i - b * T, blk = b0 + b;
+        for (int i = a.rec ? nb * T : wq; i < nb * T; i += WARPS) {
+            const int b = block_of(i), tk = TP == 1 ? 0 : i - b * T, blk = b0 + b;
             uint8_t* f0 = smem + a.frag_off + (size_t)b * (X::BLOCK * TP) + tk * X::TOKEN;
             int s;
             float xs, ssq;
-            if (a.rec) {  // the fragments lie in the record as they lie here; nobody waits for a copy before all are on their way
-                const uint8_t* src = a.rec + (size_t)tk * a.rec_stride + (size_t)blk * X::BLOCK;
-                constexpr int PIECES = X::BLOCK / 16, PER = X::TOKEN / 16;  // pieces of 16 bytes
-                const uint32_t dst = smem0 + a.frag_off + (uint32_t)(b * (X::BLOCK * TP) + tk * X::TOKEN);
-                cp16(dst + (lane / PER) * X::STEP + (lane % PER) * 16, src + lane * 16);
-                if (lane + 32 < PIECES) cp16(dst + ((lane + 32) / PER) * X::STEP + ((lane + 32) % PER) * 16, src + (lane + 32) * 16);
-                continue;
-            }
             {
                 const SplitIn in = next;
                 if (i + WARPS < nb * T) next = load(i + WARPS);
@@ -227,8 +220,19 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
             }
             F::put_sums(smem + a.sums_off + (size_t)(b * TP + tk) * X::SUMS, xs, s, lane);
         }
-        if (a.rec) {  // the scales, and the chunk sums of which every lane takes one
+        // Records: the fragments lie there as they lie here; nobody waits for a copy before all are on their way. (Apart from the other path, whose first
+        // run through its code counts: inside its loop, and with divisions by one token, Q5_K 14336 x 4096 took 12.05 us, this way 11.70.)
+        if (__builtin_expect(a.rec != nullptr, 0)) {
+            for (int i = wq; i < nb * T; i += WARPS) {
+                const int b = block_of(i), tk = TP == 1 ? 0 : i - b * T, blk = b0 + b;
+                const uint8_t* src = a.rec + (size_t)tk * a.rec_stride + (size_t)blk * X::BLOCK;
+                constexpr int PIECES = X::BLOCK / 16, PER = X::TOKEN / 16;  // pieces of 16 bytes
+                const uint32_t dst = smem0 + a.frag_off + (uint32_t)(b * (X::BLOCK * TP) + tk * X::TOKEN);
+                cp16(dst + (lane / PER) * X::STEP + (lane % PER) * 16, src + lane * 16);
+                if (lane + 32 < PIECES) cp16(dst + ((lane + 32) / PER) * X::STEP + ((lane + 32) % PER) * 16, src + (lane + 32) * 16);
+            }
             cp_commit();
+            // the scales, and the chunk sums of which every lane takes one
             constexpr int LANES = F::SUMS ? 8 : 1;
             for (int e0 = wq * 32; e0 < nb * T * LANES; e0 += THREADS) {
                 const int i = (e0 + lane) / LANES, sub = lane % LANES, at = min(i, nb * T - 1), b = at / T, tk = at - b * T, blk = b0 + b;
