@@ -210,7 +210,7 @@ def gemv_extras(be, torch, peaks, steps, only=None, use_graph=True):
         out[name] = {"us_per_gemv": us, "bytes": algo, "gbs": algo / us / 1e3, "frac_of_hbm_peak": algo / us / 1e3 / peaks["hbm_gbs"],
                      "launches_per_gemv": 1, "timing": timing}
         traffic, commit = profiled_traffic(f"gemv_{name}.txt")
-        out[name]["roofline"] = {"kernel": "gemv_mma_kernel (one matrix-vector product)",
+        out[name]["roofline"] = {"kernel": ("gemv_tc_kernel" if name.startswith(("mlx4", "q4_k", "q8_0")) else "gemv_mma_kernel") + " (one matrix-vector product)",
                                  "bound": "hbm", "achieved": algo / us / 1e3, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                                  "frac": algo / us / 1e3 / peaks["hbm_gbs"], "frac_of_nominal_8000": algo / us / 1e3 / 8000.0, "traffic": traffic,
                                  "traffic_unit": f"bytes per product, from profiles/gemv_{name}.txt" + (f" captured at {commit}" if commit else ""),

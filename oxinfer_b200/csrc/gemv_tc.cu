@@ -15,8 +15,8 @@
 // Q8_0 rows are bytes already: the instructions read them where the copies put them (two swizzled tiles of 128 k and the rows' scales), and a set's warps
 // only scale the sums (f32, per 32). Eight tokens are 32 columns then: read twice, the bytes would pass at L2's rate.
 //
-// What bounds it: HBM on large matrices, the start on small ones. The form on mma.sync (gemv_mma.cu) issued 276 warp instructions for 4096 weights (one
-// token; 367: four) and was bound by that; this one about 110 (four: 150). Of the 4.7 us of 4096 x 4096, 0.5 pass before the first copy is issued, 1.5 until
+// What bounds it: HBM on large matrices, the start on small ones. The form on mma.sync (gemv_mma.cu) was bound by instructions: 393 of a warp
+// for 4096 weights (Q4_K 14336 x 4096, one token, ncu, everything counted); here it is 225, of which the bytes, the sums and the scales are about 110. Of the 4.7 us of 4096 x 4096, 0.5 pass before the first copy is issued, 1.5 until
 // activations and weights are there, and 2 between them and the result, most of it the first fetch of each line of code: hence short code, no divisions, a pass of the
 // results' loop that stores nothing. Four sets and the whole of tensor memory: two sets in half of an SM (two CTAs) left 4096 x 14336, four tokens, at 21 us.
 // One launch after another in a stream, us, one / two / four / eight tokens, on mma.sync and here:
