@@ -7,7 +7,7 @@
 // A cluster of four CTAs takes tiles of 128 rows, CTA q the blocks q n / 4 .. of K, so the order of a row's sum depends on K alone: a
 // row shard and every row of a step of several tokens have the bits of the one-token product. A CTA:
 //   warp 0        : copies packed rows (128 x 144 bytes a block of 256 k) into a ring, filled before the kernel waits for the one ahead.
-//   warps 2 .. 17 : four sets of four, a thread a row; set s takes the CTA's blocks s, s + 4, .. of a tile: nibbles to bytes in tensor memory, the
+//   warps 2 .. 17 : four sets of four, a thread a row; set s takes the blocks s, s + 4, .. of those that the CTA has of all its tiles: nibbles to bytes in tensor memory, the
 //                   instructions, the sums back and times the scales. At the end of a tile its sums go to the CTA of the cluster that owns the rows.
 //   warp 1        : adds the sixteen sums of its rows in pairs, applies the norm's factor and the output mode, and stores.
 // All but warp 0 split the CTA's part of the activations first (an RMS norm's weights multiply before the split, its factor the results).
@@ -29,7 +29,7 @@
 //   Q8_0  4096 x 4096    6.3 / 8.7 / 9.6 / 16.9    5.2 / 5.6 / 8.0 / 9.2
 //         4096 x 14336  15.0 / 24.3 / 28.4 / 42.1  13.0 / 14.6 / 16.2 / 24.5
 //         32064 x 4096  23.9 / 27.0 / 28.1 / 54.5  23.3 / 24.6 / 24.6 / 28.0
-// (6144 x 4096, MLX-4, one token: 5.9 and 6.3: its 48 tiles take two rounds of 24 clusters. In a graph 4096 x 4096 takes 4.5 and 4.4.)
+// (One token of short rows is slower than on mma.sync: Q4_K 14336 x 1024 5.1 and 6.2 us. 6144 x 4096, MLX-4, one token: 5.9 and 6.3: its 48 tiles take two rounds of 24 clusters. In a graph 4096 x 4096 takes 4.5 and 4.4.)
 // Largest error of a result against 64 bits, in parts of the row's norm, N(0, 1) activations, K = 1024 / 4096 / 14336:
 // Q4_K 1.60 / 1.70 / 1.71e-7 on mma.sync, 1.60 / 1.65 / 1.66e-7 here; MLX-4 1.78 / 2.07 / 2.39e-7 and 1.57 / 1.65 / 1.59e-7;
 // Q8_0 1.67 / 1.72 / 1.79e-7 and 1.67 / 1.69 / 1.73e-7.
@@ -233,13 +233,15 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
         return j;
     };
     // warp 0: the next block goes to slot c_slot: block c_blk of tile c_tile
-    int c_slot = 0, c_blk = 0, c_tile = cluster, c_round = 0;
-    auto place_of = [&](int round, int blk) { return round * ((nbq - (blk & 3) + 3) >> 2) + (blk >> 2); };  // among the blocks of its set
+    int c_slot = 0, c_blk = 0, c_tile = cluster, c_n = 0;
+    auto full_of = [&](int n) { return &sh->raw_full[n & 3][(n >> 2) & (GT_MOST_SLOTS - 1)]; };  // block n: set n % 4, its n / 4th
+    auto full_parity = [&](int n) { return (uint32_t)(n >> 5) & 1; };
+    static_assert(GT_SETS == 4 && GT_MOST_SLOTS == 8, "full_of, full_parity");
     auto copy = [&] {
         if (elect_one()) {
             const int x = (b0 + c_blk) * (Q8 ? 256 : 144);
             uint8_t* dst = smem + (size_t)c_slot * RAW;
-            uint64_t* const full = &sh->raw_full[c_blk & 3][place_of(c_round, c_blk) & (GT_MOST_SLOTS - 1)];
+            uint64_t* const full = full_of(c_n);
             mbar_arrive_expect_tx(full, RAW);
             if constexpr (Q8) {  // two swizzled tiles of 128 k and the rows' eight scales; a pair's matrices 64 rows each
 #pragma unroll
@@ -260,11 +262,11 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
             }
         }
         __syncwarp();
+        c_n++;
         if (++c_slot == a.slots) c_slot = 0;
         if (++c_blk == nbq) {
             c_blk = 0;
             c_tile += clusters;
-            c_round++;
         }
     };
     const int first = min(total, a.slots);
@@ -345,17 +347,19 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
         const uint32_t base = tmem + set * GT_SET_COLS;
         const uint64_t bd = smem_desc_sw128(smem_u32(b_s)), md = smem_desc_sw128(smem_u32(min_s));
         uint32_t phase = 0;
-        int s = 0, at_n = 0, place = 0;  // the slot of block at_n; the next block among this set's
+        int s = 0, at_n = 0;  // the slot of block at_n
         bool ok = true;
         for (int i = 0; i < my_tiles && ok; i++) {
             float acc[TP], low[TP];  // the third digit's share, the others'
 #pragma unroll
             for (int t = 0; t < TP; t++) acc[t] = low[t] = 0.0f;
-            for (int lb = set; lb < nbq && ok; lb += GT_SETS) {
+            // Block n of the CTA belongs to set n % 4, so that short parts of K keep all four busy (28672 x 2048, one token, Q4_K: by the block in the tile
+            // 12.5 us, this way 10.3); the sums go by the block in the tile.
+            const int share = (set - i * nbq) & 3;
+            for (int lb = share; lb < nbq && ok; lb += GT_SETS) {
                 const int n = i * nbq + lb;
                 for (s += n - at_n, at_n = n; s >= a.slots;) s -= a.slots;
-                ok = __all_sync(0xffffffffu, gt_wait(&sh->raw_full[set][place & (GT_MOST_SLOTS - 1)], (uint32_t)((place / GT_MOST_SLOTS) & 1), sh, a.status));
-                place++;
+                ok = __all_sync(0xffffffffu, gt_wait(full_of(n), full_parity(n), sh, a.status));
                 if (!ok) break;
                 const uint8_t* const slot = smem + (size_t)s * RAW;
                 const uint4 hd = *(const uint4*)(slot + (Q8 ? GT_ROWS * 256 + r * 16 : r * 144));  // (Q8_0: eight scales)
@@ -549,7 +553,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
             const int buf = i & 1, to = PAIR ? 2 * (w & 1) + (lane >> 4) : w, row = PAIR ? 16 * (w >> 1) + (lane & 15) : lane;
             if (i >= 2) ok = __all_sync(0xffffffffu, gt_wait(&sh->in_free[to][buf], (uint32_t)(((i >> 1) - 1) & 1), sh, a.status));
             if (!ok) break;
-            gt_send(cluster_addr(&sh->in[buf][GT_SETS * rank + set][row][0], to), acc, cluster_addr(&sh->in_full[buf], to));
+            gt_send(cluster_addr(&sh->in[buf][GT_SETS * rank + share][row][0], to), acc, cluster_addr(&sh->in_full[buf], to));
         }
     } else if (warp == 0) {
         // ---------------- packed weights ----------------
@@ -562,10 +566,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
             copy();
         }
         if (sh->abort_flag)  // copies in flight land before the shared memory goes away
-            for (int n = max(0, issued - a.slots); n < issued; n++) {
-                const int round_n = n / nbq, blk = n - round_n * nbq, at = place_of(round_n, blk);
-                gt_wait(&sh->raw_full[blk & 3][at & (GT_MOST_SLOTS - 1)], (uint32_t)((at / GT_MOST_SLOTS) & 1), sh, a.status, false);
-            }
+            for (int n = max(0, issued - a.slots); n < issued; n++) gt_wait(full_of(n), full_parity(n), sh, a.status, false);
     } else if (warp == 1) {
         // ---------------- results ----------------
         float factor[TP];
