@@ -349,6 +349,9 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
         uint32_t phase = 0;
         int s = 0, at_n = 0;  // the slot of block at_n
         bool ok = true;
+        // How often the set's warps have met, MEETS times a block. (MLX-4 works it out where a wait gives up: counted, four tokens took 1 % longer.)
+        int met = 0;
+        constexpr int MEETS = MLX || (Q8 && NB == 16) ? 1 : 2;
         for (int i = 0; i < my_tiles && ok; i++) {
             float acc[TP], low[TP];  // the third digit's share, the others'
 #pragma unroll
@@ -360,7 +363,10 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
                 const int n = i * nbq + lb;
                 for (s += n - at_n, at_n = n; s >= a.slots;) s -= a.slots;
                 ok = __all_sync(0xffffffffu, gt_wait(full_of(n), full_parity(n), sh, a.status));
-                if (!ok) break;
+                if (!ok) {
+                    if constexpr (MLX) met = n >> 2;
+                    break;
+                }
                 const uint8_t* const slot = smem + (size_t)s * RAW;
                 const uint4 hd = *(const uint4*)(slot + (Q8 ? GT_ROWS * 256 + r * 16 : r * 144));  // (Q8_0: eight scales)
                 uint4 q[8];
@@ -400,6 +406,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
                     gt_st_wait();
                     tc_fence_before();
                     asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");
+                    if constexpr (!MLX) met++;
                     if (w == 0) {
                         tc_fence_after();
                         if (elect_one()) {
@@ -456,7 +463,10 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
                         for (int k = 0; k < 8; k++) gt_mma(base + GT_D + 16 * (k >> 1), base + 8 * k, b + (k >> 2) * 128 + 2 * (k & 3), idesc, k & 1);
                     });
                     sums();
-                    if (!ok) break;
+                    if (!ok) {
+                        met = (n >> 2) + 1;
+                        break;
+                    }
 #pragma unroll
                     for (int g0 = 0; g0 < 4; g0 += AT_ONCE) {
                         int c[AT_ONCE][CW];
@@ -552,8 +562,18 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
             for (int t = 0; t < TP; t++) acc[t] += low[t];
             const int buf = i & 1, to = PAIR ? 2 * (w & 1) + (lane >> 4) : w, row = PAIR ? 16 * (w >> 1) + (lane & 15) : lane;
             if (i >= 2) ok = __all_sync(0xffffffffu, gt_wait(&sh->in_free[to][buf], (uint32_t)(((i >> 1) - 1) & 1), sh, a.status));
-            if (!ok) break;
+            if (!ok) {
+                if constexpr (MLX) met = (i * nbq + nbq - set + 3) >> 2;
+                break;
+            }
             gt_send(cluster_addr(&sh->in[buf][GT_SETS * rank + share][row][0], to), acc, cluster_addr(&sh->in_full[buf], to));
+        }
+        // A warp whose wait gave up still meets the others wherever they will be waiting for it, in all of the set's blocks; and the one that issues stays
+        // until the last instructions have ended.
+        if (!ok) {
+            if (w == 0 && met > 0) gt_wait(&sh->d_full[set], (uint32_t)(met - 1) & 1, sh, a.status, false);
+            const int meets = MEETS * ((total - set + 3) >> 2);
+            for (; met < meets; met++) asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");
         }
     } else if (warp == 0) {
         // ---------------- packed weights ----------------
