@@ -353,8 +353,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
             next_slot();
             const float sa = reduce8<R>(a, l8), sb = reduce8<R>(b, l8);
             const uint32_t ka = key0 + (lane >> 3), kb = ka + 4;
-            const bool see_a = ka <= my_pos && ka < len && (p.window == 0 || ka + p.window > my_pos);
-            const bool see_b = kb <= my_pos && kb < len && (p.window == 0 || kb + p.window > my_pos);
+            const bool see_a = ka <= my_pos && ka < len && (p.window == 0 || my_pos - ka < p.window);
+            const bool see_b = kb <= my_pos && kb < len && (p.window == 0 || my_pos - kb < p.window);
             float mx = fmaxf(see_a ? sa : -INFINITY, see_b ? sb : -INFINITY);
             mx = fmaxf(mx, shfl_x(mx, 8));
             mx = fmaxf(mx, shfl_x(mx, 16));
