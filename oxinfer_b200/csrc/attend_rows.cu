@@ -256,6 +256,8 @@ attend_rows_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
             }
             if (ok && i + 1 < n) scores(s1);
         }
+        // (a share without keys: its sums, zeros, take the queries' place, which other warps may still be writing)
+        if (n == 0) mbar_wait(&sh->q_full, 0, sh, a.status, 65, 0);
         if (elect_one()) mma_commit(&sh->o_full);
         __syncwarp();
         if (n > 0 && w < tiles && !ok) mbar_wait(&sh->o_full, 0, sh, a.status, 70, 0, false);
@@ -310,7 +312,7 @@ attend_rows_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
             for (int h = 0; h < 4; h++) ar_ld32(s_at + 32 * h, v[h]);
             ar_ld_wait();
             const uint32_t j0 = (t_first + i) * AR_TILE;
-            if (j0 + AR_TILE - 1 > tile_qp || (a.window != 0 && j0 + a.window <= tile_end)) {  // some row does not see some key
+            if (j0 + AR_TILE - 1 > tile_qp || (a.window != 0 && tile_end >= j0 && tile_end - j0 >= a.window)) {  // some row does not see some key
                 const uint32_t hi = qp >= j0 ? min(qp - j0 + 1, (uint32_t)AR_TILE) : 0u, from = my_lo > j0 ? my_lo - j0 : 0u;  // keys from .. hi - 1 of the tile
                 auto below = [](uint32_t n, int h) { return n >= 32u * h + 32 ? 0xffffffffu : n <= 32u * h ? 0u : (1u << (n - 32 * h)) - 1; };  // a bit per key below n
 #pragma unroll

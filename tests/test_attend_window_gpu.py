@@ -1,4 +1,4 @@
-"""Sliding windows in the attentions (`dattn`, src/cuda_decode.cu:396-536; `attention_ext`, src/model.rs:2214-2309)
+"""Sliding windows, and rows that are not finite, in the attentions (`dattn`, src/cuda_decode.cu:396-536; `attention_ext`, src/model.rs:2214-2309)
 against 64 bits. The graphs hold nothing but RoPE and attention; the factors are cos 1 and sin 0, so a step's input is its queries, keys and values."""
 import numpy as np
 import pytest
@@ -80,4 +80,23 @@ def test_prefill_with_windows_and_shares_of_the_keys(backend, nh, nkv, hd, windo
         got, _ = pre.step_multi(pos, x, cs, want_logits=False)
         # (queries, keys, values and probabilities rounded to f16: the bound of a prefill step)
         assert row_err(got, reference(nh, nkv, hd, window, k, v, x)) < 2e-3, (pos, t)
+    pre.close()
+
+
+def test_a_share_without_keys_adds_nothing_whatever_the_queries_hold(backend):
+    """Nine key tiles in four shares: the last has none. Its sums are zeros in the place of its copy of the queries."""
+    nh, nkv, hd, pos, t = 8, 1, 128, 1100, 33
+    pre = D.decode_plan_prefill(backend, graph(nh, nkv, hd, 0), 1200, 64)
+    k, v, x, cs = inputs(nh, nkv, hd, pos, t, 70)
+    pre.kv_write(0, 0, k, v)
+    clean, _ = pre.step_multi(pos, x, cs, want_logits=False)
+    for token, head in ((0, 0), (5, 3), (15, 7), (32, 0)):
+        bad = x.copy()
+        bad[token, head * hd:(head + 1) * hd] = np.nan
+        for _ in range(20):
+            got, _ = pre.step_multi(pos, bad, cs, want_logits=False)
+            own = np.zeros((t, nh), bool)
+            own[token, head] = True
+            rows = np.isnan(got.reshape(t, nh, hd)).all(-1)
+            assert np.array_equal(rows, own) and np.array_equal(got.reshape(t, nh, hd)[~own], clean.reshape(t, nh, hd)[~own])
     pre.close()
