@@ -237,10 +237,14 @@ int b2_prepare_x_dev(b2_ctx* ctx, const float* x_dev, size_t n_in);
 int b2_matvec_prepared_dev(b2_ctx* ctx, b2_weight w, b2_weight up, const float* x_dev, float* y_dev, int mode, const float* gate_dev);
 
 /* After the caller has synchronized the stream: B2_OK, or B2_ERR_TIMEOUT when a device-side wait of
- * the tensor-core GEMM ran into its time limit (the kernel then returned early and its output is
+ * a product ran into its time limit (the kernel then returned early and its output is
  * not valid). The reference logs a failed launch and returns false (src/cuda.rs:625-628); this is
  * the same report for the device-resident calls, which do not synchronize themselves. */
 int b2_check_status(b2_ctx* ctx);
+/* For tests of a host program's handling of such failures (no counterpart in the reference): leaves, from the host, the mark that a
+ * wait leaves when it gives up, and launches nothing. The next call on ctx that looks (b2_matmul, b2_matvec_rows, b2_check_status), or, with a
+ * plan, that plan's next step, returns B2_ERR_TIMEOUT; the one behind it is as ever. */
+int b2_inject_timeout(b2_ctx* ctx, uint64_t plan);
 
 /* ---- decode plan: one token's whole forward pass in one submission ---------------------------
  * Mirrors gpu::decode (src/gpu_decode.rs): the model describes a token as a list of ops over

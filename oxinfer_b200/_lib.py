@@ -110,6 +110,7 @@ _SIGNATURES = {
     "b2_matmul_dev": (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p, C.c_int, C.c_size_t, C.c_void_p, C.c_int]),
     "b2_matvec_dev": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint64, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p]),
     "b2_check_status": (C.c_int, [C.c_void_p]),
+    "b2_inject_timeout": (C.c_int, [C.c_void_p, C.c_uint64]),
     "b2_upload_moe": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_size_t, C.c_size_t, C.POINTER(C.c_uint64)]),
     "b2_upload_moe_ex": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_size_t, C.c_size_t, C.c_int, C.c_float,
                          C.POINTER(C.c_uint64)]),

@@ -207,6 +207,10 @@ class Backend:
     def check_status(self) -> None:
         self._check(self._L.b2_check_status(self._ctx))
 
+    def inject_timeout(self, plan=None) -> None:
+        """The next call that looks (or the plan's next step) finds the mark of a wait that gave up (``b2_inject_timeout``)."""
+        self._check(self._L.b2_inject_timeout(self._ctx, plan.handle if plan is not None else 0))
+
     # -- the trait ----------------------------------------------------------------------------
     def wants(self, n_out: int, n_in: int, t: int) -> bool:
         return bool(self._L.b2_wants(self._ctx, n_out, n_in, t))

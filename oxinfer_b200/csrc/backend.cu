@@ -87,6 +87,7 @@ class Backend {
     static constexpr size_t HOST_STAGE = 256 * 1024;
     uint8_t* host_stage = nullptr;
     bool stage_busy = false;  // a call that failed half-way may have left a copy from it in flight
+    cudaEvent_t stage_full[2] = {};  // the halves of [y] in turn, for results that do not fit (parts_out)
     GemmStatus* gemm_status = nullptr;  // device
     uint32_t* wait_status = nullptr;    // page-locked: the products of a few tokens write it when a bounded wait gives up; 64 bytes on, a copy of *gemm_status
     // cached tensor maps of the tensor-core GEMM (see matmul_dev)
@@ -739,6 +740,41 @@ class Backend {
         return B2_OK;
     }
 
+    // Larger results through the stage's two halves in turn: while the host copies a part to y, the next one is on its way. The first part has
+    // come behind every kernel, so the status word is final before y is touched, and no synchronize stands between the kernels and the copies.
+    template <typename Job>
+    int parts_out(const Job* jobs, size_t n_jobs, size_t t, const std::vector<size_t>& y_off, size_t y_total, const char* what) {
+        constexpr size_t PART = HOST_STAGE / 2;
+        uint8_t* const ys = host_stage + HOST_STAGE;
+        const size_t parts = (y_total + PART - 1) / PART;
+        cudaError_t e = cudaSuccess;
+        for (int h = 0; h < 2 && e == cudaSuccess; h++)
+            if (!stage_full[h]) e = cudaEventCreateWithFlags(&stage_full[h], cudaEventDisableTiming);
+        auto ask = [&](size_t p) {
+            const size_t at = p * PART, n = std::min(PART, y_total - at);
+            e = cudaMemcpyAsync(ys + p % 2 * PART, (const uint8_t*)y_dev.p + at, n, cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaEventRecord(stage_full[p % 2], stream);
+        };
+        for (size_t p = 0; p < std::min<size_t>(2, parts) && e == cudaSuccess; p++) ask(p);
+        int rc = B2_OK;
+        size_t j = 0;
+        for (size_t p = 0; p < parts && e == cudaSuccess && !rc; p++) {
+            if ((e = cudaEventSynchronize(stage_full[p % 2])) != cudaSuccess) break;
+            if (p == 0 && (rc = check_wait_status())) break;
+            const size_t from = p * PART, to = std::min(from + PART, y_total);
+            for (;; j++) {  // the jobs with results in this part
+                const size_t a = std::max(from, y_off[j]), z = std::min(to, y_off[j] + t * jobs[j].n_out * 4);
+                if (a < z) std::memcpy((uint8_t*)jobs[j].y + (a - y_off[j]), ys + p % 2 * PART + (a - from), z - a);
+                if (j + 1 == n_jobs || y_off[j + 1] >= to) break;
+            }
+            if (p + 2 < parts) ask(p + 2);
+        }
+        if (rc || e != cudaSuccess) cudaStreamSynchronize(stream);  // (a part may still be on its way to the stage)
+        if (e != cudaSuccess) return cuda_fail(e, what);
+        stage_busy = false;
+        return rc;
+    }
+
     // ---- Backend::matmul (src/cuda.rs:1428-1493)
     int matmul(const float* x, size_t t, size_t n_in, b2_job* jobs, size_t n_jobs) {
         if (t == 0 || n_jobs == 0) return B2_OK;
@@ -874,15 +910,18 @@ class Backend {
                 return rc;
             }
         }
-        // Every launch was accepted (a refused one returned above, before any y is touched): small results follow the kernels on
-        // the stream to page-locked memory and the call synchronizes once; the copies of large ones are queued behind the kernels (a
-        // synchronize in front of them costs 14 us of 300), so that a wait that ran out shows when they have been written: the call still
-        // fails then. The kernels' and the copies' time are booked together as kernel time.
+        // Every launch was accepted (a refused one returned above, before any y is touched): the results follow the kernels on
+        // the stream to page-locked memory, small ones whole and the call synchronizes once, large ones in parts. (A synchronize between the kernels and
+        // copies to y itself costs 14 us of 300.) The kernels' and the copies' time are booked together as kernel time.
+        const char* const what = "matvec_rows kernels / copy-out";
         if (staged(y_total)) {
-            if (int rc = staged_out(jobs, n_jobs, t, y_off, y_total, in_place, "matvec_rows kernels / copy-out")) return rc;
+            if (int rc = staged_out(jobs, n_jobs, t, y_off, y_total, in_place, what)) return rc;
+        } else if (stage_host()) {
+            if (int rc = parts_out(jobs, n_jobs, t, y_off, y_total, what)) return rc;
         } else {
-            if ((e = copy_out(jobs, n_jobs, t, y_off)) != cudaSuccess) return cuda_fail(e, "matvec_rows kernels / copy-out");
+            if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(e, what);
             if (int rc = check_wait_status()) return rc;
+            if ((e = copy_out(jobs, n_jobs, t, y_off)) != cudaSuccess) return cuda_fail(e, what);
         }
         ns_gpu += since(t1);
         calls++;
@@ -1574,6 +1613,10 @@ class Backend {
         xapart.release();
         if (host_stage) cudaFreeHost(host_stage);
         host_stage = nullptr;
+        for (cudaEvent_t& ev : stage_full) {
+            if (ev) cudaEventDestroy(ev);
+            ev = nullptr;
+        }
         xrec.release();
         if (gemm_status) cudaFree(gemm_status);
         gemm_status = nullptr;
@@ -1807,11 +1850,22 @@ B2_EXPORT int b2_matvec_prepared_dev(b2_ctx* ctx, b2_weight w, b2_weight up, con
     return ctx->be.matvec_prepared(w, up, x_dev, y_dev, mode, gate_dev);
 }
 
-// Reads (and clears) the status word of the tensor-core GEMM after the caller synchronized the
-// stream: B2_OK, or B2_ERR_TIMEOUT with the place where a bounded device wait gave up.
+// Reads (and clears) the status words of the products after the caller synchronized the
+// stream: B2_OK, or B2_ERR_TIMEOUT where a bounded device wait gave up.
 B2_EXPORT int b2_check_status(b2_ctx* ctx) {
     LOCKED(ctx);
     return ctx->be.check_gemm_status();
+}
+
+B2_EXPORT int b2_inject_timeout(b2_ctx* ctx, b2_plan plan) {
+    LOCKED(ctx);
+    if (!plan) {
+        *(volatile uint32_t*)ctx->be.wait_status = 2u;
+        return B2_OK;
+    }
+    b2::DecodePlanImpl* p = ctx->be.find_plan(plan);
+    if (!p) return ctx->be.fail(B2_ERR_ARG, "[b200qmm: inject_timeout: unknown plan]");
+    return p->inject_timeout(ctx->be.err);
 }
 
 B2_EXPORT int b2_comm_unique_id(void* id_out) {

@@ -844,6 +844,12 @@ int DecodePlanImpl::capture(cudaStream_t st, bool with_head, cudaGraphExec_t* ou
     return B2_OK;
 }
 
+int DecodePlanImpl::inject_timeout(std::string& err) {
+    const uint32_t s = 2;
+    PLAN_CUDA(cudaMemcpy(status_, &s, 4, cudaMemcpyHostToDevice), "cudaMemcpy(status)");
+    return B2_OK;
+}
+
 int DecodePlanImpl::check_status(std::string& err) {
     uint32_t s = 0;
     PLAN_CUDA(cudaMemcpy(&s, status_, 4, cudaMemcpyDeviceToHost), "cudaMemcpy(status)");

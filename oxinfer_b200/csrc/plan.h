@@ -41,6 +41,7 @@ class DecodePlanImpl {
     int attach_peers(uint32_t rank, uint32_t world, const void* handles, std::string& err);
     uint64_t launches_per_step() const { return prefill_ ? prefill_launches_ : launches_; }
     uint64_t launches_per_step(size_t t) const { return prefill_ ? prefill_launches_ : t >= 2 && t <= 4 ? multi_launches_[t] : launches_; }
+    int inject_timeout(std::string& err);  // the status word as a kernel whose wait gives up leaves it
     bool uses_weight(uint64_t h) const;
 
   private:
