@@ -4,7 +4,8 @@
 // A cluster of CTAs takes up to four rows (query heads of one KV head, of one or several of the step's tokens) over all keys. Tile t of
 // 64 keys belongs to part t % 16, keys 8 w .. 8 w + 7 of a tile to warp w, so the division depends on the absolute position of a key alone, and a
 // row's sums are the same whatever rows stand beside it (keys that it may not see do not enter them). A cluster has 16 CTAs, a part each, while
-// no more than 14 of them are wanted, which is what the chip holds at two CTAs an SM (seven at one); otherwise eight, two parts each.
+// no more than 14 of them are wanted, which is what the chip holds at two CTAs an SM (seven at one); otherwise eight, two parts each. Over long caches
+// several clusters share a KV head's keys, 1024 at a time in turn (attend_shares); the last to finish adds their sums.
 // Every warp runs on its own: a ring of batches of eight keys or values in shared memory (bulk copies, started before the kernel waits for the one
 // ahead: those rows were written by earlier steps), a running softmax, and no CTA barrier between batches. The warps' sums are added in
 // shared memory, every CTA stores them into the CTAs of the cluster, a share of the outputs to each, and those add them, in a fixed order.
@@ -35,6 +36,8 @@ constexpr int ATT_BATCH = 8;                        // keys a warp takes at a ti
 constexpr int ATT_TILE = ATT_WARPS * ATT_BATCH;     // keys
 constexpr int ATT_MOST_ROWS = 4;
 constexpr int ATT_PARTS = 16;                       // of the keys
+constexpr int ATT_SPAN = ATT_PARTS * ATT_TILE;      // keys: a tile of every part
+constexpr int ATT_MOST_SHARES = 16;
 
 template <int HD, int R, typename T>
 struct AttShared {  // bytes
@@ -190,16 +193,33 @@ struct Turn {
     }
 };
 
-// Grid (C, KV heads, groups of R rows), a cluster along x. Row r of a KV head: query head r % G of token r / G. sp[0]: the position of the step's first token.
+// Clusters that share a KV head's keys: 1 << log of them, span j of the keys to cluster j % shares.
+struct AttShares {
+    int log;
+    uint32_t groups, groups_inv;  // ceil(2^16 / groups)
+    float4* part;      // [unit][share][4 outputs]{sums, {largest score, denominator, -, -}}
+    uint32_t* counts;  // [unit][CTA], zero
+};
+
+// Grid (C, KV heads, shares x groups of R rows), a cluster along x. Row r of a KV head: query head r % G of token r / G. sp[0]: the position of the step's first token.
 template <int HD, int R, typename T>
 __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __restrict__ q, T* kc, T* vc, float* __restrict__ out,
                                                                 const uint32_t* __restrict__ sp, DecAttn p, uint32_t* status, FusedRope fr, AttnTokens at,
-                                                                int g_log) {
+                                                                int g_log, AttShares sh) {
     using L = AttShared<HD, R, T>;
     constexpr int V = HD / 32, S = L::SLOTS;
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_launch_dependents();
     const uint32_t pos0 = sp[0], table0 = sp[1];
+    const uint32_t C = gridDim.x, c = blockIdx.x, kvh = blockIdx.y, my_share = blockIdx.z * sh.groups_inv >> 16, group = blockIdx.z - my_share * sh.groups, row0 = group * R;
+    const uint32_t all = (uint32_t)max(1, at.n) << g_log, g_mask = (1u << g_log) - 1;
+    const uint32_t tok_a = row0 >> g_log, tok_z = (min(row0 + R, all) - 1) >> g_log;  // the group's tokens
+    const uint32_t len = min(pos0 + tok_z + 1, p.max_len);                            // keys below len are seen by some row
+    const uint32_t lo = p.window != 0 && pos0 + tok_a + 1 > p.window ? pos0 + tok_a + 1 - p.window : 0;
+    const uint32_t span0 = lo / ATT_SPAN, spans = (len - 1) / ATT_SPAN + 1 - span0, shares_mask = (1u << sh.log) - 1;
+    __shared__ uint32_t active_s[1];  // shares that have keys
+    if (((my_share - span0) & shares_mask) >= spans) return;
+    if (threadIdx.x == 0) *active_s = min(spans, shares_mask + 1);
     constexpr int F4_LOG = L::F4 == 16 ? 4 : L::F4 == 32 ? 5 : L::F4 == 64 ? 6 : 7;
     static_assert(L::F4 == 1u << F4_LOG);
     const uint32_t share_log = F4_LOG - (gridDim.x == 16 ? 4 : 3), share = 1u << share_log;  // of the outputs
@@ -212,8 +232,6 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
     __syncwarp();
     cluster_arrive();  // (the CTAs store into one another's shared memory: all of them have to be there)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, l8 = lane & 7;
-    const uint32_t C = gridDim.x, c = blockIdx.x, kvh = blockIdx.y, row0 = blockIdx.z * R;
-    const uint32_t all = (uint32_t)max(1, at.n) << g_log, g_mask = (1u << g_log) - 1;
     uint8_t* const ring = smem + warp * L::RING;
     float* const qs = (float*)(smem + L::Q);                                // [R][HD]
     float* const pw = (float*)(smem + L::P) + warp * (ATT_BATCH + 1) * 4;   // the warp's probabilities [key][4], and what its sums shrink by
@@ -225,18 +243,19 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
     T* const own = (T*)(smem + L::OWN);                                     // the step's own keys and values [token][k | v][HD]
     uint64_t* const bars = (uint64_t*)(smem + L::BARS) + warp * S;
 
-    const uint32_t tok_a = row0 >> g_log, tok_z = (min(row0 + R, all) - 1) >> g_log;  // the group's tokens
-    const uint32_t len = min(pos0 + tok_z + 1, p.max_len);                            // keys below len are seen by some row
     const bool fused = fr.qkv != nullptr;
     const float q_scale = p.scale * 1.44269504f;  // scores in powers of two
     const uint32_t first_pos = pos0 + tok_a, last_pos = pos0 + tok_z;
     const uint32_t lo_all = p.window != 0 && last_pos + 1 > p.window ? last_pos + 1 - p.window : 0;  // keys from here to first_pos are seen by every row
-    const uint32_t lo = p.window != 0 && pos0 + tok_a + 1 > p.window ? pos0 + tok_a + 1 - p.window : 0;
     const uint32_t t_beg = lo / ATT_TILE;
     const uint32_t w_key = (tid >> 5) * ATT_BATCH, t_end = len > w_key ? (len - w_key + ATT_TILE - 1) / ATT_TILE : 0;  // (this warp's tiles end there)
     const uint32_t copied = fused ? min(len, pos0) : len;  // rows that come from the caches
-    // A warp's batches: those of part c, then (eight CTAs) of part c + 8. A part's first tile at or above t_beg:
-    auto first_of = [&](uint32_t part) { return t_beg + ((part - t_beg) & (ATT_PARTS - 1)); };
+    // A warp's batches: those of part c, then (eight CTAs) of part c + 8. A part's first tile of this share at or above t_beg, and from one to the next:
+    auto first_of = [&](uint32_t part) {
+        const uint32_t span = (t_beg + ATT_PARTS - 1 - part) / ATT_PARTS;
+        return (span + ((my_share - span) & shares_mask)) * ATT_PARTS + part;
+    };
+    const uint32_t t_step = ATT_PARTS << sh.log;
     // copies run ahead: the batch at tile `it` of the part, its keys or its values next (one lane)
     uint32_t it = first_of(c), in_flight = 0, is = 0;
     bool iv = false;
@@ -248,7 +267,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
         if (bytes) bulk_load(ring + is * L::SLOT, (iv ? v_head : k_head) + (size_t)key * HD, bytes, &bars[is]);
         is = is + 1 == S ? 0 : is + 1;
         in_flight++;
-        if (iv) it += ATT_PARTS;
+        if (iv) it += t_step;
         iv = !iv;
     };
     if (lane == 0) {
@@ -278,7 +297,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
         // takes them, all by the CTA that has their tile.
         for (uint32_t i = tid; i < 2 * PAIRS * (tok_z + 1); i += ATT_THREADS) {
             const uint32_t t = i / (2 * PAIRS), e = i % (2 * PAIRS), jj = e % PAIRS, pos = pos0 + t;
-            if (pos >= len || ((pos / ATT_TILE) & (C - 1)) != c) continue;
+            if (pos >= len || ((pos / ATT_TILE) & (C - 1)) != c || ((pos / ATT_SPAN) & shares_mask) != my_share) continue;
             const float* base = fr.qkv + t * at.act_stride;
             const size_t row = ((size_t)kvh * p.max_len + pos) * HD;
             if (e < PAIRS) {
@@ -330,7 +349,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
         for (int r = 0; r < R; r++)
 #pragma unroll
             for (int i = 0; i < V / 2; i++) o[r][i] = make_float2(0.0f, 0.0f);
-        for (uint32_t t = first_of(part); t < t_end && ok; t += ATT_PARTS) {
+        for (uint32_t t = first_of(part); t < t_end && ok; t += t_step) {
             const uint32_t key0 = t * ATT_TILE + w_key;
             // some of the batch's rows are the step's own
             auto put_own = [&](T* slot, int which) {
@@ -482,9 +501,16 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
         }
     }
     __syncwarp();
+    auto store = [&](uint32_t item, float4 a, float den) {
+        const uint32_t r = row0 + item / (HD / 4);
+        const float inv = 1.0f / den;
+        if (r < all)
+            *(float4*)(out + (r >> g_log) * at.act_stride + (size_t)((kvh << g_log) + (r & g_mask)) * HD + item % (HD / 4) * 4) = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
+    };
     // Every CTA waits for all that is meant for it, so none ends before its peers have stored.
     if (!bar_wait(all_in, 0)) atomicExch(status, 1u);
     // sixteen lanes per four outputs, one for each part's sums
+    const uint32_t unit = kvh * sh.groups + group, active = *active_s;
     if (tid < (int)(share * ATT_PARTS + 31) / 32 * 32) {  // (whole warps; the last half of one may read past its share, and stores nothing)
         float4 a = xo[tid];
         float M = xm[tid], den = xl[tid];
@@ -502,26 +528,93 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
             a.w += shfl_x(a.w, k);
             den += shfl_x(den, k);
         }
-        const uint32_t item = (c << share_log) + tid / ATT_PARTS, r = row0 + item / (HD / 4);
-        const float inv = 1.0f / den;
-        if (tid % ATT_PARTS == 0 && tid < (int)share * ATT_PARTS && r < all)
-            *(float4*)(out + (r >> g_log) * at.act_stride + (size_t)((kvh << g_log) + (r & g_mask)) * HD + item % (HD / 4) * 4) = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
+        const uint32_t item = (c << share_log) + tid / ATT_PARTS;
+        if (tid % ATT_PARTS == 0 && tid < (int)share * ATT_PARTS) {
+            if (active == 1) {
+                store(item, a, den);
+            } else {
+                float4* const to = sh.part + (((size_t)unit << sh.log) + my_share) * (2 * L::F4) + 2 * item;
+                to[0] = a;
+                to[1] = make_float4(M, den, 0.0f, 0.0f);
+            }
+        }
     }
+    if (active == 1) return;
+    // The last of the shares' CTAs that have these outputs adds them, a lane for each share.
+    __shared__ uint32_t others;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) others = atomicAdd(sh.counts + unit * ATT_PARTS + c, 1u);
+    __syncthreads();
+    if (others != active - 1) return;
+    __threadfence();
+    if (tid == 0) sh.counts[unit * ATT_PARTS + c] = 0;  // (for the next launch)
+    if (tid < (int)(share * ATT_PARTS + 31) / 32 * 32) {
+        const uint32_t item = (c << share_log) + min((uint32_t)tid / ATT_PARTS, share - 1), k = tid % ATT_PARTS;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), ml = make_float4(-INFINITY, 0.f, 0.f, 0.f);
+        if (k <= shares_mask && ((k - span0) & shares_mask) < active) {
+            const float4* const from = sh.part + (((size_t)unit << sh.log) + k) * (2 * L::F4) + 2 * item;
+            a = __ldcg(from);
+            ml = __ldcg(from + 1);
+        }
+        float M = ml.x;
+#pragma unroll
+        for (int o = 1; o < ATT_MOST_SHARES; o *= 2) M = fmaxf(M, shfl_x(M, o));
+        const float w = weight_of(ml.x, M);
+        a = make_float4(w * a.x, w * a.y, w * a.z, w * a.w);
+        float den = ml.y * w;
+#pragma unroll
+        for (int o = 1; o < ATT_MOST_SHARES; o *= 2) {
+            a.x += shfl_x(a.x, o);
+            a.y += shfl_x(a.y, o);
+            a.z += shfl_x(a.z, o);
+            a.w += shfl_x(a.w, o);
+            den += shfl_x(den, o);
+        }
+        if (k == 0 && tid < (int)share * ATT_PARTS) store(item, a, den);
+    }
+}
+
+// How many clusters share a KV head's keys: by heads and the caches' size alone, since a token's sums have to be the same in steps of one and of several
+// tokens. More of them only where that puts more CTAs to work on one token, and
+// - while the clusters of a step of four tokens still run at once (one for each head and share, some 36 of eight CTAs fit the chip), from 3072 keys a share on, where
+//   the exchange through memory (2 us) is made up for; 1536 where one token's clusters already have eight CTAs. f32 caches of 128 dimensions, 12300 keys, one and four tokens,
+//   us a launch without and with: 4 heads of 1 KV head 17.6 / 19.1 and 9.7 / 17.9, 16 of 4 19.3 / 46.2 and 16.5 / 31.4, 16 of 16 of 64 dimensions, 4100 keys, 18.6 / 18.0 and 12.9 / 14.0;
+// - or else from 16384 keys on: 32 heads of 8 KV heads, 24600 keys, f32 46.3 / 87.1 and 40.7 / 110.5, f16 45.6 / 91.0 and 33.6 / 109.4 (at 12300 keys 28.0 / 48.8, f16 28.1 / 49.7
+//   without): one token gains what four lose there.
+uint32_t attend_shares(uint32_t nh, uint32_t nkv, uint32_t max_len) {
+    const uint32_t units = nkv * ((nh / nkv + ATT_MOST_ROWS - 1) / ATT_MOST_ROWS);  // clusters of one token
+    auto ctas = [&](uint32_t s) { return units * s * (units * s > 14 ? 8 : 16); };
+    uint32_t shares = 1;
+    for (uint32_t s = 2; s <= ATT_MOST_SHARES && nh * s <= 32 && max_len >= (units > 14 ? 1536 : 3072) * s; s *= 2)
+        if (ctas(s) > ctas(shares)) shares = s;
+    for (uint32_t s = 2; shares == 1 && s <= ATT_MOST_SHARES && units * s <= 32 && max_len >= 16384; s *= 2)
+        if (ctas(s) > ctas(1)) shares = s;
+    return shares;
 }
 
 template <int HD, int R, typename T>
 cudaError_t attend_t(const float* q, void* kc, void* vc, float* out, const uint32_t* sp, const DecAttn& p, uint32_t* status, cudaStream_t st, bool pdl,
-                     const FusedRope& fr, const AttnTokens& at) {
+                     const FusedRope& fr, const AttnTokens& at, const AttScratch& scratch) {
     constexpr size_t smem = AttShared<HD, R, T>::BYTES;
     auto kern = attend_kernel<HD, R, T>;
-    const unsigned G = p.nh / p.nkv, groups = (G * (unsigned)std::max(1, at.n) + R - 1) / R, C = p.nkv * groups > 14 ? 8 : 16;
+    const unsigned G = p.nh / p.nkv, groups = (G * (unsigned)std::max(1, at.n) + R - 1) / R, shares = attend_shares(p.nh, p.nkv, p.max_len), C = p.nkv * groups * shares > 14 ? 8 : 16;
+    AttShares sh{};
+    while ((1u << sh.log) < shares) sh.log++;
+    sh.groups = groups;
+    sh.groups_inv = (65536 + groups - 1) / groups;  // (at most 8 groups x 16 shares)
+    if (shares > 1) {
+        if (!scratch.part || !scratch.counts) return cudaErrorInvalidValue;
+        sh.counts = scratch.counts;
+        sh.part = (float4*)scratch.part;
+    }
     int g_log = 0;
     while ((1u << g_log) < G) g_log++;
     if (cudaError_t e = ensure_dynamic_smem((const void*)kern, smem, 0); e != cudaSuccess) return e;
     // (clusters of more than eight CTAs have to be asked for)
     if (cudaError_t e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(C, p.nkv, groups);
+    cfg.gridDim = dim3(C, p.nkv, groups * shares);
     cfg.blockDim = dim3(ATT_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -534,16 +627,16 @@ cudaError_t attend_t(const float* q, void* kc, void* vc, float* out, const uint3
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kern, q, (T*)kc, (T*)vc, out, sp, p, status, fr, at, g_log);
+    return cudaLaunchKernelEx(&cfg, kern, q, (T*)kc, (T*)vc, out, sp, p, status, fr, at, g_log, sh);
 }
 
 template <int HD, typename T>
 cudaError_t attend_r(const float* q, void* kc, void* vc, float* out, const uint32_t* sp, const DecAttn& p, uint32_t* status, cudaStream_t st, bool pdl,
-                     const FusedRope& fr, const AttnTokens& at) {
+                     const FusedRope& fr, const AttnTokens& at, const AttScratch& scratch) {
     const uint32_t rows = p.nh / p.nkv * (uint32_t)std::max(1, at.n);
-    if (rows <= 1) return attend_t<HD, 1, T>(q, kc, vc, out, sp, p, status, st, pdl, fr, at);
-    if (rows <= 2) return attend_t<HD, 2, T>(q, kc, vc, out, sp, p, status, st, pdl, fr, at);
-    return attend_t<HD, ATT_MOST_ROWS, T>(q, kc, vc, out, sp, p, status, st, pdl, fr, at);
+    if (rows <= 1) return attend_t<HD, 1, T>(q, kc, vc, out, sp, p, status, st, pdl, fr, at, scratch);
+    if (rows <= 2) return attend_t<HD, 2, T>(q, kc, vc, out, sp, p, status, st, pdl, fr, at, scratch);
+    return attend_t<HD, ATT_MOST_ROWS, T>(q, kc, vc, out, sp, p, status, st, pdl, fr, at, scratch);
 }
 
 }  // namespace
@@ -554,8 +647,17 @@ bool attend_supports(uint32_t nh, uint32_t nkv, uint32_t hd) {
     return (hd == 64 || hd == 128) && (g == 1 || g == 2 || g == 4 || g == 8);
 }
 
+static size_t attend_units(uint32_t nh, uint32_t nkv, uint32_t tokens) { return nkv * (((size_t)(nh / nkv) * tokens + ATT_MOST_ROWS - 1) / ATT_MOST_ROWS); }
+size_t attend_part_floats(uint32_t nh, uint32_t nkv, uint32_t hd, uint32_t max_len, uint32_t tokens) {
+    const size_t shares = attend_shares(nh, nkv, max_len);
+    return shares > 1 ? attend_units(nh, nkv, tokens) * shares * (ATT_MOST_ROWS * hd / 4) * 8 : 0;
+}
+size_t attend_count_words(uint32_t nh, uint32_t nkv, uint32_t max_len, uint32_t tokens) {
+    return attend_shares(nh, nkv, max_len) > 1 ? attend_units(nh, nkv, tokens) * ATT_PARTS : 0;
+}
+
 cudaError_t launch_attend(const float* q, void* kc, void* vc, int kv_f16, float* out, const uint32_t* sp, const DecAttn& p, uint32_t* status,
-                          cudaStream_t st, bool pdl, const FusedRope* frp, const AttnTokens* atp) {
+                          const AttScratch& scratch, cudaStream_t st, bool pdl, const FusedRope* frp, const AttnTokens* atp) {
     if (!attend_supports(p.nh, p.nkv, p.hd)) return cudaErrorInvalidValue;
     AttnTokens at{};
     if (atp) at = *atp;
@@ -567,8 +669,8 @@ cudaError_t launch_attend(const float* q, void* kc, void* vc, int kv_f16, float*
             return cudaErrorInvalidValue;
     }
     if (p.hd == 64)
-        return kv_f16 ? attend_r<64, __half>(q, kc, vc, out, sp, p, status, st, pdl, fr, at) : attend_r<64, float>(q, kc, vc, out, sp, p, status, st, pdl, fr, at);
-    return kv_f16 ? attend_r<128, __half>(q, kc, vc, out, sp, p, status, st, pdl, fr, at) : attend_r<128, float>(q, kc, vc, out, sp, p, status, st, pdl, fr, at);
+        return kv_f16 ? attend_r<64, __half>(q, kc, vc, out, sp, p, status, st, pdl, fr, at, scratch) : attend_r<64, float>(q, kc, vc, out, sp, p, status, st, pdl, fr, at, scratch);
+    return kv_f16 ? attend_r<128, __half>(q, kc, vc, out, sp, p, status, st, pdl, fr, at, scratch) : attend_r<128, float>(q, kc, vc, out, sp, p, status, st, pdl, fr, at, scratch);
 }
 
 }  // namespace b2

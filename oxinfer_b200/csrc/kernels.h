@@ -263,9 +263,17 @@ struct AttnTokens {
     int n;  // 0 or 1: one token
     size_t act_stride;
 };
+// Over long caches several clusters share a KV head's keys, and add their sums through memory: `tokens` the most of a step. Counts are zeros, and every launch
+// leaves them so; one launch at a time.
+struct AttScratch {
+    float* part = nullptr;
+    uint32_t* counts = nullptr;
+};
+size_t attend_part_floats(uint32_t nh, uint32_t nkv, uint32_t hd, uint32_t max_len, uint32_t tokens);
+size_t attend_count_words(uint32_t nh, uint32_t nkv, uint32_t max_len, uint32_t tokens);
 // status: set to 1 if a bounded wait gave up.
 cudaError_t launch_attend(const float* q, void* kc, void* vc, int kv_f16, float* out, const uint32_t* sp, const DecAttn& p, uint32_t* status,
-                          cudaStream_t st, bool pdl = false, const FusedRope* fr = nullptr, const AttnTokens* tokens = nullptr);
+                          const AttScratch& scratch, cudaStream_t st, bool pdl = false, const FusedRope* fr = nullptr, const AttnTokens* tokens = nullptr);
 // Host-order rows [n][nkv][hd] f32 <-> cache rows pos0 .. pos0 + n - 1.
 cudaError_t launch_kv_rows(float* rows, void* cache, int kv_f16, bool to_cache, uint32_t nkv, uint32_t hd, uint32_t max_len, uint32_t pos0,
                            uint32_t n, cudaStream_t st);

@@ -126,7 +126,7 @@ DecodePlanImpl::~DecodePlanImpl() {
     for (void* m : peer_maps_) cudaIpcCloseMemHandle(m);
     for (auto& kv : gemm_plans_)
         for (GemmPlan* gp : kv.second) gemm_tc_plan_destroy(gp);
-    void* frees[] = {kv16_, x16_, unscale_, tmp_a_, tmp_b_, gemm_status_, xflags_, bufs_, records_, consts_, words_, rope_table_, argmax_val_, argmax_idx_, token_, out_tokens_, stage_};
+    void* frees[] = {kv16_, x16_, unscale_, tmp_a_, tmp_b_, gemm_status_, xflags_, bufs_, records_, consts_, att_scratch_.part, words_, rope_table_, argmax_val_, argmax_idx_, token_, out_tokens_, stage_};
     for (void* p : frees)
         if (p) cudaFree(p);
 }
@@ -604,7 +604,15 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
     }
 
     // ---- scratch ------------------------------------------------------------------------------------
-    const size_t n_words = 8 + 4 * T;
+    size_t part_floats = 0, count_words = 0;
+    for (const Op& o : p->ops_) {
+        if (o.kind != B2_OP_ATTEND || (prefill && !p->loop_attend_)) continue;
+        const uint32_t tokens = prefill ? 1 : (uint32_t)T;
+        part_floats = std::max(part_floats, attend_part_floats(o.attn.nh, o.attn.nkv, o.attn.hd, o.attn.max_len, tokens));
+        count_words = std::max(count_words, attend_count_words(o.attn.nh, o.attn.nkv, o.attn.max_len, tokens));
+    }
+    if (part_floats) PLAN_CUDA(cudaMalloc((void**)&p->att_scratch_.part, part_floats * sizeof(float)), "cudaMalloc(attention shares)");
+    const size_t n_words = 8 + 4 * T + count_words;
     PLAN_CUDA(cudaMalloc((void**)&p->words_, n_words * 4), "cudaMalloc(step words)");
     PLAN_CUDA(cudaMemset(p->words_, 0, n_words * 4), "cudaMemset(step words)");
     if (p->has_exchange_) {
@@ -615,6 +623,7 @@ int DecodePlanImpl::create(const b2_graph* g, const std::function<const WeightDe
     p->status_ = p->words_ + 4;
     p->argmax_counter_ = p->words_ + 5;
     p->sp_multi_ = p->words_ + 8;
+    p->att_scratch_.counts = p->words_ + 8 + 4 * T;
     size_t table = (size_t)std::max<uint32_t>(p->cs_stride_, 1) * g->max_len;
     PLAN_CUDA(cudaMalloc((void**)&p->rope_table_, table * sizeof(float)), "cudaMalloc(rope table)");
     PLAN_CUDA(cudaMemset(p->rope_table_, 0, table * sizeof(float)), "cudaMemset(rope table)");
@@ -727,9 +736,9 @@ int DecodePlanImpl::run_ops(cudaStream_t st, std::string& err, bool chained, boo
                 if (o.fr.qkv) {
                     FusedRope fr = o.fr;
                     fr.cs_table = rope_table_;
-                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, sp_, o.attn, status_, st, pdl, &fr);
+                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, sp_, o.attn, status_, att_scratch_, st, pdl, &fr);
                 } else {
-                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, sp_, o.attn, status_, st, pdl);
+                    e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, sp_, o.attn, status_, att_scratch_, st, pdl);
                 }
                 break;
             case B2_OP_GLU: e = launch_glu(o.x, o.z, o.y, o.n, o.gelu, st, pdl); break;
@@ -800,7 +809,7 @@ int DecodePlanImpl::run_ops_multi(cudaStream_t st, int nt, std::string& err, boo
                 FusedRope fr = o.fr;
                 fr.cs_table = rope_table_;
                 const bool dependent = pdl();
-                e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, sp_multi_, o.attn, status_, st, dependent && o.fr.qkv, o.fr.qkv ? &fr : nullptr,
+                e = launch_attend(o.x, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y, sp_multi_, o.attn, status_, att_scratch_, st, dependent && o.fr.qkv, o.fr.qkv ? &fr : nullptr,
                                   &at);
                 break;
             }
@@ -1054,7 +1063,7 @@ int DecodePlanImpl::run_prefill(cudaStream_t st, size_t pos, size_t t, std::stri
             case B2_OP_ATTEND:
                 if (loop_attend_) {
                     for (size_t tk = 0; tk < t && e == cudaSuccess; tk++, count++)
-                        e = launch_attend(o.x + tk * ld, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y + tk * ld, sp_multi_ + 4 * tk, o.attn, status_, st);
+                        e = launch_attend(o.x + tk * ld, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, o.y + tk * ld, sp_multi_ + 4 * tk, o.attn, status_, att_scratch_, st);
                 } else {
                     e = launch_attend_rows(o.x, o.y, ld, rows, kv_[o.kv].k, kv_[o.kv].v, kv_f16_, kv16_, (uint32_t)(pos + t), o.attn, gemm_status_, sm_count_, st);
                     count += kv_f16_ ? 1 : 2;

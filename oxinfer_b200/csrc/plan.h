@@ -130,7 +130,8 @@ class DecodePlanImpl {
     std::vector<Kv> kv_;
     uint32_t max_len_ = 0;
     int kv_f16_ = 0;
-    uint32_t* words_ = nullptr;   // sp[4] | status | argmax counter | - | - | sp[4] of each token of a step
+    AttScratch att_scratch_;      // (the counts are words)
+    uint32_t* words_ = nullptr;   // sp[4] | status | argmax counter | - | - | sp[4] of each token of a step | attention counts
     uint32_t* sp_ = nullptr;
     uint32_t* status_ = nullptr;
     uint32_t* argmax_counter_ = nullptr;

@@ -68,6 +68,32 @@ def test_steps_of_several_tokens_with_windows_at_the_edges_of_the_tiles(backend,
     many.close()
 
 
+# four shares, four (two groups of rows a token), two of sixteen heads, four of eight heads (and eight CTAs a cluster)
+@pytest.mark.parametrize("nh,nkv,hd,max_len", [(4, 2, 64, 12400), (8, 1, 128, 12400), (16, 16, 64, 3200), (8, 8, 64, 12400)])
+@pytest.mark.parametrize("window", [0, 1500])
+@pytest.mark.parametrize("kv_f16", [False, True], ids=["f32cache", "f16cache"])
+def test_clusters_that_share_a_heads_keys(backend, nh, nkv, hd, max_len, window, kv_f16):
+    """Long caches: every 1024 keys go to the next cluster. One of them, the next ones too, all; windows that leave the first ones without keys."""
+    one, many = (D.decode_plan(backend, graph(nh, nkv, hd, window), max_len, kv_f16=kv_f16), D.decode_plan_multi(backend, graph(nh, nkv, hd, window), max_len, 4, kv_f16=kv_f16))
+    for pos in (0, 5, 1021, 1024, 2046, 3071, 5120, 12390):
+        if pos + 4 > max_len:
+            continue
+        k, v, x, cs = inputs(nh, nkv, hd, pos, 4, 80 + pos)
+        if kv_f16:  # (values that f16 holds)
+            k, v, x = (a.astype(np.float16).astype(np.float32) for a in (k, v, x))
+        for p in (one, many):
+            if pos:
+                p.kv_write(0, 0, k, v)
+        want = reference(nh, nkv, hd, window, k, v, x)
+        h1 = np.stack([one.step(pos + i, x[i], cs[i], want_logits=False)[0] for i in range(4)])
+        for t in (4, 3, 2, 4):
+            hm, _ = many.step_multi(pos, x[:t], cs[:t], want_logits=False)
+            assert np.array_equal(hm, h1[:t]), (pos, t)
+        assert row_err(h1, want) < 2e-6 * max(1, hd / 64), (pos, row_err(h1, want))
+    one.close()
+    many.close()
+
+
 @pytest.mark.parametrize("nh,nkv,hd", SHAPES)
 @pytest.mark.parametrize("window", [1, 100, 700, NO_LIMIT])
 def test_prefill_with_windows_and_shares_of_the_keys(backend, nh, nkv, hd, window):
