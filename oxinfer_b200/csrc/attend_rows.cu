@@ -134,8 +134,10 @@ __device__ __forceinline__ uint32_t ar_token(const ArArgs& a, uint32_t r) { retu
 template <int HD>
 __host__ __device__ constexpr size_t attend_rows_smem() {  // queries of two tiles, two slots of keys and of values; over them the sums (f32)
     const size_t tiles = (size_t)6 * AR_TILE * HD * 2;
-    return (tiles < 120 * 1024 ? 120 * 1024 : tiles) + 1024;  // (no second CTA on the SM: it would wait for tensor memory)
+    return (tiles < TMEM_512_SMEM ? TMEM_512_SMEM : tiles) + 1024;
 }
+
+static_assert(attend_rows_smem<64>() >= TMEM_512_SMEM && attend_rows_smem<128>() >= TMEM_512_SMEM);
 
 // Grid (Z x row blocks, KV heads), Z CTAs along x a cluster.
 template <int HD>

@@ -61,6 +61,7 @@ constexpr size_t F8_SMEM = 1024 + (size_t)F8_STAGES * (F8_A_BYTES + F8_B_BYTES) 
 static_assert(F8_SMEM <= 227 * 1024, "shared memory budget");
 constexpr size_t F8_PAIR_SMEM = 1024 + (size_t)F8_PAIR_STAGES * (F8_A_BYTES + F8_B_BYTES / 2) + sizeof(F8Shared);
 static_assert(F8_PAIR_SMEM <= 227 * 1024, "shared memory budget (pair form)");
+static_assert(F8_SMEM >= TMEM_512_SMEM && F8_PAIR_SMEM >= TMEM_512_SMEM);
 
 __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {

@@ -90,6 +90,7 @@ constexpr size_t GEMM_SMEM = 1024 /*alignment slack*/ + (size_t)STAGES * (A_STAG
 static_assert(GEMM_SMEM <= 227 * 1024, "shared memory budget");
 constexpr size_t PAIR_SMEM = 1024 + (size_t)PAIR_STAGES * (A_STAGE_BYTES + PAIR_B_STAGE_BYTES) + 2 * PAIR_RAW_BYTES + sizeof(Shared);
 static_assert(PAIR_SMEM <= 227 * 1024, "shared memory budget (pair form)");
+static_assert(GEMM_SMEM >= TMEM_512_SMEM && PAIR_SMEM >= TMEM_512_SMEM);
 
 // TT: the instantiation that takes two-term operands (a_lo_row_arg, w_terms); the one-term kernel carries none of that code.
 // PAIR: the CTA-pair form (4-bit formats, one-term operands, no K split, dense launches of an even number of 256-token

@@ -53,6 +53,9 @@ constexpr size_t wp_smem(int fmt, bool two) {
 }
 static_assert(wp_smem(B2_FMT_Q4_K, false) + sizeof(WpShared) <= 227 * 1024 && wp_smem(B2_FMT_Q6_K, false) + sizeof(WpShared) <= 227 * 1024 &&
               wp_smem(B2_FMT_Q8_0, false) + sizeof(WpShared) <= 227 * 1024 && wp_smem(B2_FMT_MLX4, true) + sizeof(WpShared) <= 227 * 1024, "shared memory budget");
+static_assert(wp_smem(B2_FMT_Q4_K, false) >= TMEM_512_SMEM && wp_smem(B2_FMT_Q4_K, true) >= TMEM_512_SMEM && wp_smem(B2_FMT_MLX4, false) >= TMEM_512_SMEM &&
+              wp_smem(B2_FMT_MLX4, true) >= TMEM_512_SMEM && wp_smem(B2_FMT_Q6_K, false) >= TMEM_512_SMEM && wp_smem(B2_FMT_Q8_0, false) >= TMEM_512_SMEM &&
+              wp_smem(B2_FMT_F8E4M3, false) >= TMEM_512_SMEM);
 
 struct WpArgs {
     int K, n_out, t;

@@ -38,7 +38,7 @@ constexpr int WT_THREADS = 352;
 constexpr int WT_ROWS = 128;
 constexpr uint32_t WT_TMEM_COLS = 256, WT_SLOT_COLS = 64;  // the accumulator, 64 or 128 columns, and the A ring behind it
 constexpr int WT_MAX_RING = 8;
-constexpr size_t WT_SMEM_MAX = 113 * 1024, WT_SMEM_MIN = 77 * 1024;
+constexpr size_t WT_SMEM_MAX = 113 * 1024, WT_SMEM_MIN = TMEM_256_SMEM;
 
 struct __align__(8) WtShared {
     uint64_t a_full[4], b_full[4];

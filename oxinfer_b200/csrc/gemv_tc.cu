@@ -729,7 +729,7 @@ cudaError_t gt_launch(const WeightDev& w, const WeightDev* up, const GemvTcJob* 
     a.min_off = a.b_off + (uint32_t)nbq * (TP == 8 ? 8192 : 4096);
     a.sum_off = a.min_off + (uint32_t)(FMT == B2_FMT_Q4_K ? (nbq + 3) / 4 * 2048 : 0);
     a.xs_off = a.sum_off + (uint32_t)(nbq * TP * 16);
-    const size_t smem = fixed + (size_t)a.slots * gt_raw(FMT);
+    const size_t smem = std::max(fixed + (size_t)a.slots * gt_raw(FMT), TMEM_512_SMEM);
     auto kern = gemv_tc_kernel<FMT, PAIR, TP, JOBS>;
     if (cudaError_t e = ensure_dynamic_smem((const void*)kern, smem, 0); e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};

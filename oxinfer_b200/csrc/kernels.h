@@ -137,6 +137,11 @@ cudaError_t launch_gemv_other(const WeightDev& w, const WeightDev* up, const flo
                               const float* gate, int sm_count, cudaStream_t st, bool pdl = false);
 
 // ---- gemm_tc.cu: prefill dequant-GEMM on tcgen05 ------------------------------------------------
+// Shared memory that a CTA with 256 and with 512 columns of tensor memory asks for at least: of the first two fit an SM, beside one of the second none. So no
+// allocation finds the columns taken. One that waits has no limit to its patience, and CTAs of clusters of two kernels (other streams', other contexts') that hold
+// one SM's columns each and wait for the other's would wait for ever.
+constexpr size_t TMEM_256_SMEM = 77 * 1024, TMEM_512_SMEM = 151 * 1024;
+static_assert(3 * TMEM_256_SMEM > 227 * 1024 && TMEM_512_SMEM + TMEM_256_SMEM > 227 * 1024);
 struct GemmStatus {   // written by the kernel when a bounded wait gives up
     uint32_t code;    // 0 = ok
     uint32_t where;   // which wait
