@@ -25,12 +25,26 @@ __device__ __forceinline__ bool bar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// Acquires at cluster scope: for what the other CTAs of the cluster store.
+__device__ __forceinline__ bool bar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Bounded: false after `limit` cycles.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, long long limit = 2000000000LL) {
-    if (bar_try_wait(bar, parity)) return true;
+    auto test = [&] { return CLUSTER ? bar_try_wait_cluster(bar, parity) : bar_try_wait(bar, parity); };
+    if (test()) return true;
     const long long t0 = clock64();
     for (uint32_t spin = 1;; spin++) {
-        if (bar_try_wait(bar, parity)) return true;
+        if (test()) return true;
         if ((spin & 255) == 0 && clock64() - t0 > limit) return false;
     }
 }

@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
             *(float4*)(out + (r >> g_log) * at.act_stride + (size_t)((kvh << g_log) + (r & g_mask)) * HD + item % (HD / 4) * 4) = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
     };
     // Every CTA waits for all that is meant for it, so none ends before its peers have stored.
-    if (!bar_wait(all_in, 0)) atomicExch(status, 1u);
+    if (!bar_wait<true>(all_in, 0)) atomicExch(status, 1u);
     // sixteen lanes per four outputs, one for each part's sums
     const uint32_t unit = kvh * sh.groups + group, active = *active_s;
     if (tid < (int)(share * ATT_PARTS + 31) / 32 * 32) {  // (whole warps; the last half of one may read past its share, and stores nothing)

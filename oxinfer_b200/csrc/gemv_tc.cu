@@ -100,12 +100,14 @@ struct __align__(16) GtShared {
     volatile uint32_t abort_flag;
 };
 
-template <class Sh>
+// CLUSTER: what the barrier counts comes from the cluster's other CTAs.
+template <bool CLUSTER = false, class Sh>
 __device__ __forceinline__ bool gt_wait(uint64_t* bar, uint32_t parity, Sh* sh, uint32_t* status, bool heed_abort = true) {
-    if (mbar_try_wait(bar, parity)) return true;
+    auto test = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+    if (test()) return true;
     const long long t0 = clock64();
     for (uint32_t spin = 1;; spin++) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (test()) return true;
         if ((spin & 255) == 0) {
             if (heed_abort && sh->abort_flag) return false;
             if (clock64() - t0 > WAIT_LIMIT_CYCLES) {
@@ -561,7 +563,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
 #pragma unroll
             for (int t = 0; t < TP; t++) acc[t] += low[t];
             const int buf = i & 1, to = PAIR ? 2 * (w & 1) + (lane >> 4) : w, row = PAIR ? 16 * (w >> 1) + (lane & 15) : lane;
-            if (i >= 2) ok = __all_sync(0xffffffffu, gt_wait(&sh->in_free[to][buf], (uint32_t)(((i >> 1) - 1) & 1), sh, a.status));
+            if (i >= 2) ok = __all_sync(0xffffffffu, gt_wait<true>(&sh->in_free[to][buf], (uint32_t)(((i >> 1) - 1) & 1), sh, a.status));
             if (!ok) {
                 if constexpr (MLX) met = (i * nbq + nbq - set + 3) >> 2;
                 break;
@@ -602,7 +604,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
                 gt_send(cluster_addr(sh->ssq_in[rank], lane), q, cluster_addr(&sh->ssq_full, lane));
             }
             __syncwarp();
-            ok = __all_sync(0xffffffffu, gt_wait(&sh->ssq_full, 0, sh, a.status));
+            ok = __all_sync(0xffffffffu, gt_wait<true>(&sh->ssq_full, 0, sh, a.status));
 #pragma unroll
             for (int t = 0; t < TP; t++) {
                 const float sq = sh->ssq_in[0][t] + sh->ssq_in[1][t] + sh->ssq_in[2][t] + sh->ssq_in[3][t];
@@ -631,7 +633,7 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
                     times[t] = a.mode != B2_MODE_STORE && a.mode != B2_MODE_ADD && t < T ? 1.0f / (1.0f + __expf(-a.gate[(size_t)(t0 + t) * a.gate_stride])) : 1.0f;
                 }
             }
-            if (i >= 0) ok = __all_sync(0xffffffffu, gt_wait(&sh->in_full[buf], (uint32_t)((i >> 1) & 1), sh, a.status));
+            if (i >= 0) ok = __all_sync(0xffffffffu, gt_wait<true>(&sh->in_full[buf], (uint32_t)((i >> 1) & 1), sh, a.status));
             if (!ok) break;
             float v[TP];
 #pragma unroll
@@ -646,12 +648,14 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
                 v[t] = u[0];
                 v[t] *= factor[t];
             }
-            __syncwarp();
             if (i >= 0 && i + 2 < my_tiles) {
                 if (lane == 0) mbar_arrive_expect_tx(&sh->in_full[buf], IN_BYTES);
-                __syncwarp();
-                // (relaxed: with release at cluster scope an arrival takes 1500 cycles; the loads above enter its address)
-                if (lane < GT_CTAS) gt_arrive(cluster_addr(&sh->in_free[rank][buf], lane) + (__float_as_uint(v[TP - 1]) & (uint32_t)a.zero));
+                // (relaxed: with release at cluster scope an arrival takes 1500 cycles; what every lane has loaded enters its address)
+                uint32_t words = __float_as_uint(v[0]);
+#pragma unroll
+                for (int t = 1; t < TP; t++) words |= __float_as_uint(v[t]);
+                words = __reduce_or_sync(0xffffffffu, words) & (uint32_t)a.zero;
+                if (lane < GT_CTAS) gt_arrive(cluster_addr(&sh->in_free[rank][buf], lane) + words);
             }
 #pragma unroll
             for (int t = 0; t < TP; t++) {

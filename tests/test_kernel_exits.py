@@ -39,3 +39,14 @@ def test_every_meeting_is_counted_and_the_rest_is_made_up_for():
     assert code[q8:mlx].count("multiply(") == 1 and code[mlx:q4].count("multiply(") == 1 and code[q4:].count("multiply(") == 2
     assert "k0 < 8; k0 += CHUNKS" in code and "CHUNKS = NB == 16 ? 8 : 4" in code
     assert the(r"constexpr int MEETS = (.*);") == "MLX || (Q8 && NB == 16) ? 1 : 2"
+
+
+def test_what_peers_store_is_acquired_at_cluster_scope_and_given_back_after_every_lane_has_read_it():
+    """(Read from the source too: on one machine a missing order shows once in a great while.)"""
+    attend = (Path(__file__).resolve().parent.parent / "oxinfer_b200" / "csrc" / "attend.cu").read_text()
+    for bar in ("in_full[buf]", "in_free[to][buf]", "ssq_full"):  # (counted by the cluster's other CTAs)
+        waits = re.findall(r"gt_wait(<true>)?\(&sh->" + re.escape(bar), TEXT)
+        assert waits and all(waits), bar
+    assert "bar_wait<true>(all_in" in attend and "bar_wait(all_in" not in attend
+    give_back = TEXT[TEXT.index("uint32_t words = __float_as_uint(v[0]);"):TEXT.index("gt_arrive(cluster_addr(&sh->in_free[rank][buf]")]
+    assert "for (int t = 1; t < TP; t++) words |=" in give_back and "words = __reduce_or_sync(0xffffffffu, words) & (uint32_t)a.zero;" in give_back
