@@ -513,8 +513,11 @@ class Backend {
     // Q6_K; the forms that gemv_tc.cu took over behaved alike): 14336 x 4096 48 and 32 us, 28672 x 4096 83 and 51.
     // The second launch waits for the first, so a matrix whose tiles fill no more than half of the SMs gains nothing by it:
     // FP8 512 x 4096 10.1 us in one launch, 11.5 in two. Seven or eight tokens of Q6_K do (512 x 4096 12.7
-    // and 13.8). Matrices whose CTAs split only the part of K that they multiply (gemv_tc.cu) need no records (null), x instead, and take eight
+    // and 13.8). Products that split the activations themselves (self_split) need no records (null), x instead; those of gemv_tc.cu then take eight
     // tokens a launch (Q4_K 4096 x 4096 7.9 us, in two launches 12.4); 4-bit ones from records four, as the callers with host buffers count them.
+    // A CTA of gemv_tc.cu splits only the part of K that it multiplies; one of gemv_mma.cu all of it, up to two blocks a warp before a launch for the records
+    // pays (two and four tokens of Q6_K, records and not: 4096 x 1024 4.5 / 4.8 and 3.7 / 3.8 us, 28672 x 2048 20.9 / 21.3 and 19.2 / 19.9; three of 4096 x 4096, 48 blocks: alike).
+    static bool self_split(const WeightDev& w, size_t t) { return gemv_tc_supports(w) || split_blocks_of(w.n_in) * t <= 32; }
     int small_products(const WeightDev& w, const WeightDev* up, const uint8_t* rec, const float* x, size_t t, float* y, int mode) {
         const size_t stride = record_stride(w.n_in, gemv_mma_halves(w)), tiles = (w.n_out + 15) / 16;
         const bool narrow = 2 * tiles <= (size_t)sm_count && w.fmt == B2_FMT_Q6_K && t > 6;
@@ -587,7 +590,7 @@ class Backend {
                 for (size_t i = 0; i < t && !rc; i++) rc = matvec_dev(h, 0, xf + i * K, (float*)y + i * w->dev.n_out, B2_MODE_STORE, nullptr);
                 return rc;
             }
-            if (gemv_tc_supports(w->dev) && !records) {
+            if (self_split(w->dev, t) && !records) {
                 const float* xf = (const float*)x;
                 if (int rc = apart(xf, t * K, (const float*)y, t * w->dev.n_out)) return rc;
                 return small_products(w->dev, nullptr, nullptr, xf, t, (float*)y, B2_MODE_STORE);
@@ -896,11 +899,12 @@ class Backend {
             if (t > 1 && gemv_mma_supports(w->dev)) {  // one launch reads the weights once for all rows
                 const bool halves = gemv_mma_halves(w->dev);
                 uint8_t* rec = (uint8_t*)xrec.p + (halves ? digits : 0);
-                if (!made[halves] && !gemv_tc_supports(w->dev)) {
+                const bool self = self_split(w->dev, t);
+                if (!made[halves] && !self) {
                     rc = make_records((const float*)x_dev.p, t, n_in, halves, rec);
                     made[halves] = true;
                 }
-                if (!rc) rc = small_products(w->dev, u ? &u->dev : nullptr, gemv_tc_supports(w->dev) ? nullptr : rec, (const float*)x_dev.p, t, yj, mode);
+                if (!rc) rc = small_products(w->dev, u ? &u->dev : nullptr, self ? nullptr : rec, (const float*)x_dev.p, t, yj, mode);
             } else {
                 for (size_t i = 0; i < t && !rc; i++)
                     rc = matvec_dev(jobs[j].w, jobs[j].up, (const float*)x_dev.p + i * n_in, yj + i * jobs[j].n_out, mode, nullptr);
