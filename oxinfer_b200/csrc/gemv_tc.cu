@@ -29,7 +29,7 @@
 //   Q8_0  4096 x 4096    6.3 / 8.7 / 9.6 / 16.9    5.2 / 5.6 / 8.0 / 9.2
 //         4096 x 14336  15.0 / 24.3 / 28.4 / 42.1  13.0 / 14.6 / 16.2 / 24.5
 //         32064 x 4096  23.9 / 27.0 / 28.1 / 54.5  23.3 / 24.6 / 24.6 / 28.0
-// (One token of short rows is slower than on mma.sync: Q4_K 14336 x 1024 5.1 and 6.2 us. 6144 x 4096, MLX-4, one token: 5.9 and 6.3: its 48 tiles take two rounds of 24 clusters. In a graph 4096 x 4096 takes 4.5 and 4.4.)
+// (6144 x 4096, MLX-4, one token: 5.9 and 6.3: its 48 tiles take two rounds of 24 clusters. In a graph 4096 x 4096 takes 4.5 and 4.4.)
 // Largest error of a result against 64 bits, in parts of the row's norm, N(0, 1) activations, K = 1024 / 4096 / 14336:
 // Q4_K 1.60 / 1.70 / 1.71e-7 on mma.sync, 1.60 / 1.65 / 1.66e-7 here; MLX-4 1.78 / 2.07 / 2.39e-7 and 1.57 / 1.65 / 1.59e-7;
 // Q8_0 1.67 / 1.72 / 1.79e-7 and 1.67 / 1.69 / 1.73e-7.
@@ -805,11 +805,14 @@ GtArgs gt_args(const WeightDev& w, const GemvIn& in, int T) {
 }  // namespace
 
 // By format and K alone: all of a matrix's rows, whatever shard or token they belong to, have to take the same form. (Q8_0 up to 14336 values a row: two slots
-// beside the digits of eight tokens. Q4_K up to 36864, MLX-4 to 41984.)
+// beside the digits of eight tokens. Q4_K up to 36864, MLX-4 to 41984.) Up to 1024 values a row the form on mma.sync is faster, by itself, where it splits the
+// activations (us in a graph, one / two / four / eight tokens, on mma.sync and here: Q4_K 1024 x 1024 2.54 / 2.72 / 3.14 / 4.26 and 3.35 / 3.49 / 3.82 / 3.88, 14336 x 1024
+// 5.00 / 5.46 / 5.60 / 8.03 and 5.28 / 5.71 / 6.45 / 8.80), and more so between other kernels: six layers of hidden size 1024 with Q4_K, Q6_K and Q8_0, four tokens,
+// 309 us and 358.
 bool gemv_tc_supports(const WeightDev& w) {
     const int tp = w.fmt == B2_FMT_Q8_0 ? 8 : GT_TOKENS;
     return (w.fmt == B2_FMT_Q4_K || w.fmt == B2_FMT_MLX4 || (w.fmt == B2_FMT_Q8_0 && ((uintptr_t)w.p1 & 15) == 0)) && ((uintptr_t)w.p0 & 15) == 0 && w.n_in % 256 == 0 &&
-           w.n_in > 0 && gt_fixed(w.fmt, w.n_in, tp) + 2 * gt_raw(w.fmt) <= gt_smem(tp);
+           w.n_in > 1024 && gt_fixed(w.fmt, w.n_in, tp) + 2 * gt_raw(w.fmt) <= gt_smem(tp);
 }
 
 cudaError_t launch_gemv_tc(const WeightDev& w, const WeightDev* up, const GemvIn& in, int T, float* y, size_t y_stride, int mode, const float* gate,
