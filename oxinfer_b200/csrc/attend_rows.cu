@@ -314,7 +314,7 @@ attend_rows_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
             for (int h = 0; h < 4; h++) ar_ld32(s_at + 32 * h, v[h]);
             ar_ld_wait();
             const uint32_t j0 = (t_first + i) * AR_TILE;
-            if (j0 + AR_TILE - 1 > tile_qp || (a.window != 0 && tile_end >= j0 && tile_end - j0 >= a.window)) {  // some row does not see some key
+            if (j0 + AR_TILE - 1 > tile_qp || (a.window != 0 && j0 + a.window <= tile_end)) {  // some row does not see some key
                 const uint32_t hi = qp >= j0 ? min(qp - j0 + 1, (uint32_t)AR_TILE) : 0u, from = my_lo > j0 ? my_lo - j0 : 0u;  // keys from .. hi - 1 of the tile
                 auto below = [](uint32_t n, int h) { return n >= 32u * h + 32 ? 0xffffffffu : n <= 32u * h ? 0u : (1u << (n - 32 * h)) - 1; };  // a bit per key below n
 #pragma unroll
@@ -524,7 +524,7 @@ cudaError_t launch_attend_rows(const float* q, float* out, size_t stride, uint32
     a.g_inv = a.G == 1 ? 0u : (uint32_t)(((1ull << 32) + a.G - 1) / a.G);
     a.rows = tokens * a.G;
     a.pos0 = len - tokens;
-    a.window = p.window;
+    a.window = p.window >= p.max_len ? 0 : p.window;  // (none then, and a key's position plus the window does not wrap)
     a.q_sign = p.scale < 0.0f ? -1.0f : 1.0f;
     a.c = std::max(p.scale * a.q_sign, 1e-30f) * 1.44269504f;  // (a factor of zero would make a masked key's score NaN)
     a.status = status;
