@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(256) qk_rope_rows_kernel(const float* __restri
                                                            const float* __restrict__ cs_table, const uint32_t* __restrict__ sp, DecRope p) {
     __shared__ float buf[256];
     __shared__ float red[32];
+    pdl_launch_dependents();
     const size_t off = (size_t)blockIdx.y * stride;
     rope_head<T>(blockIdx.x, threadIdx.x, sp[0] + blockIdx.y, sp[1], qkv + off, qo + off, kc, vc, qn, kn, cs_table, p, buf, red);
 }
@@ -48,6 +49,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) qk_rope_fast_kernel(const float* __restrict__ qkv, float* __restrict__ qo, size_t stride, uint32_t rows,
                                                            T* __restrict__ kc, T* __restrict__ vc, const float* __restrict__ cs_table,
                                                            const uint32_t* __restrict__ sp, DecRope p) {
+    pdl_launch_dependents();
     const uint32_t heads = p.nh + 2 * p.nkv;
     const uint32_t unit = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (unit >= rows * heads) return;
