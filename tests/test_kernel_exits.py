@@ -49,4 +49,4 @@ def test_what_peers_store_is_acquired_at_cluster_scope_and_given_back_after_ever
         assert waits and all(waits), bar
     assert "bar_wait<true>(all_in" in attend and "bar_wait(all_in" not in attend
     give_back = TEXT[TEXT.index("uint32_t words = __float_as_uint(v[0]);"):TEXT.index("gt_arrive(cluster_addr(&sh->in_free[rank][buf]")]
-    assert "for (int t = 1; t < TP; t++) words |=" in give_back and "words = __reduce_or_sync(0xffffffffu, words) & (uint32_t)a.zero;" in give_back
+    assert "for (int t = 1; t < TP; t++) words |=" in give_back and re.search(r"words = __(ballot|reduce_or)_sync\(0xffffffffu, words[^;]*\) & \(uint32_t\)a\.zero;", give_back)
