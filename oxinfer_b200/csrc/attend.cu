@@ -202,7 +202,7 @@ struct AttShares {
 };
 
 // Grid (C, KV heads, shares x groups of R rows), a cluster along x. Row r of a KV head: query head r % G of token r / G. sp[0]: the position of the step's first token.
-template <int HD, int R, typename T>
+template <int HD, int R, typename T, bool SHARED>
 __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __restrict__ q, T* kc, T* vc, float* __restrict__ out,
                                                                 const uint32_t* __restrict__ sp, DecAttn p, uint32_t* status, FusedRope fr, AttnTokens at,
                                                                 int g_log, AttShares sh) {
@@ -211,15 +211,18 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_launch_dependents();
     const uint32_t pos0 = sp[0], table0 = sp[1];
-    const uint32_t C = gridDim.x, c = blockIdx.x, kvh = blockIdx.y, my_share = blockIdx.z * sh.groups_inv >> 16, group = blockIdx.z - my_share * sh.groups, row0 = group * R;
+    const uint32_t C = gridDim.x, c = blockIdx.x, kvh = blockIdx.y, my_share = SHARED ? blockIdx.z * sh.groups_inv >> 16 : 0, group = blockIdx.z - my_share * sh.groups, row0 = group * R;
     const uint32_t all = (uint32_t)max(1, at.n) << g_log, g_mask = (1u << g_log) - 1;
     const uint32_t tok_a = row0 >> g_log, tok_z = (min(row0 + R, all) - 1) >> g_log;  // the group's tokens
     const uint32_t len = min(pos0 + tok_z + 1, p.max_len);                            // keys below len are seen by some row
     const uint32_t lo = p.window != 0 && pos0 + tok_a + 1 > p.window ? pos0 + tok_a + 1 - p.window : 0;
-    const uint32_t span0 = lo / ATT_SPAN, spans = (len - 1) / ATT_SPAN + 1 - span0, shares_mask = (1u << sh.log) - 1;
+    const uint32_t span0 = lo / ATT_SPAN, shares_mask = SHARED ? (1u << sh.log) - 1 : 0;
     __shared__ uint32_t active_s[1];  // shares that have keys
-    if (((my_share - span0) & shares_mask) >= spans) return;
-    if (threadIdx.x == 0) *active_s = min(spans, shares_mask + 1);
+    if constexpr (SHARED) {
+        const uint32_t spans = (len - 1) / ATT_SPAN + 1 - span0;
+        if (((my_share - span0) & shares_mask) >= spans) return;
+        if (threadIdx.x == 0) *active_s = min(spans, shares_mask + 1);
+    }
     constexpr int F4_LOG = L::F4 == 16 ? 4 : L::F4 == 32 ? 5 : L::F4 == 64 ? 6 : 7;
     static_assert(L::F4 == 1u << F4_LOG);
     const uint32_t share_log = F4_LOG - (gridDim.x == 16 ? 4 : 3), share = 1u << share_log;  // of the outputs
@@ -252,10 +255,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
     const uint32_t copied = fused ? min(len, pos0) : len;  // rows that come from the caches
     // A warp's batches: those of part c, then (eight CTAs) of part c + 8. A part's first tile of this share at or above t_beg, and from one to the next:
     auto first_of = [&](uint32_t part) {
+        if constexpr (!SHARED) return t_beg + ((part - t_beg) & (ATT_PARTS - 1));
         const uint32_t span = (t_beg + ATT_PARTS - 1 - part) / ATT_PARTS;
         return (span + ((my_share - span) & shares_mask)) * ATT_PARTS + part;
     };
-    const uint32_t t_step = ATT_PARTS << sh.log;
+    const uint32_t t_step = SHARED ? ATT_PARTS << sh.log : ATT_PARTS;
     // copies run ahead: the batch at tile `it` of the part, its keys or its values next (one lane)
     uint32_t it = first_of(c), in_flight = 0, is = 0;
     bool iv = false;
@@ -297,7 +301,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
         // takes them, all by the CTA that has their tile.
         for (uint32_t i = tid; i < 2 * PAIRS * (tok_z + 1); i += ATT_THREADS) {
             const uint32_t t = i / (2 * PAIRS), e = i % (2 * PAIRS), jj = e % PAIRS, pos = pos0 + t;
-            if (pos >= len || ((pos / ATT_TILE) & (C - 1)) != c || ((pos / ATT_SPAN) & shares_mask) != my_share) continue;
+            if (pos >= len || ((pos / ATT_TILE) & (C - 1)) != c || (SHARED && ((pos / ATT_SPAN) & shares_mask) != my_share)) continue;
             const float* base = fr.qkv + t * at.act_stride;
             const size_t row = ((size_t)kvh * p.max_len + pos) * HD;
             if (e < PAIRS) {
@@ -510,7 +514,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
     // Every CTA waits for all that is meant for it, so none ends before its peers have stored.
     if (!bar_wait<true>(all_in, 0)) atomicExch(status, 1u);
     // sixteen lanes per four outputs, one for each part's sums
-    const uint32_t unit = kvh * sh.groups + group, active = *active_s;
+    const uint32_t unit = kvh * sh.groups + group, active = SHARED ? *active_s : 1;
     if (tid < (int)(share * ATT_PARTS + 31) / 32 * 32) {  // (whole warps; the last half of one may read past its share, and stores nothing)
         float4 a = xo[tid];
         float M = xm[tid], den = xl[tid];
@@ -539,6 +543,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
             }
         }
     }
+    if constexpr (!SHARED) return;
     if (active == 1) return;
     // The last of the shares' CTAs that have these outputs adds them, a lane for each share.
     __shared__ uint32_t others;
@@ -597,7 +602,7 @@ template <int HD, int R, typename T>
 cudaError_t attend_t(const float* q, void* kc, void* vc, float* out, const uint32_t* sp, const DecAttn& p, uint32_t* status, cudaStream_t st, bool pdl,
                      const FusedRope& fr, const AttnTokens& at, const AttScratch& scratch) {
     constexpr size_t smem = AttShared<HD, R, T>::BYTES;
-    auto kern = attend_kernel<HD, R, T>;
+    auto kern = attend_kernel<HD, R, T, false>;
     const unsigned G = p.nh / p.nkv, groups = (G * (unsigned)std::max(1, at.n) + R - 1) / R, shares = attend_shares(p.nh, p.nkv, p.max_len), C = p.nkv * groups * shares > 14 ? 8 : 16;
     AttShares sh{};
     while ((1u << sh.log) < shares) sh.log++;
@@ -607,6 +612,7 @@ cudaError_t attend_t(const float* q, void* kc, void* vc, float* out, const uint3
         if (!scratch.part || !scratch.counts) return cudaErrorInvalidValue;
         sh.counts = scratch.counts;
         sh.part = (float4*)scratch.part;
+        kern = attend_kernel<HD, R, T, true>;  // (code of its own: what the shares ask costs the others 2 %)
     }
     int g_log = 0;
     while ((1u << g_log) < G) g_log++;
