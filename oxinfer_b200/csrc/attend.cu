@@ -101,7 +101,8 @@ __device__ __forceinline__ void score(float2 (&a)[R], float2 (&b)[R], const __ha
 }
 
 // Where the queries' dimension d lies in shared memory: eight lanes' quads side by side as they read them. (f16 keys come eight dimensions a lane; with the
-// queries in order two lanes met in a bank: 32 heads of 8 KV heads of 128, one / four tokens, 8200 keys 22.0 / 38.9 us, this way 18.3 / 36.6, 16000 keys 37.3 / 72.7 and 31.8 / 61.1.)
+// queries in order two lanes met in a bank: 32 heads of 8 KV heads of 128, one / four tokens, 8200 keys 22.0 / 38.9 us, this way 18.3 / 36.6, 16000
+// keys 37.3 / 72.7 and 31.8 / 61.1.)
 template <typename T>
 __device__ __forceinline__ uint32_t q_at(uint32_t d) { return sizeof(T) == 2 ? (d & ~63u) + 32 * ((d >> 2) & 1) + 4 * ((d >> 3) & 7) + (d & 3) : d; }
 
@@ -201,7 +202,8 @@ struct AttShares {
     uint32_t* counts;  // [unit][CTA], zero
 };
 
-// Grid (C, KV heads, shares x groups of R rows), a cluster along x. Row r of a KV head: query head r % G of token r / G. sp[0]: the position of the step's first token.
+// Grid (C, KV heads, shares x groups of R rows), a cluster along x. Row r of a KV head: query head r % G of token r / G. sp[0]: the position of the
+// step's first token.
 template <int HD, int R, typename T, bool SHARED>
 __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __restrict__ q, T* kc, T* vc, float* __restrict__ out,
                                                                 const uint32_t* __restrict__ sp, DecAttn p, uint32_t* status, FusedRope fr, AttnTokens at,
@@ -582,10 +584,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
 
 // How many clusters share a KV head's keys: by heads and the caches' size alone, since a token's sums have to be the same in steps of one and of several
 // tokens. More of them only where that puts more CTAs to work on one token, and
-// - while the clusters of a step of four tokens still run at once (one for each head and share, some 36 of eight CTAs fit the chip), from 3072 keys a share on, where
-//   the exchange through memory (2 us) is made up for; 1536 where one token's clusters already have eight CTAs. f32 caches of 128 dimensions, 12300 keys, one and four tokens,
-//   us a launch without and with: 4 heads of 1 KV head 17.6 / 19.1 and 9.7 / 17.9, 16 of 4 19.3 / 46.2 and 16.5 / 31.4, 16 of 16 of 64 dimensions, 4100 keys, 18.6 / 18.0 and 12.9 / 14.0;
-// - or else from 16384 keys on: 32 heads of 8 KV heads, 24600 keys, f32 46.3 / 87.1 and 40.7 / 110.5, f16 45.6 / 91.0 and 33.6 / 109.4 (at 12300 keys 28.0 / 48.8, f16 28.1 / 49.7
+// - while the clusters of a step of four tokens still run at once (one for each head and share, some 36 of eight CTAs fit the chip), from 3072 keys
+// a share on, where
+//   the exchange through memory (2 us) is made up for; 1536 where one token's clusters already have eight CTAs. f32 caches of 128 dimensions, 12300
+//   keys, one and four tokens,
+//   us a launch without and with: 4 heads of 1 KV head 17.6 / 19.1 and 9.7 / 17.9, 16 of 4 19.3 / 46.2 and 16.5 / 31.4, 16 of 16 of 64 dimensions,
+//   4100 keys, 18.6 / 18.0 and 12.9 / 14.0;
+// - or else from 16384 keys on: 32 heads of 8 KV heads, 24600 keys, f32 46.3 / 87.1 and 40.7 / 110.5, f16 45.6 / 91.0 and 33.6 / 109.4 (at 12300
+// keys 28.0 / 48.8, f16 28.1 / 49.7
 //   without): one token gains what four lose there.
 uint32_t attend_shares(uint32_t nh, uint32_t nkv, uint32_t max_len) {
     const uint32_t units = nkv * ((nh / nkv + ATT_MOST_ROWS - 1) / ATT_MOST_ROWS);  // clusters of one token

@@ -483,7 +483,8 @@ cudaError_t attend_rows_t(const CUtensorMap& k, const CUtensorMap& v, const ArAr
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    // Dependent where the CTAs run at once: the start (tensor memory, barriers, maps) under the kernel ahead. (f16 caches, 32 query and 8 KV heads of 128, RoPE and attention
+    // Dependent where the CTAs run at once: the start (tensor memory, barriers, maps) under the kernel ahead. (f16 caches, 32 query and 8 KV heads
+    // of 128, RoPE and attention
     // of 8 / 128 / 600 tokens: 14.9 / 19.4 / 36.5 us, dependent 10.9 / 17.2 / 33.9, on mma.sync 12.9 / 21.3 / 56; of 2048, 256 CTAs: 120 and 123.)
     cfg.numAttrs = cfg.gridDim.x * nkv <= (unsigned)sm_count ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, k, v, a);

@@ -516,7 +516,8 @@ class Backend {
     // and 13.8). Products that split the activations themselves (self_split) need no records (null), x instead; those of gemv_tc.cu then take eight
     // tokens a launch (Q4_K 4096 x 4096 7.9 us, in two launches 12.4); 4-bit ones from records four, as the callers with host buffers count them.
     // A CTA of gemv_tc.cu splits only the part of K that it multiplies; one of gemv_mma.cu all of it, up to two blocks a warp before a launch for the records
-    // pays (two and four tokens of Q6_K, records and not: 4096 x 1024 4.5 / 4.8 and 3.7 / 3.8 us, 28672 x 2048 20.9 / 21.3 and 19.2 / 19.9; three of 4096 x 4096, 48 blocks: alike).
+    // pays (two and four tokens of Q6_K, records and not: 4096 x 1024 4.5 / 4.8 and 3.7 / 3.8 us, 28672 x 2048 20.9 / 21.3 and 19.2 / 19.9; three of
+    // 4096 x 4096, 48 blocks: alike).
     static bool self_split(const WeightDev& w, size_t t) { return gemv_tc_supports(w) || split_blocks_of(w.n_in) * t <= 32; }
     int small_products(const WeightDev& w, const WeightDev* up, const uint8_t* rec, const float* x, size_t t, float* y, int mode) {
         const size_t stride = record_stride(w.n_in, gemv_mma_halves(w)), tiles = (w.n_out + 15) / 16;

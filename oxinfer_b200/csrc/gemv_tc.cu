@@ -7,7 +7,8 @@
 // A cluster of four CTAs takes tiles of 128 rows, CTA q the blocks q n / 4 .. of K, so the order of a row's sum depends on K alone: a
 // row shard and every row of a step of several tokens have the bits of the one-token product. A CTA:
 //   warp 0        : copies packed rows (128 x 144 bytes a block of 256 k) into a ring, filled before the kernel waits for the one ahead.
-//   warps 2 .. 17 : four sets of four, a thread a row; set s takes the blocks s, s + 4, .. of those that the CTA has of all its tiles: nibbles to bytes in tensor memory, the
+//   warps 2 .. 17 : four sets of four, a thread a row; set s takes the blocks s, s + 4, .. of those that the CTA has of all its tiles: nibbles to
+//   bytes in tensor memory, the
 //                   instructions, the sums back and times the scales. At the end of a tile its sums go to the CTA of the cluster that owns the rows.
 //   warp 1        : adds the sixteen sums of its rows in pairs, applies the norm's factor and the output mode, and stores.
 // All but warp 0 split the CTA's part of the activations first (an RMS norm's weights multiply before the split, its factor the results).
@@ -16,8 +17,10 @@
 // only scale the sums (f32, per 32). Eight tokens are 32 columns then: read twice, the bytes would pass at L2's rate.
 //
 // What bounds it: HBM on large matrices, the start on small ones. The form on mma.sync (gemv_mma.cu) was bound by instructions: 393 of a warp
-// for 4096 weights (Q4_K 14336 x 4096, one token, ncu, everything counted); here it is 225, of which the bytes, the sums and the scales are about 110. Of the 4.7 us of 4096 x 4096, 0.5 pass before the first copy is issued, 1.5 until
-// activations and weights are there, and 2 between them and the result, most of it the first fetch of each line of code: hence short code, no divisions, a pass of the
+// for 4096 weights (Q4_K 14336 x 4096, one token, ncu, everything counted); here it is 225, of which the bytes, the sums and the scales are about
+// 110. Of the 4.7 us of 4096 x 4096, 0.5 pass before the first copy is issued, 1.5 until
+// activations and weights are there, and 2 between them and the result, most of it the first fetch of each line of code: hence short code, no
+// divisions, a pass of the
 // results' loop that stores nothing. Four sets and the whole of tensor memory: two sets in half of an SM (two CTAs) left 4096 x 14336, four tokens, at 21 us.
 // One launch after another in a stream, us, one / two / four / eight tokens, on mma.sync and here:
 //   Q4_K  4096 x 4096    5.2 / 8.8 / 11.0 / 16.1   5.1 / 5.5 / 6.1 / 7.9
@@ -284,7 +287,18 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
     float* const xs_s = (float*)(smem + a.xs_off);    // [block][TP]
     float* const ssq_s = xs_s + nbq * TP;
     const int items = nbq * T;
-    auto block_of = [&](int i) { return TP == 1 ? i : TP == 2 ? i >> 1 : T == 4 ? i >> 2 : T == 3 ? (i * 21846) >> 16 : T == 2 ? i >> 1 : T == 1 ? i : T == 8 ? i >> 3 : T == 7 ? (i * 9363) >> 16 : T == 6 ? (i * 10923) >> 16 : (i * 13108) >> 16; };  // i / T
+    auto block_of = [&](int i) {  // i / T (i < 512: times ceil(2^16 / T) where T is no power of two)
+        if constexpr (TP == 1) return i;
+        if constexpr (TP == 2) return i >> 1;
+        return T == 4   ? i >> 2
+               : T == 3 ? (i * 21846) >> 16
+               : T == 2 ? i >> 1
+               : T == 1 ? i
+               : T == 8 ? i >> 3
+               : T == 7 ? (i * 9363) >> 16
+               : T == 6 ? (i * 10923) >> 16
+                        : (i * 13108) >> 16;
+    };
     auto load = [&](int i) {
         const int lb = block_of(i), tk = i - lb * T, blk = b0 + lb;
         return split_load(a.x + (size_t)(t0 + tk) * a.x_stride + (size_t)blk * 256, a.nw ? a.nw + (size_t)blk * 256 : nullptr, 256, lane);
@@ -658,7 +672,8 @@ gemv_tc_kernel(const __grid_constant__ GtMats<JOBS, FMT == B2_FMT_Q8_0> mats, co
             }
             if (i >= 0 && i + 2 < my_tiles) {
                 if (lane == 0) mbar_arrive_expect_tx(&sh->in_full[buf], IN_BYTES);
-                // (relaxed: with release at cluster scope an arrival takes 1500 cycles; what every lane has loaded enters its address, by a vote: an OR over the words took
+                // (relaxed: with release at cluster scope an arrival takes 1500 cycles; what every lane has loaded enters its address, by a vote: an
+                // OR over the words took
                 // 1 % of a launch)
                 uint32_t words = __float_as_uint(v[0]);
 #pragma unroll
@@ -807,7 +822,8 @@ GtArgs gt_args(const WeightDev& w, const GemvIn& in, int T) {
 
 // By format and K alone: all of a matrix's rows, whatever shard or token they belong to, have to take the same form. (Q8_0 up to 14336 values a row: two slots
 // beside the digits of eight tokens. Q4_K up to 36864, MLX-4 to 41984.) Up to 1024 values a row the form on mma.sync is faster, by itself, where it splits the
-// activations (us in a graph, one / two / four / eight tokens, on mma.sync and here: Q4_K 1024 x 1024 2.54 / 2.72 / 3.14 / 4.26 and 3.35 / 3.49 / 3.82 / 3.88, 14336 x 1024
+// activations (us in a graph, one / two / four / eight tokens, on mma.sync and here: Q4_K 1024 x 1024 2.54 / 2.72 / 3.14 / 4.26 and 3.35 / 3.49 /
+// 3.82 / 3.88, 14336 x 1024
 // 5.00 / 5.46 / 5.60 / 8.03 and 5.28 / 5.71 / 6.45 / 8.80), and more so between other kernels: six layers of hidden size 1024 with Q4_K, Q6_K and Q8_0, four tokens,
 // 309 us and 358.
 bool gemv_tc_supports(const WeightDev& w) {
@@ -848,7 +864,8 @@ cudaError_t launch_gemv_tc_jobs(const GemvTcJob* jobs, int n_jobs, const GemvIn&
     for (int j = 0; j < n_jobs; j++)
         if (!gemv_tc_supports(*jobs[j].w) || w.fmt == B2_FMT_Q8_0 || jobs[j].w->fmt != w.fmt || jobs[j].w->n_in != w.n_in) return cudaErrorInvalidValue;
     const GtArgs a = gt_args(w, in, T);
-    return w.fmt == B2_FMT_MLX4 ? gt_tokens<B2_FMT_MLX4, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs) : gt_tokens<B2_FMT_Q4_K, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs);
+    return w.fmt == B2_FMT_MLX4 ? gt_tokens<B2_FMT_MLX4, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs)
+                                : gt_tokens<B2_FMT_Q4_K, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs);
 }
 
 }  // namespace b2
