@@ -178,8 +178,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
             return split_load(a.x + xr * a.x_stride + k, a.nw ? a.nw + k : nullptr, (int)a.w.n_in - k, lane);
         };
         SplitIn next;
-        if (!a.rec && wq < nb * T) next = load(wq);
-        for (int i = a.rec ? nb * T : wq; i < nb * T; i += WARPS) {
+        constexpr bool RECORDS = X::COLUMNS <= 3;  // (there are none of four digits)
+        if (!(RECORDS && a.rec) && wq < nb * T) next = load(wq);
+        for (int i = RECORDS && a.rec ? nb * T : wq; i < nb * T; i += WARPS) {
             const int b = block_of(i), tk = TP == 1 ? 0 : i - b * T, blk = b0 + b;
             uint8_t* f0 = smem + a.frag_off + (size_t)b * (X::BLOCK * TP) + tk * X::TOKEN;
             int s;
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
         }
         // Records: the fragments lie there as they lie here; nobody waits for a copy before all are on their way. (Apart from the other path, whose first
         // run through its code counts: inside its loop, and with divisions by one token, Q5_K 14336 x 4096 took 12.05 us, this way 11.70.)
-        if (__builtin_expect(a.rec != nullptr, 0)) {
+        if (RECORDS && __builtin_expect(a.rec != nullptr, 0)) {
             for (int i = wq; i < nb * T; i += WARPS) {
                 const int b = block_of(i), tk = TP == 1 ? 0 : i - b * T, blk = b0 + b;
                 const uint8_t* src = a.rec + (size_t)tk * a.rec_stride + (size_t)blk * X::BLOCK;
