@@ -417,7 +417,8 @@ int b2_moe_ep(b2_ctx* ctx, b2_moe_handle m, size_t n_experts_global, const float
  * in its shared memory; n_in is limited to B2_NOALLOC_MAX_K, larger inputs are refused with
  * B2_ERR_ARG and a message, and go through b2_matvec_dev instead. y_dev may overlap x_dev: such calls
  * copy x into one fixed array of the library (65,536 bytes per GPU for as long as it is loaded) and
- * race on it where they may overlap on the GPU; the others share nothing.
+ * race on it where they may overlap on the GPU; the others share nothing. Above 1024 values a row the sums are added in another
+ * order than b2_matvec_dev's (no wait of its kernel has a status word): the same accuracy, not the same bits.
  *   w_blocks_dev : raw GGUF Q4_K super-blocks on the device, [n_out][n_in/256][144], 16-byte aligned
  *   x_dev, y_dev : f32 on the device; cuda_stream : the stream to launch on (NULL = default)
  *   err, err_len : optional buffer that receives the error text

@@ -97,9 +97,9 @@ def test_clusters_that_share_a_heads_keys(backend, nh, nkv, hd, max_len, window,
 @pytest.mark.parametrize("nh,nkv,hd", SHAPES)
 @pytest.mark.parametrize("window", [1, 100, 700, NO_LIMIT])
 def test_prefill_with_windows_and_shares_of_the_keys(backend, nh, nkv, hd, window):
-    pre = D.decode_plan_prefill(backend, graph(nh, nkv, hd, window), 4500, 300)
+    pre = D.decode_plan_prefill(backend, graph(nh, nkv, hd, window), 9100, 300)
     # whole tiles (128 keys) outside the window; two, four and eight shares, most of them empty where the window is short
-    for pos, t in ((0, 130), (127, 2), (500, 12), (1100, 33), (2100, 5), (4096, 300)):
+    for pos, t in ((0, 130), (127, 2), (500, 12), (1100, 33), (2100, 5), (4096, 300), (9050, 7)):
         k, v, x, cs = inputs(nh, nkv, hd, pos, t, 60 + pos)
         if pos:
             pre.kv_write(0, 0, k, v)
