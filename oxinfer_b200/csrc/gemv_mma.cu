@@ -93,8 +93,8 @@ cudaError_t launch_gemv_mma(const WeightDev& w, const WeightDev* up, const GemvI
     a.mode = mode;
     a.T = T;
     switch (w.fmt) {
-        case B2_FMT_MLX4: return launch_f<F4<true>>(a, pair, sm_count, st, pdl);
-        case B2_FMT_Q4_K: return launch_f<F4<false>>(a, pair, sm_count, st, pdl);
+        case B2_FMT_MLX4: return launch_f<F4<true, true>>(a, pair, sm_count, st, pdl);
+        case B2_FMT_Q4_K: return launch_f<F4<false, false>>(a, pair, sm_count, st, pdl);
         case B2_FMT_Q6_K: return launch_f<F6>(a, pair, sm_count, st, pdl);
         case B2_FMT_Q8_0: return launch_f<F8B<false>>(a, pair, sm_count, st, pdl);
         case B2_FMT_F8E4M3: return launch_f<F8B<true>>(a, pair, sm_count, st, pdl);
@@ -104,7 +104,7 @@ cudaError_t launch_gemv_mma(const WeightDev& w, const WeightDev* up, const GemvI
 
 // The most rows of K values that a group's activations fit for beside the rings (launch_t: two warp groups' sums are 16 KB).
 int gemv_groups_most(size_t K) {
-    const size_t nb = split_blocks(K), fixed = (size_t)WARPS * F4<false>::SLOTS * F4<false>::UNIT_BYTES + 16384 + 512;
+    const size_t nb = split_blocks(K), fixed = (size_t)WARPS * F4<false, false>::SLOTS * F4<false, false>::UNIT_BYTES + 16384 + 512;
     for (size_t tp : {8, 4, 1})
         if (fixed + nb * tp * (SPLIT_DIGITS + 4 + 4 + 32) <= SMEM_MAX) return (int)tp;
     return 0;
@@ -124,8 +124,8 @@ cudaError_t launch_gemv_groups(const WeightDev& w, const WeightDev* up, const fl
     a.y_stride = y_stride;
     a.mode = mode;
     a.T = most;
-    if (w.fmt == B2_FMT_MLX4) return launch_f<F4<true>>(a, pair, sm_count, st, true, &groups);
-    if (w.fmt == B2_FMT_Q4_K) return launch_f<F4<false>>(a, pair, sm_count, st, true, &groups);
+    if (w.fmt == B2_FMT_MLX4) return launch_f<F4<true, false>>(a, pair, sm_count, st, true, &groups);
+    if (w.fmt == B2_FMT_Q4_K) return launch_f<F4<false, false>>(a, pair, sm_count, st, true, &groups);
     return cudaErrorInvalidValue;
 }
 

@@ -391,12 +391,13 @@ cudaError_t launch_t(Args& a, int sm_count, cudaStream_t st, bool pdl, const Gem
     a.sums_off = take(part * TP * X::SUMS + 64);
     a.ssq_off = take(ssq);
     a.xs_off = take(part * TP * 4 + 64);
-    if constexpr (std::is_same<F, F4<true>>::value || std::is_same<F, F4<false>>::value)
+    if constexpr (std::is_same<F, F4<true, false>>::value || std::is_same<F, F4<false, false>>::value) {
         if (gt) {
             auto kern = gemv_mma_kernel<F, PAIR, TP, false, GemvGroups>;
             if (cudaError_t e = ensure_dynamic_smem((const void*)kern, at); e != cudaSuccess) return e;
             return launch_k(kern, dim3((unsigned)grid), dim3(THREADS), at, st, pdl, a, *gt);
         }
+    }
     auto kern = gemv_mma_kernel<F, PAIR, TP, false, NoGroups>;
     if constexpr (F::PARTS) {
         if (parts) kern = gemv_mma_kernel<F, PAIR, TP, true, NoGroups>;

@@ -62,7 +62,7 @@ struct Fo {
     static constexpr int BLOCK_BYTES = 16 * STRIDE, UNIT_BYTES = BLOCK_BYTES;
     // One: eight sums of 32 times the block scale. Q5_K: as for Q4_K.
     __device__ static __forceinline__ void put_sums(uint8_t* e, float xs, int s, int lane) {
-        if (FMT == B2_FMT_Q5_K) F4<false>::put_sums(e, xs, s, lane);
+        if (FMT == B2_FMT_Q5_K) F4<false, false>::put_sums(e, xs, s, lane);
         else if (ONE && lane < 8) ((float*)e)[lane] = xs * (float)s;
     }
     // Q3_K: whether block 0 of rows g (bit 0) and g + 8 (bit 1) starts in the middle of a word
