@@ -858,7 +858,7 @@ class Backend {
         bool one = n_jobs <= (size_t)GEMV_TC_JOBS;
         for (size_t j = 0; j < n_jobs; j++) {
             const WeightDev& w = find(jobs[j].w)->dev;
-            one = one && gemv_tc_supports(w) && w.fmt == find(jobs[0].w)->dev.fmt && (n_jobs == 1 || (!jobs[j].up && w.fmt != B2_FMT_Q8_0));
+            one = one && w.fmt == find(jobs[0].w)->dev.fmt && (n_jobs == 1 ? gemv_tc_supports(w) : !jobs[j].up && gemv_tc_jobs_supports(w));
         }
         const bool in_place = one && staged(y_total);
         cudaError_t e = x_dev.reserve(t * n_in * 4);

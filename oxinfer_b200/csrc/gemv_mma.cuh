@@ -111,7 +111,8 @@ template <bool MLX, bool SIGNED>
 struct F4 {
     template <int TP>
     using X = XView<TP, false>;
-    static constexpr bool HALVES = false, SUMS = true, PARTS = true;
+    // IN_PAIRS: four slices' sums are added as gemv_tc.cu adds its four parts', so that a launch of several jobs there has the same bits (gemv_tc_jobs_supports).
+    static constexpr bool HALVES = false, SUMS = true, PARTS = true, IN_PAIRS = true;
     static constexpr int BLOCK_K = 256, SLOTS = 2, MAX_BLOCKS = 2;  // a unit is one or two blocks
     static constexpr int BLOCK_BYTES = 16 * 144, UNIT_BYTES = MAX_BLOCKS * BLOCK_BYTES;
     static constexpr bool SUMS_BY_COLUMN = !MLX;
@@ -287,7 +288,7 @@ template <bool FP8>
 struct F8B {
     template <int TP>
     using X = XView<TP, FP8>;
-    static constexpr bool HALVES = FP8, SUMS = false, SUMS_BY_COLUMN = false, PARTS = true;
+    static constexpr bool HALVES = FP8, SUMS = false, SUMS_BY_COLUMN = false, PARTS = true, IN_PAIRS = false;
     static constexpr int BLOCK_K = 128, SLOTS = 2, MAX_BLOCKS = 2;
     static constexpr int BLOCK_BYTES = 16 * 144, UNIT_BYTES = MAX_BLOCKS * BLOCK_BYTES;
     __device__ static __forceinline__ void put_sums(uint8_t*, float, int, int) {}
@@ -440,7 +441,7 @@ struct F8B {
 struct F6 {
     template <int TP>
     using X = XView<TP, false>;
-    static constexpr bool HALVES = false, SUMS = false, SUMS_BY_COLUMN = false, PARTS = true;
+    static constexpr bool HALVES = false, SUMS = false, SUMS_BY_COLUMN = false, PARTS = true, IN_PAIRS = false;
     static constexpr int BLOCK_K = 256, SLOTS = 3, MAX_BLOCKS = 1;
     static constexpr int BLOCK_BYTES = 16 * 208 + 64, UNIT_BYTES = BLOCK_BYTES;
     __device__ static __forceinline__ void put_sums(uint8_t*, float, int, int) {}

@@ -305,9 +305,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_mma_kernel(const __grid_const
                 if (row < first || row >= n_out) continue;  // (the last tile's halves overlap the rows before them)
                 const float* pv = c0 + (size_t)tl * slices * RES + (TP == 1 ? r : token / X::PER * 16 * X::PER + r * X::PER + token % X::PER);
                 float v = 0.0f, v2 = 0.0f;
-                for (int s = 0; s < slices; s++) {
-                    v += pv[s * RES];
-                    if (PAIR) v2 += pv[s * RES + 8 * (TP == 1 ? 1 : X::PER)];
+                constexpr int SECOND = 8 * (TP == 1 ? 1 : X::PER);  // (of a pair)
+                if (!GROUPED && F::IN_PAIRS && slices == 4) {
+                    v = (pv[0] + pv[RES]) + (pv[2 * RES] + pv[3 * RES]);
+                    if (PAIR) v2 = (pv[SECOND] + pv[RES + SECOND]) + (pv[2 * RES + SECOND] + pv[3 * RES + SECOND]);
+                } else {
+                    for (int s = 0; s < slices; s++) {
+                        v += pv[s * RES];
+                        if (PAIR) v2 += pv[s * RES + SECOND];
+                    }
                 }
                 if (a.norm) {
                     float sq = 0.0f;

@@ -48,7 +48,7 @@ struct Fo {
     template <int TP>
     using X = XView<TP, false, 4>;  // (four digits: the float kernel, which these formats had before, rounds nothing of x)
     static constexpr bool ONE = FMT == B2_FMT_Q4_1 || FMT == B2_FMT_Q5_1;  // a float minimum per 32
-    static constexpr bool HALVES = false, SUMS = ONE || FMT == B2_FMT_Q5_K, SUMS_BY_COLUMN = FMT == B2_FMT_Q5_K;
+    static constexpr bool HALVES = false, SUMS = ONE || FMT == B2_FMT_Q5_K, SUMS_BY_COLUMN = FMT == B2_FMT_Q5_K, IN_PAIRS = false;
     static constexpr int BS = FMT == B2_FMT_Q2_K || FMT == B2_FMT_Q3_K || FMT == B2_FMT_Q5_K || FMT == B2_FMT_IQ4_XS ? 256 : FMT == B2_FMT_NVFP4 ? 64 : 32;
     static constexpr int TS = FMT == B2_FMT_NVFP4 ? 36 : FMT == B2_FMT_Q4_0 || FMT == B2_FMT_IQ4_NL ? 18 : FMT == B2_FMT_Q4_1 ? 20 : FMT == B2_FMT_Q5_0 ? 22 : FMT == B2_FMT_Q5_1 ? 24
                               : FMT == B2_FMT_Q2_K ? 84 : FMT == B2_FMT_Q3_K ? 110 : FMT == B2_FMT_Q5_K ? 176 : FMT == B2_FMT_IQ4_XS ? 136 : 17;

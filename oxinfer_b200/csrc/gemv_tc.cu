@@ -826,10 +826,17 @@ GtArgs gt_args(const WeightDev& w, const GemvIn& in, int T) {
 // 3.82 / 3.88, 14336 x 1024
 // 5.00 / 5.46 / 5.60 / 8.03 and 5.28 / 5.71 / 6.45 / 8.80), and more so between other kernels: six layers of hidden size 1024 with Q4_K, Q6_K and Q8_0, four tokens,
 // 309 us and 358.
-bool gemv_tc_supports(const WeightDev& w) {
+static bool gt_fits(const WeightDev& w) {
     const int tp = w.fmt == B2_FMT_Q8_0 ? 8 : GT_TOKENS;
     return (w.fmt == B2_FMT_Q4_K || w.fmt == B2_FMT_MLX4 || (w.fmt == B2_FMT_Q8_0 && ((uintptr_t)w.p1 & 15) == 0)) && ((uintptr_t)w.p0 & 15) == 0 && w.n_in % 256 == 0 &&
-           w.n_in > 1024 && gt_fixed(w.fmt, w.n_in, tp) + 2 * gt_raw(w.fmt) <= gt_smem(tp);
+           w.n_in > 0 && gt_fixed(w.fmt, w.n_in, tp) + 2 * gt_raw(w.fmt) <= gt_smem(tp);
+}
+
+bool gemv_tc_supports(const WeightDev& w) { return w.n_in > 1024 && gt_fits(w); }
+// Several matrices in one launch: shorter rows too where their sums have one order here and there, a block a part (one, two or four blocks; q / k / v of one token
+// from host to host, K = 1024: 27.5 us, in a launch each 32).
+bool gemv_tc_jobs_supports(const WeightDev& w) {
+    return w.fmt != B2_FMT_Q8_0 && gt_fits(w) && (w.n_in > 1024 || w.n_in == 256 || w.n_in == 512 || w.n_in == 1024);
 }
 
 cudaError_t launch_gemv_tc(const WeightDev& w, const WeightDev* up, const GemvIn& in, int T, float* y, size_t y_stride, int mode, const float* gate,
@@ -862,7 +869,7 @@ cudaError_t launch_gemv_tc_jobs(const GemvTcJob* jobs, int n_jobs, const GemvIn&
     if (n_jobs < 1 || n_jobs > GEMV_TC_JOBS || !in.status || T < 1 || T > 2 * GT_TOKENS) return cudaErrorInvalidValue;
     const WeightDev& w = *jobs[0].w;
     for (int j = 0; j < n_jobs; j++)
-        if (!gemv_tc_supports(*jobs[j].w) || w.fmt == B2_FMT_Q8_0 || jobs[j].w->fmt != w.fmt || jobs[j].w->n_in != w.n_in) return cudaErrorInvalidValue;
+        if (!gemv_tc_jobs_supports(*jobs[j].w) || jobs[j].w->fmt != w.fmt || jobs[j].w->n_in != w.n_in) return cudaErrorInvalidValue;
     const GtArgs a = gt_args(w, in, T);
     return w.fmt == B2_FMT_MLX4 ? gt_tokens<B2_FMT_MLX4, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs)
                                 : gt_tokens<B2_FMT_Q4_K, false, true>(w, nullptr, a, sm_count, st, pdl, jobs, n_jobs);

@@ -98,6 +98,7 @@ cudaError_t launch_gemv_tc(const WeightDev& w, const WeightDev* up, const GemvIn
                            size_t gate_stride, int sm_count, cudaStream_t st, bool pdl);
 // Up to four matrices of one format and K by the same T (1 .. 8) rows, in one launch; results one after another, [T][n_out] each.
 constexpr int GEMV_TC_JOBS = 4;
+bool gemv_tc_jobs_supports(const WeightDev& w);
 struct GemvTcJob {
     const WeightDev* w;
     float* y;

@@ -41,3 +41,23 @@ def test_rows_keep_their_bits_with_and_without_records(backend, fmt, n_out, n_in
         y = np.full((t, n_out), np.nan, np.float32)
         assert backend.matmul(x[:t], [ob.Job(dev, y)])
         assert np.array_equal(y, ones[:t]), t
+
+
+# one, two, three and four blocks of activations, and five (the form on tcgen05 for every call)
+@pytest.mark.parametrize("fmt", ["q4_k", "mlx4"])
+@pytest.mark.parametrize("n_in", [256, 512, 768, 1024, 1280])
+def test_jobs_of_short_rows_have_the_bits_of_each_by_itself(backend, fmt, n_in):
+    """Several matrices of a call may share a launch of the other form; extreme activations, whose sums round everywhere, among them."""
+    outs = [1, 129, 700, 64]
+    devs = [backend.upload(make_pair(fmt, n, n_in, 60 + n % 53)[0], n, n_in) for n in outs]
+    for seed, scale in ((71, 1.0), (72, 1e6), (73, 1e-6)):
+        x = synth.activations(4, n_in, seed) * np.float32(scale)
+        x[:, ::97] *= 1000.0
+        for t in (1, 2, 4):
+            alone = [np.full((t, n), np.nan, np.float32) for n in outs]
+            for d, y in zip(devs, alone):
+                assert backend.matvec_rows(x[:t], [ob.RowsJob(d, y)])
+            ys = [np.full((t, n), np.nan, np.float32) for n in outs]
+            assert backend.matvec_rows(x[:t], [ob.RowsJob(d, y) for d, y in zip(devs, ys)])
+            for a, y in zip(alone, ys):
+                assert np.array_equal(a, y), (scale, t, a.shape)
