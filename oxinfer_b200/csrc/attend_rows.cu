@@ -129,6 +129,8 @@ __device__ __forceinline__ float ar_peer_f(const void* p, uint32_t cta) {
     return v;
 }
 
+// The first key that a query at position qp sees.
+__device__ __forceinline__ uint32_t ar_first_key(const ArArgs& a, uint32_t qp) { return a.window != 0 && qp + 1 > a.window ? qp + 1 - a.window : 0; }
 // Row r's token (r G < 2^32).
 __device__ __forceinline__ uint32_t ar_token(const ArArgs& a, uint32_t r) { return a.g_inv ? __umulhi(r, a.g_inv) : r; }
 
@@ -158,7 +160,7 @@ attend_rows_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     const uint32_t r_end = min(r_block + 2 * AR_TILE, a.rows);
     const int tiles = r_block + AR_TILE < r_end ? 2 : 1;
     const uint32_t first_qp = a.pos0 + ar_token(a, r_block), last_qp = a.pos0 + ar_token(a, r_end - 1);
-    const uint32_t lo = a.window != 0 && first_qp + 1 > a.window ? first_qp + 1 - a.window : 0;
+    const uint32_t lo = ar_first_key(a, first_qp);
     const uint32_t all_0 = lo / AR_TILE, all_n = last_qp / AR_TILE + 1 - all_0, share = (all_n + a.Z - 1) / a.Z;
     const uint32_t t_first = all_0 + z * share;
     const int n = (int)min(share, all_0 + all_n > t_first ? all_0 + all_n - t_first : 0u);  // this CTA's key tiles
@@ -242,6 +244,10 @@ attend_rows_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
             tc_fence_after();
             return ok;
         };
+        // 64 keys that no row of the tile sees are left out: their probabilities are zeros, but a value that is not finite would still reach the sums
+        const uint32_t tile_0 = min(r_block + w * AR_TILE, a.rows - 1), see_to = a.pos0 + ar_token(a, min(tile_0 + AR_TILE - 1, a.rows - 1));
+        const uint32_t see_from = ar_first_key(a, a.pos0 + ar_token(a, tile_0));
+        uint32_t started = 0;
         if (ok && wait(&sh->q_full, 0, 65, 0) && wait(&sh->k_full[0], 0, 66, 0)) scores(0);
         for (int i = 0; i < n && ok; i++) {
             const int s = i & 1, s1 = s ^ 1;
@@ -250,12 +256,17 @@ attend_rows_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
 #pragma unroll
             for (int h = 0; h < 2; h++) {  // (the first half's products run under the second half's exponentials)
                 if (!wait(&sh->p_full[w][h], (uint32_t)(i & 1), 69, i)) break;
+                const uint32_t j = (t_first + i) * AR_TILE + 64 * h;
+                const bool seen = j <= see_to && j + 63 >= see_from;
                 if (elect_one()) {
                     const uint64_t v = vd + (s * TILE_BYTES >> 4) + 512 * h;
+                    if (seen) {
 #pragma unroll
-                    for (int kk = 0; kk < AR_TILE / 32; kk++) ar_mma_ts(o_at, s_at + 32 * h + 8 * kk, v + 128 * kk, idesc_pv, i > 0 || h > 0 || kk > 0);
+                        for (int kk = 0; kk < AR_TILE / 32; kk++) ar_mma_ts(o_at, s_at + 32 * h + 8 * kk, v + 128 * kk, idesc_pv, started | kk);
+                    }
                     if (h) mma_commit(&sh->v_empty[s]);
                 }
+                started |= seen;
                 __syncwarp();
             }
             if (ok && i + 1 < n) scores(s1);
@@ -303,7 +314,7 @@ attend_rows_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         const uint32_t row = (uint32_t)((warp & 3) * 32 + lane), r = min(r_block + w * AR_TILE + row, a.rows - 1), qp = a.pos0 + ar_token(a, r);
         const uint32_t tile_qp = a.pos0 + ar_token(a, min(r_block + w * AR_TILE, a.rows - 1));                          // the tile's first position
         const uint32_t tile_end = a.pos0 + ar_token(a, min(r_block + w * AR_TILE + AR_TILE - 1, a.rows - 1));           // and its last
-        const uint32_t my_lo = a.window != 0 && qp + 1 > a.window ? qp + 1 - a.window : 0;
+        const uint32_t my_lo = ar_first_key(a, qp);
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16, s_at = tmem + lane_base + w * AR_TILE, o_at = tmem + lane_base + 2 * AR_TILE + w * HD;
         float m = -INFINITY, l = 0.0f;
         bool ok = true;
@@ -377,6 +388,8 @@ attend_rows_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         if (ok && live) {
             tc_fence_after();
             float4* const dst = (float4*)(smem + (size_t)(w * AR_TILE + row) * HD * 4);
+            // (the tile's rows may see none of this CTA's keys: there are no sums then)
+            const bool none = n == 0 || tile_end < t_first * AR_TILE || ar_first_key(a, tile_qp) >= (t_first + n) * AR_TILE;
 #pragma unroll
             for (int h = 0; h < HD / 32; h++) {
                 uint32_t o[32];
@@ -384,8 +397,8 @@ attend_rows_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
                 ar_ld_wait();
 #pragma unroll
                 for (int e = 0; e < 8; e++)
-                    dst[(8 * h + e) ^ (row & 7)] = n == 0 ? make_float4(0.f, 0.f, 0.f, 0.f)
-                                                          : make_float4(__uint_as_float(o[4 * e]), __uint_as_float(o[4 * e + 1]), __uint_as_float(o[4 * e + 2]), __uint_as_float(o[4 * e + 3]));
+                    dst[(8 * h + e) ^ (row & 7)] = none ? make_float4(0.f, 0.f, 0.f, 0.f)
+                                                        : make_float4(__uint_as_float(o[4 * e]), __uint_as_float(o[4 * e + 1]), __uint_as_float(o[4 * e + 2]), __uint_as_float(o[4 * e + 3]));
             }
             sh->m[w * AR_TILE + row] = m;
             sh->l[w * AR_TILE + row] = a.Z > 1 ? l : l > 0.0f ? 1.0f / l : 0.0f;

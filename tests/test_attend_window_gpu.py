@@ -126,3 +126,24 @@ def test_a_share_without_keys_adds_nothing_whatever_the_queries_hold(backend):
             rows = np.isnan(got.reshape(t, nh, hd)).all(-1)
             assert np.array_equal(rows, own) and np.array_equal(got.reshape(t, nh, hd)[~own], clean.reshape(t, nh, hd)[~own])
     pre.close()
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 64), (8, 1, 128)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_values_of_later_and_of_forgotten_tokens_reach_nobody(backend, nh, nkv, hd, window):
+    """An infinite value (or one that f16 does not hold) is in nobody's sums who does not see its 64 keys."""
+    pre = D.decode_plan_prefill(backend, graph(nh, nkv, hd, window), 512, 300)
+    k, v, x, cs = inputs(nh, nkv, hd, 0, 300, 90)
+    clean, _ = pre.step_multi(0, x, cs, want_logits=False)
+    for token, value in ((70, np.inf), (129, 1e6), (255, -np.inf), (299, np.nan)):
+        bad = x.copy()
+        bad[token, (nh + nkv) * hd:] = value
+        got, _ = pre.step_multi(0, bad, cs, want_logits=False)
+        first = token // 64 * 64
+        assert np.array_equal(got[:first], clean[:first]), token
+        assert not np.isfinite(got[token]).any()
+        if window:  # 64 keys that end before the windows of a tile of rows (128 / G tokens) begin
+            tile = 128 // (nh // nkv)
+            behind = -(-(first + 63 + window) // tile) * tile
+            assert np.array_equal(got[behind:], clean[behind:]), token
+    pre.close()
