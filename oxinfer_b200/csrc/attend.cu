@@ -585,14 +585,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) attend_kernel(const float* __r
 // How many clusters share a KV head's keys: by heads and the caches' size alone, since a token's sums have to be the same in steps of one and of several
 // tokens. More of them only where that puts more CTAs to work on one token, and
 // - while the clusters of a step of four tokens still run at once (one for each head and share, some 36 of eight CTAs fit the chip), from 3072 keys
-// a share on, where
-//   the exchange through memory (2 us) is made up for; 1536 where one token's clusters already have eight CTAs. f32 caches of 128 dimensions, 12300
-//   keys, one and four tokens,
-//   us a launch without and with: 4 heads of 1 KV head 17.6 / 19.1 and 9.7 / 17.9, 16 of 4 19.3 / 46.2 and 16.5 / 31.4, 16 of 16 of 64 dimensions,
-//   4100 keys, 18.6 / 18.0 and 12.9 / 14.0;
-// - or else from 16384 keys on: 32 heads of 8 KV heads, 24600 keys, f32 46.3 / 87.1 and 40.7 / 110.5, f16 45.6 / 91.0 and 33.6 / 109.4 (at 12300
-// keys 28.0 / 48.8, f16 28.1 / 49.7
-//   without): one token gains what four lose there.
+//   a share on, where the exchange through memory (2 us) is made up for; 1536 where one token's clusters already have eight CTAs. f32 caches of 128
+//   dimensions, 12300 keys, one and four tokens, us a launch without and with: 4 heads of 1 KV head 17.6 / 19.1 and 9.7 / 17.9, 16 of 4 19.3 / 46.2
+//   and 16.5 / 31.4, 16 of 16 of 64 dimensions, 4100 keys, 18.6 / 18.0 and 12.9 / 14.0;
+// - or else from 16384 keys on, where one to three tokens gain more than four lose (two waves of clusters). 32 heads of 8 KV heads, one, two, three
+//   and four tokens: f32, 24600 keys 42 / 86 / 88 / 88 and 35 / 63 / 84 / 111, 32000 keys 58 / 112 / 111 / 112 and 47 / 69 / 101 / 135, of 64
+//   dimensions 42 / 82 / 82 / 82 and 29 / 54 / 77 / 102; f16, 24600 keys, one and four 45.6 / 91.0 and 33.6 / 109.4. (12300 keys 28.0 / 48.8, f16
+//   28.1 / 49.7 without.)
 uint32_t attend_shares(uint32_t nh, uint32_t nkv, uint32_t max_len) {
     const uint32_t units = nkv * ((nh / nkv + ATT_MOST_ROWS - 1) / ATT_MOST_ROWS);  // clusters of one token
     auto ctas = [&](uint32_t s) { return units * s * (units * s > 14 ? 8 : 16); };
@@ -609,7 +608,8 @@ cudaError_t attend_t(const float* q, void* kc, void* vc, float* out, const uint3
                      const FusedRope& fr, const AttnTokens& at, const AttScratch& scratch) {
     constexpr size_t smem = AttShared<HD, R, T>::BYTES;
     auto kern = attend_kernel<HD, R, T, false>;
-    const unsigned G = p.nh / p.nkv, groups = (G * (unsigned)std::max(1, at.n) + R - 1) / R, shares = attend_shares(p.nh, p.nkv, p.max_len), C = p.nkv * groups * shares > 14 ? 8 : 16;
+    const unsigned G = p.nh / p.nkv, groups = (G * (unsigned)std::max(1, at.n) + R - 1) / R, shares = attend_shares(p.nh, p.nkv, p.max_len);
+    const unsigned C = p.nkv * groups * shares > 14 ? 8 : 16;
     AttShares sh{};
     while ((1u << sh.log) < shares) sh.log++;
     sh.groups = groups;

@@ -8,8 +8,8 @@
 // row shard and every row of a step of several tokens have the bits of the one-token product. A CTA:
 //   warp 0        : copies packed rows (128 x 144 bytes a block of 256 k) into a ring, filled before the kernel waits for the one ahead.
 //   warps 2 .. 17 : four sets of four, a thread a row; set s takes the blocks s, s + 4, .. of those that the CTA has of all its tiles: nibbles to
-//   bytes in tensor memory, the
-//                   instructions, the sums back and times the scales. At the end of a tile its sums go to the CTA of the cluster that owns the rows.
+//                   bytes in tensor memory, the instructions, the sums back and times the scales. At the end of a tile its sums go to the CTA of
+//                   the cluster that owns the rows.
 //   warp 1        : adds the sixteen sums of its rows in pairs, applies the norm's factor and the output mode, and stores.
 // All but warp 0 split the CTA's part of the activations first (an RMS norm's weights multiply before the split, its factor the results).
 // Five to eight tokens: every other cluster has those from the fifth on, and the second reading of the weights comes from L2.
@@ -18,10 +18,9 @@
 //
 // What bounds it: HBM on large matrices, the start on small ones. The form on mma.sync (gemv_mma.cu) was bound by instructions: 393 of a warp
 // for 4096 weights (Q4_K 14336 x 4096, one token, ncu, everything counted); here it is 225, of which the bytes, the sums and the scales are about
-// 110. Of the 4.7 us of 4096 x 4096, 0.5 pass before the first copy is issued, 1.5 until
-// activations and weights are there, and 2 between them and the result, most of it the first fetch of each line of code: hence short code, no
-// divisions, a pass of the
-// results' loop that stores nothing. Four sets and the whole of tensor memory: two sets in half of an SM (two CTAs) left 4096 x 14336, four tokens, at 21 us.
+// 110. Of the 4.7 us of 4096 x 4096, 0.5 pass before the first copy is issued, 1.5 until activations and weights are there, and 2 between them and
+// the result, most of it the first fetch of each line of code: hence short code, no divisions, a pass of the results' loop that stores nothing. Four
+// sets and the whole of tensor memory: two sets in half of an SM (two CTAs) left 4096 x 14336, four tokens, at 21 us.
 // One launch after another in a stream, us, one / two / four / eight tokens, on mma.sync and here:
 //   Q4_K  4096 x 4096    5.2 / 8.8 / 11.0 / 16.1   5.1 / 5.5 / 6.1 / 7.9
 //         4096 x 14336  12.8 / 21.7 / 25.7 / 41.1  9.6 / 11.2 / 14.2 / 19.6
@@ -32,9 +31,10 @@
 //   Q8_0  4096 x 4096    6.3 / 8.7 / 9.6 / 16.9    5.2 / 5.6 / 8.0 / 9.2
 //         4096 x 14336  15.0 / 24.3 / 28.4 / 42.1  13.0 / 14.6 / 16.2 / 24.5
 //         32064 x 4096  23.9 / 27.0 / 28.1 / 54.5  23.3 / 24.6 / 24.6 / 28.0
-// (6144 x 4096, MLX-4, one token: 5.9 and 6.3: its 48 tiles take two rounds of 24 clusters. In a graph 4096 x 4096 takes 4.5 and 4.4.)
+// (6144 x 4096, MLX-4, one token: 5.9 and 6.3: its 48 tiles take two rounds of 24 clusters. In a graph 4096 x 4096 takes 4.5 and 4.4. K of 1024 and
+// less: gemv_tc_supports.)
 // Largest error of a result against 64 bits, in parts of the row's norm, N(0, 1) activations, K = 1024 / 4096 / 14336:
-// Q4_K 1.60 / 1.70 / 1.71e-7 on mma.sync, 1.60 / 1.65 / 1.66e-7 here; MLX-4 1.78 / 2.07 / 2.39e-7 and 1.57 / 1.65 / 1.59e-7;
+// Q4_K 1.60 / 1.70 / 1.71e-7 on mma.sync, 1.60 / 1.65 / 1.66e-7 here; MLX-4, unsigned there, 1.78 / 2.07 / 2.39e-7 and 1.57 / 1.65 / 1.59e-7;
 // Q8_0 1.67 / 1.72 / 1.79e-7 and 1.67 / 1.69 / 1.73e-7.
 #include <cuda.h>
 
@@ -820,12 +820,11 @@ GtArgs gt_args(const WeightDev& w, const GemvIn& in, int T) {
 
 }  // namespace
 
-// By format and K alone: all of a matrix's rows, whatever shard or token they belong to, have to take the same form. (Q8_0 up to 14336 values a row: two slots
-// beside the digits of eight tokens. Q4_K up to 36864, MLX-4 to 41984.) Up to 1024 values a row the form on mma.sync is faster, by itself, where it splits the
-// activations (us in a graph, one / two / four / eight tokens, on mma.sync and here: Q4_K 1024 x 1024 2.54 / 2.72 / 3.14 / 4.26 and 3.35 / 3.49 /
-// 3.82 / 3.88, 14336 x 1024
-// 5.00 / 5.46 / 5.60 / 8.03 and 5.28 / 5.71 / 6.45 / 8.80), and more so between other kernels: six layers of hidden size 1024 with Q4_K, Q6_K and Q8_0, four tokens,
-// 309 us and 358.
+// By format and K alone: all of a matrix's rows, whatever shard or token they belong to, have to take the same form. (Q8_0 up to 14336 values a row: two
+// slots beside the digits of eight tokens. Q4_K up to 36864, MLX-4 to 41984.) Up to 1024 values a row the form on mma.sync is faster, by itself, where
+// it splits the activations (us in a graph, one / two / four / eight tokens, on mma.sync and here: Q4_K 1024 x 1024 2.54 / 2.72 / 3.14 / 4.26 and 3.35 /
+// 3.49 / 3.82 / 3.88, 14336 x 1024 5.00 / 5.46 / 5.60 / 8.03 and 5.28 / 5.71 / 6.45 / 8.80), and more so between other kernels: six layers of hidden size
+// 1024 with Q4_K, Q6_K and Q8_0, four tokens, 309 us and 358.
 static bool gt_fits(const WeightDev& w) {
     const int tp = w.fmt == B2_FMT_Q8_0 ? 8 : GT_TOKENS;
     return (w.fmt == B2_FMT_Q4_K || w.fmt == B2_FMT_MLX4 || (w.fmt == B2_FMT_Q8_0 && ((uintptr_t)w.p1 & 15) == 0)) && ((uintptr_t)w.p0 & 15) == 0 && w.n_in % 256 == 0 &&
@@ -833,8 +832,8 @@ static bool gt_fits(const WeightDev& w) {
 }
 
 bool gemv_tc_supports(const WeightDev& w) { return w.n_in > 1024 && gt_fits(w); }
-// Several matrices in one launch: shorter rows too where their sums have one order here and there, a block a part (one, two or four blocks; q / k / v of one token
-// from host to host, K = 1024: 27.5 us, in a launch each 32).
+// Several matrices in one launch: shorter rows too where their sums have one order here and there, a block a part (one, two or four blocks; q / k / v of
+// one token from host to host, K = 1024: 27.5 us, in a launch each 32).
 bool gemv_tc_jobs_supports(const WeightDev& w) {
     return w.fmt != B2_FMT_Q8_0 && gt_fits(w) && (w.n_in > 1024 || w.n_in == 256 || w.n_in == 512 || w.n_in == 1024);
 }
